@@ -1,14 +1,18 @@
-"""Build recipe of libb2fil.so: nvcc for sm_100a, in-tree output under cuml_b200/lib/.
+"""Build recipe of libb2fil.so (nvcc for sm_100a) and of the torch call path beside it; in-tree
+output under cuml_b200/lib/.
 
 `python -m cuml_b200.build [--force] [--verbose]` (also called by `__graft_entry__.build()`).
 The register / shared-memory report of ptxas is written to cuml_b200/lib/ptxas.log.
 """
 from __future__ import annotations
 
+import importlib.metadata
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SRC = os.path.join(HERE, "csrc")
@@ -23,6 +27,30 @@ HEADERS = ["forest.hpp", "kernels.hpp", "kernels_q.hpp", "device_common.cuh", "d
            os.path.join("..", "..", "include", "b2fil.h")]
 
 
+# Native call path for torch tensors: a CPython module compiled against the installed torch, whose
+# version is part of the file name (another torch needs another build).
+TORCH_SOURCE = os.path.join(SRC, "torch_call.cpp")
+
+
+def torch_module_path():
+    """Path of the compiled torch module, or None where torch is not installed."""
+    try:
+        return os.path.join(LIB_DIR, f"b2fil_torch-{importlib.metadata.version('torch')}.so")
+    except importlib.metadata.PackageNotFoundError:
+        return None
+
+
+def _torch_command(out: str) -> list:
+    root = os.path.dirname(importlib.util.find_spec("torch").origin)  # without importing torch
+    inc, lib = os.path.join(root, "include"), os.path.join(root, "lib")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    dirs = [inc, os.path.join(inc, "torch", "csrc", "api", "include"), cuda,
+            sysconfig.get_paths()["include"]]
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall"] + ["-I" + d for d in dirs] +
+            [TORCH_SOURCE, "-o", out, "-L" + lib, "-lc10", "-lc10_cuda", "-ltorch_cpu",
+             "-ltorch_cuda", "-ltorch_python", "-ltorch"])
+
+
 def _nvcc() -> str:
     exe = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(exe):
@@ -33,9 +61,16 @@ def _nvcc() -> str:
 def up_to_date() -> bool:
     if not os.path.exists(LIB):
         return False
-    t = os.path.getmtime(LIB)
-    deps = [os.path.join(SRC, s) for s in SOURCES + HEADERS] + [os.path.abspath(__file__)]
-    return all((not os.path.exists(d)) or os.path.getmtime(d) <= t for d in deps)
+    me = os.path.abspath(__file__)
+
+    def newer(target, deps):
+        t = os.path.getmtime(target)
+        return all((not os.path.exists(d)) or os.path.getmtime(d) <= t for d in deps)
+
+    module = torch_module_path()
+    if module and not (os.path.exists(module) and newer(module, [TORCH_SOURCE, me])):
+        return False
+    return newer(LIB, [os.path.join(SRC, s) for s in SOURCES + HEADERS] + [me])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -56,6 +91,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
         cmd = base + ["-c", os.path.join(SRC, src), "-o", obj]
         out = open(obj + ".log", "w+")  # a file, not a pipe: nothing blocks while others run
         jobs.append((cmd, obj, subprocess.Popen(cmd, stdout=out, stderr=subprocess.STDOUT), out))
+    module = torch_module_path()
+    if module:
+        cmd = _torch_command(module)
+        out = open(os.path.join(obj_dir, "torch_call.log"), "w+")
+        jobs.append((cmd, None, subprocess.Popen(cmd, stdout=out, stderr=subprocess.STDOUT), out))
     log, failed = [], False
     for cmd, obj, proc, out in jobs:
         proc.wait()
@@ -65,7 +105,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         failed |= proc.returncode != 0
     if not failed:
         cmd = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", LIB]
-        cmd += [obj for _, obj, _, _ in jobs]
+        cmd += [obj for _, obj, _, _ in jobs if obj]
         proc = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         log.append(" ".join(cmd) + "\n" + proc.stdout)
         failed = proc.returncode != 0

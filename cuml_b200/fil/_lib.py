@@ -2,6 +2,8 @@
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 from ._desc import CCreateOpts, CForestDesc, CInfo
@@ -82,6 +84,30 @@ def load() -> C.CDLL:
                                           C.POINTER(i64), i64, vp, i32, C.c_double]
     _lib = lib
     return lib
+
+
+_torch_module = None
+
+
+def torch_module():
+    """The compiled call path for torch tensors (csrc/torch_call.cpp).  torch must be importable."""
+    global _torch_module
+    if _torch_module is None:
+        from .. import build as _build
+
+        import torch  # noqa: F401  (its shared libraries must be loaded first)
+
+        load()  # builds both libraries when they are missing
+        path = _build.torch_module_path()
+        if path is None or not os.path.exists(path):
+            raise ImportError(f"{path} is missing and could not be built; "
+                              "run `python -m cuml_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("b2fil_torch", path)
+        spec = importlib.util.spec_from_file_location("b2fil_torch", path, loader=loader)
+        module = importlib.util.module_from_spec(spec)
+        loader.exec_module(module)
+        _torch_module = module
+    return _torch_module
 
 
 def last_variant() -> str:

@@ -37,6 +37,7 @@ class _Forest:
         info = CInfo()
         _lib.check(_lib.load().b2fil_forest_info(self.handle, C.byref(info)))
         self.info = info
+        self._device_call = None
 
     @classmethod
     def create(cls, desc: ForestDesc, precision: int, layout: int, storage: int,
@@ -59,7 +60,18 @@ class _Forest:
         """dtype callers must cast inputs to (randomforestclassifier.py:333)."""
         return np.float32 if self.info.precision == F32 else np.float64
 
+    def device_call(self):
+        """The compiled call path of this forest for torch tensors (created on first use)."""
+        if self._device_call is None:
+            i = self.info
+            predict = C.cast(_lib.load().b2fil_predict, C.c_void_p).value
+            self._device_call = _lib.torch_module().DeviceCall(
+                predict, self.handle.value, i.n_features, i.n_trees, i.n_outputs, i.device_id,
+                i.precision != F32, i.leaf_vector_len > 1)
+        return self._device_call
+
     def close(self):
+        self._device_call = None
         if self.handle:
             _lib.load().b2fil_forest_free(self.handle)
             self.handle = C.c_void_p()
@@ -192,9 +204,10 @@ class ForestInference:
     # -- properties -----------------------------------------------------------------------------
     @property
     def forest(self) -> _Forest:
-        if self._forest is None:
+        f = self._forest
+        if f is None:
             raise RuntimeError("no model loaded")
-        return self._forest
+        return f
 
     @property
     def n_outputs(self) -> int:
@@ -252,18 +265,28 @@ class ForestInference:
         return (n, k), dt
 
     def _run(self, X, kind: int, chunk_size: Optional[int], threshold: float = 0.5, preds=None):
-        lib = _lib.load()
         f = self.forest
-        dt = self._np_dt
         cs = int(chunk_size or self.default_chunk_size or 0)
         if cs and (cs < 1 or cs & (cs - 1)):
             raise ValueError("chunk_size must be a positive power of two")
+        # CUDA tensors that need no conversion: one native call (None: not such a call)
+        call = f._device_call
+        if call is not None and self.output_type != "numpy":
+            out = call(X, preds, kind, cs, threshold)
+            if out is not None:
+                if type(out) is int:
+                    _lib.check(out)
+                return out
+        lib = _lib.load()
+        dt = self._np_dt
         torch = None
         is_torch = False
         if not isinstance(X, np.ndarray):
             torch = _torch()
             if isinstance(X, torch.Tensor):
                 is_torch = True
+                if X.is_cuda:
+                    f.device_call()  # from the next call on
             elif hasattr(X, "__cuda_array_interface__"):
                 X = torch.as_tensor(X, device=f"cuda:{self._dev}")
                 is_torch = True
