@@ -78,8 +78,8 @@ struct DenseWalker {
                                               int64_t row, int lane, uint32_t bars,
                                               uint32_t stages, uint32_t stage_bytes,
                                               uint32_t row_addr, uint32_t stride_b, T* acc_group,
-                                              int R, RingPos& pos, Running<T>& run, int b_begin,
-                                              int b_end)
+                                              int R, RingPos& pos, Running<T>& run, int t_begin,
+                                              int t_end)
   {
     const ForestView& f    = p.f;
     const int D            = f.dense_depth;
@@ -87,12 +87,12 @@ struct DenseWalker {
     const uint32_t width_b = (1u << D) * TR::NB;  // bytes of the node array of one tree
     const int per_batch    = G * NT;
     bool ok                = true;
-    for (int b = b_begin; b < b_end; ++b) {
+    for (int batch = t_begin; batch < t_end; batch += per_batch) {
       const uint32_t s = pos.stage;
       if (ok) ok = mbar_wait(bars + 8u * s, pos.phase);
       if (ok) {
-        const int first = b * per_batch + g * NT;
-        const int n_act = min(NT, f.n_trees - first);
+        const int first = batch + g * NT;
+        const int n_act = min(NT, t_end - first);
         if (n_act > 0) {
           uint32_t base[NT], a[NT];
 #pragma unroll
@@ -135,10 +135,16 @@ struct DenseWalker {
   }
 };
 
+// n_splits > 1 (small batches): the trees of a row tile are split over n_splits CTAs, each of
+// which streams and walks only its share.  Reduced outputs launch those CTAs as a cluster and
+// meet in its distributed shared memory (finish_cluster_rows); per-tree outputs need no meeting.
+// What bounds such a launch is latency: launch, tile, trees, walk, sum, one after the other.  So
+// the barriers are set up and the trees requested before grid_wait(), while the kernel before
+// this one may still be running, and the row tile arrives by asynchronous copies.
 template <typename T, bool CAT, int MODE, int NT>
 __global__ void __launch_bounds__(544, 1)
-dense_kernel(const PredictParams p, const int R, const int G, const int S, const int n_splits,
-             T* __restrict__ partial)
+dense_kernel(const __grid_constant__ PredictParams p, const int R, const int G, const int S,
+             const int n_splits)
 {
   using TR = Traits<T>;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -164,12 +170,11 @@ dense_kernel(const PredictParams p, const int R, const int G, const int S, const
   const uint32_t tstride    = static_cast<uint32_t>(f.tree_stride);
   const int per_batch       = G * NT;
   const uint32_t stage_bytes = per_batch * tstride;
-  const int n_batches       = (f.n_trees + per_batch - 1) / per_batch;
-  // small batches split the forest over blockIdx.y: every CTA streams and walks only its share
-  // of the tree batches and leaves raw partial sums for finish_kernel
-  const int b_begin = static_cast<int>(static_cast<int64_t>(n_batches) * blockIdx.y / n_splits);
-  const int b_end   = static_cast<int>(static_cast<int64_t>(n_batches) * (blockIdx.y + 1) / n_splits);
+  const int split           = static_cast<int>(blockIdx.x) % n_splits;
+  const int t_begin         = static_cast<int>(static_cast<int64_t>(f.n_trees) * split / n_splits);
+  const int t_end           = static_cast<int>(static_cast<int64_t>(f.n_trees) * (split + 1) / n_splits);
   const int64_t n_tiles     = (p.n_rows + R - 1) / R;
+  const int64_t tile_step   = gridDim.x / n_splits;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -181,6 +186,7 @@ dense_kernel(const PredictParams p, const int R, const int G, const int S, const
     mbar_fence_init();
   }
   __syncthreads();
+  grid_release();
 
   if (warp == n_cw) {
     // ---- producer: one thread streams tree batches into the stage ring ----------------------
@@ -188,15 +194,14 @@ dense_kernel(const PredictParams p, const int R, const int G, const int S, const
       const unsigned char* src = static_cast<const unsigned char*>(f.nodes);
       RingPos pos;
       bool primed = false;  // every stage has been filled once
-      for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-        for (int b = b_begin; b < b_end; ++b) {
+      for (int64_t t = blockIdx.x / n_splits; t < n_tiles; t += tile_step) {
+        for (int first = t_begin; first < t_end; first += per_batch) {
           const uint32_t s = pos.stage;
           if (primed && !mbar_wait(bars + 8u * (kMaxStages + s), pos.phase ^ 1u)) {
             atomicExch(p.status, 1);
             return;
           }
-          const int first      = b * per_batch;
-          const int count      = min(per_batch, f.n_trees - first);
+          const int count      = min(per_batch, t_end - first);
           const uint32_t bytes = count * tstride;
           mbar_expect_tx(bars + 8u * s, bytes);
           bulk_copy_g2s(stages + s * stage_bytes, src + static_cast<size_t>(first) * tstride,
@@ -216,13 +221,20 @@ dense_kernel(const PredictParams p, const int R, const int G, const int S, const
   const uint32_t row_addr = tile + r * TR::ES;
   RingPos pos;
   bool ok               = true;
-  for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+  grid_wait();
+  for (int64_t t = blockIdx.x / n_splits; t < n_tiles; t += tile_step) {
     const int64_t row0 = t * R;
-    const bool saw_nan = stage_rows<T>(p, tile, R, row0, warp, lane, n_cw);
+    bool saw_nan       = true;
+    if (n_splits > 1) {
+      stage_rows_async<T>(p, tile, R, row0, warp, lane, n_cw);
+    } else {
+      saw_nan = stage_rows<T>(p, tile, R, row0, warp, lane, n_cw);
+    }
     if (MODE <= MODE_VECTOR) {
       for (int i = threadIdx.x; i < G * NC * R; i += n_ct) acc[i] = T(0);
     }
     if (__any_sync(0xffffffffu, saw_nan) && lane == 0) flags[0] = 1;
+    if (n_splits > 1) cp_async_wait_all();
     consumer_sync(n_ct);
     const bool nans = flags[0] != 0;
     Running<T> run{T(0), 0, {}};
@@ -230,69 +242,27 @@ dense_kernel(const PredictParams p, const int R, const int G, const int S, const
       if (CAT || nans) {
         ok = DenseWalker<T, CAT, MODE, NT>::template walk<true>(
           p, G, S, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b, acc_group,
-          R, pos, run, b_begin, b_end);
+          R, pos, run, t_begin, t_end);
       } else {
         ok = DenseWalker<T, CAT, MODE, NT>::template walk<false>(
           p, G, S, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b, acc_group,
-          R, pos, run, b_begin, b_end);
+          R, pos, run, t_begin, t_end);
       }
       if (!ok) atomicExch(p.status, 2);
     }
     flush_running<T, MODE>(f, run, acc_group, R, r);
     consumer_sync(n_ct);
     if (MODE <= MODE_VECTOR) {
-      if (threadIdx.x < R) {
-        if (n_splits == 1) {
-          finish_row<T>(p, acc, R, G, threadIdx.x, row0 + threadIdx.x);
-        } else if (row0 + threadIdx.x < p.n_rows) {
-          // raw sums of this CTA's trees, laid out [split][output][row]
-          for (int c = 0; c < NC; ++c) {
-            T sum = acc[c * R + threadIdx.x];
-            for (int gg = 1; gg < G; ++gg) sum += acc[(gg * NC + c) * R + threadIdx.x];
-            partial[(static_cast<int64_t>(blockIdx.y) * NC + c) * p.n_rows + row0 + threadIdx.x] = sum;
-          }
-        }
+      if (n_splits > 1) {
+        finish_cluster_rows<T>(p, acc, R, G, row0, n_ct, n_splits, split);
+        cluster_wait();
+      } else if (threadIdx.x < R) {
+        finish_row<T>(p, acc, R, G, threadIdx.x, row0 + threadIdx.x);
       }
     }
     if (threadIdx.x == 0) flags[0] = 0;
     consumer_sync(n_ct);
   }
-}
-
-// Second step of a split prediction: one warp per row adds the partial sums of the splits - lane
-// l takes splits l, l + 32, ..., then a shuffle tree: a fixed order, and the loads of a row are
-// in flight together (one thread per row spent 6 us on 63 dependent loads for a one-row batch) -
-// and lane 0 applies averaging, base score, postprocessor and the output conversion.
-// `partial` is laid out [split][output][row], which is the accumulator layout finish_row expects
-// with the row count as the row stride; the sums of a row replace its split-0 slots.
-template <typename T>
-__global__ void __launch_bounds__(256)
-finish_kernel(const PredictParams p, T* __restrict__ partial, const int n_splits)
-{
-  const int64_t row = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane    = threadIdx.x & 31;
-  if (row >= p.n_rows) return;  // whole warps
-  const int NC = p.f.n_outputs;
-  for (int c = 0; c < NC; ++c) {
-    T sum = T(0);
-    for (int g = lane; g < n_splits; g += 32)
-      sum += partial[(static_cast<int64_t>(g) * NC + c) * p.n_rows + row];
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, off);
-    if (lane == 0) partial[static_cast<int64_t>(c) * p.n_rows + row] = sum;
-  }
-  if (lane == 0) finish_row<T>(p, partial, static_cast<int>(p.n_rows), 1, static_cast<int>(row), row);
-}
-
-// The same with one thread per row, for the larger of the small batches: a handful of splits,
-// thousands of rows.
-template <typename T>
-__global__ void __launch_bounds__(256)
-finish_few_splits_kernel(const PredictParams p, T* __restrict__ partial, const int n_splits)
-{
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (row >= p.n_rows) return;
-  finish_row<T>(p, partial, static_cast<int>(p.n_rows), n_splits, static_cast<int>(row), row);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -719,41 +689,22 @@ int set_smem(K kernel, size_t bytes, std::string& err)
 }
 
 template <typename T, bool CAT, int MODE>
-int launch_dense_mode(const PredictParams& p, const DenseCfg& c, dim3 grid, int n_splits,
-                      void* partial, cudaStream_t stream, std::string& err)
+int launch_dense_mode(const PredictParams& p, const DenseCfg& c, const SplitLaunch& l, int n_splits,
+                      std::string& err)
 {
-  int rc;
-  T* part = static_cast<T*>(partial);
-  if (c.trees_in_flight == 2) {
-    auto k = dense_kernel<T, CAT, MODE, 2>;
-    if ((rc = set_smem(k, c.smem_bytes, err)) != B2FIL_OK) return rc;
-    k<<<grid, c.threads, c.smem_bytes, stream>>>(p, c.rows_per_tile, c.tree_groups, c.stages,
-                                                 n_splits, part);
-  } else {
-    auto k = dense_kernel<T, CAT, MODE, 1>;
-    if ((rc = set_smem(k, c.smem_bytes, err)) != B2FIL_OK) return rc;
-    k<<<grid, c.threads, c.smem_bytes, stream>>>(p, c.rows_per_tile, c.tree_groups, c.stages,
-                                                 n_splits, part);
-  }
-  if (n_splits > 1 && MODE <= MODE_VECTOR) {
-    launch_finish_rows(p, part, n_splits, sizeof(T) == 8, stream);
-  }
-  return B2FIL_OK;
+  auto k = c.trees_in_flight == 2 ? dense_kernel<T, CAT, MODE, 2> : dense_kernel<T, CAT, MODE, 1>;
+  return launch_split(l, err, k, p, c.rows_per_tile, c.tree_groups, c.stages, n_splits);
 }
 
 template <typename T, bool CAT>
-int launch_dense_cat(const PredictParams& p, int mode, const DenseCfg& c, dim3 grid, int n_splits,
-                     void* partial, cudaStream_t stream, std::string& err)
+int launch_dense_cat(const PredictParams& p, int mode, const DenseCfg& c, const SplitLaunch& l,
+                     int n_splits, std::string& err)
 {
   switch (mode) {
-    case MODE_SCALAR:
-      return launch_dense_mode<T, CAT, MODE_SCALAR>(p, c, grid, n_splits, partial, stream, err);
-    case MODE_VECTOR:
-      return launch_dense_mode<T, CAT, MODE_VECTOR>(p, c, grid, n_splits, partial, stream, err);
-    case MODE_PERTREE:
-      return launch_dense_mode<T, CAT, MODE_PERTREE>(p, c, grid, n_splits, partial, stream, err);
-    default:
-      return launch_dense_mode<T, CAT, MODE_LEAFID>(p, c, grid, n_splits, partial, stream, err);
+    case MODE_SCALAR: return launch_dense_mode<T, CAT, MODE_SCALAR>(p, c, l, n_splits, err);
+    case MODE_VECTOR: return launch_dense_mode<T, CAT, MODE_VECTOR>(p, c, l, n_splits, err);
+    case MODE_PERTREE: return launch_dense_mode<T, CAT, MODE_PERTREE>(p, c, l, n_splits, err);
+    default: return launch_dense_mode<T, CAT, MODE_LEAFID>(p, c, l, n_splits, err);
   }
 }
 
@@ -1153,30 +1104,6 @@ std::mutex g_tuning_mu;
 std::map<std::string, int> g_tuning;
 }  // namespace
 
-namespace {
-template <typename T>
-void finish_rows(const PredictParams& p, T* part, int n_splits, cudaStream_t stream)
-{
-  if (n_splits > 4) {
-    const int blocks = static_cast<int>((p.n_rows + 7) / 8);  // a warp per row
-    finish_kernel<T><<<blocks, 256, 0, stream>>>(p, part, n_splits);
-  } else {
-    const int blocks = static_cast<int>((p.n_rows + 255) / 256);
-    finish_few_splits_kernel<T><<<blocks, 256, 0, stream>>>(p, part, n_splits);
-  }
-}
-}  // namespace
-
-void launch_finish_rows(const PredictParams& p, void* partial, int n_splits, bool f64,
-                        cudaStream_t stream)
-{
-  if (f64) {
-    finish_rows<double>(p, static_cast<double*>(partial), n_splits, stream);
-  } else {
-    finish_rows<float>(p, static_cast<float*>(partial), n_splits, stream);
-  }
-}
-
 int tuning_value(const char* key, int fallback)
 {
   std::lock_guard<std::mutex> lock(g_tuning_mu);
@@ -1216,10 +1143,6 @@ bool dense_config(int depth, int precision, int n_features, int n_outputs, bool 
                   int64_t n_rows, int chunk_size, int sm_count, DenseCfg& cfg)
 {
   int want = pick_rows_per_tile(n_rows, chunk_size, sm_count);
-  // small batches get their parallelism from splitting the forest across CTAs, not from many
-  // small row tiles: every tile has to stream the trees it walks, so fewer, larger tiles win
-  if (chunk_size <= 0 && n_rows <= static_cast<int64_t>(64) * sm_count)
-    want = n_rows <= 32 ? 32 : (n_rows <= 64 ? 64 : 128);
   for (int R = want; R >= 32; R /= 2) {
     const int rw = R / 32;
     for (int G = 16 / rw; G >= 1; G /= 2) {
@@ -1236,6 +1159,96 @@ bool dense_config(int depth, int precision, int n_features, int n_outputs, bool 
     }
   }
   return false;
+}
+
+// Small batches: fewer 128-row tiles than half the SMs.
+bool n_rows_small(int64_t n_rows, int sm_count) { return (n_rows + 127) / 128 * 2 <= sm_count; }
+
+// Launch shape of a small batch: row tiles of R rows, each shared by n_splits CTAs that walk their
+// part of the forest.  Takes the shape with the least estimated time (in SM cycles):
+//   waves x (fixed + rows + max(walk, trees))
+// `fixed` is what every CTA spends on starting, meeting and finishing, `rows` and `trees` the time
+// to bring the row tile and the CTA's trees in at the 48 bytes per cycle an SM gets from L2, `walk`
+// the steps of its tree batches, each bound by the latency of two dependent shared-memory loads
+// or by the wavefronts of all its warps (5.6 per warp and step in fp32, 9 in fp64).  Checked
+// against all shapes of four forests (100 depth-6 to 1000 depth-8 trees; 1,000 and 4,000 rows): it
+// picked the fastest each time (5.5 / 7.1 / 17.1 / 36.1 us).
+struct SplitShape {
+  DenseCfg c;
+  int n_splits;
+};
+// `rows_per_tile` > 0 asks for that R (the caller's chunk_size).
+bool pick_split_shape(const ForestView& f, int mode, int precision, int64_t n_rows,
+                      int rows_per_tile, int sm_count, SplitShape& best)
+{
+  const bool reduce   = mode <= MODE_VECTOR;
+  const double es     = precision == B2FIL_F32 ? 4 : 8;
+  const double stride = static_cast<double>(dense_tree_stride(f.dense_depth, precision));
+  const double wave_w = precision == B2FIL_F32 ? 5.6 : 9.0;
+  const int depth     = std::max(1, f.dense_depth);
+  double best_cost    = 1e300;
+  for (int R = 32; R <= 128; R *= 2) {
+    if (rows_per_tile > 0 ? R != rows_per_tile : (R > 32 && n_rows <= R / 2)) continue;
+    const int rw          = R / 32;
+    const int64_t n_tiles = (n_rows + R - 1) / R;
+    for (int G = 16 / rw; G >= 1; G /= 2) {
+      for (int NT = 2; NT >= 1; --NT) {
+        int S    = 3;
+        size_t b = dense_smem(f.dense_depth, precision, f.n_features, f.n_outputs, reduce, R, G, NT, S);
+        if (b > kMaxSmemBytes)
+          b = dense_smem(f.dense_depth, precision, f.n_features, f.n_outputs, reduce, R, G, NT, S = 2);
+        if (b > kMaxSmemBytes) continue;
+        for (int C = 1; C <= (reduce ? kMaxCluster : 64) && C <= f.n_trees; C *= 2) {
+          // one CTA per SM and wave: a second one shares the SM's bandwidth, and clusters of eight
+          // that overlap the previous launch (half the SMs taken) wait for a whole free GPC slice
+          const double waves = std::ceil(static_cast<double>(n_tiles) * C /
+                                         cluster_ctas(sm_count, reduce ? C : 1));
+          const int trees    = (f.n_trees + C - 1) / C;
+          const int batches  = (trees + G * NT - 1) / (G * NT);
+          const double walk  = batches * depth * std::max(120.0, rw * G * NT * wave_w);
+          const double rows  = static_cast<double>(R) * f.n_features * es / 48.0;
+          const double load  = trees * stride / 48.0;
+          const double cost  = waves * (4000.0 + rows + std::max(walk, load));
+          if (cost < best_cost) {
+            best_cost     = cost;
+            best.c        = DenseCfg{R, G, NT, S, b, (rw * G + 1) * 32, 1, 0};
+            best.n_splits = C;
+          }
+        }
+      }
+    }
+  }
+  return best_cost < 1e300;
+}
+
+// The same from a small per-thread table of recent answers: the search takes a few microseconds,
+// and a serving loop asks for the same few shapes again and again.
+bool split_shape(const ForestView& f, int mode, int precision, int64_t n_rows, int rows_per_tile,
+                 int sm_count, SplitShape& out)
+{
+  struct Entry {
+    int32_t depth, precision, mode, n_features, n_outputs, n_trees, rows_per_tile, sm_count;
+    int64_t n_rows;
+    bool found;
+    SplitShape shape;
+  };
+  static thread_local Entry table[8] = {};
+  static thread_local int next       = 0;
+  for (const Entry& e : table) {
+    if (e.n_rows == n_rows && e.depth == f.dense_depth && e.precision == precision &&
+        e.mode == mode && e.n_features == f.n_features && e.n_outputs == f.n_outputs &&
+        e.n_trees == f.n_trees && e.rows_per_tile == rows_per_tile && e.sm_count == sm_count) {
+      out = e.shape;
+      return e.found;
+    }
+  }
+  Entry& e = table[next];
+  next     = (next + 1) % 8;
+  e        = Entry{f.dense_depth, precision, mode, f.n_features, f.n_outputs, f.n_trees,
+                   rows_per_tile, sm_count, n_rows, false, {}};
+  e.found  = pick_split_shape(f, mode, precision, n_rows, rows_per_tile, sm_count, e.shape);
+  out      = e.shape;
+  return e.found;
 }
 
 int dense_ok(int depth, int precision, int n_features, int n_outputs)
@@ -1284,7 +1297,7 @@ int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStr
     dense_fmt && dense_ok(f.dense_depth, f.format == FMT_DENSE_F ? B2FIL_F32 : B2FIL_F64,
                           f.n_features, f.n_outputs) != 1;
   if (dense_fmt && f.q_enabled && p.row_stride < (int64_t(1) << 22) && pool != nullptr &&
-      (chunk_size > 0 || ranks_only || (p.n_rows + 127) / 128 * 2 > sm_count)) {
+      (chunk_size > 0 || ranks_only || !n_rows_small(p.n_rows, sm_count))) {
     rc = launch_dense_q(p, mode, chunk_size, sm_count, stream, pool, err, launches);
     if (rc != B2FIL_OK) return rc;
     const cudaError_t e = cudaGetLastError();
@@ -1297,35 +1310,23 @@ int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStr
   if (f.format == FMT_DENSE_F || f.format == FMT_DENSE_D) {
     const int precision = f.format == FMT_DENSE_F ? B2FIL_F32 : B2FIL_F64;
     DenseCfg c;
-    if (!dense_config(f.dense_depth, precision, f.n_features, f.n_outputs, reduce, p.n_rows,
-                      chunk_size, sm_count, c)) {
+    int n_splits = 1;
+    // small batches split the forest over CTAs: a CTA then streams only its share of the trees
+    if (SplitShape s; n_rows_small(p.n_rows, sm_count) &&
+                      split_shape(f, mode, precision, p.n_rows,
+                                  chunk_size > 0 ? pick_rows_per_tile(p.n_rows, chunk_size, sm_count) : 0,
+                                  sm_count, s)) {
+      c        = s.c;
+      n_splits = s.n_splits;
+    } else if (!dense_config(f.dense_depth, precision, f.n_features, f.n_outputs, reduce, p.n_rows,
+                             chunk_size, sm_count, c)) {
       err = "no dense launch shape fits shared memory";
       return B2FIL_ERR_UNSUPPORTED;
     }
     const int64_t n_tiles = (p.n_rows + c.rows_per_tile - 1) / c.rows_per_tile;
-    const int gx          = static_cast<int>(std::min<int64_t>(n_tiles, sm_count));
-    // batches with fewer row tiles than SMs split the forest across CTAs (blockIdx.y): a CTA then
-    // streams only its share of the trees; reduced outputs take a tiny second kernel
-    const int per_batch = c.tree_groups * c.trees_in_flight;
-    const int n_batches = (f.n_trees + per_batch - 1) / per_batch;
-    int n_splits        = 1;
-    if (n_tiles * 2 <= sm_count && (pool != nullptr || !reduce)) {  // no pool: never allocate
-      // one wave of CTAs: tiles x splits fills the SMs once
-      n_splits = static_cast<int>(std::min<int64_t>(n_batches, sm_count / n_tiles));
-      n_splits = std::max(1, n_splits);
-    }
-    void* partial = nullptr;
-    if (n_splits > 1 && reduce) {
-      const size_t es    = precision == B2FIL_F32 ? 4 : 8;
-      const size_t bytes = static_cast<size_t>(n_splits) * f.n_outputs * p.n_rows * es;
-      const cudaError_t e = cudaMallocFromPoolAsync(&partial, bytes, pool, stream);
-      if (e != cudaSuccess) {
-        cudaGetLastError();
-        err = std::string("scratch allocation for split prediction failed: ") + cudaGetErrorString(e);
-        return e == cudaErrorMemoryAllocation ? B2FIL_ERR_NO_MEMORY : B2FIL_ERR_CUDA;
-      }
-    }
-    const dim3 grid(gx, n_splits);
+    const int64_t ctas    = n_splits > 1 ? n_tiles * n_splits : std::min<int64_t>(n_tiles, sm_count);
+    const SplitLaunch l{static_cast<int>(ctas), c.threads, c.smem_bytes, stream,
+                        reduce ? n_splits : 1, n_splits > 1};
     {
       LaunchRecord& rec = g_last_launch;
       rec               = LaunchRecord{};
@@ -1340,19 +1341,14 @@ int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStr
       rec.splits        = n_splits;
     }
     if (precision == B2FIL_F32) {
-      rc = f.has_categorical
-             ? launch_dense_cat<float, true>(p, mode, c, grid, n_splits, partial, stream, err)
-             : launch_dense_cat<float, false>(p, mode, c, grid, n_splits, partial, stream, err);
+      rc = f.has_categorical ? launch_dense_cat<float, true>(p, mode, c, l, n_splits, err)
+                             : launch_dense_cat<float, false>(p, mode, c, l, n_splits, err);
     } else {
-      rc = f.has_categorical
-             ? launch_dense_cat<double, true>(p, mode, c, grid, n_splits, partial, stream, err)
-             : launch_dense_cat<double, false>(p, mode, c, grid, n_splits, partial, stream, err);
+      rc = f.has_categorical ? launch_dense_cat<double, true>(p, mode, c, l, n_splits, err)
+                             : launch_dense_cat<double, false>(p, mode, c, l, n_splits, err);
     }
-    if (partial) cudaFreeAsync(partial, stream);
-    if (launches && n_splits > 1 && reduce) ++*launches;
   } else if (CompactCfg cc; compact_config(f, reduce, pick_rows_per_tile(p.n_rows, chunk_size, sm_count),
-                                          p.n_rows, sm_count,
-                                          chunk_size <= 0 && (pool != nullptr || !reduce), cc)) {
+                                          p.n_rows, sm_count, chunk_size <= 0, cc)) {
     // deep / ragged forests with a compact image: heaps of the top levels through shared memory,
     // 8-byte internal nodes below
     LaunchRecord& rec = g_last_launch;
@@ -1367,7 +1363,7 @@ int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStr
     rec.G             = cc.tree_groups;
     rec.S             = cc.stages;
     rec.splits        = cc.splits;
-    rc = launch_sparse_compact(p, mode, cc, stream, pool, err, launches);
+    rc = launch_sparse_compact(p, mode, cc, stream, err);
   } else {
     const size_t es = f.format == FMT_SPARSE_16D ? 8 : 4;
     int R           = pick_rows_per_tile(p.n_rows, chunk_size, sm_count);
@@ -1535,7 +1531,7 @@ std::string last_launch_variant()
   s += "> R=" + std::to_string(r.R) + " G=" + std::to_string(r.G);
   if (r.S) s += " S=" + std::to_string(r.S);
   if (r.K) s += " K=" + std::to_string(r.K);
-  if (r.splits > 1) s += " forest_splits=" + std::to_string(r.splits) + " + finish_kernel";
+  if (r.splits > 1) s += " forest_splits=" + std::to_string(r.splits);
   return s;
 }
 

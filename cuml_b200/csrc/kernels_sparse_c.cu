@@ -24,8 +24,8 @@
 // threshold from a side array.  So fp64 forests run on 4-byte tiles and float compares and still
 // decide every test exactly.  (fp32 forests: xl = x, lo = threshold, only a missing value is open.)
 // Categories survive the rounding too: integers below 2^24 are floats, so trunc(xl) = trunc(x).
-// Small batches split the tree batches of a row tile over CTAs (blockIdx.y) and leave raw sums
-// for finish_kernel, like the dense kernel does.
+// Small batches split the tree batches of a row tile over the CTAs of a cluster, like the dense
+// kernel does.
 #include "device_common.cuh"
 #include "kernels_q.hpp"
 
@@ -159,29 +159,41 @@ static_assert(CMETA_SWAPPED == 0x08000000u && CMETA_SECOND_LEAF == 0x10000000u &
 
 // Stage rows [row0, row0 + R) feature-major as floats (fp64 inputs rounded down).  A warp reads 32
 // consecutive features of one row and scatters them to 32 different banks.  Rows past the end of
-// the batch become zeros.
+// the batch become zeros.  fp32 rows are asynchronous copies, fp64 rows pass through registers
+// eight loads at a time: with one load and one store in turn every 32 values cost a memory latency.
 template <typename T>
 __device__ __forceinline__ void stage_rows_as_float(const PredictParams& p, uint32_t tile, int R,
                                                     int64_t row0, int warp, int lane, int n_warps)
 {
-  const int F             = p.f.n_features;
-  const uint32_t stride_b = (R + 1) * 4u;
-  const T* X              = static_cast<const T*>(p.X);
-  for (int rr = warp; rr < R; rr += n_warps) {
-    const int64_t row = row0 + rr;
-    const bool live   = row < p.n_rows;
-    const T* src      = X + row * p.row_stride;
-    for (int c = lane; c < F; c += 32) {
-      float v = 0.f;
-      if (live) {
-        const T raw = __ldg(src + c);
-        if constexpr (sizeof(T) == 8) {
-          v = __double2float_rd(raw);
-        } else {
-          v = raw;
+  if constexpr (sizeof(T) == 4) {
+    stage_rows_async<T>(p, tile, R, row0, warp, lane, n_warps);
+    cp_async_wait_all();
+  } else {
+    const int F             = p.f.n_features;
+    const uint32_t stride_b = (R + 1) * 4u;
+    const T* X              = static_cast<const T*>(p.X);
+    constexpr int U         = 8;
+    int rr = warp, cb = 0;  // next row of the warp, next run of 32 features
+    while (rr < R) {
+      T v[U];
+      uint32_t dst[U];  // 0: nothing to store (the tile does not start at address 0)
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int c       = cb + lane;
+        const bool have   = rr < R && c < F;
+        const int64_t row = row0 + rr;
+        dst[u]            = have ? tile + c * stride_b + rr * 4u : 0u;
+        v[u]              = (have && row < p.n_rows) ? __ldg(X + row * p.row_stride + c) : T(0);
+        cb += 32;
+        if (cb >= F) {
+          cb = 0;
+          rr += n_warps;
         }
       }
-      Traits<float>::st_real(tile + c * stride_b + rr * 4u, v);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (dst[u] != 0u) Traits<float>::st_real(dst[u], __double2float_rd(v[u]));
+      }
     }
   }
 }
@@ -189,8 +201,8 @@ __device__ __forceinline__ void stage_rows_as_float(const PredictParams& p, uint
 // Shared memory: [mbarriers 256 B][row tile][accumulators][16 B][S stages of G * NT heaps].
 template <typename T, bool CAT, int MODE, int NT, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1)
-sparse_compact_kernel(const PredictParams p, const int R, const int G, const int S,
-                      const int n_splits, T* __restrict__ partial)
+sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, const int G, const int S,
+                      const int n_splits)
 {
   using TR  = Traits<T>;
   using Val = typename TR::Val;
@@ -221,11 +233,14 @@ sparse_compact_kernel(const PredictParams p, const int R, const int G, const int
   const int per_batch        = G * NT;
   const uint32_t stage_bytes = per_batch * top_stride;
   const int n_batches        = (f.n_trees + per_batch - 1) / per_batch;
-  // small batches: blockIdx.y splits the tree batches over CTAs (n_splits = gridDim.y); a CTA
-  // then streams and walks only its share and leaves raw sums for finish_kernel
-  const int b_begin = static_cast<int>(static_cast<int64_t>(n_batches) * blockIdx.y / n_splits);
-  const int b_end   = static_cast<int>(static_cast<int64_t>(n_batches) * (blockIdx.y + 1) / n_splits);
-  const int64_t n_tiles      = (p.n_rows + R - 1) / R;
+  // small batches: the tree batches of a row tile are split over n_splits CTAs, like in
+  // dense_kernel (reduced outputs: a cluster)
+  const int split   = static_cast<int>(blockIdx.x) % n_splits;
+  const int b_begin = static_cast<int>(static_cast<int64_t>(n_batches) * split / n_splits);
+  const int b_end   = static_cast<int>(static_cast<int64_t>(n_batches) * (split + 1) / n_splits);
+  const int64_t n_tiles   = (p.n_rows + R - 1) / R;
+  const int64_t tile0     = blockIdx.x / n_splits;
+  const int64_t tile_step = gridDim.x / n_splits;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -235,6 +250,7 @@ sparse_compact_kernel(const PredictParams p, const int R, const int G, const int
     mbar_fence_init();
   }
   __syncthreads();
+  grid_release();
 
   if (warp == n_cw) {
     // ---- producer: one thread streams the heaps of tree batches into the stage ring ------------
@@ -242,7 +258,7 @@ sparse_compact_kernel(const PredictParams p, const int R, const int G, const int
       const unsigned char* src = f.c_top;
       RingPos pos;
       bool primed = false;  // every stage has been filled once
-      for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+      for (int64_t t = tile0; t < n_tiles; t += tile_step) {
         for (int b = b_begin; b < b_end; ++b) {
           const uint32_t s = pos.stage;
           if (primed && !mbar_wait(bars + 8u * (kMaxStages + s), pos.phase ^ 1u)) {
@@ -272,7 +288,8 @@ sparse_compact_kernel(const PredictParams p, const int R, const int G, const int
   const CompactNode* __restrict__ nodes = f.c_nodes;
   RingPos pos;
   bool ok = true;
-  for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+  grid_wait();
+  for (int64_t t = tile0; t < n_tiles; t += tile_step) {
     const int64_t row0 = t * R;
     const int64_t row  = row0 + r;
     stage_rows_as_float<T>(p, tile, R, row0, warp, lane, n_cw);
@@ -282,7 +299,7 @@ sparse_compact_kernel(const PredictParams p, const int R, const int G, const int
     consumer_sync(n_ct);
     {
       // ask the L2 for the rows of this CTA's next tile, so that staging them does not wait on HBM
-      const int64_t next0 = row0 + static_cast<int64_t>(gridDim.x) * R;
+      const int64_t next0 = row0 + tile_step * R;
       const int row_bytes = F * static_cast<int>(sizeof(T));
       const int lines     = (row_bytes + 127) >> 7;
       for (int i = threadIdx.x; i < R * lines; i += n_ct) {
@@ -479,17 +496,11 @@ sparse_compact_kernel(const PredictParams p, const int R, const int G, const int
     flush_running<T, MODE>(f, run, acc_group, R, r);
     consumer_sync(n_ct);
     if (MODE <= MODE_VECTOR) {
-      if (threadIdx.x < R) {
-        if (n_splits == 1) {
-          finish_row<T>(p, acc, R, G, threadIdx.x, row0 + threadIdx.x);
-        } else if (row0 + threadIdx.x < p.n_rows) {
-          // raw sums of this CTA's trees, laid out [split][output][row]
-          for (int c = 0; c < NC; ++c) {
-            T sum = acc[c * R + threadIdx.x];
-            for (int gg = 1; gg < G; ++gg) sum += acc[(gg * NC + c) * R + threadIdx.x];
-            partial[(static_cast<int64_t>(blockIdx.y) * NC + c) * p.n_rows + row0 + threadIdx.x] = sum;
-          }
-        }
+      if (n_splits > 1) {
+        finish_cluster_rows<T>(p, acc, R, G, row0, n_ct, n_splits, split);
+        cluster_wait();
+      } else if (threadIdx.x < R) {
+        finish_row<T>(p, acc, R, G, threadIdx.x, row0 + threadIdx.x);
       }
     }
     consumer_sync(n_ct);
@@ -507,36 +518,25 @@ size_t compact_smem(const ForestView& f, size_t es, bool reduce, int R, int G, i
 }
 
 template <typename T, bool CAT, int MODE>
-int launch_mode(const PredictParams& p, const CompactCfg& c, void* partial, cudaStream_t stream,
-                std::string& err)
+int launch_mode(const PredictParams& p, const CompactCfg& c, cudaStream_t stream, std::string& err)
 {
-  const dim3 grid(c.grid, c.splits);
-  T* part = static_cast<T*>(partial);
-  if (c.threads > kCompactThreads) {
-    auto k       = sparse_compact_kernel<T, CAT, MODE, kCompactTreesInFlight, kCompactThreadsBig>;
-    const int rc = set_smem_bytes(reinterpret_cast<const void*>(k), c.smem_bytes, err);
-    if (rc != B2FIL_OK) return rc;
-    k<<<grid, c.threads, c.smem_bytes, stream>>>(p, c.rows_per_tile, c.tree_groups, c.stages,
-                                                 c.splits, part);
-    return B2FIL_OK;
-  }
-  auto k       = sparse_compact_kernel<T, CAT, MODE, kCompactTreesInFlight, kCompactThreads>;
-  const int rc = set_smem_bytes(reinterpret_cast<const void*>(k), c.smem_bytes, err);
-  if (rc != B2FIL_OK) return rc;
-  k<<<grid, c.threads, c.smem_bytes, stream>>>(p, c.rows_per_tile, c.tree_groups, c.stages,
-                                               c.splits, part);
-  return B2FIL_OK;
+  auto k = c.threads > kCompactThreads
+             ? sparse_compact_kernel<T, CAT, MODE, kCompactTreesInFlight, kCompactThreadsBig>
+             : sparse_compact_kernel<T, CAT, MODE, kCompactTreesInFlight, kCompactThreads>;
+  const SplitLaunch l{c.grid * c.splits, c.threads, c.smem_bytes, stream,
+                      MODE <= MODE_VECTOR ? c.splits : 1, c.splits > 1};
+  return launch_split(l, err, k, p, c.rows_per_tile, c.tree_groups, c.stages, c.splits);
 }
 
 template <typename T, bool CAT>
-int launch_cat(const PredictParams& p, int mode, const CompactCfg& c, void* partial,
-               cudaStream_t stream, std::string& err)
+int launch_cat(const PredictParams& p, int mode, const CompactCfg& c, cudaStream_t stream,
+               std::string& err)
 {
   switch (mode) {
-    case MODE_SCALAR: return launch_mode<T, CAT, MODE_SCALAR>(p, c, partial, stream, err);
-    case MODE_VECTOR: return launch_mode<T, CAT, MODE_VECTOR>(p, c, partial, stream, err);
-    case MODE_PERTREE: return launch_mode<T, CAT, MODE_PERTREE>(p, c, partial, stream, err);
-    default: return launch_mode<T, CAT, MODE_LEAFID>(p, c, partial, stream, err);
+    case MODE_SCALAR: return launch_mode<T, CAT, MODE_SCALAR>(p, c, stream, err);
+    case MODE_VECTOR: return launch_mode<T, CAT, MODE_VECTOR>(p, c, stream, err);
+    case MODE_PERTREE: return launch_mode<T, CAT, MODE_PERTREE>(p, c, stream, err);
+    default: return launch_mode<T, CAT, MODE_LEAFID>(p, c, stream, err);
   }
 }
 
@@ -549,11 +549,16 @@ bool compact_config(const ForestView& f, bool reduce, int rows_per_tile, int64_t
   const size_t es = f.format == FMT_SPARSE_16D ? 8 : 4;
   // Small batches (fewer row tiles than half the SMs): one CTA per tile would walk the whole
   // forest batch after batch, which is what bounds their latency.  The tree batches are split
-  // over CTAs instead (tiles x splits fills the SMs once) with few tree groups per CTA, so that
-  // there are enough batches to split.
+  // over CTAs instead (tiles x splits fills the SMs once; reduced outputs: the CTAs of a cluster)
+  // with few tree groups per CTA, so that there are enough batches to split.
   const int64_t small_tiles = (n_rows + 31) / 32;
   if (may_split && small_tiles * 2 <= sm_count && tuning_value("compact_R", 0) == 0) {
-    const int want_splits = static_cast<int>(sm_count / small_tiles);
+    int want_splits = static_cast<int>(sm_count / small_tiles);
+    if (reduce) {
+      int c = kMaxCluster;
+      while (c > want_splits) c /= 2;
+      want_splits = c;
+    }
     const int n_quads     = (f.n_trees + kCompactTreesInFlight - 1) / kCompactTreesInFlight;
     int G                 = std::max(1, std::min(31, (n_quads + want_splits - 1) / want_splits));
     for (; G >= 1; --G) {
@@ -561,7 +566,9 @@ bool compact_config(const ForestView& f, bool reduce, int rows_per_tile, int64_t
       if (b > kMaxSmemBytes) continue;
       const int per_batch = G * kCompactTreesInFlight;
       const int n_batches = (f.n_trees + per_batch - 1) / per_batch;
-      const int splits    = std::max(1, std::min(n_batches, want_splits));
+      int splits          = std::max(1, std::min(n_batches, want_splits));
+      if (reduce)  // whole clusters at once, or fewer CTAs per cluster
+        while (splits > 1 && cluster_ctas(sm_count, splits) < small_tiles * splits) --splits;
       cfg = CompactCfg{32, G, 1, b, (G + 1) * 32, static_cast<int>(small_tiles), splits};
       return true;
     }
@@ -604,37 +611,14 @@ bool compact_config(const ForestView& f, bool reduce, int rows_per_tile, int64_t
 }
 
 int launch_sparse_compact(const PredictParams& p, int mode, const CompactCfg& c,
-                          cudaStream_t stream, cudaMemPool_t pool, std::string& err,
-                          int64_t* launches)
+                          cudaStream_t stream, std::string& err)
 {
   const ForestView& f = p.f;
-  const bool f64      = f.format == FMT_SPARSE_16D;
-  void* partial       = nullptr;
-  if (c.splits > 1 && mode <= MODE_VECTOR) {
-    const size_t bytes  = static_cast<size_t>(c.splits) * f.n_outputs * p.n_rows * (f64 ? 8 : 4);
-    const cudaError_t e = cudaMallocFromPoolAsync(&partial, bytes, pool, stream);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      err = std::string("scratch allocation for split prediction failed: ") + cudaGetErrorString(e);
-      return e == cudaErrorMemoryAllocation ? B2FIL_ERR_NO_MEMORY : B2FIL_ERR_CUDA;
-    }
-  }
-  int rc;
-  if (f64) {
-    rc = f.has_categorical ? launch_cat<double, true>(p, mode, c, partial, stream, err)
-                           : launch_cat<double, false>(p, mode, c, partial, stream, err);
-  } else {
-    rc = f.has_categorical ? launch_cat<float, true>(p, mode, c, partial, stream, err)
-                           : launch_cat<float, false>(p, mode, c, partial, stream, err);
-  }
-  if (partial) {
-    if (rc == B2FIL_OK) {
-      launch_finish_rows(p, partial, c.splits, f64, stream);
-      if (launches) ++*launches;
-    }
-    cudaFreeAsync(partial, stream);
-  }
-  return rc;
+  if (f.format == FMT_SPARSE_16D)
+    return f.has_categorical ? launch_cat<double, true>(p, mode, c, stream, err)
+                             : launch_cat<double, false>(p, mode, c, stream, err);
+  return f.has_categorical ? launch_cat<float, true>(p, mode, c, stream, err)
+                           : launch_cat<float, false>(p, mode, c, stream, err);
 }
 
 }  // namespace b2fil

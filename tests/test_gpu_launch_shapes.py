@@ -1,0 +1,24 @@
+"""Launch shapes of the prediction kernels at the sizes where they change: every output kind against
+the CPU oracle."""
+import pytest
+
+from tests.helpers import random_forest_desc, random_rows
+from tests.test_gpu_parity import _all_kinds
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("storage", ["dense", "sparse"])
+@pytest.mark.parametrize("kw", [dict(n_trees=3, postproc="sigmoid"),
+                                dict(n_trees=67, n_outputs=3, postproc="softmax"),
+                                dict(n_trees=130, n_outputs=5, vector=True, average=True),
+                                dict(n_trees=40, categorical=True, n_features=37)])
+def test_small_batches_split_over_clusters(kw, storage, precision):
+    """Row counts around the edges of a tile and of every cluster size, forests with fewer trees
+    than CTAs in a cluster and with a tree count no cluster size divides."""
+    desc = random_forest_desc(90, max_depth=6, **kw)
+    for n in (1, 33, 128, 481, 1057, 4737):
+        X = random_rows(n, n, desc.n_features, "float64", nan_frac=0.03,
+                        categories=22 if kw.get("categorical") else None)
+        _all_kinds(desc, X, precision, "depth_first", storage)
