@@ -12,13 +12,18 @@ namespace {
 // ---------------------------------------------------------------------------------------------
 // DENSE kernel on rank-quantised rows
 // ---------------------------------------------------------------------------------------------
-// Shared memory: [mbarriers 128 B][row tile F x R uint16][accumulators][flags 16 B][S tree stages].
-// The row tile arrives with one bulk copy per tile (the pre-pass already stored it feature-major);
+// Shared memory: [mbarriers][1 or 2 row tiles F x R uint16][1 or 2 sets of accumulators][16 B]
+// [S tree stages].
+// The row tile arrives with one bulk copy per tile (the pre-pass already stored it feature-major),
+// where there is room for two while the tile before it is being walked (forests whose trees last
+// only a few microseconds per tile spend a fifth of them waiting for it otherwise);
 // tree batches stream through the stage ring exactly as in dense_kernel.  A node is 4 bytes
 // (rank j << 17 | default-right << 16 | feature << 2 | categorical) and a test is one signed
 // subtraction.
-constexpr int kBarTileFull  = 2 * kMaxStages;      // mbarrier slots after the stage ring
-constexpr int kBarTileEmpty = 2 * kMaxStages + 1;
+constexpr int NAN_NONE = 0, NAN_TESTED = 1, NAN_COLUMNS = 2;
+
+constexpr int kBarTileFull  = 2 * kMaxStages;      // mbarrier slots after the stage ring: two each
+constexpr int kBarTileEmpty = 2 * kMaxStages + 2;
 
 // node - (q << 17) in one multiply-add: the sign of (j - rank) lands in bit 31.
 __device__ __forceinline__ uint32_t rank_diff(uint32_t node, uint32_t q)
@@ -62,14 +67,19 @@ struct DenseQWalker {
   using TR = Traits<T>;
   // Walk the warp's 32 rows through all trees.  A stage of the ring holds K sub-batches of G * NT
   // trees; the warp waits once per stage and walks its NT trees of every sub-batch.
-  template <bool NANS>
+  // MISSING says what a missing value costs: nothing (NAN_NONE: there is none, or NAN_COLUMNS: the
+  // doubled columns of the tile take care of it; only the top nodes, which exist once, pick the
+  // column by their direction) or a comparison per test (NAN_TESTED).
+  template <int MISSING>
   static __device__ __forceinline__ bool walk(const PredictParams& p, int G, int S, int K, int g,
                                               int r, int64_t row, int lane, uint32_t bars,
                                               uint32_t stages, uint32_t stage_bytes,
                                               uint32_t row_addr, uint32_t stride_b, T* acc_group,
                                               int R, RingPos& pos, Running<T>& run,
-                                              const QTop* top)
+                                              const QTop* top, int b_begin, int b_end,
+                                              uint32_t copy_off)
   {
+    constexpr bool NANS = MISSING == NAN_TESTED;
     static_assert(!TOPC || (DEPTH >= 2 && !CAT), "top nodes need two plain levels");
     static_assert(!PAIR || (!CAT && !TOPC && MODE == MODE_SCALAR && sizeof(T) == 4),
                   "the child-pair walk exists for fp32 scalar leaves without categorical tests");
@@ -87,7 +97,6 @@ struct DenseQWalker {
     const uint32_t fstride = stride_b >> Q_FEATURE_SHIFT;  // R / 2 <= 128: fits a byte
     const int per_sub      = G * NT;
     const int per_batch    = per_sub * K;
-    const int n_batches    = (f.n_trees + per_batch - 1) / per_batch;
     const uint32_t mine    = static_cast<uint32_t>(g * NT) * tstride;  // this warp's trees in a sub-batch
     const uint32_t sub_b   = static_cast<uint32_t>(per_sub) * tstride;
     bool ok                = true;
@@ -117,14 +126,19 @@ struct DenseQWalker {
       // the NT walks are independent: all node loads are issued first, then all rank loads,
       // so that their shared-memory latencies overlap inside one warp.
       // test(): the rows' ranks against NT nodes; the sign bit of d[k] is the step to the right.
-      auto test = [&](const uint32_t(&node)[NT], const uint32_t(&bits)[CAT ? NT : 1], uint32_t(&d)[NT]) {
+      auto test = [&](const uint32_t(&node)[NT], const uint32_t(&bits)[CAT ? NT : 1], uint32_t(&d)[NT],
+                      auto is_top) {
         uint32_t q[NT];
 #pragma unroll
-        for (int k = 0; k < NT; ++k)
+        for (int k = 0; k < NT; ++k) {
+          uint32_t from = row_addr;
+          if (decltype(is_top)::value && MISSING == NAN_COLUMNS && !(node[k] & Q_DEFAULT_RIGHT))
+            from += copy_off;
           // the low half of a node is feature * 4: one dot-product instruction (low half x byte 0
           // of fstride, high half x byte 1 = 0) turns it into the address of the row's rank of
           // that feature
-          q[k] = lds_u16(__dp2a_lo(node[k], fstride, row_addr));
+          q[k] = lds_u16(__dp2a_lo(node[k], fstride, from));
+        }
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           // rank j in the high half: x < T[j] <=> rank(x) <= j, so right <=> j - rank < 0
@@ -162,7 +176,7 @@ struct DenseQWalker {
             node[k] = lds_u32(a[k]);
           }
         }
-        test(node, bits, d);
+        test(node, bits, d, std::false_type{});
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           // heap index 2i + right in one funnel shift: (i << 1) | (d >> 31)
@@ -182,7 +196,7 @@ struct DenseQWalker {
           uint2 pair[NT];
 #pragma unroll
           for (int k = 0; k < NT; ++k) pair[k] = lds_u32x2(base[k] + idx[k] * 8u);
-          test(node, reinterpret_cast<const uint32_t(&)[CAT ? NT : 1]>(no_bits), d);
+          test(node, reinterpret_cast<const uint32_t(&)[CAT ? NT : 1]>(no_bits), d, std::false_type{});
 #pragma unroll
           for (int k = 0; k < NT; ++k) {
             idx[k]  = __funnelshift_l(d[k], idx[k], 1);
@@ -206,13 +220,13 @@ struct DenseQWalker {
           n2[k]       = top->w[t + 1];
           n3[k]       = top->w[t + 2];
         }
-        test(n1, reinterpret_cast<const uint32_t(&)[CAT ? NT : 1]>(no_bits), d);
+        test(n1, reinterpret_cast<const uint32_t(&)[CAT ? NT : 1]>(no_bits), d, std::true_type{});
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           node[k] = static_cast<int32_t>(d[k]) < 0 ? n3[k] : n2[k];
           idx[k]  = __funnelshift_l(d[k], 1u, 1);
         }
-        test(node, reinterpret_cast<const uint32_t(&)[CAT ? NT : 1]>(no_bits), d);
+        test(node, reinterpret_cast<const uint32_t(&)[CAT ? NT : 1]>(no_bits), d, std::true_type{});
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           idx[k] = __funnelshift_l(d[k], idx[k], 1);
@@ -334,7 +348,7 @@ struct DenseQWalker {
       }
     };
 
-    for (int b = 0; b < n_batches; ++b) {
+    for (int b = b_begin; b < b_end; ++b) {
       const uint32_t s = pos.stage;
       if (ok) ok = mbar_wait(bars + 8u * s, pos.phase);
       if (ok) {
@@ -360,16 +374,117 @@ struct DenseQWalker {
   }
 };
 
+// Which (row tile, tree batches) a CTA walks.  The row tiles of a launch, each with all its tree
+// batches, form one line of units that is cut into equal parts, one per CTA: a CTA walks the end
+// of one tile, some whole tiles, and the beginning of another, so that a launch takes the time of
+// its average CTA however few tiles there are (157 tiles on 148 SMs used to take two rounds, the
+// second almost empty).  Tiles that are cut leave partial sums (finish_shared_tile).  When sums
+// cannot be exchanged (QArgs::partial is null and outputs are reduced) only whole tiles are dealt.
+struct QSegments {
+  int32_t tile, begin;           // current tile, and the first tree batch of the segment
+  int32_t last_tile, last_end;   // the CTA's part ends before batch last_end of tile last_tile
+  int32_t n_batches;
+  __device__ __forceinline__ QSegments(int64_t n_tiles, int nb, bool cut) : n_batches(nb)
+  {
+    int64_t u0 = n_tiles * blockIdx.x / gridDim.x, u1 = n_tiles * (blockIdx.x + 1) / gridDim.x;
+    if (cut) {
+      const int64_t units = n_tiles * nb;
+      u0        = units * blockIdx.x / gridDim.x;
+      u1        = units * (blockIdx.x + 1) / gridDim.x;
+      tile      = static_cast<int32_t>(u0 / nb);
+      begin     = static_cast<int32_t>(u0 - static_cast<int64_t>(tile) * nb);
+      last_tile = static_cast<int32_t>(u1 / nb);
+      last_end  = static_cast<int32_t>(u1 - static_cast<int64_t>(last_tile) * nb);
+    } else {
+      tile      = static_cast<int32_t>(u0);
+      last_tile = static_cast<int32_t>(u1);
+      begin = last_end = 0;
+    }
+  }
+  __device__ __forceinline__ int32_t end() const { return tile < last_tile ? n_batches : last_end; }
+  __device__ __forceinline__ bool live() const
+  {
+    return tile < last_tile || (tile == last_tile && begin < last_end);
+  }
+  // does another segment follow this one?
+  __device__ __forceinline__ bool more() const
+  {
+    return tile + 1 < last_tile || (tile + 1 == last_tile && last_end > 0);
+  }
+  __device__ __forceinline__ bool whole() const { return begin == 0 && tile < last_tile; }
+  __device__ __forceinline__ void next()
+  {
+    ++tile;
+    begin = 0;
+  }
+};
+
+// A tile that several CTAs share.  The CTA leaves its sums in global memory; the one that arrives
+// last adds all of them in CTA order (a fixed order whoever is last) and finishes the rows.
+// Called by the consumer threads, `sums` = the CTA's accumulators [group][output][row].
+template <typename T>
+__device__ __forceinline__ void finish_shared_tile(const PredictParams& p, const QArgs& q,
+                                                   const QSegments& seg, bool first_segment,
+                                                   T* sums, volatile int* last_flag, int n_ct,
+                                                   int64_t n_tiles)
+{
+  const int NC    = p.f.n_outputs;
+  const int R     = q.R;
+  T* partial      = static_cast<T*>(q.partial);
+  T* mine         = partial + static_cast<int64_t>(2 * blockIdx.x + (first_segment ? 0 : 1)) * NC * R;
+  for (int i = threadIdx.x; i < NC * R; i += n_ct) {
+    T s = sums[i];
+    for (int g = 1; g < q.G; ++g) s += sums[g * NC * R + i];
+    __stcg(mine + i, s);
+  }
+  __threadfence();
+  consumer_sync(n_ct);
+  if (threadIdx.x == 0) {
+    const int n    = seg.end() - seg.begin;
+    const int seen = atomicAdd(q.arrived + seg.tile, n);
+    __threadfence();
+    *last_flag = seen + n == seg.n_batches;
+  }
+  consumer_sync(n_ct);
+  if (*last_flag == 0) return;
+  // CTAs that share the tile: those whose units overlap [tile * n_batches, (tile + 1) * n_batches)
+  const int64_t units = n_tiles * seg.n_batches;
+  const int64_t u     = static_cast<int64_t>(seg.tile) * seg.n_batches;
+  const int lo        = static_cast<int>(((u + 1) * gridDim.x - 1) / units);
+  const int hi        = static_cast<int>(((u + seg.n_batches) * gridDim.x - 1) / units);
+  // the tile is the first segment of every one of them but, perhaps, the first
+  const int lo_slot = units * lo / gridDim.x >= u ? 2 * lo : 2 * lo + 1;
+  const int64_t stride = static_cast<int64_t>(2) * NC * R;  // between the first segments of two CTAs
+  for (int i = threadIdx.x; i < NC * R; i += n_ct) {
+    T s           = __ldcg(partial + static_cast<int64_t>(lo_slot) * NC * R + i);
+    const T* from = partial + stride * (lo + 1) + i;
+    for (int k0 = lo + 1; k0 <= hi; k0 += 8, from += 8 * stride) {
+      T part[8];  // loads in flight together
+#pragma unroll
+      for (int k = 0; k < 8; ++k) part[k] = k0 + k <= hi ? __ldcg(from + k * stride) : T(0);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) s += part[k];
+    }
+    sums[i] = s;
+  }
+  consumer_sync(n_ct);
+  if (threadIdx.x < R)
+    finish_row<T>(p, sums, R, 1, threadIdx.x, static_cast<int64_t>(seg.tile) * R + threadIdx.x);
+}
+
 template <typename T, int MODE, int NT, int DEPTH, bool CAT, bool TOPC, bool PAIR = false,
           bool LEAFG = false>
-__device__ __forceinline__ void dense_q_body(const PredictParams& p, const uint16_t* __restrict__ Q,
-                                             const int32_t* __restrict__ tile_flags, const int R,
-                                             const int G, const int S, const int K,
+__device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs& q,
                                              const QTop* top)
 {
   using TR = Traits<T>;
+  using Walker = DenseQWalker<T, MODE, NT, DEPTH, CAT, TOPC, PAIR, LEAFG>;
   extern __shared__ __align__(128) unsigned char smem[];
   const ForestView& f = p.f;
+  const int R         = q.R;
+  const int G         = q.G;
+  const int S         = q.S;
+  const int K         = q.K;
   const int F         = f.n_features;
   const int NC        = f.n_outputs;
   const int rw        = R >> 5;
@@ -377,13 +492,16 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const uint1
   const int n_ct      = n_cw * 32;
   const int warp      = threadIdx.x >> 5;
   const int lane      = threadIdx.x & 31;
+  constexpr bool REDUCE = MODE <= MODE_VECTOR;
 
   const uint32_t stride_b    = R * 2u;  // bytes between features in the tile
   const uint32_t tile_bytes  = static_cast<uint32_t>(F) * stride_b;  // multiple of 64
-  const size_t acc_bytes     = (MODE <= MODE_VECTOR) ? align16(static_cast<size_t>(G) * NC * R * TR::ES) : 0;
+  const uint32_t acc_bytes   = REDUCE ? static_cast<uint32_t>(align16(static_cast<size_t>(G) * NC * R * TR::ES)) : 0u;
   unsigned char* tile_ptr    = smem + kBarBytes;
-  T* acc                     = reinterpret_cast<T*>(tile_ptr + tile_bytes);
-  unsigned char* stage_ptr   = tile_ptr + tile_bytes + acc_bytes + 16;
+  const uint32_t tile_room   = tile_bytes * (q.nan_columns ? 2u : 1u);  // per buffer
+  unsigned char* acc_ptr     = tile_ptr + q.tile_bufs * tile_room;
+  volatile int* last_flag    = reinterpret_cast<volatile int*>(acc_ptr + q.acc_bufs * acc_bytes);
+  unsigned char* stage_ptr   = acc_ptr + q.acc_bufs * acc_bytes + 16;
   const uint32_t bars        = smem_addr(smem);
   const uint32_t tile        = smem_addr(tile_ptr);
   const uint32_t stages      = smem_addr(stage_ptr);
@@ -402,52 +520,81 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const uint1
       mbar_init(bars + 8u * s, 1);
       mbar_init(bars + 8u * (kMaxStages + s), n_cw);
     }
-    mbar_init(bar_tfull, 1);
-    mbar_init(bar_tempty, n_cw);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar_tfull + 8u * i, 1);
+      mbar_init(bar_tempty + 8u * i, n_cw);
+    }
     mbar_fence_init();
   }
   __syncthreads();
+  grid_release();
+  QSegments seg(n_tiles, n_batches, !REDUCE || q.partial != nullptr);
+
+  // does the tile hold a missing value?  (asked by whole warps)
+  auto has_nan = [&](int t) {
+    uint32_t bits = 0;
+    for (int i = lane; i < q.flag_words; i += 32)
+      bits |= __ldg(q.flags + static_cast<int64_t>(t) * q.flag_words + i);
+    return __any_sync(0xffffffffu, bits != 0u);
+  };
 
   if (warp == n_cw) {
-    // ---- producer: row tile, then the tree batches of that tile ------------------------------
-    if (lane == 0) {
-      // predictions that report leaves stream the image whose payload slots hold the leaf ids
-      const unsigned char* src  = static_cast<const unsigned char*>(
-        MODE == MODE_LEAFID ? f.q_nodes_ids : f.q_nodes);
-      const unsigned char* qsrc = reinterpret_cast<const unsigned char*>(Q);
-      RingPos pos;
-      bool primed               = false;  // every stage has been filled once
-      uint32_t n_done           = 0;
-      for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x, ++n_done) {
-        // the tile buffer is free once every consumer warp has left the previous tile's trees
-        if (n_done > 0 && !mbar_wait(bar_tempty, (n_done - 1) & 1u)) {
-          atomicExch(p.status, 3);
-          return;
+    // ---- producer: row tiles, and the tree batches of each of them -----------------------------
+    // predictions that report leaves stream the image whose payload slots hold the leaf ids
+    const void* image         = MODE == MODE_LEAFID ? f.q_nodes_ids : f.q_nodes;
+    const unsigned char* qsrc = reinterpret_cast<const unsigned char*>(q.Q);
+    RingPos pos;
+    bool primed = false;  // every stage has been filled once
+    RingPos tpos;         // buffer of the next tile to request, and the parity of its use
+    bool tprimed = false;
+    auto request_tile = [&](int t) {
+      // a buffer is free once every consumer warp has left the trees of the tile it held
+      if (tprimed && !mbar_wait(bar_tempty + 8u * tpos.stage, tpos.phase ^ 1u)) {
+        atomicExch(p.status, 3);
+        return false;
+      }
+      const uint32_t bar = bar_tfull + 8u * tpos.stage;
+      mbar_expect_tx(bar, tile_bytes);
+      bulk_copy_g2s(tile + tpos.stage * tile_room, qsrc + static_cast<size_t>(t) * tile_bytes,
+                    tile_bytes, bar);
+      tpos.advance(q.tile_bufs);
+      if (tpos.stage == 0) tprimed = true;
+      return true;
+    };
+    grid_wait();
+    bool going = seg.live();
+    if (lane == 0 && going) going = request_tile(seg.tile);
+    for (; seg.live(); seg.next()) {
+      const bool nan_image = q.nan_columns && has_nan(seg.tile);
+      if (lane != 0 || !going) continue;
+      const unsigned char* src = static_cast<const unsigned char*>(nan_image ? f.q_nodes_nan : image);
+      const bool more = seg.more();
+      const int end   = seg.end();
+      // with two buffers the next tile is requested once the ring is full of this tile's trees
+      const int ask_at = q.tile_bufs == 2 ? min(end, seg.begin + S) - 1 : end - 1;
+      for (int b = seg.begin; b < end && going; ++b) {
+        const uint32_t s = pos.stage;
+        if (primed && !mbar_wait(bars + 8u * (kMaxStages + s), pos.phase ^ 1u)) {
+          atomicExch(p.status, 1);
+          going = false;
+          break;
         }
-        mbar_expect_tx(bar_tfull, tile_bytes);
-        bulk_copy_g2s(tile, qsrc + static_cast<size_t>(t) * tile_bytes, tile_bytes, bar_tfull);
-        for (int b = 0; b < n_batches; ++b) {
-          const uint32_t s = pos.stage;
-          if (primed && !mbar_wait(bars + 8u * (kMaxStages + s), pos.phase ^ 1u)) {
-            atomicExch(p.status, 1);
-            return;
-          }
-          const int first      = b * per_batch;
-          const int count      = min(per_batch, f.n_trees - first);
-          const uint32_t bytes = count * tstride;
-          mbar_expect_tx(bars + 8u * s, bytes);
-          if (LEAFG) {
-            // one copy per tree: the node half of its block
-            for (int i = 0; i < count; ++i)
-              bulk_copy_g2s(stages + s * stage_bytes + i * tstride,
-                            src + static_cast<size_t>(first + i) * gstride, tstride, bars + 8u * s);
-          } else {
-            bulk_copy_g2s(stages + s * stage_bytes, src + static_cast<size_t>(first) * gstride,
-                          bytes, bars + 8u * s);
-          }
-          pos.advance(S);
-          if (pos.stage == 0) primed = true;
+        const int first      = b * per_batch;
+        const int count      = min(per_batch, f.n_trees - first);
+        const uint32_t bytes = count * tstride;
+        mbar_expect_tx(bars + 8u * s, bytes);
+        if (LEAFG) {
+          // one copy per tree: the node half of its block
+          for (int i = 0; i < count; ++i)
+            bulk_copy_g2s(stages + s * stage_bytes + i * tstride,
+                          src + static_cast<size_t>(first + i) * gstride, tstride, bars + 8u * s);
+        } else {
+          bulk_copy_g2s(stages + s * stage_bytes, src + static_cast<size_t>(first) * gstride, bytes,
+                        bars + 8u * s);
         }
+        pos.advance(S);
+        if (pos.stage == 0) primed = true;
+        if (more && b == ask_at) going = request_tile(seg.tile + 1);
       }
     }
     return;
@@ -456,82 +603,111 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const uint1
   // ---- consumers ------------------------------------------------------------------------------
   const int g             = warp / rw;
   const int r             = (warp % rw) * 32 + lane;
-  T* acc_group            = acc + static_cast<size_t>(g) * NC * R;
-  const uint32_t row_addr = tile + q_slot(r, R) * 2u;
-  RingPos pos;
-  uint32_t n_done         = 0;
+  const uint32_t row_slot = tile + q_slot(r, R) * 2u;
+  // sums that the walk keeps in registers to its end are stored, others are added to zeroed ones
+  const bool stored       = MODE == MODE_SCALAR ? NC == 1 : NC <= kRegClasses;
+  RingPos pos, tpos;
+  int acc_set             = 0;
+  int finisher            = 0;     // the tree group that finishes the rows of the tile
+  bool first_segment      = true;
   bool ok                 = true;
-  for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x, ++n_done) {
-    const int64_t row0 = t * R;
-    if (MODE <= MODE_VECTOR) {
-      for (int i = threadIdx.x; i < G * NC * R; i += n_ct) acc[i] = T(0);
+  grid_wait();
+  for (; seg.live(); seg.next()) {
+    const int64_t row0 = static_cast<int64_t>(seg.tile) * R;
+    T* acc             = reinterpret_cast<T*>(acc_ptr + acc_set * acc_bytes);
+    T* acc_group       = acc + static_cast<size_t>(g) * NC * R;
+    if (REDUCE && !stored) {
+      for (int c = 0; c < NC; ++c) acc_group[c * R + r] = T(0);  // nobody else's
     }
-    const bool nans = __ldg(tile_flags + t) != 0;
-    consumer_sync(n_ct);
-    if (ok) ok = mbar_wait(bar_tfull, n_done & 1u);
+    const bool nans = has_nan(seg.tile);
+    if (ok) ok = mbar_wait(bar_tfull + 8u * tpos.stage, tpos.phase);
     Running<T> run{T(0), 0, {}};
+    const uint32_t at_tile = tpos.stage * tile_room;
+    if (nans && q.nan_columns) {
+      // the second set of columns: the NaN code moves from "right" to "left"
+      for (uint32_t i = threadIdx.x * 16u; i < tile_bytes; i += n_ct * 16u) {
+        uint4* from = reinterpret_cast<uint4*>(tile_ptr + at_tile + i);
+        uint4 v     = *from;
+        uint32_t* w = &v.x;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          w[k] |= __vcmpeq2(w[k], Q_NAN_CODE * 0x10001u) & Q_NAN_LEFT_BIT * 0x10001u;
+        *reinterpret_cast<uint4*>(tile_ptr + at_tile + tile_bytes + i) = v;
+      }
+      consumer_sync(n_ct);
+    }
     if (ok) {
-      if (nans) {
-        ok = DenseQWalker<T, MODE, NT, DEPTH, CAT, TOPC, PAIR, LEAFG>::template walk<true>(
-          p, G, S, K, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b,
-          acc_group, R, pos, run, top);
+      const uint32_t row_addr = row_slot + at_tile;
+      auto go = [&](auto missing) {
+        return Walker::template walk<decltype(missing)::value>(
+          p, G, S, K, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b, acc_group,
+          R, pos, run, top, seg.begin, seg.end(), tile_bytes);
+      };
+      if (nans && !q.nan_columns) {
+        ok = go(std::integral_constant<int, NAN_TESTED>{});
+      } else if (TOPC && nans) {
+        ok = go(std::integral_constant<int, TOPC ? NAN_COLUMNS : NAN_NONE>{});
       } else {
-        ok = DenseQWalker<T, MODE, NT, DEPTH, CAT, TOPC, PAIR, LEAFG>::template walk<false>(
-          p, G, S, K, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b,
-          acc_group, R, pos, run, top);
+        // (without top nodes in the parameter block the walk over doubled columns is the same one)
+        ok = go(std::integral_constant<int, NAN_NONE>{});
       }
       if (!ok) atomicExch(p.status, 2);
     }
     __syncwarp();
-    if (lane == 0) mbar_arrive(bar_tempty);
-    flush_running<T, MODE>(f, run, acc_group, R, r);
-    consumer_sync(n_ct);
-    if (MODE <= MODE_VECTOR) {
-      if (threadIdx.x < R) finish_row<T>(p, acc, R, G, threadIdx.x, row0 + threadIdx.x);
+    if (lane == 0) mbar_arrive(bar_tempty + 8u * tpos.stage);
+    tpos.advance(q.tile_bufs);
+    if (REDUCE) {
+      flush_running<T, MODE>(f, run, acc_group, R, r, stored);
+      consumer_sync(n_ct);
+      if (seg.whole()) {
+        if (g == finisher) finish_row<T>(p, acc, R, G, r, row0 + r);
+        if (++finisher == G) finisher = 0;
+      } else {
+        finish_shared_tile<T>(p, q, seg, first_segment, acc, last_flag, n_ct, n_tiles);
+      }
+      first_segment = false;
+      // with two sets of accumulators the next meeting is early enough: by then the finishers
+      // have read this set
+      if (q.acc_bufs == 2) {
+        acc_set ^= 1;
+      } else {
+        consumer_sync(n_ct);
+      }
     }
-    consumer_sync(n_ct);
   }
 }
 
 
 template <typename T, int MODE, int NT, int DEPTH, bool CAT>
 __global__ void __launch_bounds__(NT > 4 ? 800 : 1024, 1)
-dense_q_kernel(const PredictParams p, const uint16_t* __restrict__ Q,
-               const int32_t* __restrict__ tile_flags, const int R, const int G, const int S,
-               const int K)
+dense_q_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q)
 {
-  dense_q_body<T, MODE, NT, DEPTH, CAT, false>(p, Q, tile_flags, R, G, S, K, nullptr);
+  dense_q_body<T, MODE, NT, DEPTH, CAT, false>(p, q, nullptr);
 }
 
 // Same kernel with the child-pair walk (see DenseQWalker).
 template <int NT>
 __global__ void __launch_bounds__(1024, 1)
-dense_q_pair_kernel(const PredictParams p, const uint16_t* __restrict__ Q,
-                    const int32_t* __restrict__ tile_flags, const int R, const int G, const int S,
-                    const int K)
+dense_q_pair_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q)
 {
-  dense_q_body<float, MODE_SCALAR, NT, 0, false, false, true>(p, Q, tile_flags, R, G, S, K, nullptr);
+  dense_q_body<float, MODE_SCALAR, NT, 0, false, false, true>(p, q, nullptr);
 }
 
 // Same kernel with the leaf payloads left in global memory (see DenseQWalker).
 template <int NT, int DEPTH>
 __global__ void __launch_bounds__(1024, 1)
-dense_q_leafg_kernel(const PredictParams p, const uint16_t* __restrict__ Q,
-                     const int32_t* __restrict__ tile_flags, const int R, const int G, const int S,
-                     const int K)
+dense_q_leafg_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q)
 {
-  dense_q_body<float, MODE_SCALAR, NT, DEPTH, false, false, false, true>(p, Q, tile_flags, R, G, S,
-                                                                         K, nullptr);
+  dense_q_body<float, MODE_SCALAR, NT, DEPTH, false, false, false, true>(p, q, nullptr);
 }
 
 // Same kernel with the top nodes of every tree in the parameter block.
 template <typename T, int MODE, int NT, int DEPTH>
 __global__ void __launch_bounds__(NT > 4 ? 800 : 1024, 1)
-dense_q_top_kernel(const __grid_constant__ PredictParams p, const uint16_t* __restrict__ Q,
-                   const int32_t* __restrict__ tile_flags, const int R, const int G, const int S,
-                   const int K, const __grid_constant__ QTop top)
+dense_q_top_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q,
+                   const __grid_constant__ QTop top)
 {
-  dense_q_body<T, MODE, NT, DEPTH, false, true>(p, Q, tile_flags, R, G, S, K, &top);
+  dense_q_body<T, MODE, NT, DEPTH, false, true>(p, q, &top);
 }
 
 // Launch one instantiation of dense_q_kernel.
@@ -539,12 +715,7 @@ template <typename T, int MODE, int NT, int DEPTH, bool CAT>
 int launch_q(const QLaunch& L, std::string& err)
 {
   auto k = dense_q_kernel<T, MODE, NT, DEPTH, CAT>;
-  const int rc = set_smem_bytes(reinterpret_cast<const void*>(k), L.c.smem_bytes, err);
-  if (rc != B2FIL_OK) return rc;
-  k<<<L.grid, L.c.threads, L.c.smem_bytes, L.stream>>>(L.p, L.Q, L.flags, L.c.rows_per_tile,
-                                                       L.c.tree_groups, L.c.stages,
-                                                       L.c.sub_batches);
-  return B2FIL_OK;
+  return launch_split(L.shape(), err, k, L.p, L.q);
 }
 
 // One case per output mode of the generic-depth kernels.

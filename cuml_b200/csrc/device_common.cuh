@@ -464,23 +464,21 @@ __device__ __forceinline__ void finish_cluster_rows(const PredictParams& p, T* a
   cluster_arrive();
   cluster_wait();
   // rows [begin, end) of the tile are this CTA's to finish; nobody else reads their sums here
-  const int begin = R * rank / n_splits, end = R * (rank + 1) / n_splits;
-  for (int j = begin + threadIdx.x; j < end; j += n_ct) {
-    for (int c = 0; c < NC; ++c) {
-      const uint32_t a = smem_addr(acc + c * R + j);
-      T s              = T(0);
-      for (int k0 = 0; k0 < n_splits; k0 += 8) {
-        T part[8];  // loads in flight together
+  const int begin = R * rank / n_splits, n_mine = R * (rank + 1) / n_splits - begin;
+  for (int i = threadIdx.x; i < NC * n_mine; i += n_ct) {
+    T* at            = acc + i / n_mine * R + begin + i % n_mine;
+    const uint32_t a = smem_addr(at);
+    T part[8];  // loads in flight together (a cluster has at most eight CTAs)
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-          part[k] = k0 + k < n_splits ? cluster_ld(cluster_map(a, k0 + k), T(0)) : T(0);
+    for (int k = 0; k < 8; ++k) part[k] = k < n_splits ? cluster_ld(cluster_map(a, k), T(0)) : T(0);
+    T s = part[0];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) s += part[k];
-      }
-      acc[c * R + j] = s;
-    }
-    finish_row<T>(p, acc, R, 1, j, row0 + j);
+    for (int k = 1; k < 8; ++k) s += part[k];
+    *at = s;
   }
+  consumer_sync(n_ct);
+  if (threadIdx.x < n_mine)
+    finish_row<T>(p, acc, R, 1, begin + threadIdx.x, row0 + begin + threadIdx.x);
   cluster_arrive();
 }
 
@@ -575,16 +573,23 @@ __device__ __forceinline__ void take_leaf(const PredictParams& p, int tree,
   }
 }
 
-// Add a thread's running sums to its accumulators in shared memory (end of a row tile).
+// Add a thread's running sums to its accumulators in shared memory (end of a row tile), or store
+// them where nothing else was added to the tile's accumulators.
 template <typename T, int MODE>
 __device__ __forceinline__ void flush_running(const ForestView& f, const Running<T>& run,
-                                              T* acc_group, int R, int r)
+                                              T* acc_group, int R, int r, bool store = false)
 {
-  if (MODE == MODE_SCALAR) acc_group[run.cls * R + r] += run.sum;
+  if (MODE == MODE_SCALAR) {
+    T* at = acc_group + run.cls * R + r;
+    *at   = store ? run.sum : *at + run.sum;
+  }
   if (MODE == MODE_VECTOR && f.n_outputs <= kRegClasses) {
 #pragma unroll
     for (int c = 0; c < kRegClasses; ++c) {
-      if (c < f.n_outputs) acc_group[c * R + r] += run.v[c];
+      if (c < f.n_outputs) {
+        T* at = acc_group + c * R + r;
+        *at   = store ? run.v[c] : *at + run.v[c];
+      }
     }
   }
 }

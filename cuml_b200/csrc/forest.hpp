@@ -84,6 +84,13 @@ struct SparseNode16D {  // fp64
 // to know, and the low half of every node stays a clean feature * 4 for the address arithmetic.)  The sets are stored bit-reversed (category c in bit 31 - c) and a categorical node
 // carries the largest rank, so its rank comparison always says "left" and the walk can simply OR
 // the two answers: sign(node - (code << 17)) | sign(set << code).
+// Row tiles that hold missing values are walked with a second image of the nodes where room allows
+// (q_nodes_nan).  Beside the tile's columns there is then a copy of each in which the NaN code has
+// bit 14 set: 0x3FFF in the first set is a rank above every j (the test says "right"), 0x7FFF in
+// the copy is -1 in the 15 bits of the subtraction (the test says "left"), and a node reads its
+// feature from the set of its own missing direction (copies are numbered n_features and up).  So
+// missing values cost no instruction in the walk.  Categorical nodes carry j = 0x3FFE there, below
+// the NaN code and not below any other code.
 // The rank is found through a per-feature bucket table: bucket(x) = clamp(int(fma(x, scale,
 // offset)), 0, n_buckets-1) is monotone in x, lut[b] is the number of thresholds in buckets below
 // b (all of them are <= x), thresholds of higher buckets are all > x, so the rank is lut[b] plus
@@ -123,6 +130,7 @@ struct QGroup {        // 32 bytes
   uint32_t pad[3];
 };
 constexpr uint32_t Q_NAN_CODE      = 0x3FFFu;
+constexpr uint32_t Q_NAN_LEFT_BIT  = 0x4000u;  // set in the NaN codes of the second set of columns
 constexpr uint32_t Q_MAX_RANK      = 0x3FFEu;
 constexpr uint32_t Q_NO_CATEGORY   = 0x3FFEu;
 constexpr uint32_t Q_MAX_FEATURES  = 0x4000u;
@@ -248,12 +256,14 @@ struct ForestView {
   int32_t q_leaf_bytes;         // bytes per leaf payload: the element size (scalar, or index of the
                                 // leaf's vector), or n_outputs elements when the vectors of a
                                 // forest with few outputs sit in the tree blocks themselves
-  int32_t q_pad_;
+  int32_t q_any_default_left;   // 0: missing values go right in every test
   int64_t q_tree_stride;        // bytes between trees: 2^D * (node bytes + leaf bytes), 16-byte multiple
   const void* q_nodes;          // [n_trees] blocks of [2^D nodes][2^D leaf payloads]; a node is a
                                 // uint32, or {uint32 node, uint32 category set} when q_has_cat
   const void* q_nodes_ids;      // same blocks with the leaf id (uint32) in every leaf payload slot:
                                 // what the traversal streams when it reports leaf ids
+  const void* q_nodes_nan;      // q_nodes for tiles with missing values and doubled columns (see
+                                // above), or null
   int64_t q_max_blob_bytes;     // largest group blob
   const unsigned char* q_blob;  // group blobs
   const QGroup* q_groups;       // [q_n_groups]
@@ -291,6 +301,7 @@ struct PackedForest {
   std::vector<uint8_t> out_bias;
   std::vector<uint8_t> q_nodes;
   std::vector<uint8_t> q_nodes_ids;  // q_nodes with leaf ids in the payload slots
+  std::vector<uint8_t> q_nodes_nan;  // q_nodes for doubled columns, or empty
   std::vector<uint32_t> q_top;  // root and its two children of every tree (3 words per tree), or empty
   std::vector<uint8_t> q_thresholds;
   std::vector<uint16_t> q_lut;

@@ -35,7 +35,7 @@ struct LaunchRecord {
   const char* kernel  = nullptr;  // traversal kernel family
   const char* real    = "";       // float / double
   int mode = 0, nt = 0, depth = -1, cat = -1, fmt = -1, top = -1;
-  int R = 0, G = 0, S = 0, K = 0, splits = 1;
+  int R = 0, G = 0, S = 0, K = 0, splits = 1, tiles = 1, nan_columns = 0;
 };
 thread_local LaunchRecord g_last_launch;
 
@@ -135,8 +135,8 @@ struct DenseWalker {
   }
 };
 
-// n_splits > 1 (small batches): the trees of a row tile are split over n_splits CTAs, each of
-// which streams and walks only its share.  Reduced outputs launch those CTAs as a cluster and
+// small: a small batch.  With n_splits > 1 the trees of a row tile are split over n_splits CTAs,
+// each of which streams and walks only its share.  Reduced outputs launch those CTAs as a cluster and
 // meet in its distributed shared memory (finish_cluster_rows); per-tree outputs need no meeting.
 // What bounds such a launch is latency: launch, tile, trees, walk, sum, one after the other.  So
 // the barriers are set up and the trees requested before grid_wait(), while the kernel before
@@ -144,7 +144,7 @@ struct DenseWalker {
 template <typename T, bool CAT, int MODE, int NT>
 __global__ void __launch_bounds__(544, 1)
 dense_kernel(const __grid_constant__ PredictParams p, const int R, const int G, const int S,
-             const int n_splits)
+             const int n_splits, const bool small)
 {
   using TR = Traits<T>;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -225,7 +225,7 @@ dense_kernel(const __grid_constant__ PredictParams p, const int R, const int G, 
   for (int64_t t = blockIdx.x / n_splits; t < n_tiles; t += tile_step) {
     const int64_t row0 = t * R;
     bool saw_nan       = true;
-    if (n_splits > 1) {
+    if (small) {
       stage_rows_async<T>(p, tile, R, row0, warp, lane, n_cw);
     } else {
       saw_nan = stage_rows<T>(p, tile, R, row0, warp, lane, n_cw);
@@ -234,7 +234,7 @@ dense_kernel(const __grid_constant__ PredictParams p, const int R, const int G, 
       for (int i = threadIdx.x; i < G * NC * R; i += n_ct) acc[i] = T(0);
     }
     if (__any_sync(0xffffffffu, saw_nan) && lane == 0) flags[0] = 1;
-    if (n_splits > 1) cp_async_wait_all();
+    if (small) cp_async_wait_all();
     consumer_sync(n_ct);
     const bool nans = flags[0] != 0;
     Running<T> run{T(0), 0, {}};
@@ -289,12 +289,18 @@ __device__ __forceinline__ void for_each_constant(F&& f, std::integer_sequence<i
 // Q_NAN_CODE and raises the tile's flag.
 // Shared memory: [mbarrier 16 B][blob].
 
+// Where the pre-pass reports NaN and what it clears for the traversal.
+struct QFlags {
+  uint8_t* bytes;     // [tile][group][32 warps], each written by its warp; or
+  int32_t* words;     // one word per tile, zeroed by the caller
+  int32_t* arrived;   // counters of shared row tiles to zero, one per tile, or null
+};
+
 // NU = slots of a tile each thread owns (R * GF / threads, at least 1).  GFC > 0 fixes the group
 // size at compile time (table strides become immediates), GFC == 0 reads it from the group.
 template <typename T, int STEPS, int NU, int GFC>
 __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGroup& grp,
-                                               uint16_t* __restrict__ Q,
-                                               int32_t* __restrict__ tile_flags, int R,
+                                               uint16_t* __restrict__ Q, const QFlags& flags, int R,
                                                uint32_t blob_a, const QFeatRec* rec)
 {
   using TR               = Traits<T>;
@@ -326,6 +332,12 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
   const uint32_t e32     = e1 * 32u;
   const uint32_t e_mine  = b * e1 + grp.f_begin + i;
   const T* X             = static_cast<const T*>(p.X);
+
+  // one lane per warp reports NaN in a byte of its own: nothing has to be zeroed beforehand
+  uint8_t* my_flag = nullptr;
+  if (flags.bytes != nullptr && (tid & 31) == 0)
+    my_flag = flags.bytes + (static_cast<int64_t>(blockIdx.x) * gridDim.y + blockIdx.y) * 32 + (tid >> 5);
+  const uint32_t flag_step = gridDim.x * gridDim.y * 32u;
 
   T xs[NU];
   // loads chunk c (slots s0 + c * CH ...) of tile t
@@ -448,34 +460,39 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
         *dst = static_cast<uint16_t>(packed[0]);
       }
     }
-    if (__any_sync(0xffffffffu, saw_nan) && (tid & 31) == 0) atomicOr(tile_flags + t, 1);
+    const bool warp_nan = __any_sync(0xffffffffu, saw_nan);
+    if (my_flag != nullptr) {
+      *my_flag = warp_nan ? 1 : 0;
+      my_flag += flag_step;
+    } else if (flags.words != nullptr && warp_nan && (tid & 31) == 0) {
+      atomicOr(flags.words + t, 1);
+    }
   }
 }
 
 template <typename T, int STEPS>
 __device__ __forceinline__ void quantise_rows(const PredictParams& p, const QGroup& grp,
-                                              uint16_t* __restrict__ Q,
-                                              int32_t* __restrict__ tile_flags, int R,
+                                              uint16_t* __restrict__ Q, const QFlags& flags, int R,
                                               uint32_t blob_a, const QFeatRec* rec)
 {
   const int GF         = static_cast<int>(grp.f_end - grp.f_begin);
   const int per_thread = (R * GF) / static_cast<int>(blockDim.x);
   // full-width groups on large tiles, the shape of big batches, get the group size baked in
   if (GF == 32 && STEPS >= 2 && per_thread == 8) {
-    quantise_tiles<T, STEPS, 8, 32>(p, grp, Q, tile_flags, R, blob_a, rec);
+    quantise_tiles<T, STEPS, 8, 32>(p, grp, Q, flags, R, blob_a, rec);
     return;
   }
   switch (per_thread) {
-    case 8: quantise_tiles<T, STEPS, 8, 0>(p, grp, Q, tile_flags, R, blob_a, rec); break;
-    case 4: quantise_tiles<T, STEPS, 4, 0>(p, grp, Q, tile_flags, R, blob_a, rec); break;
-    case 2: quantise_tiles<T, STEPS, 2, 0>(p, grp, Q, tile_flags, R, blob_a, rec); break;
-    default: quantise_tiles<T, STEPS, 1, 0>(p, grp, Q, tile_flags, R, blob_a, rec); break;
+    case 8: quantise_tiles<T, STEPS, 8, 0>(p, grp, Q, flags, R, blob_a, rec); break;
+    case 4: quantise_tiles<T, STEPS, 4, 0>(p, grp, Q, flags, R, blob_a, rec); break;
+    case 2: quantise_tiles<T, STEPS, 2, 0>(p, grp, Q, flags, R, blob_a, rec); break;
+    default: quantise_tiles<T, STEPS, 1, 0>(p, grp, Q, flags, R, blob_a, rec); break;
   }
 }
 
 template <typename T>
 __global__ void __launch_bounds__(1024, 1)
-quantise_kernel(const PredictParams p, uint16_t* __restrict__ Q, int32_t* __restrict__ tile_flags,
+quantise_kernel(const __grid_constant__ PredictParams p, uint16_t* __restrict__ Q, const QFlags flags,
                 const int R)
 {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -493,19 +510,32 @@ quantise_kernel(const PredictParams p, uint16_t* __restrict__ Q, int32_t* __rest
     bulk_copy_g2s(blob_a, f.q_blob + grp.blob_off, grp.blob_bytes, bar);
   }
   __syncthreads();
+  grid_release();
+  grid_wait();  // the tables are part of the forest; rows and scratch may still be in use
+  // while the tables arrive, ask the L2 for the rows of the CTA's first tile
+  if (threadIdx.x < R) {
+    const int64_t row = static_cast<int64_t>(blockIdx.x) * R + threadIdx.x;
+    if (row < p.n_rows)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const T*>(p.X) + row * p.row_stride + grp.f_begin));
+  }
+  if (flags.arrived != nullptr && blockIdx.y == 0) {
+    const int64_t n_tiles = (p.n_rows + R - 1) / R;
+    for (int64_t t = blockIdx.x * 1024ll + threadIdx.x; t < n_tiles; t += gridDim.x * 1024ll)
+      flags.arrived[t] = 0;
+  }
   if (!mbar_wait(bar, 0)) {
     if (threadIdx.x == 0) atomicExch(p.status, 4);
     return;
   }
   // the number of halvings is fixed per group: pick the unrolled body once
   switch (grp.steps) {
-    case 0: quantise_rows<T, 0>(p, grp, Q, tile_flags, R, blob_a, rec); break;
-    case 1: quantise_rows<T, 1>(p, grp, Q, tile_flags, R, blob_a, rec); break;
-    case 2: quantise_rows<T, 2>(p, grp, Q, tile_flags, R, blob_a, rec); break;
-    case 3: quantise_rows<T, 3>(p, grp, Q, tile_flags, R, blob_a, rec); break;
-    case 4: quantise_rows<T, 4>(p, grp, Q, tile_flags, R, blob_a, rec); break;
-    case 5: quantise_rows<T, 5>(p, grp, Q, tile_flags, R, blob_a, rec); break;
-    default: quantise_rows<T, -1>(p, grp, Q, tile_flags, R, blob_a, rec); break;
+    case 0: quantise_rows<T, 0>(p, grp, Q, flags, R, blob_a, rec); break;
+    case 1: quantise_rows<T, 1>(p, grp, Q, flags, R, blob_a, rec); break;
+    case 2: quantise_rows<T, 2>(p, grp, Q, flags, R, blob_a, rec); break;
+    case 3: quantise_rows<T, 3>(p, grp, Q, flags, R, blob_a, rec); break;
+    case 4: quantise_rows<T, 4>(p, grp, Q, flags, R, blob_a, rec); break;
+    case 5: quantise_rows<T, 5>(p, grp, Q, flags, R, blob_a, rec); break;
+    default: quantise_rows<T, -1>(p, grp, Q, flags, R, blob_a, rec); break;
   }
 }
 
@@ -693,7 +723,7 @@ int launch_dense_mode(const PredictParams& p, const DenseCfg& c, const SplitLaun
                       std::string& err)
 {
   auto k = c.trees_in_flight == 2 ? dense_kernel<T, CAT, MODE, 2> : dense_kernel<T, CAT, MODE, 1>;
-  return launch_split(l, err, k, p, c.rows_per_tile, c.tree_groups, c.stages, n_splits);
+  return launch_split(l, err, k, p, c.rows_per_tile, c.tree_groups, c.stages, n_splits, l.overlap);
 }
 
 template <typename T, bool CAT>
@@ -732,12 +762,12 @@ int launch_sparse_fmt(const PredictParams& p, int mode, int R, int G, int rows_i
 }
 
 size_t dense_q_smem(size_t qstride, int precision, int F, int NC, bool reduce, int R, int G, int NT,
-                    int S, int K)
+                    int S, int K, int tile_bufs = 1, int acc_bufs = 1, int columns = 1)
 {
   const size_t es = precision == B2FIL_F32 ? 4 : 8;
   size_t b        = kBarBytes;
-  b += static_cast<size_t>(F) * R * 2;
-  if (reduce) b += align16(static_cast<size_t>(G) * NC * R * es);
+  b += static_cast<size_t>(tile_bufs) * columns * F * R * 2;
+  if (reduce) b += acc_bufs * align16(static_cast<size_t>(G) * NC * R * es);
   b += 16;
   b += static_cast<size_t>(S) * G * NT * K * qstride;
   return b;
@@ -761,6 +791,18 @@ int q_max_trees_in_flight(const ForestView& f, int mode)
   return specialised ? 6 : 4;
 }
 
+// Can tiles with missing values be walked with doubled columns?
+bool has_nan_image(const ForestView& f, int mode)
+{
+  return f.q_nodes_nan != nullptr && mode != MODE_LEAFID;
+}
+// Words of NaN flags per row tile that the traversal has to look at: none when every test sends
+// missing values to the right, where the NaN code compares to by itself.
+int nan_flag_words(const ForestView& f, int words)
+{
+  return (f.q_any_default_left || f.q_has_cat) ? words : 0;
+}
+
 // Launch shape of the quantised dense kernel: the largest row tile that fits, then as many warps
 // as fit (31 consumer warps at most), then as many trees in flight per warp as there is a kernel
 // for, then the deepest tree ring that still fits.
@@ -769,13 +811,19 @@ int q_max_trees_in_flight(const ForestView& f, int mode)
 // puts at least a third more walks in flight.
 bool dense_q_config(size_t qstride, int max_nt, int precision, int F, int NC, bool reduce,
                     int64_t n_rows, int chunk_size, int sm_count, DenseCfg& cfg,
-                    int depth_hint = 0, size_t node_stride = 0)
+                    int depth_hint, size_t node_stride, int64_t visits_per_row, bool nan_image)
 {
   int want = 256;
   if (chunk_size > 0) {
     want = std::min(256, std::max(32, 32 * chunk_size));
   } else {
-    while (want > 32 && n_rows < static_cast<int64_t>(want) * sm_count) want /= 2;
+    // tiles are cut between CTAs, so their number need not fill the SMs; larger ones stream the
+    // forest less often.  Smaller ones serve forests with few visits per row, which have too few
+    // tree batches to cut, and small batches with many outputs, where the sums of a cut tile
+    // are the larger part.
+    if (n_rows < static_cast<int64_t>(256) * sm_count &&
+        (visits_per_row < 1000 || (NC > 4 && n_rows < static_cast<int64_t>(32) * sm_count)))
+      want = 128;
   }
   // tuning aid "R,G,NT,S,K": from the environment (read once per process) or, taking
   // precedence, from the knobs q_R, q_G, q_NT, q_S, q_K of b2fil_set_tuning
@@ -858,13 +906,25 @@ bool dense_q_config(size_t qstride, int max_nt, int precision, int F, int NC, bo
     }
     if (best_g == 0) continue;
     // a stage holds K sub-batches so that a warp waits and signals once per K * NT trees.
-    // Two stages already hide the bulk copies (measured: S = 2 and S = 3 run alike).
-    for (int K = 2; K >= 1; K /= 2) {
-      for (int S = 3; S >= 2; --S) {
-        const size_t b = dense_q_smem(stride, precision, F, NC, reduce, R, best_g, best_nt, S, K);
-        if (b <= kMaxSmemBytes) {
-          cfg = DenseCfg{R, best_g, best_nt, S, b, (rw * best_g + 1) * 32, K, leafg};
-          return true;
+    // Two stages already hide the bulk copies (measured: S = 2 and S = 3 run alike), so a second
+    // row tile and room for doubled columns come first - the tile where the trees of a row last only
+    // a few microseconds -, and a second set of accumulators takes what is left.
+    const bool tile_first = visits_per_row < 4000;
+    for (int pass = 0; pass < 4; ++pass) {
+      const int tiles   = (pass == 0 || pass == (tile_first ? 1 : 2)) ? 2 : 1;
+      const int columns = (pass == 0 || pass == (tile_first ? 2 : 1)) ? 2 : 1;
+      if (columns == 2 && !nan_image) continue;
+      for (int K = 2; K >= 1; K /= 2) {
+        for (int S = 3; S >= 2; --S) {
+          for (int accs = reduce ? 2 : 1; accs >= 1; --accs) {
+            const size_t b = dense_q_smem(stride, precision, F, NC, reduce, R, best_g, best_nt, S,
+                                          K, tiles, accs, columns);
+            if (b <= kMaxSmemBytes) {
+              cfg = DenseCfg{R, best_g, best_nt, S, b, (rw * best_g + 1) * 32, K, leafg, tiles, accs,
+                             columns - 1};
+              return true;
+            }
+          }
         }
       }
     }
@@ -887,6 +947,8 @@ int launch_dense_q_kernel(const QLaunch& L, int mode, bool f64, std::string& err
   rec.real            = f64 ? "double" : "float";
   rec.mode            = mode;
   rec.nt              = L.c.trees_in_flight;
+  rec.tiles           = L.c.tile_bufs;
+  rec.nan_columns     = L.c.nan_columns;
   rec.depth           = 0;  // read at run time unless a specialised body is picked below
   rec.cat             = f.q_has_cat ? 1 : 0;
   rec.R               = L.c.rows_per_tile;
@@ -941,26 +1003,44 @@ int launch_dense_q_kernel(const QLaunch& L, int mode, bool f64, std::string& err
   return launch_q_generic(L, mode, f64, err);
 }
 
-// CTAs per feature group of the rank pre-pass.  Every CTA holds the tables of one group, so the
-// grid is (CTAs per group) x (groups) and the SMs take it in waves of one CTA each.  With g
-// groups on s SMs, s / g CTAs per group fill one wave but leave s mod g SMs idle (64 groups on
-// 148 SMs: 20 idle); more, shorter CTAs per group waste less: the count that minimises
-// waves / (CTAs per group) is taken, among up to 48 or one wave's worth (a CTA loads its group's
-// tables once, about 200 KB from L2).
-int quantise_ctas_per_group(int n_groups, int sm_count, int64_t n_tiles)
+// CTAs per feature group of the rank pre-pass.  Every CTA loads the tables of one group (about 200 KB
+// of an SM's 48 bytes per cycle from L2) and then ranks its share of the group's tiles; the SMs take
+// the grid in waves of one CTA each.  Taken is the count with the least estimated time,
+//   waves x (start and tables + tiles of a CTA x time per tile),
+// a warp ranking 32 values in 17.4 SM cycles (measured on 1 M rows of 256 features).  With large
+// batches many short CTAs fill the last wave (64 groups on 148 SMs: 37 CTAs per group), with
+// 20,000 rows loading the tables twice on an SM costs more than it evens out.
+int quantise_ctas_per_group(const ForestView& f, int R, int sm_count, int64_t n_tiles)
 {
+  const int n_groups   = std::max(1, f.q_n_groups);
+  const double tables  = 3000.0 + static_cast<double>(f.q_max_blob_bytes) / 48.0;
+  const double per_tile = 17.4 * R * f.n_features / n_groups / 32.0 + 100.0;
   int best = 1;
-  double best_cost = 1e30;
-  const int most = std::max(48, sm_count / std::max(1, n_groups));
+  double best_cost = 1e300;
+  const int most = static_cast<int>(std::min<int64_t>(n_tiles, std::max(48, sm_count / n_groups)));
   for (int gx = 1; gx <= most; ++gx) {
     const int waves   = (gx * n_groups + sm_count - 1) / sm_count;
-    const double cost = static_cast<double>(waves) / gx;
-    if (cost < best_cost * 0.99) {  // ties and near ties: fewer CTAs
+    const double cost = waves * (tables + static_cast<double>((n_tiles + gx - 1) / gx) * per_tile);
+    if (cost < best_cost * 0.995) {  // ties and near ties: fewer CTAs
       best_cost = cost;
       best      = gx;
     }
   }
-  return static_cast<int>(std::min<int64_t>(n_tiles, best));
+  return best;
+}
+
+// Enqueue the rank pre-pass of p's rows.  The kernel may start while the one before it in the
+// stream is still running, unless that is a copy or memset.
+int launch_quantise(const PredictParams& p, uint16_t* Q, const QFlags& flags, int R, bool f64,
+                    int sm_count, cudaStream_t stream, std::string& err)
+{
+  const ForestView& f = p.f;
+  // shared memory: mbarrier and the largest group blob
+  const size_t smem = 16 + static_cast<size_t>(f.q_max_blob_bytes);
+  const int gx      = quantise_ctas_per_group(f, R, sm_count, (p.n_rows + R - 1) / R);
+  const SplitLaunch l{dim3(gx, f.q_n_groups), 1024, smem, stream, 1, true};
+  return f64 ? launch_split(l, err, quantise_kernel<double>, p, Q, flags, R)
+             : launch_split(l, err, quantise_kernel<float>, p, Q, flags, R);
 }
 
 // Rank-quantised prediction: rows are processed in chunks of whole waves of tiles; for each
@@ -975,7 +1055,8 @@ int launch_dense_q(const PredictParams& p, int mode, int chunk_size, int sm_coun
   DenseCfg c;
   if (!dense_q_config(static_cast<size_t>(f.q_tree_stride), q_max_trees_in_flight(f, mode), precision,
                       f.n_features, f.n_outputs, reduce, p.n_rows, chunk_size, sm_count, c,
-                      f.dense_depth, q_node_only_stride(f, mode))) {
+                      f.dense_depth, q_node_only_stride(f, mode),
+                      static_cast<int64_t>(f.n_trees) * f.dense_depth, has_nan_image(f, mode))) {
     err = "no quantised launch shape fits shared memory";
     return B2FIL_ERR_UNSUPPORTED;
   }
@@ -998,21 +1079,27 @@ int launch_dense_q(const PredictParams& p, int mode, int chunk_size, int sm_coun
   const int64_t waves    = std::max<int64_t>(1, static_cast<int64_t>(target / (tile_b * sm_count)));
   const int64_t chunk    = std::min<int64_t>(wave * waves, (p.n_rows + R - 1) / R * R);
   const int64_t ch_tiles = (chunk + R - 1) / R;
+  // scratch: ranks, sums of shared tiles, NaN flags and arrival counters (zeroed together)
+  const int per_batch    = c.tree_groups * c.trees_in_flight * c.sub_batches;
+  const int64_t batches  = (f.n_trees + per_batch - 1) / per_batch;
   const size_t q_bytes   = static_cast<size_t>(ch_tiles) * tile_b;
-  const size_t fl_bytes  = (static_cast<size_t>(ch_tiles) * 4 + 255) / 256 * 256;
+  const size_t sum_bytes =
+    reduce ? align16(static_cast<size_t>(2 * sm_count) * f.n_outputs * R * es) : 0;
+  const int flag_words   = f.q_n_groups * 8;  // a byte per warp of the pre-pass
+  const size_t fl_bytes  = static_cast<size_t>(ch_tiles) * flag_words * 4;
+  const size_t arr_bytes = reduce ? static_cast<size_t>(ch_tiles) * 4 : 0;
   unsigned char* scratch = nullptr;
-  cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch), q_bytes + fl_bytes,
-                                          pool, stream);
+  cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch),
+                                          q_bytes + sum_bytes + fl_bytes + arr_bytes, pool, stream);
   if (e != cudaSuccess) {
     cudaGetLastError();
     err = std::string("scratch allocation for quantised rows failed: ") + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? B2FIL_ERR_NO_MEMORY : B2FIL_ERR_CUDA;
   }
-  uint16_t* Q    = reinterpret_cast<uint16_t*>(scratch);
-  int32_t* flags = reinterpret_cast<int32_t*>(scratch + q_bytes);
-  // shared memory of the pre-pass: mbarrier and the largest group blob
-  const size_t q_smem = 16 + static_cast<size_t>(f.q_max_blob_bytes);
-  int rc = B2FIL_OK;
+  uint16_t* Q     = reinterpret_cast<uint16_t*>(scratch);
+  uint8_t* flags  = scratch + q_bytes + sum_bytes;
+  int32_t* arrive = reduce ? reinterpret_cast<int32_t*>(flags + fl_bytes) : nullptr;
+  int rc          = B2FIL_OK;
   const size_t out_row_b =
     (p.kind == B2FIL_INFER_LEAF_ID ? size_t(4) * f.n_trees
      : p.kind == B2FIL_INFER_CLASS ? size_t(4)
@@ -1026,27 +1113,14 @@ int launch_dense_q(const PredictParams& p, int mode, int chunk_size, int sm_coun
     pc.X             = static_cast<const unsigned char*>(p.X) + static_cast<size_t>(r0) * p.row_stride * es;
     pc.out           = static_cast<unsigned char*>(p.out) + static_cast<size_t>(r0) * out_row_b;
     const int64_t n_tiles = (pc.n_rows + R - 1) / R;
-    e = cudaMemsetAsync(flags, 0, static_cast<size_t>(n_tiles) * 4, stream);
-    if (e != cudaSuccess) {
-      err = std::string("cudaMemsetAsync: ") + cudaGetErrorString(e);
-      rc  = B2FIL_ERR_CUDA;
-      break;
-    }
-    const int gx = quantise_ctas_per_group(f.q_n_groups, sm_count, n_tiles);
-    const dim3 qgrid(gx, f.q_n_groups);
-    const dim3 qblock(1024);
-    if (precision == B2FIL_F32) {
-      auto k = quantise_kernel<float>;
-      if ((rc = set_smem(k, q_smem, err)) != B2FIL_OK) break;
-      k<<<qgrid, qblock, q_smem, stream>>>(pc, Q, flags, R);
-    } else {
-      auto k = quantise_kernel<double>;
-      if ((rc = set_smem(k, q_smem, err)) != B2FIL_OK) break;
-      k<<<qgrid, qblock, q_smem, stream>>>(pc, Q, flags, R);
-    }
-    const int grid = static_cast<int>(std::min<int64_t>(n_tiles, sm_count));
-    rc = launch_dense_q_kernel(QLaunch{pc, Q, flags, c, grid, stream}, mode,
-                               precision != B2FIL_F32, err);
+    rc = launch_quantise(pc, Q, QFlags{flags, nullptr, arrive}, R, precision != B2FIL_F32,
+                         sm_count, stream, err);
+    if (rc != B2FIL_OK) break;
+    const int grid = static_cast<int>(std::min<int64_t>(n_tiles * batches, sm_count));
+    const QArgs qa{Q, reinterpret_cast<const uint32_t*>(flags), nan_flag_words(f, flag_words),
+                   reduce ? scratch + q_bytes : nullptr, arrive, R, c.tree_groups, c.stages,
+                   c.sub_batches, c.tile_bufs, c.nan_columns, c.acc_bufs};
+    rc = launch_dense_q_kernel(QLaunch{pc, qa, c, grid, stream}, mode, precision != B2FIL_F32, err);
     if (launches) *launches += 2;
   }
   cudaFreeAsync(scratch, stream);
@@ -1161,8 +1235,24 @@ bool dense_config(int depth, int precision, int n_features, int n_outputs, bool 
   return false;
 }
 
-// Small batches: fewer 128-row tiles than half the SMs.
-bool n_rows_small(int64_t n_rows, int sm_count) { return (n_rows + 127) / 128 * 2 <= sm_count; }
+// Small batches: at most one round of 128-row tiles.
+bool n_rows_small(int64_t n_rows, int sm_count) { return n_rows <= int64_t(128) * sm_count; }
+
+// Measured time of small batches per estimated SM cycle (1000 depth-8 trees x 4,000 rows: 36 us
+// for 51,000 cycles).
+constexpr double kDenseUsPerCycle = 0.0007;
+
+// Estimated time of the same batch on the rank path: two kernels with their start-up, the ranks of
+// every value, the node visits at the pace of large batches.
+double rank_path_us(const ForestView& f, int mode, int64_t n_rows, int sm_count)
+{
+  const bool plain    = f.format == FMT_DENSE_F && !f.q_has_cat && mode == MODE_SCALAR;
+  const double visits = static_cast<double>(n_rows) * f.n_trees * std::max(1, f.dense_depth);
+  const double values = static_cast<double>(n_rows) * f.n_features;
+  const double sms    = sm_count / 148.0;  // the rates are those of 148 SMs
+  const double fixed  = mode <= MODE_VECTOR ? 13.0 : 7.5;  // per-tree outputs: no sums to meet
+  return fixed + (visits / (plain ? 3.0e6 : 2.0e6) + values / 5.2e5) / sms;
+}
 
 // Launch shape of a small batch: row tiles of R rows, each shared by n_splits CTAs that walk their
 // part of the forest.  Takes the shape with the least estimated time (in SM cycles):
@@ -1176,6 +1266,7 @@ bool n_rows_small(int64_t n_rows, int sm_count) { return (n_rows + 127) / 128 * 
 struct SplitShape {
   DenseCfg c;
   int n_splits;
+  double us;  // estimated time
 };
 // `rows_per_tile` > 0 asks for that R (the caller's chunk_size).
 bool pick_split_shape(const ForestView& f, int mode, int precision, int64_t n_rows,
@@ -1184,7 +1275,8 @@ bool pick_split_shape(const ForestView& f, int mode, int precision, int64_t n_ro
   const bool reduce   = mode <= MODE_VECTOR;
   const double es     = precision == B2FIL_F32 ? 4 : 8;
   const double stride = static_cast<double>(dense_tree_stride(f.dense_depth, precision));
-  const double wave_w = precision == B2FIL_F32 ? 5.6 : 9.0;
+  const double wave_w = (precision == B2FIL_F32 ? 5.6 : 9.0) * (f.has_categorical ? 2.0 : 1.0);
+  const double leaf_w = mode == MODE_SCALAR ? 4.0 : (mode == MODE_VECTOR ? 32.0 : 64.0);
   const int depth     = std::max(1, f.dense_depth);
   double best_cost    = 1e300;
   for (int R = 32; R <= 128; R *= 2) {
@@ -1205,12 +1297,14 @@ bool pick_split_shape(const ForestView& f, int mode, int precision, int64_t n_ro
                                          cluster_ctas(sm_count, reduce ? C : 1));
           const int trees    = (f.n_trees + C - 1) / C;
           const int batches  = (trees + G * NT - 1) / (G * NT);
-          const double walk  = batches * depth * std::max(120.0, rw * G * NT * wave_w);
+          const double walk  = std::max(batches * (150.0 + depth * 120.0),
+                                        rw * trees * (depth * wave_w + leaf_w));
           const double rows  = static_cast<double>(R) * f.n_features * es / 48.0;
           const double load  = trees * stride / 48.0;
           const double cost  = waves * (4000.0 + rows + std::max(walk, load));
           if (cost < best_cost) {
             best_cost     = cost;
+            best.us       = cost * kDenseUsPerCycle;
             best.c        = DenseCfg{R, G, NT, S, b, (rw * G + 1) * 32, 1, 0};
             best.n_splits = C;
           }
@@ -1296,8 +1390,15 @@ int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStr
   const bool ranks_only =
     dense_fmt && dense_ok(f.dense_depth, f.format == FMT_DENSE_F ? B2FIL_F32 : B2FIL_F64,
                           f.n_features, f.n_outputs) != 1;
+  // (other small batches take whichever of the two kernels is estimated to be faster)
+  const int prec = f.format == FMT_DENSE_F ? B2FIL_F32 : B2FIL_F64;
+  SplitShape split;
+  bool have_split =
+    dense_fmt && !ranks_only && n_rows_small(p.n_rows, sm_count) &&
+    split_shape(f, mode, prec, p.n_rows,
+                chunk_size > 0 ? pick_rows_per_tile(p.n_rows, chunk_size, sm_count) : 0, sm_count, split);
   if (dense_fmt && f.q_enabled && p.row_stride < (int64_t(1) << 22) && pool != nullptr &&
-      (chunk_size > 0 || ranks_only || !n_rows_small(p.n_rows, sm_count))) {
+      (chunk_size > 0 || !have_split || split.us > rank_path_us(f, mode, p.n_rows, sm_count))) {
     rc = launch_dense_q(p, mode, chunk_size, sm_count, stream, pool, err, launches);
     if (rc != B2FIL_OK) return rc;
     const cudaError_t e = cudaGetLastError();
@@ -1312,21 +1413,19 @@ int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStr
     DenseCfg c;
     int n_splits = 1;
     // small batches split the forest over CTAs: a CTA then streams only its share of the trees
-    if (SplitShape s; n_rows_small(p.n_rows, sm_count) &&
-                      split_shape(f, mode, precision, p.n_rows,
-                                  chunk_size > 0 ? pick_rows_per_tile(p.n_rows, chunk_size, sm_count) : 0,
-                                  sm_count, s)) {
-      c        = s.c;
-      n_splits = s.n_splits;
+    const bool small = have_split;
+    if (have_split) {
+      c        = split.c;
+      n_splits = split.n_splits;
     } else if (!dense_config(f.dense_depth, precision, f.n_features, f.n_outputs, reduce, p.n_rows,
                              chunk_size, sm_count, c)) {
       err = "no dense launch shape fits shared memory";
       return B2FIL_ERR_UNSUPPORTED;
     }
     const int64_t n_tiles = (p.n_rows + c.rows_per_tile - 1) / c.rows_per_tile;
-    const int64_t ctas    = n_splits > 1 ? n_tiles * n_splits : std::min<int64_t>(n_tiles, sm_count);
-    const SplitLaunch l{static_cast<int>(ctas), c.threads, c.smem_bytes, stream,
-                        reduce ? n_splits : 1, n_splits > 1};
+    const int64_t ctas    = small ? n_tiles * n_splits : std::min<int64_t>(n_tiles, sm_count);
+    const SplitLaunch l{dim3(static_cast<unsigned>(ctas)), c.threads, c.smem_bytes, stream,
+                        reduce ? n_splits : 1, small};
     {
       LaunchRecord& rec = g_last_launch;
       rec               = LaunchRecord{};
@@ -1458,7 +1557,8 @@ int launch_predict_fixed_scratch(const PredictParams& p, int chunk_size, int sm_
   DenseCfg c;
   if (!dense_q_config(static_cast<size_t>(f.q_tree_stride), q_max_trees_in_flight(f, mode), precision,
                       f.n_features, f.n_outputs, mode <= MODE_VECTOR, p.n_rows, chunk_size,
-                      sm_count, c, f.dense_depth, q_node_only_stride(f, mode))) {
+                      sm_count, c, f.dense_depth, q_node_only_stride(f, mode),
+                      static_cast<int64_t>(f.n_trees) * f.dense_depth, has_nan_image(f, mode))) {
     err = "no quantised launch shape fits shared memory";
     return B2FIL_ERR_UNSUPPORTED;
   }
@@ -1488,22 +1588,15 @@ int launch_predict_fixed_scratch(const PredictParams& p, int chunk_size, int sm_
     err = std::string("cudaMemsetAsync: ") + cudaGetErrorString(e);
     return B2FIL_ERR_CUDA;
   }
-  const size_t q_smem = 16 + static_cast<size_t>(f.q_max_blob_bytes);
-  const int gx = quantise_ctas_per_group(f.q_n_groups, sm_count, n_tiles);
-  const dim3 qgrid(gx, f.q_n_groups);
-  const dim3 qblock(1024);
-  if (precision == B2FIL_F32) {
-    auto k = quantise_kernel<float>;
-    if ((rc = set_smem(k, q_smem, err)) != B2FIL_OK) return rc;
-    k<<<qgrid, qblock, q_smem, stream>>>(p, Q, flags, R);
-  } else {
-    auto k = quantise_kernel<double>;
-    if ((rc = set_smem(k, q_smem, err)) != B2FIL_OK) return rc;
-    k<<<qgrid, qblock, q_smem, stream>>>(p, Q, flags, R);
-  }
+  rc = launch_quantise(p, Q, QFlags{nullptr, flags, nullptr}, R, precision != B2FIL_F32, sm_count,
+                       stream, err);
+  if (rc != B2FIL_OK) return rc;
   const int grid = static_cast<int>(std::min<int64_t>(n_tiles, sm_count));
-  rc = launch_dense_q_kernel(QLaunch{p, Q, flags, c, grid, stream}, mode, precision != B2FIL_F32,
-                             err);
+  // (the array holds nothing but ranks and flags: row tiles are not shared by CTAs)
+  const QArgs qa{Q, reinterpret_cast<const uint32_t*>(flags), nan_flag_words(f, 1), nullptr,
+                 nullptr, R, c.tree_groups, c.stages, c.sub_batches, c.tile_bufs, c.nan_columns,
+                 c.acc_bufs};
+  rc = launch_dense_q_kernel(QLaunch{p, qa, c, grid, stream}, mode, precision != B2FIL_F32, err);
   if (rc != B2FIL_OK) return rc;
   e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -1531,6 +1624,8 @@ std::string last_launch_variant()
   s += "> R=" + std::to_string(r.R) + " G=" + std::to_string(r.G);
   if (r.S) s += " S=" + std::to_string(r.S);
   if (r.K) s += " K=" + std::to_string(r.K);
+  if (r.tiles > 1) s += " tiles=" + std::to_string(r.tiles);
+  if (r.nan_columns) s += " nan_columns";
   if (r.splits > 1) s += " forest_splits=" + std::to_string(r.splits);
   return s;
 }

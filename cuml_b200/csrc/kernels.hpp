@@ -34,6 +34,9 @@ struct DenseCfg {
   int threads;
   int sub_batches;     // K: sub-batches of G * NT trees per stage (quantised kernel)
   int leaves_global;   // quantised kernel: the stages hold test nodes only, payloads stay in global memory
+  int tile_bufs = 1;   // quantised kernel: row-tile buffers and sets of accumulators (QArgs)
+  int acc_bufs  = 1;
+  int nan_columns = 0; // quantised kernel: room for doubled columns (QArgs)
 };
 
 // Largest dynamic shared memory a CTA may use on sm_100 (227 KiB).

@@ -10,23 +10,13 @@
 
 namespace b2fil {
 
-// One launch of a quantised traversal kernel.
-struct QLaunch {
-  PredictParams p;
-  const uint16_t* Q;      // rank image of the chunk
-  const int32_t* flags;   // per tile: non-zero when the tile holds a NaN
-  DenseCfg c;
-  int grid;
-  cudaStream_t stream;
-};
-
 // Raise the dynamic shared memory limit of `kernel` on the current device to `bytes` (cached per
 // device and kernel).
 int set_smem_bytes(const void* kernel, size_t bytes, std::string& err);
 
 // A launch that may be split over clusters and may overlap the tail of the kernel before it.
 struct SplitLaunch {
-  int grid;             // CTAs, a multiple of `cluster`
+  dim3 grid;            // CTAs; grid.x is a multiple of `cluster`
   int threads;
   size_t smem_bytes;
   cudaStream_t stream;
@@ -41,7 +31,7 @@ int launch_split(const SplitLaunch& l, std::string& err, void (*kernel)(Params..
   if (rc != B2FIL_OK) return rc;
   cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim          = dim3(l.grid);
+  cfg.gridDim          = l.grid;
   cfg.blockDim         = dim3(l.threads);
   cfg.dynamicSmemBytes = l.smem_bytes;
   cfg.stream           = l.stream;
@@ -64,6 +54,36 @@ int launch_split(const SplitLaunch& l, std::string& err, void (*kernel)(Params..
   }
   return B2FIL_OK;
 }
+// What the quantised traversal kernels take beside the prediction itself; passed by value.
+struct QArgs {
+  const uint16_t* Q;      // rank image of the chunk
+  // which tiles hold a NaN: flag_words 32-bit words per tile, any of them non-zero
+  const uint32_t* flags;
+  int32_t flag_words;
+  // Reduced outputs of a balanced launch (see dense_q_body): sums of row tiles that several CTAs
+  // share, [2 per CTA][output][row] of the forest precision, and per tile the tree batches that
+  // have arrived (zeroed by the pre-pass).  Null: every row tile belongs to one CTA.
+  void* partial;
+  int32_t* arrived;
+  int32_t R, G, S, K;
+  int32_t tile_bufs;      // row-tile buffers: 2 bring the next tile in during the walk of this one
+  int32_t nan_columns;    // 1: tiles with missing values are walked with doubled columns (room for them)
+  int32_t acc_bufs;       // sets of accumulators: with 2 the CTA meets once per tile, not twice
+};
+
+// One launch of a quantised traversal kernel.
+struct QLaunch {
+  PredictParams p;
+  QArgs q;
+  DenseCfg c;
+  int grid;
+  cudaStream_t stream;
+  SplitLaunch shape() const
+  {
+    return SplitLaunch{dim3(grid), c.threads, c.smem_bytes, stream, 1, true};
+  }
+};
+
 // CTAs of a launch in clusters of `cluster` that run at the same time, one per SM.  Clusters live
 // inside one GPC, so the larger they are the more SMs stay idle: measured on 148 SMs, 148 CTAs in
 // pairs, 132 in fours, 120 in eights.

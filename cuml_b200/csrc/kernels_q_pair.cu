@@ -8,12 +8,7 @@ template <int NT>
 int launch_pair(const QLaunch& L, std::string& err)
 {
   auto k = dense_q_pair_kernel<NT>;
-  const int rc = set_smem_bytes(reinterpret_cast<const void*>(k), L.c.smem_bytes, err);
-  if (rc != B2FIL_OK) return rc;
-  k<<<L.grid, L.c.threads, L.c.smem_bytes, L.stream>>>(L.p, L.Q, L.flags, L.c.rows_per_tile,
-                                                       L.c.tree_groups, L.c.stages,
-                                                       L.c.sub_batches);
-  return B2FIL_OK;
+  return launch_split(L.shape(), err, k, L.p, L.q);
 }
 }  // namespace
 

@@ -7,12 +7,7 @@ template <int DEPTH>
 int launch_top(const QLaunch& L, const QTop& top, std::string& err)
 {
   auto k = dense_q_top_kernel<float, MODE_SCALAR, 6, DEPTH>;
-  const int rc = set_smem_bytes(reinterpret_cast<const void*>(k), L.c.smem_bytes, err);
-  if (rc != B2FIL_OK) return rc;
-  k<<<L.grid, L.c.threads, L.c.smem_bytes, L.stream>>>(L.p, L.Q, L.flags, L.c.rows_per_tile,
-                                                       L.c.tree_groups, L.c.stages,
-                                                       L.c.sub_batches, top);
-  return B2FIL_OK;
+  return launch_split(L.shape(), err, k, L.p, L.q, top);
 }
 }  // namespace
 

@@ -523,7 +523,7 @@ int launch_mode(const PredictParams& p, const CompactCfg& c, cudaStream_t stream
   auto k = c.threads > kCompactThreads
              ? sparse_compact_kernel<T, CAT, MODE, kCompactTreesInFlight, kCompactThreadsBig>
              : sparse_compact_kernel<T, CAT, MODE, kCompactTreesInFlight, kCompactThreads>;
-  const SplitLaunch l{c.grid * c.splits, c.threads, c.smem_bytes, stream,
+  const SplitLaunch l{dim3(c.grid * c.splits), c.threads, c.smem_bytes, stream,
                       MODE <= MODE_VECTOR ? c.splits : 1, c.splits > 1};
   return launch_split(l, err, k, p, c.rows_per_tile, c.tree_groups, c.stages, c.splits);
 }

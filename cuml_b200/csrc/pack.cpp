@@ -633,6 +633,32 @@ struct Packer {
         std::memcpy(leaves + s * lbytes, &id, 4);
       }
     }
+    // the same nodes for tiles with missing values: features of tests whose missing values go
+    // left are read from the second set of columns
+    bool any_left = false;
+    for (int p = 0; p < nt && !any_left; ++p) {
+      const uint8_t* src = out.q_nodes.data() + static_cast<size_t>(qstride) * p;
+      for (int64_t i = 1; i < width && !any_left; ++i) {
+        uint32_t node;
+        std::memcpy(&node, src + i * qnb, 4);
+        any_left = (node & Q_DEFAULT_RIGHT) == 0u;
+      }
+    }
+    out.view.q_any_default_left = any_left ? 1 : 0;
+    if (any_left && 2 * F <= static_cast<int>(Q_MAX_FEATURES)) {
+      out.q_nodes_nan = out.q_nodes;
+      for (int p = 0; p < nt; ++p) {
+        uint8_t* dst = out.q_nodes_nan.data() + static_cast<size_t>(qstride) * p;
+        for (int64_t i = 1; i < width; ++i) {
+          uint32_t node;
+          std::memcpy(&node, dst + i * qnb, 4);
+          if (node >> Q_RANK_SHIFT == Q_MAX_RANK_FIELD)  // categorical
+            node -= 1u << Q_RANK_SHIFT;
+          if ((node & Q_DEFAULT_RIGHT) == 0u) node += static_cast<uint32_t>(F) << Q_FEATURE_SHIFT;
+          std::memcpy(dst + i * qnb, &node, 4);
+        }
+      }
+    }
     bool in_order = true;
     for (int p = 0; p < nt; ++p) in_order = in_order && out.tree_orig[p] == p;
     out.view.q_trees_in_order = in_order ? 1 : 0;
@@ -1107,6 +1133,7 @@ int pack_forest(const b2fil_forest_desc& desc, const b2fil_create_opts& opts,
       out.q_thresholds.clear();
       out.q_top.clear();
       out.q_nodes_ids.clear();
+      out.q_nodes_nan.clear();
       out.q_lut.clear();
       out.q_feats.clear();
       out.q_groups.clear();
