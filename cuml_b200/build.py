@@ -23,7 +23,7 @@ SOURCES = ["api.cu", "kernels.cu", "kernels_q_top6.cu", "kernels_q_plain6.cu", "
            "kernels_q_vec.cu",
            "kernels_sparse_c.cu",
            "pack.cpp"]
-HEADERS = ["forest.hpp", "kernels.hpp", "kernels_q.hpp", "device_common.cuh", "dense_q.cuh",
+HEADERS = ["forest.hpp", "host_pool.hpp", "kernels.hpp", "kernels_q.hpp", "device_common.cuh", "dense_q.cuh",
            os.path.join("..", "..", "include", "b2fil.h")]
 
 

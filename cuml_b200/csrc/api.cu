@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "forest.hpp"
+#include "host_pool.hpp"
 #include "kernels.hpp"
 #include "kernels_q.hpp"
 
@@ -104,36 +105,30 @@ struct ShardTiming {
 };
 thread_local ShardTiming g_shard_timing;
 
-// Pipeline shape of b2fil_predict_host (tuning aids B2FIL_HOST_BLOCK_MB / B2FIL_HOST_SLOTS, read
-// from the environment once).
+// Pipeline shape of b2fil_predict_host (tuning aids B2FIL_HOST_BLOCK_MB / B2FIL_HOST_SLOTS /
+// B2FIL_HOST_STAGED_BLOCK_MB / B2FIL_HOST_COPY_THREADS, read from the environment once).
 constexpr int kMaxHostSlots = 4;
 struct HostPipeCfg {
-  size_t block_bytes = size_t(256) << 20;
-  int slots          = 2;
-  // pageable arrays: smaller blocks through three pinned staging buffers, filled by a few threads
+  // rows predicted by one launch: pinned arrays, and pageable arrays, which are staged
+  size_t block_bytes        = size_t(256) << 20;
   size_t staged_block_bytes = size_t(64) << 20;
-  int staged_slots          = 3;
+  int slots                 = 3;  // such blocks in flight
   int copy_threads          = 0;
   HostPipeCfg()
   {
     const unsigned hw = std::thread::hardware_concurrency();
     copy_threads      = static_cast<int>(std::max(1u, std::min(8u, hw / 2)));
-    if (const char* e = getenv("B2FIL_HOST_COPY_THREADS")) {
-      const long n = atol(e);
-      if (n >= 1 && n <= 64) copy_threads = static_cast<int>(n);
-    }
-    if (const char* e = getenv("B2FIL_HOST_STAGED_BLOCK_MB")) {
-      const long mb = atol(e);
-      if (mb >= 1 && mb <= 1024) staged_block_bytes = static_cast<size_t>(mb) << 20;
-    }
-    if (const char* e = getenv("B2FIL_HOST_BLOCK_MB")) {
-      const long mb = atol(e);
-      if (mb >= 1 && mb <= 4096) block_bytes = static_cast<size_t>(mb) << 20;
-    }
-    if (const char* e = getenv("B2FIL_HOST_SLOTS")) {
-      const long n = atol(e);
-      if (n >= 1 && n <= kMaxHostSlots) slots = static_cast<int>(n);
-    }
+    auto number = [](const char* name, long lo, long hi, auto set) {
+      const char* e = getenv(name);
+      if (!e) return;
+      const long v = atol(e);
+      if (v >= lo && v <= hi) set(v);
+    };
+    number("B2FIL_HOST_COPY_THREADS", 1, 64, [&](long v) { copy_threads = static_cast<int>(v); });
+    number("B2FIL_HOST_STAGED_BLOCK_MB", 1, 1024,
+           [&](long v) { staged_block_bytes = static_cast<size_t>(v) << 20; });
+    number("B2FIL_HOST_BLOCK_MB", 1, 4096, [&](long v) { block_bytes = static_cast<size_t>(v) << 20; });
+    number("B2FIL_HOST_SLOTS", 1, kMaxHostSlots, [&](long v) { slots = static_cast<int>(v); });
   }
 };
 const HostPipeCfg& host_pipe_cfg()
@@ -144,6 +139,78 @@ const HostPipeCfg& host_pipe_cfg()
 
 }  // namespace
 
+namespace {
+// Scratch of predictions comes from one stream-ordered memory pool per device, shared by the
+// forests on it: creating and first growing a pool costs milliseconds, which every newly loaded
+// model would otherwise pay.  It keeps what was freed for the next call (a pool of its own leaves
+// the settings of the device's default pool alone) and is destroyed with the last forest.
+struct ScratchPool {
+  cudaMemPool_t pool = nullptr;
+  int users          = 0;
+};
+std::mutex g_pool_mu;
+std::map<int, ScratchPool> g_pools;
+
+cudaError_t acquire_scratch_pool(int device, cudaMemPool_t* out)
+{
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  ScratchPool& s = g_pools[device];
+  if (!s.pool) {
+    cudaMemPoolProps props{};
+    props.allocType     = cudaMemAllocationTypePinned;
+    props.handleTypes   = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id   = device;
+    cudaError_t e       = cudaMemPoolCreate(&s.pool, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = ~uint64_t(0);
+    e = cudaMemPoolSetAttribute(s.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(s.pool);
+      s.pool = nullptr;
+      return e;
+    }
+  }
+  ++s.users;
+  *out = s.pool;
+  return cudaSuccess;
+}
+void release_scratch_pool(int device)
+{
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  ScratchPool& s = g_pools[device];
+  if (--s.users == 0) {
+    cudaMemPoolDestroy(s.pool);
+    s.pool = nullptr;
+  }
+}
+
+// Status words live in pinned host memory, so that the host reads one without a copy (12 us per
+// call).  A page of them serves a thousand forests; pages are kept.
+std::mutex g_status_mu;
+std::vector<int32_t*> g_status_free;
+cudaError_t acquire_status_word(int32_t** out)
+{
+  std::lock_guard<std::mutex> lock(g_status_mu);
+  if (g_status_free.empty()) {
+    void* page          = nullptr;
+    const size_t bytes  = 4096;
+    const cudaError_t e = cudaHostAlloc(&page, bytes, cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e != cudaSuccess) return e;
+    for (size_t i = bytes / 4; i-- > 0;) g_status_free.push_back(static_cast<int32_t*>(page) + i);
+  }
+  *out = g_status_free.back();
+  g_status_free.pop_back();
+  **out = 0;
+  return cudaSuccess;
+}
+void release_status_word(int32_t* word)
+{
+  std::lock_guard<std::mutex> lock(g_status_mu);
+  g_status_free.push_back(word);
+}
+}  // namespace
+
 // One slot of the host-buffer pipeline: device staging buffers and the stream that orders them.
 struct HostSlot {
   cudaStream_t stream = nullptr;
@@ -152,46 +219,64 @@ struct HostSlot {
   size_t x_bytes      = 0;
   size_t out_bytes    = 0;
   cudaEvent_t ev[3]   = {nullptr, nullptr, nullptr};  // sharded prediction: begin, kernels done, gathered
-  // pageable host arrays: pinned staging on the host side of the copies
-  void* pin_in         = nullptr;
-  void* pin_out        = nullptr;
-  size_t pin_in_bytes  = 0;
+  void* pin_out        = nullptr;  // results for pageable arrays pass through here
   size_t pin_out_bytes = 0;
   int64_t pending_r0   = -1;  // rows whose results sit in pin_out, not yet handed to the caller
   int64_t pending_n    = 0;
 };
+
+// One piece of pinned memory through which pageable inputs pass.
+struct StageChunk {
+  void* ptr        = nullptr;
+  size_t bytes     = 0;
+  cudaEvent_t free = nullptr;  // its last copy to the device is done
+};
+constexpr int kStageChunks = 4;
 
 struct b2fil_forest {
   ForestView view{};
   int32_t precision = B2FIL_F32, storage = 0, layout = 0, align_bytes = 0, node_bytes = 0;
   int32_t device = 0, sm_count = 0, default_chunk = 0;
   int64_t n_nodes_in = 0, n_nodes_packed = 0, device_bytes = 0;
-  int32_t* status = nullptr;
-  cudaMemPool_t pool = nullptr;  // stream-ordered scratch of the rank-quantised path
+  int32_t* status = nullptr;     // pinned host word that kernels set when a bounded wait runs out
+  cudaMemPool_t pool = nullptr;  // the device's scratch pool (shared, see acquire_scratch_pool)
+  mutable std::atomic<int64_t> scratch_peak{0};  // most scratch one prediction took from it
+  void* arena = nullptr;         // device memory of all blocks
+  size_t arena_bytes = 0;
   std::vector<uint32_t> q_top;   // host copy of the three top nodes per tree (may be empty)
   struct Block {
-    void* ptr;
-    size_t bytes;
+    size_t at;           // offset in the arena
     size_t view_offset;  // offset of the pointer member inside ForestView
   };
+  void place_blocks()
+  {
+    for (const Block& b : blocks) {
+      void* d = static_cast<char*>(arena) + b.at;
+      std::memcpy(reinterpret_cast<char*>(&view) + b.view_offset, &d, sizeof(void*));
+    }
+  }
   std::vector<Block> blocks;
   int32_t clone_src_device = -1;  // device this forest was replicated from, or -1
   int32_t clone_direct     = -1;  // 1: that replication went over a direct peer path
   std::mutex host_mu;  // serialises the calls that use the slots below
   HostSlot slots[kMaxHostSlots];
+  StageChunk chunks[kStageChunks];
   ~b2fil_forest()
   {
     DeviceGuard g(device);
-    for (auto& b : blocks) cudaFree(b.ptr);
-    if (status) cudaFree(status);
-    if (pool) cudaMemPoolDestroy(pool);
+    if (arena) cudaFree(arena);
+    if (status) release_status_word(status);
+    if (pool) release_scratch_pool(device);
+    for (auto& c : chunks) {
+      if (c.ptr) cudaFreeHost(c.ptr);
+      if (c.free) cudaEventDestroy(c.free);
+    }
     for (auto& s : slots) {
       if (s.x) cudaFree(s.x);
       if (s.out) cudaFree(s.out);
       if (s.stream) cudaStreamDestroy(s.stream);
       for (auto& e : s.ev)
         if (e) cudaEventDestroy(e);
-      if (s.pin_in) cudaFreeHost(s.pin_in);
       if (s.pin_out) cudaFreeHost(s.pin_out);
     }
   }
@@ -199,43 +284,56 @@ struct b2fil_forest {
 
 namespace {
 
+// Device memory of a forest: its arrays, one after the other in a single allocation (fifteen
+// allocations and frees of their own took most of the time of loading a small model).
+struct Upload {
+  const void* data;
+  size_t bytes, view_offset;
+};
 template <typename V>
-int upload(b2fil_forest* f, const V& host, size_t view_offset)
+void add_upload(std::vector<Upload>& list, const V& host, size_t view_offset)
 {
-  if (host.empty()) return B2FIL_OK;
-  const size_t bytes = host.size() * sizeof(typename V::value_type);
-  void* d            = nullptr;
-  cudaError_t e      = cudaMalloc(&d, bytes);
+  if (!host.empty())
+    list.push_back({host.data(), host.size() * sizeof(typename V::value_type), view_offset});
+}
+
+int allocate_arena(b2fil_forest* f, size_t bytes)
+{
+  const cudaError_t e = cudaMalloc(&f->arena, std::max<size_t>(bytes, 256));
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
     return set_error(B2FIL_ERR_NO_MEMORY, "device allocation of " + std::to_string(bytes) +
                                             " bytes for the forest failed");
   }
   if (e != cudaSuccess) return cuda_error("cudaMalloc", e);
-  f->blocks.push_back({d, bytes, view_offset});
-  f->device_bytes += static_cast<int64_t>(bytes);
-  B2FIL_CUDA(cudaMemcpy(d, host.data(), bytes, cudaMemcpyHostToDevice));
-  std::memcpy(reinterpret_cast<char*>(&f->view) + view_offset, &d, sizeof(void*));
+  f->arena_bytes = bytes;
+  return B2FIL_OK;
+}
+
+int upload_all(b2fil_forest* f, const std::vector<Upload>& list)
+{
+  size_t total = 0;
+  for (const Upload& u : list) {
+    f->blocks.push_back({total, u.view_offset});
+    f->device_bytes += static_cast<int64_t>(u.bytes);
+    total += (u.bytes + 255) / 256 * 256;
+  }
+  const int rc = allocate_arena(f, total);
+  if (rc != B2FIL_OK) return rc;
+  for (size_t i = 0; i < list.size(); ++i)
+    B2FIL_CUDA(cudaMemcpy(static_cast<char*>(f->arena) + f->blocks[i].at, list[i].data,
+                          list[i].bytes, cudaMemcpyHostToDevice));
+  f->place_blocks();
   return B2FIL_OK;
 }
 
 int init_device_state(b2fil_forest* f)
 {
-  cudaDeviceProp prop;
-  B2FIL_CUDA(cudaGetDeviceProperties(&prop, f->device));
-  f->sm_count = prop.multiProcessorCount;
-  B2FIL_CUDA(cudaMalloc(&f->status, sizeof(int32_t)));
-  B2FIL_CUDA(cudaMemset(f->status, 0, sizeof(int32_t)));
-  // a pool of its own keeps freed scratch cached between predictions without touching the
-  // settings of the device's default pool
-  cudaMemPoolProps props{};
-  props.allocType     = cudaMemAllocationTypePinned;
-  props.handleTypes   = cudaMemHandleTypeNone;
-  props.location.type = cudaMemLocationTypeDevice;
-  props.location.id   = f->device;
-  B2FIL_CUDA(cudaMemPoolCreate(&f->pool, &props));
-  uint64_t keep = ~uint64_t(0);
-  B2FIL_CUDA(cudaMemPoolSetAttribute(f->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+  int sms = 0;
+  B2FIL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, f->device));
+  f->sm_count = sms;
+  B2FIL_CUDA(acquire_status_word(&f->status));
+  B2FIL_CUDA(acquire_scratch_pool(f->device, &f->pool));
   return B2FIL_OK;
 }
 
@@ -289,15 +387,15 @@ int enqueue(const b2fil_forest* f, int kind, const void* X, int64_t n_rows, int6
   p.q_top      = f->q_top.empty() ? nullptr : f->q_top.data();
   std::string err;
   int64_t n = 0;
-  const int rc =
-    launch_predict(p, chunk_size > 0 ? chunk_size : f->default_chunk, f->sm_count, stream, f->pool,
-                   err, &n);
+  const Scratch scratch{f->pool, &f->scratch_peak};
+  const int rc = launch_predict(p, chunk_size > 0 ? chunk_size : f->default_chunk, f->sm_count,
+                                stream, &scratch, err, &n);
   g_launches += n;
   if (rc != B2FIL_OK) return set_error(rc, err);
   return B2FIL_OK;
 }
 
-int ensure_slot(b2fil_forest* f, HostSlot& s, size_t x_bytes, size_t out_bytes)
+int ensure_slot(HostSlot& s, size_t x_bytes, size_t out_bytes)
 {
   if (!s.stream) B2FIL_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
   if (s.x_bytes < x_bytes) {
@@ -314,17 +412,16 @@ int ensure_slot(b2fil_forest* f, HostSlot& s, size_t x_bytes, size_t out_bytes)
     B2FIL_CUDA(cudaMalloc(&s.out, out_bytes));
     s.out_bytes = out_bytes;
   }
-  (void)f;
   return B2FIL_OK;
 }
 
 // Read and clear the status word.  The caller has already waited for the work it cares about.
 int read_status_word(const b2fil_forest* f, int32_t* status)
 {
-  B2FIL_CUDA(cudaMemcpy(status, f->status, sizeof(int32_t), cudaMemcpyDeviceToHost));
+  volatile int32_t* word = f->status;
+  *status                = *word;
   if (*status != 0) {
-    // reported once: the next prediction starts from a clean word
-    B2FIL_CUDA(cudaMemset(f->status, 0, sizeof(int32_t)));
+    *word = 0;  // reported once: the next prediction starts from a clean word
     static const char* const where[] = {"", "tree ring (producer)", "tree ring (consumer)",
                                         "row-tile buffer", "rank tables", "self test"};
     const char* w = (*status >= 1 && *status <= 5) ? where[*status] : "unknown";
@@ -337,13 +434,16 @@ int read_status_word(const b2fil_forest* f, int32_t* status)
 // True when the CUDA runtime does not know the host pointer: ordinary (pageable) memory.  Copies
 // from such memory are staged by the driver through a small internal buffer and run at a
 // fraction of the link; the library stages them itself instead.
-bool is_pageable(const void* p)
+// `mapped`: the address kernels reach it at, or null.
+bool is_pageable(const void* p, void** mapped)
 {
   cudaPointerAttributes a{};
+  *mapped = nullptr;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return true;
   }
+  if (a.type == cudaMemoryTypeHost) *mapped = a.devicePointer;
   return a.type == cudaMemoryTypeUnregistered;
 }
 
@@ -363,11 +463,15 @@ int ensure_pinned(void** buf, size_t* have, size_t want)
 }
 
 // Copy `n_rows` rows of `row_bytes` bytes (source rows `src_stride` bytes apart) into a dense
-// buffer with `threads` host threads: one thread cannot fill a PCIe 5 link from pageable memory.
-void parallel_rows_copy(char* dst, const char* src, int64_t n_rows, size_t row_bytes,
-                        size_t src_stride, int threads)
+// buffer, in pieces that the copy threads share.
+void copy_rows(char* dst, const char* src, int64_t n_rows, size_t row_bytes, size_t src_stride)
 {
-  auto work = [=](int64_t b, int64_t e) {
+  const size_t total  = static_cast<size_t>(n_rows) * row_bytes;
+  const size_t piece  = std::min(size_t(128) << 10, std::max(size_t(16) << 10, total / 16));
+  const int64_t step  = std::max<int64_t>(1, static_cast<int64_t>(piece / std::max<size_t>(1, row_bytes)));
+  const size_t pieces = static_cast<size_t>((n_rows + step - 1) / step);
+  CopyPool::get(host_pipe_cfg().copy_threads).run(pieces, [&](size_t i) {
+    const int64_t b = static_cast<int64_t>(i) * step, e = std::min(n_rows, b + step);
     if (src_stride == row_bytes) {
       std::memcpy(dst + static_cast<size_t>(b) * row_bytes, src + static_cast<size_t>(b) * src_stride,
                   static_cast<size_t>(e - b) * row_bytes);
@@ -376,95 +480,272 @@ void parallel_rows_copy(char* dst, const char* src, int64_t n_rows, size_t row_b
         std::memcpy(dst + static_cast<size_t>(r) * row_bytes, src + static_cast<size_t>(r) * src_stride,
                     row_bytes);
     }
-  };
-  const int64_t min_rows = std::max<int64_t>(1, static_cast<int64_t>((size_t(4) << 20) / std::max<size_t>(1, row_bytes)));
-  const int t = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(threads, n_rows / min_rows)));
-  if (t <= 1) {
-    work(0, n_rows);
-    return;
-  }
-  std::vector<std::thread> pool;
-  pool.reserve(t - 1);
-  for (int i = 1; i < t; ++i) pool.emplace_back(work, n_rows * i / t, n_rows * (i + 1) / t);
-  work(0, n_rows / t);
-  for (auto& th : pool) th.join();
+  });
 }
 
-// Host-array prediction for pageable inputs: row blocks are gathered into pinned staging buffers
-// by several host threads while the previous blocks are copied and predicted; results come back
-// through pinned buffers too.  The caller holds the forest's host mutex and has made its device
-// current.
-int predict_host_staged(b2fil_forest* f, int infer_kind, const char* xin, int64_t n_rows,
-                        int64_t row_stride, char* yout, int chunk_size, double threshold)
-{
-  const HostPipeCfg& pipe = host_pipe_cfg();
-  const size_t es        = elem_bytes(f);
-  const int64_t F        = f->view.n_features;
-  const size_t in_row_b  = static_cast<size_t>(F) * es;
-  const size_t out_row_b = static_cast<size_t>(out_elems(f, infer_kind)) * out_elem_bytes(f, infer_kind);
-  int64_t block_rows = static_cast<int64_t>(
-    std::max<size_t>(1, pipe.staged_block_bytes / std::max(in_row_b, out_row_b)));
-  block_rows = std::max<int64_t>(block_rows / 128 * 128, 128);
-  block_rows = std::min(block_rows, n_rows);
-  const int S = pipe.staged_slots;
-  int rc      = B2FIL_OK;
-  for (int i = 0; i < S && rc == B2FIL_OK; ++i) {
-    HostSlot& s = f->slots[i];
-    rc = ensure_slot(f, s, static_cast<size_t>(block_rows) * in_row_b,
-                     static_cast<size_t>(block_rows) * out_row_b);
-    if (rc == B2FIL_OK) rc = ensure_pinned(&s.pin_in, &s.pin_in_bytes, static_cast<size_t>(block_rows) * in_row_b);
-    if (rc == B2FIL_OK) rc = ensure_pinned(&s.pin_out, &s.pin_out_bytes, static_cast<size_t>(block_rows) * out_row_b);
-    s.pending_r0 = -1;
+// Host-array prediction, in one of three ways by the size of the input:
+//  in_place (up to 16 KiB): the kernel reads its rows over the link and writes its results back over
+//    it; pinned host memory is mapped, and no copy starts as fast as that.
+//  short_call (up to 8 MiB): a kernel fetches the rows from pinned memory, piece by piece while the
+//    copy threads fill the next one.  Between kernels of a stream there is about a microsecond; a
+//    copy-engine transfer costs 5 us to start and again to hand over (1,000 rows of 50 features:
+//    46 -> 30 us).
+//  blocks: row blocks are copied to the device, predicted and copied back on a few streams, so that
+//    the copies of one block overlap the kernels of another; about eight blocks per call keep the
+//    last block's kernels, which nothing overlaps, short.  Pinned inputs are copied from where they
+//    are.  Pageable ones pass through four pinned chunks of at most 4 MiB: the copy threads fill one
+//    (they stay in the host's cache, 100 GB/s) while another is on the link (large enough for 52 of
+//    its 55 GB/s); the driver's own staging of pageable memory reaches 12 to 19 GB/s.
+// The caller holds the forest's host mutex and has made its device current.
+class HostPrediction {
+ public:
+  HostPrediction(b2fil_forest* f, int kind, const void* X, int64_t n_rows, int64_t row_stride,
+                 void* out, int chunk_size, double threshold)
+      : f_(f), kind_(kind), x_(static_cast<const char*>(X)), out_(static_cast<char*>(out)),
+        n_rows_(n_rows), chunk_size_(chunk_size), threshold_(threshold)
+  {
+    in_row_b_   = static_cast<size_t>(f->view.n_features) * elem_bytes(f);
+    in_stride_  = static_cast<size_t>(row_stride) * elem_bytes(f);
+    out_row_b_  = static_cast<size_t>(out_elems(f, kind)) * out_elem_bytes(f, kind);
+    in_bytes_   = static_cast<size_t>(n_rows) * in_row_b_;
+    out_bytes_  = static_cast<size_t>(n_rows) * out_row_b_;
+    in_pinned_  = !is_pageable(X, &in_mapped_);
+    out_pinned_ = !is_pageable(out, &out_mapped_);
   }
-  if (rc != B2FIL_OK) return rc;  // nothing has been enqueued yet
-  // hand a slot's finished results to the caller (after its stream has drained)
-  auto flush = [&](HostSlot& s) -> int {
-    if (s.pending_r0 < 0) return B2FIL_OK;
-    const cudaError_t e = cudaStreamSynchronize(s.stream);
-    if (e != cudaSuccess) return cuda_error("cudaStreamSynchronize", e);
-    std::memcpy(yout + static_cast<size_t>(s.pending_r0) * out_row_b, s.pin_out,
-                static_cast<size_t>(s.pending_n) * out_row_b);
-    s.pending_r0 = -1;
-    return B2FIL_OK;
-  };
-  int which = 0;
-  for (int64_t r0 = 0; r0 < n_rows && rc == B2FIL_OK; r0 += block_rows, which = (which + 1) % S) {
-    HostSlot& s     = f->slots[which];
-    const int64_t n = std::min(block_rows, n_rows - r0);
-    if ((rc = flush(s)) != B2FIL_OK) break;  // also frees the slot's staging buffers for reuse
-    parallel_rows_copy(static_cast<char*>(s.pin_in), xin + static_cast<size_t>(r0) * row_stride * es,
-                       n, in_row_b, static_cast<size_t>(row_stride) * es, pipe.copy_threads);
-    cudaError_t e = cudaMemcpyAsync(s.x, s.pin_in, static_cast<size_t>(n) * in_row_b,
-                                    cudaMemcpyHostToDevice, s.stream);
-    if (e != cudaSuccess) {
-      rc = cuda_error("host-to-device copy of a row block", e);
-      break;
+
+  int run()
+  {
+    int rc;
+    if (in_bytes_ <= kInPlaceIn && out_bytes_ <= (per_tree() ? kPerTreeOut : kInPlaceOut)) {
+      rc = in_place();
+    } else if (in_bytes_ <= kShortIn && out_bytes_ <= kShortIn) {
+      rc = short_call();
+    } else {
+      rc = blocks();
     }
-    rc = enqueue(f, infer_kind, s.x, n, F, s.out, chunk_size, threshold, s.stream);
-    if (rc != B2FIL_OK) break;
-    e = cudaMemcpyAsync(s.pin_out, s.out, static_cast<size_t>(n) * out_row_b, cudaMemcpyDeviceToHost,
-                        s.stream);
-    if (e != cudaSuccess) {
-      rc = cuda_error("device-to-host copy of a result block", e);
-      break;
-    }
-    s.pending_r0 = r0;
-    s.pending_n  = n;
-  }
-  // drain every slot, also after an error: copies in flight still use the staging buffers
-  for (int i = 0; i < S; ++i) {
-    HostSlot& s = f->slots[i];
-    if (rc == B2FIL_OK) {
-      rc = flush(s);
-    } else if (s.stream) {
-      cudaStreamSynchronize(s.stream);
+    // also after an error: work already enqueued still uses the caller's arrays and the staging
+    for (HostSlot& s : f_->slots) {
+      if (!s.stream) continue;
+      const int drained = rc == B2FIL_OK ? flush(s) : (cudaStreamSynchronize(s.stream), B2FIL_OK);
+      if (rc == B2FIL_OK) rc = drained;
       s.pending_r0 = -1;
     }
+    if (rc != B2FIL_OK) return rc;
+    int32_t status = 0;
+    return read_status_word(f_, &status);
   }
-  if (rc != B2FIL_OK) return rc;
-  int32_t status = 0;
-  return read_status_word(f, &status);
-}
+
+ private:
+  static constexpr size_t kInPlaceIn  = size_t(16) << 10;
+  static constexpr size_t kInPlaceOut = size_t(64) << 10;
+  static constexpr size_t kShortIn    = size_t(8) << 20;
+  static constexpr size_t kShortOut   = size_t(256) << 10;  // results that the kernel writes to the host itself
+  static constexpr size_t kPerTreeOut = size_t(2) << 10;
+  static constexpr size_t kChunkMax   = size_t(4) << 20;
+  bool per_tree() const { return kind_ == B2FIL_INFER_LEAF_ID || kind_ == B2FIL_INFER_PER_TREE; }
+
+  int in_place()
+  {
+    HostSlot& s   = f_->slots[0];
+    StageChunk& c = f_->chunks[0];
+    int rc        = ensure_slot(s, 0, 0);
+    if (rc == B2FIL_OK) rc = ensure_chunk(c, kInPlaceIn);
+    if (rc == B2FIL_OK) rc = ensure_pinned(&s.pin_out, &s.pin_out_bytes, kInPlaceOut);
+    if (rc != B2FIL_OK) return rc;
+    copy_rows(static_cast<char*>(c.ptr), x_, n_rows_, in_row_b_, in_stride_);
+    rc = enqueue(f_, kind_, c.ptr, n_rows_, f_->view.n_features, s.pin_out, chunk_size_, threshold_,
+                 s.stream);
+    s.pending_r0 = 0;
+    s.pending_n  = n_rows_;
+    return rc;
+  }
+
+  int short_call()
+  {
+    HostSlot& s       = f_->slots[0];
+    StageChunk& c     = f_->chunks[0];
+    const bool direct = in_mapped_ != nullptr && in_stride_ == in_row_b_ &&
+                        reinterpret_cast<uintptr_t>(in_mapped_) % 16 == 0;
+    // results without a copy: consecutive ones, not a store of its own per row and tree
+    const bool write  = out_bytes_ <= (per_tree() ? kPerTreeOut : kShortOut);
+    int rc            = ensure_slot(s, (in_bytes_ + 15) / 16 * 16, write ? 0 : out_bytes_);
+    if (rc == B2FIL_OK && !direct) rc = ensure_chunk(c, (in_bytes_ + 15) / 16 * 16);
+    const bool to_pin = write ? out_mapped_ == nullptr : !out_pinned_;
+    if (rc == B2FIL_OK && to_pin)
+      rc = ensure_pinned(&s.pin_out, &s.pin_out_bytes, std::max(out_bytes_, kShortOut));
+    if (rc != B2FIL_OK) return rc;
+    std::string err;
+    if (direct) {
+      rc = launch_fetch(s.x, in_mapped_, in_bytes_, f_->sm_count, s.stream, err);
+    } else {
+      rc = stage_and_fetch(static_cast<char*>(c.ptr), static_cast<char*>(s.x), s.stream, err);
+    }
+    if (rc != B2FIL_OK) return set_error(rc, err);
+    void* to = to_pin ? s.pin_out : (write ? out_mapped_ : static_cast<void*>(out_));
+    rc = enqueue(f_, kind_, s.x, n_rows_, f_->view.n_features, write ? to : s.out, chunk_size_,
+                 threshold_, s.stream);
+    if (rc != B2FIL_OK) return rc;
+    if (!write) B2FIL_CUDA(cudaMemcpyAsync(to, s.out, out_bytes_, cudaMemcpyDeviceToHost, s.stream));
+    s.pending_r0 = 0;
+    s.pending_n  = to_pin ? n_rows_ : 0;
+    return B2FIL_OK;
+  }
+
+  // All rows to pinned memory and, part by part as the copy threads get on, to the device.
+  int stage_and_fetch(char* pinned, char* device, cudaStream_t stream, std::string& err)
+  {
+    // items of whole rows, and parts of whole items, that start on 16-byte boundaries
+    const int64_t unit  = in_row_b_ % 16 == 0 ? 1 : 4;
+    auto rows_of = [&](size_t bytes) {
+      return std::max(unit, static_cast<int64_t>(bytes / in_row_b_) / unit * unit);
+    };
+    const int64_t item_rows = rows_of(std::min(size_t(64) << 10, std::max(size_t(16) << 10, in_bytes_ / 32)));
+    const size_t n_items    = static_cast<size_t>((n_rows_ + item_rows - 1) / item_rows);
+    // Few parts, each twice the one before: every transfer kernel adds the link's latency, and the
+    // copy threads are faster than the link, so a larger part is ready when a smaller one is over.
+    constexpr size_t kMost = 4;
+    size_t part_end[kMost], n_parts = 0;
+    for (size_t end = 0, size = std::max(size_t(256) << 10, in_bytes_ / 7); end < n_items; size *= 2) {
+      end += std::max<size_t>(1, static_cast<size_t>(rows_of(size) / item_rows));
+      if (n_parts == kMost - 1 || end + end / 2 > n_items) end = n_items;
+      part_end[n_parts++] = end;
+    }
+    std::atomic<size_t> done[kMost] = {};
+    size_t sent = 0;
+    int rc      = B2FIL_OK;
+    auto copy = [&](size_t i) {
+      const int64_t b = static_cast<int64_t>(i) * item_rows, e = std::min(n_rows_, b + item_rows);
+      if (in_stride_ == in_row_b_) {
+        std::memcpy(pinned + static_cast<size_t>(b) * in_row_b_, x_ + static_cast<size_t>(b) * in_row_b_,
+                    static_cast<size_t>(e - b) * in_row_b_);
+      } else {
+        for (int64_t r = b; r < e; ++r)
+          std::memcpy(pinned + static_cast<size_t>(r) * in_row_b_,
+                      x_ + static_cast<size_t>(r) * in_stride_, in_row_b_);
+      }
+      size_t part = 0;
+      while (i >= part_end[part]) ++part;
+      done[part].fetch_add(1);
+    };
+    auto send = [&] {
+      for (; sent < n_parts; ++sent) {
+        const size_t first = sent > 0 ? part_end[sent - 1] : 0, last = part_end[sent];
+        if (done[sent].load() < last - first) return false;
+        const size_t at  = first * static_cast<size_t>(item_rows) * in_row_b_;
+        const size_t end = std::min(in_bytes_, last * static_cast<size_t>(item_rows) * in_row_b_);
+        if (rc == B2FIL_OK)
+          rc = launch_fetch(device + at, pinned + at, end - at, f_->sm_count, stream, err);
+      }
+      return true;
+    };
+    CopyPool::get(host_pipe_cfg().copy_threads).run(n_items, copy, send);
+    return rc;
+  }
+
+  int blocks()
+  {
+    const HostPipeCfg& pipe = host_pipe_cfg();
+    const size_t row_b      = std::max(in_row_b_, out_row_b_);
+    const size_t most       = in_pinned_ ? pipe.block_bytes : pipe.staged_block_bytes;
+    const size_t want       = std::max<size_t>(static_cast<size_t>(n_rows_) * row_b / 8, size_t(8) << 20);
+    int64_t block_rows      = static_cast<int64_t>(std::max<size_t>(1, std::min(most, want) / row_b));
+    block_rows              = std::max<int64_t>(block_rows / 256 * 256, 256);
+    block_rows              = std::min(block_rows, n_rows_);
+    const int n_slots       = static_cast<int>(std::min<int64_t>(pipe.slots, (n_rows_ + block_rows - 1) / block_rows));
+    for (int i = 0; i < n_slots; ++i) {
+      HostSlot& s = f_->slots[i];
+      int rc      = ensure_slot(s, static_cast<size_t>(block_rows) * in_row_b_,
+                                static_cast<size_t>(block_rows) * out_row_b_);
+      if (rc == B2FIL_OK && !out_pinned_)
+        rc = ensure_pinned(&s.pin_out, &s.pin_out_bytes, static_cast<size_t>(block_rows) * out_row_b_);
+      if (rc != B2FIL_OK) return rc;
+    }
+    int which = 0;
+    for (int64_t r0 = 0; r0 < n_rows_; r0 += block_rows, which = (which + 1) % n_slots) {
+      HostSlot& s     = f_->slots[which];
+      const int64_t n = std::min(block_rows, n_rows_ - r0);
+      // stream order makes the slot's previous block finish before its device buffers are reused
+      int rc = flush(s);
+      if (rc == B2FIL_OK) rc = in_pinned_ ? send(s, r0, n) : send_staged(s, r0, n);
+      if (rc == B2FIL_OK)
+        rc = enqueue(f_, kind_, s.x, n, f_->view.n_features, s.out, chunk_size_, threshold_, s.stream);
+      if (rc != B2FIL_OK) return rc;
+      void* to = out_pinned_ ? out_ + static_cast<size_t>(r0) * out_row_b_ : static_cast<char*>(s.pin_out);
+      B2FIL_CUDA(cudaMemcpyAsync(to, s.out, static_cast<size_t>(n) * out_row_b_,
+                                 cudaMemcpyDeviceToHost, s.stream));
+      s.pending_r0 = r0;
+      s.pending_n  = out_pinned_ ? 0 : n;
+    }
+    return B2FIL_OK;
+  }
+
+  // Rows [r0, r0 + n) of a pinned array to the slot's device buffer.
+  int send(HostSlot& s, int64_t r0, int64_t n)
+  {
+    const char* from = x_ + static_cast<size_t>(r0) * in_stride_;
+    if (in_stride_ == in_row_b_) {
+      B2FIL_CUDA(cudaMemcpyAsync(s.x, from, static_cast<size_t>(n) * in_row_b_,
+                                 cudaMemcpyHostToDevice, s.stream));
+    } else {
+      B2FIL_CUDA(cudaMemcpy2DAsync(s.x, in_row_b_, from, in_stride_, in_row_b_,
+                                   static_cast<size_t>(n), cudaMemcpyHostToDevice, s.stream));
+    }
+    return B2FIL_OK;
+  }
+  // The same through pinned chunks.
+  int send_staged(HostSlot& s, int64_t r0, int64_t n)
+  {
+    for (int64_t b = 0, m; b < n; b += m) {
+      // the first chunks of a call are smaller: the link waits for the first one to be filled
+      const size_t size = std::min(kChunkMax, next_size_);
+      next_size_        = size * 2;
+      m = std::min(std::max<int64_t>(1, static_cast<int64_t>(size / in_row_b_)), n - b);
+      const size_t bytes = static_cast<size_t>(m) * in_row_b_;
+      StageChunk& c      = f_->chunks[next_chunk_];
+      next_chunk_        = (next_chunk_ + 1) % kStageChunks;
+      int rc             = ensure_chunk(c, std::max(bytes, kChunkMax));
+      if (rc != B2FIL_OK) return rc;
+      B2FIL_CUDA(cudaEventSynchronize(c.free));
+      copy_rows(static_cast<char*>(c.ptr), x_ + static_cast<size_t>(r0 + b) * in_stride_, m,
+                in_row_b_, in_stride_);
+      B2FIL_CUDA(cudaMemcpyAsync(static_cast<char*>(s.x) + static_cast<size_t>(b) * in_row_b_, c.ptr,
+                                 bytes, cudaMemcpyHostToDevice, s.stream));
+      B2FIL_CUDA(cudaEventRecord(c.free, s.stream));
+    }
+    return B2FIL_OK;
+  }
+  // Wait for a slot and hand its results to the caller.
+  int flush(HostSlot& s)
+  {
+    if (s.pending_r0 < 0) return B2FIL_OK;
+    B2FIL_CUDA(cudaStreamSynchronize(s.stream));
+    if (s.pending_n > 0)
+      copy_rows(out_ + static_cast<size_t>(s.pending_r0) * out_row_b_,
+                static_cast<const char*>(s.pin_out), s.pending_n, out_row_b_, out_row_b_);
+    s.pending_r0 = -1;
+    return B2FIL_OK;
+  }
+  int ensure_chunk(StageChunk& c, size_t bytes)
+  {
+    if (!c.free) B2FIL_CUDA(cudaEventCreateWithFlags(&c.free, cudaEventDisableTiming));
+    if (c.bytes >= bytes) return B2FIL_OK;
+    B2FIL_CUDA(cudaEventSynchronize(c.free));  // the old memory may still be on its way
+    return ensure_pinned(&c.ptr, &c.bytes, bytes);
+  }
+
+  b2fil_forest* f_;
+  int kind_;
+  const char* x_;
+  char* out_;
+  int64_t n_rows_;
+  int chunk_size_;
+  double threshold_;
+  size_t in_row_b_, in_stride_, out_row_b_, in_bytes_, out_bytes_;
+  bool in_pinned_, out_pinned_;
+  void *in_mapped_ = nullptr, *out_mapped_ = nullptr;
+  int next_chunk_ = 0;
+  size_t next_size_ = size_t(1) << 20;  // bytes of the next staged chunk
+};
 
 }  // namespace
 
@@ -512,41 +793,33 @@ int b2fil_forest_create(const b2fil_forest_desc* desc, const b2fil_create_opts* 
     f->n_nodes_packed = pf.n_nodes_packed;
     f->default_chunk  = std::max(0, opts->default_chunk_size);
     if ((rc = init_device_state(f.get())) != B2FIL_OK) return rc;
-    if ((rc = upload(f.get(), pf.nodes, offsetof(ForestView, nodes))) != B2FIL_OK) return rc;
-    if ((rc = upload(f.get(), pf.roots, offsetof(ForestView, roots))) != B2FIL_OK) return rc;
-    if ((rc = upload(f.get(), pf.leaf_ids, offsetof(ForestView, leaf_ids))) != B2FIL_OK) return rc;
-    if ((rc = upload(f.get(), pf.cat_pool, offsetof(ForestView, cat_pool))) != B2FIL_OK) return rc;
-    if ((rc = upload(f.get(), pf.tree_class, offsetof(ForestView, tree_class))) != B2FIL_OK)
-      return rc;
-    if ((rc = upload(f.get(), pf.tree_orig, offsetof(ForestView, tree_orig))) != B2FIL_OK)
-      return rc;
-    if ((rc = upload(f.get(), pf.leaf_vectors, offsetof(ForestView, leaf_vectors))) != B2FIL_OK)
-      return rc;
-    if ((rc = upload(f.get(), pf.out_scale, offsetof(ForestView, out_scale))) != B2FIL_OK)
-      return rc;
-    if ((rc = upload(f.get(), pf.out_bias, offsetof(ForestView, out_bias))) != B2FIL_OK) return rc;
+    std::vector<Upload> list;
+    add_upload(list, pf.nodes, offsetof(ForestView, nodes));
+    add_upload(list, pf.roots, offsetof(ForestView, roots));
+    add_upload(list, pf.leaf_ids, offsetof(ForestView, leaf_ids));
+    add_upload(list, pf.cat_pool, offsetof(ForestView, cat_pool));
+    add_upload(list, pf.tree_class, offsetof(ForestView, tree_class));
+    add_upload(list, pf.tree_orig, offsetof(ForestView, tree_orig));
+    add_upload(list, pf.leaf_vectors, offsetof(ForestView, leaf_vectors));
+    add_upload(list, pf.out_scale, offsetof(ForestView, out_scale));
+    add_upload(list, pf.out_bias, offsetof(ForestView, out_bias));
     if (pf.view.c_enabled) {
-      if ((rc = upload(f.get(), pf.c_nodes, offsetof(ForestView, c_nodes))) != B2FIL_OK) return rc;
-      if ((rc = upload(f.get(), pf.c_exact, offsetof(ForestView, c_exact))) != B2FIL_OK) return rc;
-      if ((rc = upload(f.get(), pf.c_leaf_payload, offsetof(ForestView, c_leaf_payload))) != B2FIL_OK)
-        return rc;
-      if ((rc = upload(f.get(), pf.c_leaf_ids, offsetof(ForestView, c_leaf_ids))) != B2FIL_OK)
-        return rc;
-      if ((rc = upload(f.get(), pf.c_top, offsetof(ForestView, c_top))) != B2FIL_OK) return rc;
-      if ((rc = upload(f.get(), pf.c_top_src, offsetof(ForestView, c_top_src))) != B2FIL_OK)
-        return rc;
+      add_upload(list, pf.c_nodes, offsetof(ForestView, c_nodes));
+      add_upload(list, pf.c_exact, offsetof(ForestView, c_exact));
+      add_upload(list, pf.c_leaf_payload, offsetof(ForestView, c_leaf_payload));
+      add_upload(list, pf.c_leaf_ids, offsetof(ForestView, c_leaf_ids));
+      add_upload(list, pf.c_top, offsetof(ForestView, c_top));
+      add_upload(list, pf.c_top_src, offsetof(ForestView, c_top_src));
     }
     if (pf.view.q_enabled) {
-      if ((rc = upload(f.get(), pf.q_nodes, offsetof(ForestView, q_nodes))) != B2FIL_OK) return rc;
-      if ((rc = upload(f.get(), pf.q_nodes_ids, offsetof(ForestView, q_nodes_ids))) != B2FIL_OK)
-        return rc;
-      if ((rc = upload(f.get(), pf.q_nodes_nan, offsetof(ForestView, q_nodes_nan))) != B2FIL_OK)
-        return rc;
-      if ((rc = upload(f.get(), pf.q_blob, offsetof(ForestView, q_blob))) != B2FIL_OK) return rc;
-      if ((rc = upload(f.get(), pf.q_groups, offsetof(ForestView, q_groups))) != B2FIL_OK)
-        return rc;
+      add_upload(list, pf.q_nodes, offsetof(ForestView, q_nodes));
+      add_upload(list, pf.q_nodes_ids, offsetof(ForestView, q_nodes_ids));
+      add_upload(list, pf.q_nodes_nan, offsetof(ForestView, q_nodes_nan));
+      add_upload(list, pf.q_blob, offsetof(ForestView, q_blob));
+      add_upload(list, pf.q_groups, offsetof(ForestView, q_groups));
       f->q_top = std::move(pf.q_top);
     }
+    if ((rc = upload_all(f.get(), list)) != B2FIL_OK) return rc;
     *out = f.release();
     return B2FIL_OK;
   } catch (const std::bad_alloc&) {
@@ -583,21 +856,12 @@ int b2fil_forest_clone_to_device(const b2fil_forest* src, int device_id, b2fil_f
     if ((rc = init_device_state(f.get())) != B2FIL_OK) return rc;
     f->clone_src_device = src->device;
     f->clone_direct     = enable_peer_pair(device_id, src->device);
-    for (const auto& b : src->blocks) {
-      void* d       = nullptr;
-      cudaError_t e = cudaMalloc(&d, b.bytes);
-      if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        return set_error(B2FIL_ERR_NO_MEMORY, "device allocation for the forest copy failed");
-      }
-      if (e != cudaSuccess) return cuda_error("cudaMalloc", e);
-      f->blocks.push_back({d, b.bytes, b.view_offset});
-      f->device_bytes += static_cast<int64_t>(b.bytes);
-      // direct over the peer path when it could be enabled above, staged through the host
-      // otherwise
-      B2FIL_CUDA(cudaMemcpyPeer(d, device_id, b.ptr, src->device, b.bytes));
-      std::memcpy(reinterpret_cast<char*>(&f->view) + b.view_offset, &d, sizeof(void*));
-    }
+    if ((rc = allocate_arena(f.get(), src->arena_bytes)) != B2FIL_OK) return rc;
+    f->blocks       = src->blocks;
+    f->device_bytes = src->device_bytes;
+    // direct over the peer path when it could be enabled above, staged through the host otherwise
+    B2FIL_CUDA(cudaMemcpyPeer(f->arena, device_id, src->arena, src->device, src->arena_bytes));
+    f->place_blocks();
     *out = f.release();
     return B2FIL_OK;
   } catch (const std::bad_alloc&) {
@@ -636,13 +900,7 @@ int b2fil_forest_info(const b2fil_forest* f, b2fil_info* info)
   info->top_levels         = f->view.c_enabled ? f->view.c_top_levels : 0;
   info->peer_direct        = f->clone_direct;
   info->clone_src_device   = f->clone_src_device;
-  if (f->pool) {
-    uint64_t reserved = 0;
-    if (cudaMemPoolGetAttribute(f->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess)
-      info->scratch_pool_bytes = static_cast<int64_t>(reserved);
-    else
-      cudaGetLastError();
-  }
+  info->scratch_pool_bytes = f->scratch_peak.load();
   return B2FIL_OK;
 }
 
@@ -770,62 +1028,12 @@ int b2fil_predict_host(b2fil_forest* f, int infer_kind, const void* X_host, int6
   std::lock_guard<std::mutex> lock(f->host_mu);
   DeviceGuard guard(f->device);
   if (!guard.ok) return set_error(B2FIL_ERR_CUDA, "cudaSetDevice failed");
-  const size_t es        = elem_bytes(f);
-  const int64_t F        = f->view.n_features;
-  const size_t in_row_b  = static_cast<size_t>(F) * es;
-  const size_t out_row_b = static_cast<size_t>(out_elems(f, infer_kind)) * out_elem_bytes(f, infer_kind);
-  // ordinary (pageable) arrays of some size go through the library's own pinned staging
-  if (static_cast<size_t>(n_rows) * in_row_b >= (size_t(8) << 20) && is_pageable(X_host))
-    return predict_host_staged(f, infer_kind, static_cast<const char*>(X_host), n_rows, row_stride,
-                               static_cast<char*>(out_host), chunk_size, threshold);
-  // row blocks of about 256 MiB of input (and at most 256 MiB of output) keep both copy engines
-  // and the SMs busy while two blocks are in flight
-  const HostPipeCfg& pipe = host_pipe_cfg();
-  const size_t budget     = pipe.block_bytes;
-  int64_t block_rows  = static_cast<int64_t>(std::max<size_t>(1, budget / std::max(in_row_b, out_row_b)));
-  block_rows          = std::max<int64_t>(block_rows / 128 * 128, 128);
-  block_rows          = std::min(block_rows, n_rows);
-  for (int i = 0; i < pipe.slots; ++i) {
-    rc = ensure_slot(f, f->slots[i], static_cast<size_t>(block_rows) * in_row_b,
-                     static_cast<size_t>(block_rows) * out_row_b);
-    if (rc != B2FIL_OK) return rc;  // nothing has been enqueued yet
+  try {
+    return HostPrediction(f, infer_kind, X_host, n_rows, row_stride, out_host, chunk_size, threshold)
+      .run();
+  } catch (const std::exception& ex) {
+    return set_error(B2FIL_ERR_NO_MEMORY, std::string("host-array prediction: ") + ex.what());
   }
-  const char* xin = static_cast<const char*>(X_host);
-  char* yout      = static_cast<char*>(out_host);
-  int which       = 0;
-  for (int64_t r0 = 0; r0 < n_rows && rc == B2FIL_OK; r0 += block_rows, which = (which + 1) % pipe.slots) {
-    HostSlot& s     = f->slots[which];
-    const int64_t n = std::min(block_rows, n_rows - r0);
-    // stream order makes the slot's previous block finish before its buffers are reused
-    cudaError_t e;
-    if (row_stride == F) {
-      e = cudaMemcpyAsync(s.x, xin + static_cast<size_t>(r0) * in_row_b,
-                          static_cast<size_t>(n) * in_row_b, cudaMemcpyHostToDevice, s.stream);
-    } else {
-      e = cudaMemcpy2DAsync(s.x, in_row_b, xin + static_cast<size_t>(r0) * row_stride * es,
-                            static_cast<size_t>(row_stride) * es, in_row_b, static_cast<size_t>(n),
-                            cudaMemcpyHostToDevice, s.stream);
-    }
-    if (e != cudaSuccess) {
-      rc = cuda_error("host-to-device copy of a row block", e);
-      break;
-    }
-    rc = enqueue(f, infer_kind, s.x, n, F, s.out, chunk_size, threshold, s.stream);
-    if (rc != B2FIL_OK) break;
-    e = cudaMemcpyAsync(yout + static_cast<size_t>(r0) * out_row_b, s.out,
-                        static_cast<size_t>(n) * out_row_b, cudaMemcpyDeviceToHost, s.stream);
-    if (e != cudaSuccess) rc = cuda_error("device-to-host copy of a result block", e);
-  }
-  // Also after an error: copies already enqueued still read and write the caller's buffers, so
-  // the call may not return before they are done.
-  for (int i = 0; i < pipe.slots; ++i) {
-    if (!f->slots[i].stream) continue;
-    const cudaError_t e = cudaStreamSynchronize(f->slots[i].stream);
-    if (e != cudaSuccess && rc == B2FIL_OK) rc = cuda_error("cudaStreamSynchronize", e);
-  }
-  if (rc != B2FIL_OK) return rc;
-  int32_t status = 0;
-  return read_status_word(f, &status);
 }
 
 int b2fil_predict_sharded(b2fil_forest* const* forests, int n_devices, int infer_kind,
@@ -877,7 +1085,7 @@ int b2fil_predict_sharded(b2fil_forest* const* forests, int n_devices, int infer
     row_off += n;
     if (n == 0) continue;
     const bool local = f->device == f0->device;
-    int rc = ensure_slot(f, s, 0, local ? 0 : static_cast<size_t>(n) * out_row_b);
+    int rc = ensure_slot(s, 0, local ? 0 : static_cast<size_t>(n) * out_row_b);
     for (auto& ev : s.ev) {
       if (rc == B2FIL_OK && !ev && cudaEventCreate(&ev) != cudaSuccess)
         rc = set_error(B2FIL_ERR_CUDA, "cudaEventCreate failed");

@@ -550,7 +550,7 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
     auto request_tile = [&](int t) {
       // a buffer is free once every consumer warp has left the trees of the tile it held
       if (tprimed && !mbar_wait(bar_tempty + 8u * tpos.stage, tpos.phase ^ 1u)) {
-        atomicExch(p.status, 3);
+        report_status(p.status, 3);
         return false;
       }
       const uint32_t bar = bar_tfull + 8u * tpos.stage;
@@ -575,7 +575,7 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
       for (int b = seg.begin; b < end && going; ++b) {
         const uint32_t s = pos.stage;
         if (primed && !mbar_wait(bars + 8u * (kMaxStages + s), pos.phase ^ 1u)) {
-          atomicExch(p.status, 1);
+          report_status(p.status, 1);
           going = false;
           break;
         }
@@ -651,7 +651,7 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
         // (without top nodes in the parameter block the walk over doubled columns is the same one)
         ok = go(std::integral_constant<int, NAN_NONE>{});
       }
-      if (!ok) atomicExch(p.status, 2);
+      if (!ok) report_status(p.status, 2);
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_tempty + 8u * tpos.stage);

@@ -84,6 +84,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
 {
   return mbar_wait_limited(bar, parity, kSpinLimit);
 }
+// Set the forest's status word (pinned host memory) after a wait that ran out.
+__device__ __forceinline__ void report_status(int32_t* status, int32_t code)
+{
+  *reinterpret_cast<volatile int32_t*>(status) = code;
+}
 // Position in a ring of S stages: the stage index and the parity of its current use, advanced
 // without a division.
 struct RingPos {

@@ -61,7 +61,29 @@ __global__ void bounded_wait_selftest_kernel(int32_t* status, const uint32_t tri
     mbar_fence_init();
   }
   __syncthreads();
-  if (threadIdx.x == 0 && !mbar_wait_limited(bar, 0, tries)) atomicExch(status, 5);
+  if (threadIdx.x == 0 && !mbar_wait_limited(bar, 0, tries)) report_status(status, 5);
+}
+
+// ---------------------------------------------------------------------------------------------
+// rows from mapped host memory
+// ---------------------------------------------------------------------------------------------
+// Bound by the link (45 of its 55 GB/s from 4 MB on): four 16-byte loads in flight per thread and a
+// thread for every 64 bytes, as long as the SMs hold them, cover its 1.5 us.
+__global__ void __launch_bounds__(256)
+fetch_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, const uint32_t n)
+{
+  grid_release();
+  grid_wait();  // the kernel before this one may still be reading what dst held
+  const uint32_t step = gridDim.x * 256u;
+  for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += 4u * step) {
+    uint4 v[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+      if (i + k * step < n) v[k] = __ldcs(src + i + k * step);
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+      if (i + k * step < n) dst[i + k * step] = v[k];
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -198,7 +220,7 @@ dense_kernel(const __grid_constant__ PredictParams p, const int R, const int G, 
         for (int first = t_begin; first < t_end; first += per_batch) {
           const uint32_t s = pos.stage;
           if (primed && !mbar_wait(bars + 8u * (kMaxStages + s), pos.phase ^ 1u)) {
-            atomicExch(p.status, 1);
+            report_status(p.status, 1);
             return;
           }
           const int count      = min(per_batch, t_end - first);
@@ -248,7 +270,7 @@ dense_kernel(const __grid_constant__ PredictParams p, const int R, const int G, 
           p, G, S, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b, acc_group,
           R, pos, run, t_begin, t_end);
       }
-      if (!ok) atomicExch(p.status, 2);
+      if (!ok) report_status(p.status, 2);
     }
     flush_running<T, MODE>(f, run, acc_group, R, r);
     consumer_sync(n_ct);
@@ -524,7 +546,7 @@ quantise_kernel(const __grid_constant__ PredictParams p, uint16_t* __restrict__ 
       flags.arrived[t] = 0;
   }
   if (!mbar_wait(bar, 0)) {
-    if (threadIdx.x == 0) atomicExch(p.status, 4);
+    if (threadIdx.x == 0) report_status(p.status, 4);
     return;
   }
   // the number of halvings is fixed per group: pick the unrolled body once
@@ -1047,7 +1069,8 @@ int launch_quantise(const PredictParams& p, uint16_t* Q, const QFlags& flags, in
 // chunk the pre-pass writes the ranks into stream-ordered scratch and the traversal kernel reads
 // them back.
 int launch_dense_q(const PredictParams& p, int mode, int chunk_size, int sm_count,
-                   cudaStream_t stream, cudaMemPool_t pool, std::string& err, int64_t* launches)
+                   cudaStream_t stream, const Scratch& pool, std::string& err,
+                   int64_t* launches)
 {
   const ForestView& f = p.f;
   const int precision = f.format == FMT_DENSE_F ? B2FIL_F32 : B2FIL_F64;
@@ -1088,13 +1111,17 @@ int launch_dense_q(const PredictParams& p, int mode, int chunk_size, int sm_coun
   const int flag_words   = f.q_n_groups * 8;  // a byte per warp of the pre-pass
   const size_t fl_bytes  = static_cast<size_t>(ch_tiles) * flag_words * 4;
   const size_t arr_bytes = reduce ? static_cast<size_t>(ch_tiles) * 4 : 0;
+  const size_t need      = q_bytes + sum_bytes + fl_bytes + arr_bytes;
   unsigned char* scratch = nullptr;
   cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch),
-                                          q_bytes + sum_bytes + fl_bytes + arr_bytes, pool, stream);
+                                          need, pool.pool, stream);
   if (e != cudaSuccess) {
     cudaGetLastError();
     err = std::string("scratch allocation for quantised rows failed: ") + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? B2FIL_ERR_NO_MEMORY : B2FIL_ERR_CUDA;
+  }
+  for (int64_t seen = pool.peak->load(); seen < static_cast<int64_t>(need) &&
+                                         !pool.peak->compare_exchange_weak(seen, need);) {
   }
   uint16_t* Q     = reinterpret_cast<uint16_t*>(scratch);
   uint8_t* flags  = scratch + q_bytes + sum_bytes;
@@ -1360,7 +1387,7 @@ int dense_ok(int depth, int precision, int n_features, int n_outputs)
 }
 
 int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStream_t stream,
-                   cudaMemPool_t pool, std::string& err, int64_t* launches)
+                   const Scratch* scratch, std::string& err, int64_t* launches)
 {
   const ForestView& f = p.f;
   if (p.n_rows == 0) return B2FIL_OK;
@@ -1397,9 +1424,9 @@ int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStr
     dense_fmt && !ranks_only && n_rows_small(p.n_rows, sm_count) &&
     split_shape(f, mode, prec, p.n_rows,
                 chunk_size > 0 ? pick_rows_per_tile(p.n_rows, chunk_size, sm_count) : 0, sm_count, split);
-  if (dense_fmt && f.q_enabled && p.row_stride < (int64_t(1) << 22) && pool != nullptr &&
+  if (dense_fmt && f.q_enabled && p.row_stride < (int64_t(1) << 22) && scratch != nullptr &&
       (chunk_size > 0 || !have_split || split.us > rank_path_us(f, mode, p.n_rows, sm_count))) {
-    rc = launch_dense_q(p, mode, chunk_size, sm_count, stream, pool, err, launches);
+    rc = launch_dense_q(p, mode, chunk_size, sm_count, stream, *scratch, err, launches);
     if (rc != B2FIL_OK) return rc;
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -1605,6 +1632,16 @@ int launch_predict_fixed_scratch(const PredictParams& p, int chunk_size, int sm_
   }
   if (launches) *launches += 2;
   return B2FIL_OK;
+}
+
+int launch_fetch(void* dst, const void* src_mapped, size_t bytes, int sm_count, cudaStream_t stream,
+                 std::string& err)
+{
+  const uint32_t n   = static_cast<uint32_t>((bytes + 15) / 16);
+  const int blocks   = static_cast<int>(std::min<uint32_t>((n + 1023) / 1024, sm_count * 8u));
+  const SplitLaunch l{dim3(std::max(1, blocks)), 256, 0, stream, 1, true};
+  return launch_split(l, err, fetch_kernel, static_cast<uint4*>(dst),
+                      static_cast<const uint4*>(src_mapped), n);
 }
 
 std::string last_launch_variant()

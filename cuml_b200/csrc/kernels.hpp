@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <string>
 
 #include "forest.hpp"
@@ -50,17 +51,28 @@ bool dense_config(int depth, int precision, int n_features, int n_outputs, bool 
 // rank-quantised rows.
 int dense_ok(int depth, int precision, int n_features, int n_outputs);
 
+// Where predictions take stream-ordered scratch from, and the most that one has taken.
+struct Scratch {
+  cudaMemPool_t pool;
+  std::atomic<int64_t>* peak;
+};
+
 // Enqueue a prediction on `stream`.  Returns B2FIL_OK or an error code with `err` set.
 // `launches` (optional) is incremented by the number of kernels enqueued.
-// Forests with rank-quantised rows take stream-ordered scratch for the ranks from `pool`.
+// Forests with rank-quantised rows take stream-ordered scratch for the ranks from `scratch`.
 int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStream_t stream,
-                   cudaMemPool_t pool, std::string& err, int64_t* launches);
+                   const Scratch* scratch, std::string& err, int64_t* launches);
 
 // Same as launch_predict for forests that predict on rank-quantised rows, except that the rank
 // image goes into a fixed device array inside the library instead of pool memory: nothing is
 // allocated.  `device` is the ordinal of the current device.  The whole batch must fit the array.
 int launch_predict_fixed_scratch(const PredictParams& p, int chunk_size, int sm_count, int device,
                                  cudaStream_t stream, std::string& err, int64_t* launches);
+
+// Enqueue a kernel that copies `bytes` bytes from mapped host memory to the device.  Both addresses are
+// 16-byte aligned, and both buffers may be read / written up to the next multiple of 16.
+int launch_fetch(void* dst, const void* src_mapped, size_t bytes, int sm_count, cudaStream_t stream,
+                 std::string& err);
 
 // What the calling thread's most recent launch_predict* call enqueued: kernel family, template
 // arguments and launch shape, e.g. "quantise_kernel<float> + dense_q_top_kernel<float,scalar,

@@ -262,7 +262,7 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
         for (int b = b_begin; b < b_end; ++b) {
           const uint32_t s = pos.stage;
           if (primed && !mbar_wait(bars + 8u * (kMaxStages + s), pos.phase ^ 1u)) {
-            atomicExch(p.status, 1);
+            report_status(p.status, 1);
             return;
           }
           const int first      = b * per_batch;
@@ -492,7 +492,7 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
         }
       }
     }
-    if (!ok) atomicExch(p.status, 2);
+    if (!ok) report_status(p.status, 2);
     flush_running<T, MODE>(f, run, acc_group, R, r);
     consumer_sync(n_ct);
     if (MODE <= MODE_VECTOR) {

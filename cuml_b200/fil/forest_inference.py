@@ -29,6 +29,11 @@ def _torch():
     return torch
 
 
+def _address(a: np.ndarray) -> int:
+    """Address of an array's data (`a.ctypes.data` without the object in between)."""
+    return a.__array_interface__["data"][0]
+
+
 class _Forest:
     """Owner of one `b2fil_forest` handle (one device)."""
 
@@ -340,8 +345,10 @@ class ForestInference:
                 raise ValueError("preds has the wrong shape, dtype or layout")
         else:
             out = np.empty(shape, odt)
-        _lib.check(lib.b2fil_predict_host(f.handle, kind, Xh.ctypes.data, n, Xh.shape[1],
-                                          out.ctypes.data, cs, float(threshold)))
+        rc = lib.b2fil_predict_host(f.handle, kind, _address(Xh), n, self._nf, _address(out), cs,
+                                    threshold)
+        if rc != 0:
+            _lib.check(rc)
         if want == "torch" or (want == "input" and is_torch):
             return _torch().from_numpy(out)
         return out

@@ -167,8 +167,9 @@ typedef struct b2fil_info {
   int32_t clone_src_device; /* device the forest was replicated from, or -1                     */
   int32_t compact_image;    /* 1: sparse forest with the compact image                          */
   int32_t top_levels;       /* levels of every tree kept as a heap for shared memory, else 0    */
-  int64_t scratch_pool_bytes; /* device memory the forest's scratch pool holds right now (grows
-                                 with the largest batch b2fil_predict has seen; never touched by
+  int64_t scratch_pool_bytes; /* most device memory one prediction of this forest took from its
+                                 device's scratch pool, which keeps it for the next one (grows with
+                                 the largest batch b2fil_predict has seen; never touched by
                                  b2fil_predict_fixed_scratch)                                    */
 } b2fil_info;
 
