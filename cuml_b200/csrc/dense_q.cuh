@@ -268,8 +268,9 @@ struct DenseQWalker {
         // One output per (row, tree).  The payload slot holds what is reported: the leaf value,
         // or the leaf id when the CTA streams the image made for that (MODE_LEAFID).  With four
         // live trees that are also the caller's trees first..first+3, a row's four outputs are
-        // contiguous and leave as 16-byte stores: scalar 4-byte stores at a stride of a whole
-        // output row cost one sector request each and bound these predictions otherwise.
+        // contiguous and leave as 16-byte stores, or, where the rows are not aligned for that,
+        // four lanes at a time (store_quads): scalar 4-byte stores at a stride of a whole output
+        // row cost one sector request each and bound these predictions otherwise.
         typename TR::Val val[NT];
         uint32_t leaf_at[NT];
 #pragma unroll
@@ -279,24 +280,27 @@ struct DenseQWalker {
           val[k]              = TR::ld_val(leaf_at[k]);
         }
         const bool scalar_out = MODE == MODE_LEAFID || f.leaf_vector_len <= 1;
-        const bool wide = FULL && NT == 4 && scalar_out && f.q_trees_in_order != 0 &&
-                          (f.n_trees & 3) == 0 &&
-                          (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
-        if (wide) {
+        const bool quad = FULL && NT == 4 && scalar_out && f.q_trees_in_order != 0;
+        using Out = std::conditional_t<MODE == MODE_LEAFID, uint32_t, typename TR::Val>;
+        Out* out  = static_cast<Out*>(p.out);
+        if (quad && (f.n_trees & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0) {
           if (row < p.n_rows) {
-            if (MODE == MODE_LEAFID || TR::ES == 4) {
-              uint32_t* dst = static_cast<uint32_t*>(p.out) + row * f.n_trees + first;
+            Out* dst = out + row * f.n_trees + first;
+            if constexpr (sizeof(Out) == 4) {
               *reinterpret_cast<uint4*>(dst) =
                 make_uint4(TR::low32(val[0]), TR::low32(val[NT > 1 ? 1 : 0]),
                            TR::low32(val[NT > 2 ? 2 : 0]), TR::low32(val[NT > 3 ? 3 : 0]));
             } else {
-              uint64_t* dst = static_cast<uint64_t*>(p.out) + row * f.n_trees + first;
               *reinterpret_cast<ulonglong2*>(dst) =
                 make_ulonglong2(val[0], val[NT > 1 ? 1 : 0]);
               *reinterpret_cast<ulonglong2*>(dst + 2) =
                 make_ulonglong2(val[NT > 2 ? 2 : 0], val[NT > 3 ? 3 : 0]);
             }
           }
+        } else if (quad) {
+          store_quads<Out>(out, f.n_trees, row, p.n_rows, first, static_cast<Out>(val[0]),
+                           static_cast<Out>(val[NT > 1 ? 1 : 0]), static_cast<Out>(val[NT > 2 ? 2 : 0]),
+                           static_cast<Out>(val[NT > 3 ? 3 : 0]));
         } else {
 #pragma unroll
           for (int k = 0; k < NT; ++k) {
@@ -317,6 +321,16 @@ struct DenseQWalker {
                 take_leaf<T, MODE>(p, first + k, val[k], 0u, acc_group, R, r, row, run);
               }
             }
+          }
+        }
+      } else if (MODE == MODE_VECTOR && inline_vec && f.n_outputs == 2 && sizeof(T) == 4) {
+        // two classes, the common random-forest classifier: one 8-byte load per leaf
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          if (FULL || k < n_act) {
+            const uint2 v = lds_u32x2(base[k] + width_b + (idx[k] - (1u << D)) * 8u);
+            run.v[0] += static_cast<T>(__uint_as_float(v.x));
+            run.v[1] += static_cast<T>(__uint_as_float(v.y));
           }
         }
       } else {
@@ -708,6 +722,29 @@ dense_q_top_kernel(const __grid_constant__ PredictParams p, const __grid_constan
                    const __grid_constant__ QTop top)
 {
   dense_q_body<T, MODE, NT, DEPTH, false, true>(p, q, &top);
+}
+
+// Launch one instantiation of dense_q_top_kernel.
+template <typename T, int MODE, int NT, int DEPTH>
+int launch_q_top(const QLaunch& L, std::string& err)
+{
+  // the three top nodes of every tree travel in the parameter block
+  static thread_local QTop top;
+  std::memcpy(top.w, L.p.q_top, static_cast<size_t>(L.p.f.n_trees) * 3 * sizeof(uint32_t));
+  return launch_split(L.shape(), err, dense_q_top_kernel<T, MODE, NT, DEPTH>, L.p, L.q, top);
+}
+template <typename T, int MODE, int NT>
+int launch_q_top_depth(const QLaunch& L, std::string& err)
+{
+  switch (L.p.f.dense_depth) {
+    case 4: return launch_q_top<T, MODE, NT, 4>(L, err);
+    case 5: return launch_q_top<T, MODE, NT, 5>(L, err);
+    case 6: return launch_q_top<T, MODE, NT, 6>(L, err);
+    case 7: return launch_q_top<T, MODE, NT, 7>(L, err);
+    case 8: return launch_q_top<T, MODE, NT, 8>(L, err);
+    case 9: return launch_q_top<T, MODE, NT, 9>(L, err);
+    default: return launch_q_top<T, MODE, NT, 10>(L, err);
+  }
 }
 
 // Launch one instantiation of dense_q_kernel.

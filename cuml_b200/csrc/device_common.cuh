@@ -578,6 +578,33 @@ __device__ __forceinline__ void take_leaf(const PredictParams& p, int tree,
   }
 }
 
+// Four consecutive outputs of every lane's row (outputs c..c+3 of a row-major array with `width` outputs
+// per row) where a row does not start on a 16-byte boundary.  The 4 x 4 values of four lanes are
+// transposed with shuffles, then a store covers eight rows x four neighbouring outputs: 11 sectors on
+// average instead of the 32 of a store of one output per row.  Called by whole warps; `row` is the
+// lane's row and `n_rows` the end of the batch.
+template <typename V>
+__device__ __forceinline__ void store_quads(V* out, int64_t width, int64_t row, int64_t n_rows, int c,
+                                            V v0, V v1, V v2, V v3)
+{
+  const int lane = threadIdx.x & 31;
+  auto swap = [&](bool upper, int mask, V& a, V& b) {
+    const V got = __shfl_xor_sync(0xffffffffu, upper ? a : b, mask);
+    (upper ? a : b) = got;
+  };
+  swap(lane & 1, 1, v0, v1);
+  swap(lane & 1, 1, v2, v3);
+  swap(lane & 2, 2, v0, v2);
+  swap(lane & 2, 2, v1, v3);
+  // v<j> is now output c + (lane & 3) of the j-th row of the four lanes
+  const int64_t first = row - (lane & 3);
+  V* at               = out + first * width + c + (lane & 3);
+  if (first < n_rows) at[0] = v0;
+  if (first + 1 < n_rows) at[width] = v1;
+  if (first + 2 < n_rows) at[2 * width] = v2;
+  if (first + 3 < n_rows) at[3 * width] = v3;
+}
+
 // Add a thread's running sums to its accumulators in shared memory (end of a row tile), or store
 // them where nothing else was added to the tile's accumulators.
 template <typename T, int MODE>

@@ -998,17 +998,27 @@ int launch_dense_q_kernel(const QLaunch& L, int mode, bool f64, std::string& err
     rec.depth  = f.dense_depth;
     return launch_q_leafg(L, err);
   }
-  if (!f64 && mode == MODE_VECTOR && f.dense_depth >= 4 && f.dense_depth <= 10 &&
-      (L.c.trees_in_flight == 6 || L.c.trees_in_flight == 4)) {
+  const bool unrolled = !f64 && f.dense_depth >= 4 && f.dense_depth <= 10;
+  const bool has_top  = L.p.q_top != nullptr && f.n_trees <= kQTopTrees;
+  if (unrolled && mode >= MODE_PERTREE && has_top && L.c.trees_in_flight == 4) {
+    rec.depth  = f.dense_depth;
+    rec.kernel = "dense_q_top_kernel";
+    return launch_q_top_out(L, mode, err);
+  }
+  if (unrolled && mode == MODE_VECTOR && (L.c.trees_in_flight == 6 || L.c.trees_in_flight == 4)) {
     rec.depth = f.dense_depth;
+    if (has_top && L.c.trees_in_flight == 6) {
+      rec.kernel = "dense_q_top_kernel";
+      return launch_q_top_vec(L, err);
+    }
     return launch_q_vec(L, err);
   }
-  const bool specialised = !f64 && mode == MODE_SCALAR && f.dense_depth >= 4 && f.dense_depth <= 10;
+  const bool specialised = unrolled && mode == MODE_SCALAR;
   if (specialised && L.c.trees_in_flight == 6) {
     // the common boosted-tree shapes: depth-specialised bodies with six trees in flight
     // (q_max_trees_in_flight offers six only for them)
     rec.depth = f.dense_depth;
-    if (L.p.q_top != nullptr && f.n_trees <= kQTopTrees) {
+    if (has_top) {
       rec.kernel = "dense_q_top_kernel";
       return launch_q_top6(L, err);
     }

@@ -98,6 +98,9 @@ constexpr int kMaxCluster = 8;  // largest portable cluster
 // top nodes of every tree from p.q_top (at most kQTopTrees trees).
 int launch_q_top6(const QLaunch& L, std::string& err);
 int launch_q_plain6(const QLaunch& L, std::string& err);
+// The same with vector leaves, and (four trees in flight) with one output per row and tree.
+int launch_q_top_vec(const QLaunch& L, std::string& err);
+int launch_q_top_out(const QLaunch& L, int mode, std::string& err);
 // fp32, scalar leaves, no categorical tests, depth 4..10, four trees in flight.
 int launch_q_plain4(const QLaunch& L, std::string& err);
 // fp32, scalar leaves, no categorical tests, depth 9..10, two or three trees in flight.

@@ -437,16 +437,20 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
           int orig[NT];
 #pragma unroll
           for (int kk = 0; kk < NT; ++kk) orig[kk] = __ldg(f.tree_orig + first + min(kk, n_act - 1));
-          bool wide = NT == 4 && n_act == NT && (orig[0] & 3) == 0 && (f.n_trees & 3) == 0 &&
-                      (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
+          bool quad = NT == 4 && n_act == NT;
 #pragma unroll
-          for (int kk = 1; kk < NT; ++kk) wide = wide && orig[kk] == orig[0] + kk;
+          for (int kk = 1; kk < NT; ++kk) quad = quad && orig[kk] == orig[0] + kk;
+          const bool wide = quad && (orig[0] & 3) == 0 && (f.n_trees & 3) == 0 &&
+                            (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
           if (wide) {
             if (row < p.n_rows) {
               uint32_t* dst = static_cast<uint32_t*>(p.out) + row * f.n_trees + orig[0];
               *reinterpret_cast<uint4*>(dst) =
                 make_uint4(id[0], id[NT > 1 ? 1 : 0], id[NT > 2 ? 2 : 0], id[NT > 3 ? 3 : 0]);
             }
+          } else if (quad) {
+            store_quads<uint32_t>(static_cast<uint32_t*>(p.out), f.n_trees, row, p.n_rows, orig[0], id[0],
+                                  id[NT > 1 ? 1 : 0], id[NT > 2 ? 2 : 0], id[NT > 3 ? 3 : 0]);
           } else {
 #pragma unroll
             for (int kk = 0; kk < NT; ++kk) {
@@ -460,16 +464,17 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
           for (int kk = 0; kk < NT; ++kk) {
             pay[kk] = __ldg(static_cast<const Val*>(f.c_leaf_payload) + L[kk]);
           }
-          bool wide = false;
+          bool quad = false, wide = false;
           int first_orig = 0;
           if (MODE == MODE_PERTREE) {
-            // per-tree scalar outputs: the same 16-byte stores as for leaf ids
+            // per-tree scalar outputs: the same stores as for leaf ids
             first_orig = __ldg(f.tree_orig + first);
-            wide = NT == 4 && n_act == NT && f.leaf_vector_len <= 1 && (first_orig & 3) == 0 &&
-                   (f.n_trees & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
+            quad       = NT == 4 && n_act == NT && f.leaf_vector_len <= 1;
 #pragma unroll
             for (int kk = 1; kk < NT; ++kk)
-              wide = wide && __ldg(f.tree_orig + first + min(kk, n_act - 1)) == first_orig + kk;
+              quad = quad && __ldg(f.tree_orig + first + min(kk, n_act - 1)) == first_orig + kk;
+            wide = quad && (first_orig & 3) == 0 && (f.n_trees & 3) == 0 &&
+                   (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
           }
           if (MODE == MODE_PERTREE && wide) {
             if (row < p.n_rows) {
@@ -483,6 +488,9 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
                                                                           pay[NT > 3 ? 3 : 0]);
               }
             }
+          } else if (MODE == MODE_PERTREE && quad) {
+            store_quads<Val>(static_cast<Val*>(p.out), f.n_trees, row, p.n_rows, first_orig, pay[0],
+                             pay[NT > 1 ? 1 : 0], pay[NT > 2 ? 2 : 0], pay[NT > 3 ? 3 : 0]);
           } else {
 #pragma unroll
             for (int kk = 0; kk < NT; ++kk) {

@@ -22,3 +22,15 @@ def test_small_batches_split_over_clusters(kw, storage, precision):
         X = random_rows(n, n, desc.n_features, "float64", nan_frac=0.03,
                         categories=22 if kw.get("categorical") else None)
         _all_kinds(desc, X, precision, "depth_first", storage)
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("n_trees", [4, 7, 29, 30])
+def test_one_output_per_tree_at_every_alignment(n_trees, precision):
+    """Leaf ids and per-tree outputs leave as 16-byte stores, four lanes at a time or one by one,
+    whatever the tree count and wherever the batch ends inside a group of four rows."""
+    for storage, depth in (("dense", 4), ("dense", 7), ("sparse", 9)):
+        desc = random_forest_desc(92, n_trees=n_trees, n_features=9, max_depth=depth, p_leaf=0.05)
+        for n in (11_001, 11_002, 11_003):
+            _all_kinds(desc, random_rows(n, n, 9, "float64", nan_frac=0.02), precision,
+                       "depth_first", storage)
