@@ -112,12 +112,12 @@ struct HostPipeCfg {
   // rows predicted by one launch: pinned arrays, and pageable arrays, which are staged
   size_t block_bytes        = size_t(256) << 20;
   size_t staged_block_bytes = size_t(64) << 20;
-  int slots                 = 3;  // such blocks in flight
+  int slots                 = 4;  // such blocks in flight
   int copy_threads          = 0;
   HostPipeCfg()
   {
     const unsigned hw = std::thread::hardware_concurrency();
-    copy_threads      = static_cast<int>(std::max(1u, std::min(8u, hw / 2)));
+    copy_threads      = static_cast<int>(std::max(1u, std::min(6u, hw / 2)));
     auto number = [](const char* name, long lo, long hi, auto set) {
       const char* e = getenv(name);
       if (!e) return;
@@ -486,7 +486,7 @@ void copy_rows(char* dst, const char* src, int64_t n_rows, size_t row_bytes, siz
 // Host-array prediction, in one of three ways by the size of the input:
 //  in_place (up to 16 KiB): the kernel reads its rows over the link and writes its results back over
 //    it; pinned host memory is mapped, and no copy starts as fast as that.
-//  short_call (up to 8 MiB): a kernel fetches the rows from pinned memory, piece by piece while the
+//  short_call (up to 16 MiB): a kernel fetches the rows from pinned memory, piece by piece while the
 //    copy threads fill the next one.  Between kernels of a stream there is about a microsecond; a
 //    copy-engine transfer costs 5 us to start and again to hand over (1,000 rows of 50 features:
 //    46 -> 30 us).
@@ -538,7 +538,7 @@ class HostPrediction {
  private:
   static constexpr size_t kInPlaceIn  = size_t(16) << 10;
   static constexpr size_t kInPlaceOut = size_t(64) << 10;
-  static constexpr size_t kShortIn    = size_t(8) << 20;
+  static constexpr size_t kShortIn    = size_t(16) << 20;
   static constexpr size_t kShortOut   = size_t(256) << 10;  // results that the kernel writes to the host itself
   static constexpr size_t kPerTreeOut = size_t(2) << 10;
   static constexpr size_t kChunkMax   = size_t(4) << 20;
@@ -817,6 +817,7 @@ int b2fil_forest_create(const b2fil_forest_desc* desc, const b2fil_create_opts* 
       add_upload(list, pf.q_nodes_nan, offsetof(ForestView, q_nodes_nan));
       add_upload(list, pf.q_blob, offsetof(ForestView, q_blob));
       add_upload(list, pf.q_groups, offsetof(ForestView, q_groups));
+      add_upload(list, pf.q_bundles, offsetof(ForestView, q_bundles));
       f->q_top = std::move(pf.q_top);
     }
     if ((rc = upload_all(f.get(), list)) != B2FIL_OK) return rc;

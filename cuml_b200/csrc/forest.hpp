@@ -129,6 +129,16 @@ struct QGroup {        // 32 bytes
   uint32_t steps;      // halvings of the window search, shared by the group's features
   uint32_t pad[3];
 };
+// What one CTA of the pre-pass ranks: consecutive groups with at most kQMaxGroupFeatures features and
+// one CTA's shared memory in all (a tail of 28 features is groups of 16, 8 and 4).  The CTA's threads
+// are dealt evenly to `width` features (a power of two, the last few may be missing), its tables come
+// with one bulk copy.
+struct QBundle {        // 32 bytes
+  uint32_t first_group, n_groups;
+  uint32_t blob_off, blob_bytes;
+  uint32_t width, n_features;
+  uint32_t pad[2];
+};
 constexpr uint32_t Q_NAN_CODE      = 0x3FFFu;
 constexpr uint32_t Q_NAN_LEFT_BIT  = 0x4000u;  // set in the NaN codes of the second set of columns
 constexpr uint32_t Q_MAX_RANK      = 0x3FFEu;
@@ -250,7 +260,7 @@ struct ForestView {
   double ratio_c;
   // rank-quantised copy of a dense forest (q_enabled != 0)
   int32_t q_enabled;
-  int32_t q_n_groups;
+  int32_t q_n_bundles;
   int32_t q_has_cat;            // 1: tree blocks carry a third array of 32-bit category sets
   int32_t q_trees_in_order;     // 1: packed tree t is the caller's tree t (tree_orig is the identity)
   int32_t q_leaf_bytes;         // bytes per leaf payload: the element size (scalar, or index of the
@@ -264,9 +274,12 @@ struct ForestView {
                                 // what the traversal streams when it reports leaf ids
   const void* q_nodes_nan;      // q_nodes for tiles with missing values and doubled columns (see
                                 // above), or null
-  int64_t q_max_blob_bytes;     // largest group blob
+  int64_t q_max_blob_bytes;     // largest bundle of group blobs
+  int32_t q_bundle_features;    // features of the widest bundle
+  int32_t q_last_features;      // features of the last one
   const unsigned char* q_blob;  // group blobs
-  const QGroup* q_groups;       // [q_n_groups]
+  const QGroup* q_groups;
+  const QBundle* q_bundles;     // [q_n_bundles]
   // compact image of a sparse forest (c_enabled != 0), see above
   int32_t c_enabled;
   int32_t c_top_levels;         // T
@@ -307,6 +320,7 @@ struct PackedForest {
   std::vector<uint16_t> q_lut;
   std::vector<QFeature> q_feats;
   std::vector<QGroup> q_groups;
+  std::vector<QBundle> q_bundles;
   std::vector<uint8_t> q_blob;
   std::vector<uint32_t> c_nodes;          // two words per internal node
   std::vector<uint32_t> c_leaves_before;  // L of every internal node (host only: the exits carry it)

@@ -298,116 +298,123 @@ __device__ __forceinline__ void for_each_constant(F&& f, std::integer_sequence<i
   (f(std::integral_constant<int, Ks>{}), ...);
 }
 
-// One CTA owns one feature group: the group's blob (feature records, bucket tables, sorted
-// thresholds, both tables interleaved across the group's features) arrives in shared memory with
-// one bulk copy, then the CTA loops over row tiles.  The group size GF is a power of two that
-// divides the thread count, so a thread keeps one feature for good (its record sits in registers)
-// and with 32-feature groups a warp reads 128 contiguous bytes of one row per load and its 32
-// table lookups never share a bank.  A thread owns NU consecutive slots of the rank tile (slot =
-// q_slot(row)); it ranks them four at a time while the loads of its next tile are in flight,
-// packs the ranks two per word and writes its piece of Q[tile][feature][slot] (uint16) with one
-// vector store, the layout the traversal kernel pulls into shared memory with a single bulk
-// copy.  Nothing is exchanged between threads, so the tile loop has no barrier.  NaN becomes
-// Q_NAN_CODE and raises the tile's flag.
-// Shared memory: [mbarrier 16 B][blob].
+// One CTA owns a bundle of feature groups (usually one group of 32 features; a narrow tail is several
+// groups, dealt to its warps): the groups' blobs (feature records, bucket tables, sorted thresholds,
+// both tables interleaved across the group's features) arrive in shared memory with one bulk copy,
+// then the CTA loops over row tiles.  The group size GF is a power of two, so a thread keeps one
+// feature for good (its record sits in registers) and with 32-feature groups a warp reads 128
+// contiguous bytes of one row per load and its 32 table lookups never share a bank.  A thread owns NU
+// consecutive slots of the rank tile (slot = q_slot(row)), packs their ranks two per word and writes
+// its piece of Q[tile][feature][slot] (uint16) with one vector store, the layout the traversal kernel
+// pulls into shared memory with a single bulk copy.  Groups or tiles too small to occupy the CTA's
+// threads that way are ranked several tiles at a time.  Nothing is exchanged between threads, so the
+// tile loop has no barrier.
+// Bound by issue slots: 46 instructions per 32 values in the first version, of which the search
+// (table entry, four halvings) is 17.  So values are ranked where they were loaded (the next tile's
+// load follows in the same registers), the conversion to a bucket saturates instead of clamping,
+// ranks are made relative two at a time, and NaN and categories are fixed up off the common path.
+// Shared memory: [mbarrier 16 B][blobs].
 
 // Where the pre-pass reports NaN and what it clears for the traversal.
 struct QFlags {
-  uint8_t* bytes;     // [tile][group][32 warps], each written by its warp; or
+  // [tile][n_features, rounded up to a multiple of 4]: a group reports in the bytes of its features;
+  // every byte is written, nothing has to be zeroed beforehand; or
+  uint8_t* bytes;
   int32_t* words;     // one word per tile, zeroed by the caller
   int32_t* arrived;   // counters of shared row tiles to zero, one per tile, or null
 };
 
-// NU = slots of a tile each thread owns (R * GF / threads, at least 1).  GFC > 0 fixes the group
-// size at compile time (table strides become immediates), GFC == 0 reads it from the group.
+// Bucket of a value, the same as q_bucket_host: fma, truncation that saturates at zero (also for NaN),
+// clamp to the last bucket.
+__device__ __forceinline__ uint32_t q_bucket(float x, float scale, float offset, uint32_t last)
+{
+  return min(__float2uint_rz(fmaf(x, scale, offset)), last);
+}
+__device__ __forceinline__ uint32_t q_bucket(double x, double scale, double offset, uint32_t last)
+{
+  // (a double NaN would not convert to zero)
+  return min(__double2uint_rz(fmax(fma(x, scale, offset), 0.0)), last);
+}
+
+// GFC > 0 fixes the group size at compile time (table strides become immediates), GFC == 0 reads it
+// from the group.  `tid`: the thread's number among those of its group; `tiles_par`: tiles that the
+// CTA ranks at a time; it takes every `step`-th batch of them.
 template <typename T, int STEPS, int NU, int GFC>
 __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGroup& grp,
                                                uint16_t* __restrict__ Q, const QFlags& flags, int R,
-                                               uint32_t blob_a, const QFeatRec* rec)
+                                               uint32_t blob_a, const QFeatRec* rec, int tid,
+                                               int step, int tiles_par)
 {
   using TR               = Traits<T>;
-  constexpr int CH       = NU < 4 ? NU : 4;  // values ranked side by side
-  constexpr int NCH      = NU / CH;
+  constexpr int CH       = 4;  // values ranked side by side
   const int GF           = GFC > 0 ? GFC : static_cast<int>(grp.f_end - grp.f_begin);
-  const int tid          = threadIdx.x;
   const int gshift       = 31 - __clz(GF);
   const int i            = tid & (GF - 1);
-  const uint32_t s0      = static_cast<uint32_t>(tid >> gshift) * NU;  // first slot of the thread
-  const bool active      = s0 < static_cast<uint32_t>(R);  // false only when a tile has fewer values than threads
+  const int per_tile     = R * GF / NU;  // threads of a tile, a power of two
+  const int sub          = tid >> (31 - __clz(per_tile));
+  const int in_tile      = tid & (per_tile - 1);
+  const uint32_t s0      = static_cast<uint32_t>(in_tile >> gshift) * NU;  // first slot of the thread
   const QFeatRec mine    = rec[i];
   const T scale          = static_cast<T>(mine.scale);
   const T offset         = static_cast<T>(mine.offset);
-  const T nbm1           = static_cast<T>(mine.nbm1);
+  const uint32_t last    = mine.nbm1;
   const uint32_t lut_row = static_cast<uint32_t>(GF) * 2u;      // bytes between table entries
   const uint32_t thr_row = static_cast<uint32_t>(GF) * TR::ES;  // bytes between thresholds
   const int eshift       = gshift + (TR::ES == 4 ? 2 : 3);      // log2(thr_row)
   const uint32_t lut     = blob_a + mine.lut_off;
   const uint32_t thr_m1  = blob_a + mine.thr_off - thr_row;
+  const uint32_t zero2   = (thr_m1 >> eshift) * 0x10001u;  // two ranks of 0, before they are made relative
   const bool any_cat     = __any_sync(0xffffffffu, mine.is_cat != 0);
-  const int64_t tile_elems = static_cast<int64_t>(p.f.n_features) * R;  // ranks per tile
-  const uint32_t q_mine  = (grp.f_begin + i) * static_cast<uint32_t>(R) + s0;  // thread's first rank in a tile
-  const int64_t n_tiles  = (p.n_rows + R - 1) / R;
-  // slots s0 + j, j = 0..NU-1, hold rows b + (j >> 1) + 32 * (j & 1) (NU >= 2 implies R >= 64 and
-  // an even s0); element offsets inside a tile fit 32 bits (the host sizes row chunks accordingly)
-  const uint32_t b       = q_row_of_slot(s0, R);
-  const uint32_t e1      = static_cast<uint32_t>(p.row_stride);
-  const uint32_t e32     = e1 * 32u;
-  const uint32_t e_mine  = b * e1 + grp.f_begin + i;
-  const T* X             = static_cast<const T*>(p.X);
-
-  // one lane per warp reports NaN in a byte of its own: nothing has to be zeroed beforehand
-  uint8_t* my_flag = nullptr;
-  if (flags.bytes != nullptr && (tid & 31) == 0)
-    my_flag = flags.bytes + (static_cast<int64_t>(blockIdx.x) * gridDim.y + blockIdx.y) * 32 + (tid >> 5);
-  const uint32_t flag_step = gridDim.x * gridDim.y * 32u;
+  const uint32_t tile_elems = static_cast<uint32_t>(p.f.n_features) * R;  // ranks per tile
+  const int n_rows       = static_cast<int>(p.n_rows);  // a chunk of the batch
+  const int n_tiles      = (n_rows + R - 1) / R;
+  const int stride       = step * tiles_par;  // tiles between two rounds of the CTA
+  // slots s0 + j, j = 0..NU-1, hold rows b + (j >> 1) * pair + (j & 1) * odd (see q_slot)
+  const int b            = static_cast<int>(q_row_of_slot(s0, R));
+  const int pair         = R >= 64 ? 1 : 2;
+  const int odd          = R >= 64 ? 32 : 1;
+  int base               = blockIdx.x * tiles_par;  // first tile of the round
+  const T* src  = static_cast<const T*>(p.X) +
+                 (static_cast<int64_t>(base + sub) * R + b) * p.row_stride + grp.f_begin + i;
+  uint16_t* dst = Q + static_cast<int64_t>(base + sub) * tile_elems + (grp.f_begin + i) * R + s0;
+  const uint32_t rs      = static_cast<uint32_t>(p.row_stride);  // below 2^22: offsets inside a tile fit 32 bits
+  const int64_t advance  = static_cast<int64_t>(stride) * R * p.row_stride;
 
   T xs[NU];
-  // loads chunk c (slots s0 + c * CH ...) of tile t
-  auto fetch = [&](int64_t t, int c) {
-    const int64_t row0 = t * R;
-    const T* tb        = X + row0 * p.row_stride;  // same for the whole CTA
-    const uint32_t cb  = e_mine + static_cast<uint32_t>(c * (CH / 2)) * e1;
-    if (row0 + R <= p.n_rows) {
+  // loads chunk c (slots s0 + c * CH ...) of the round that starts at tile `first`
+  auto fetch = [&](const T* at, int first, int c) {
+    if (first + tiles_par <= n_rows / R) {
 #pragma unroll
-      for (int u = 0; u < CH; ++u)
-        xs[c * CH + u] = active ? TR::ldg_here(tb + (cb + (u >> 1) * e1 + (u & 1) * e32)) : T(0);
+      for (int j = c * CH; j < c * CH + CH; ++j)
+        xs[j] = TR::ldg_here(at + static_cast<uint32_t>((j >> 1) * pair + (j & 1) * odd) * rs);
     } else {
+      const int row = (first + sub) * R + b;
 #pragma unroll
-      for (int u = 0; u < CH; ++u) {
-        const int64_t row = row0 + b + c * (CH / 2) + (u >> 1) + 32 * (u & 1);
-        xs[c * CH + u] =
-          (active && row < p.n_rows) ? TR::ldg_here(tb + (cb + (u >> 1) * e1 + (u & 1) * e32)) : T(0);
+      for (int j = c * CH; j < c * CH + CH; ++j) {
+        const int off = (j >> 1) * pair + (j & 1) * odd;
+        xs[j] = row + off < n_rows ? TR::ldg_here(at + static_cast<uint32_t>(off) * rs) : T(0);
       }
     }
   };
-  if (blockIdx.x < n_tiles) {
+  if (base < n_tiles) {
 #pragma unroll
-    for (int c = 0; c < NCH; ++c) fetch(blockIdx.x, c);
+    for (int c = 0; c < NU / CH; ++c) fetch(src, base, c);
   }
-  for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-    uint32_t packed[NU > 1 ? NU / 2 : 1];
+  for (; base < n_tiles; base += stride) {
+    src += advance;
+    uint32_t packed[NU / 2];
     bool saw_nan = false;
 #pragma unroll
-    for (int c = 0; c < NCH; ++c) {
-      T cur[CH];
-#pragma unroll
-      for (int u = 0; u < CH; ++u) cur[u] = xs[c * CH + u];
-      // the same chunk of the CTA's next tile is requested right away, so a whole tile of loads
-      // per thread stays in flight (an additional L2 prefetch further ahead measured slower)
-      if (t + gridDim.x < n_tiles) fetch(t + gridDim.x, c);
+    for (int c = 0; c < NU / CH; ++c) {
+      const T* cur = xs + c * CH;
       // rank of the CH values, step by step across all of them so that the dependent
       // shared-memory lookups of different values overlap.  A NaN walks the same code (bucket 0,
       // every comparison false) and is replaced by Q_NAN_CODE at the end; so does a categorical
       // value (its feature has empty tables), replaced by its category.
       uint32_t a[CH];  // address of the threshold below the current window
 #pragma unroll
-      for (int u = 0; u < CH; ++u) {
-        // same expression as q_bucket_host: fma, clamp (NaN becomes 0), truncate
-        T v = fma(cur[u], scale, offset);
-        v   = fmax(v, T(0));
-        v   = fmin(v, nbm1);
-        a[u] = (lds_u16(lut + static_cast<uint32_t>(v) * lut_row) << eshift) + thr_m1;
-      }
+      for (int u = 0; u < CH; ++u)
+        a[u] = (lds_u16(lut + q_bucket(cur[u], scale, offset, last) * lut_row) << eshift) + thr_m1;
       if (STEPS > 0 && GFC > 0) {
         // group size and step count known: the probe offsets are immediates of the loads
         for_each_constant(
@@ -438,56 +445,58 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
           for (int u = 0; u < CH; ++u) TR::add_if_le(a[u], TR::ld_real(a[u] + s_b), cur[u], s_b);
         }
       }
-      uint32_t code[CH];
+      uint32_t* two = packed + c * (CH / 2);
+      bool special  = any_cat;
 #pragma unroll
-      for (int u = 0; u < CH; ++u) code[u] = (a[u] - thr_m1) >> eshift;
-      if (any_cat) {
-        // groups with categorical features only (the warp-wide barrier keeps this a real branch
-        // instead of conversions and selects that every group would execute): the code of a
-        // categorical value is the category itself (truncated value); negative and huge values
-        // match no listed category
-        __syncwarp();
+      for (int u = 0; u < CH; u += 2) {
+        two[u >> 1] = ((a[u + 1] >> eshift) << 16) + (a[u] >> eshift) - zero2;
+        special     = special || cur[u] != cur[u] || cur[u + 1] != cur[u + 1];
+      }
+      if (__any_sync(0xffffffffu, special)) {
 #pragma unroll
         for (int u = 0; u < CH; ++u) {
-          const bool in_range = (cur[u] >= T(0)) && (cur[u] < T(Q_NO_CATEGORY));
-          if (mine.is_cat) code[u] = in_range ? static_cast<uint32_t>(cur[u]) : Q_NO_CATEGORY;
+          const T x     = cur[u];
+          uint32_t code = (two[u >> 1] >> (16 * (u & 1))) & 0xffffu;
+          // the code of a categorical value is the category itself (truncated value); negative and
+          // huge values match no listed category
+          if (mine.is_cat)
+            code = (x >= T(0)) && (x < T(Q_NO_CATEGORY)) ? static_cast<uint32_t>(x) : Q_NO_CATEGORY;
+          if (x != x) {
+            code    = Q_NAN_CODE;
+            saw_nan = true;
+          }
+          two[u >> 1] = (u & 1) ? (two[u >> 1] & 0xffffu) | (code << 16) : (two[u >> 1] & 0xffff0000u) | code;
         }
       }
-#pragma unroll
-      for (int u = 0; u < CH; ++u) {
-        const bool is_nan = cur[u] != cur[u];
-        saw_nan |= is_nan;
-        const uint32_t cd = is_nan ? Q_NAN_CODE : code[u];
-        const int j       = c * CH + u;
-        if (NU == 1) {
-          packed[0] = cd;
-        } else if (j & 1) {
-          packed[j >> 1] |= cd << 16;
-        } else {
-          packed[j >> 1] = cd;
-        }
-      }
+      // the same chunk of the CTA's next round goes into the registers just read, so a whole round of
+      // loads per thread stays in flight (an additional L2 prefetch further ahead measured slower)
+      if (base + stride < n_tiles) fetch(src, base + stride, c);
     }
+    const bool live = base + sub < n_tiles;
     // Q[tile][feature][slot]: the thread's NU consecutive slots of its feature in one store
-    if (active) {
-      uint16_t* dst = Q + t * tile_elems + q_mine;
-      if (NU == 8) {
-        *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[NU > 2 ? 1 : 0],
-                                                    packed[NU > 4 ? 2 : 0], packed[NU > 6 ? 3 : 0]);
-      } else if (NU == 4) {
-        *reinterpret_cast<uint2*>(dst) = make_uint2(packed[0], packed[NU > 2 ? 1 : 0]);
-      } else if (NU == 2) {
-        *reinterpret_cast<uint32_t*>(dst) = packed[0];
+    if (live) {
+      if constexpr (NU == 8) {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[NU > 4 ? 2 : 0], packed[NU > 4 ? 3 : 0]);
       } else {
-        *dst = static_cast<uint16_t>(packed[0]);
+        *reinterpret_cast<uint2*>(dst) = make_uint2(packed[0], packed[1]);
       }
     }
-    const bool warp_nan = __any_sync(0xffffffffu, saw_nan);
-    if (my_flag != nullptr) {
-      *my_flag = warp_nan ? 1 : 0;
-      my_flag += flag_step;
-    } else if (flags.words != nullptr && warp_nan && (tid & 31) == 0) {
-      atomicOr(flags.words + t, 1);
+    dst += static_cast<int64_t>(stride) * tile_elems;
+    // NaN flags.  The lanes of a warp rank one tile, or (groups of few features) several
+    const uint32_t nan_lanes = __ballot_sync(0xffffffffu, saw_nan);
+    if (flags.bytes != nullptr) {
+      const int lanes = min(32, per_tile);
+      if ((in_tile & (lanes - 1)) == 0 && live) {
+        const uint32_t mask = lanes == 32 ? 0xffffffffu : ((1u << lanes) - 1u) << (tid & 31);
+        const int n         = max(1, lanes * GF / per_tile);  // bytes: the lanes' share of the group's
+        uint8_t* at = flags.bytes + static_cast<int64_t>(base + sub) * ((p.f.n_features + 3) & ~3) +
+                      grp.f_begin + in_tile / lanes * n;
+        for (int k = 0; k < n; ++k) at[k] = (nan_lanes & mask) != 0u ? 1 : 0;
+        if (grp.f_end == static_cast<uint32_t>(p.f.n_features) && in_tile == 0)
+          for (uint32_t k = grp.f_end; k & 3u; ++k) at[k - grp.f_begin] = 0;  // the padding
+      }
+    } else if (saw_nan) {
+      flags.words[base + sub] = 1;
     }
   }
 }
@@ -495,69 +504,87 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
 template <typename T, int STEPS>
 __device__ __forceinline__ void quantise_rows(const PredictParams& p, const QGroup& grp,
                                               uint16_t* __restrict__ Q, const QFlags& flags, int R,
-                                              uint32_t blob_a, const QFeatRec* rec)
+                                              uint32_t blob_a, const QFeatRec* rec, int tid, int step,
+                                              int slots, int tiles_par)
 {
-  const int GF         = static_cast<int>(grp.f_end - grp.f_begin);
-  const int per_thread = (R * GF) / static_cast<int>(blockDim.x);
   // full-width groups on large tiles, the shape of big batches, get the group size baked in
-  if (GF == 32 && STEPS >= 2 && per_thread == 8) {
-    quantise_tiles<T, STEPS, 8, 32>(p, grp, Q, flags, R, blob_a, rec);
-    return;
-  }
-  switch (per_thread) {
-    case 8: quantise_tiles<T, STEPS, 8, 0>(p, grp, Q, flags, R, blob_a, rec); break;
-    case 4: quantise_tiles<T, STEPS, 4, 0>(p, grp, Q, flags, R, blob_a, rec); break;
-    case 2: quantise_tiles<T, STEPS, 2, 0>(p, grp, Q, flags, R, blob_a, rec); break;
-    default: quantise_tiles<T, STEPS, 1, 0>(p, grp, Q, flags, R, blob_a, rec); break;
+  if (grp.f_end - grp.f_begin == 32 && STEPS >= 2 && slots == 8) {
+    quantise_tiles<T, STEPS, 8, 32>(p, grp, Q, flags, R, blob_a, rec, tid, step, tiles_par);
+  } else if (slots == 8) {
+    quantise_tiles<T, STEPS, 8, 0>(p, grp, Q, flags, R, blob_a, rec, tid, step, tiles_par);
+  } else {
+    quantise_tiles<T, STEPS, 4, 0>(p, grp, Q, flags, R, blob_a, rec, tid, step, tiles_par);
   }
 }
 
 template <typename T>
 __global__ void __launch_bounds__(1024, 1)
 quantise_kernel(const __grid_constant__ PredictParams p, uint16_t* __restrict__ Q, const QFlags flags,
-                const int R)
+                const int R, const int slots, const int last_ctas)
 {
   extern __shared__ __align__(128) unsigned char smem[];
   const ForestView& f   = p.f;
-  const QGroup grp      = f.q_groups[blockIdx.y];
   const uint32_t bar    = smem_addr(smem);
   unsigned char* blob   = smem + 16;
   const uint32_t blob_a = smem_addr(blob);
-  const QFeatRec* rec   = reinterpret_cast<const QFeatRec*>(blob);
-
+  const QBundle bundle  = f.q_bundles[blockIdx.y];
+  const int64_t n_tiles = (p.n_rows + R - 1) / R;
+  // every feature has 1024 / width threads and every thread `slots` slots of a tile
+  const int threads_per_feature = 1024 / static_cast<int>(bundle.width);
+  const int tiles_par           = threads_per_feature * slots / R;
+  // the last bundle may have fewer features, and then takes fewer CTAs
+  const int step = blockIdx.y + 1 == gridDim.y ? last_ctas : static_cast<int>(gridDim.x);
+  if (static_cast<int>(blockIdx.x) >= step || static_cast<int64_t>(blockIdx.x) * tiles_par >= n_tiles) return;
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     mbar_fence_init();
-    mbar_expect_tx(bar, grp.blob_bytes);
-    bulk_copy_g2s(blob_a, f.q_blob + grp.blob_off, grp.blob_bytes, bar);
+    mbar_expect_tx(bar, bundle.blob_bytes);
+    bulk_copy_g2s(blob_a, f.q_blob + bundle.blob_off, bundle.blob_bytes, bar);
   }
+  // which of the bundle's groups is the thread's?
+  int tid       = threadIdx.x;  // the thread's number among those of its group
+  QGroup grp    = f.q_groups[bundle.first_group];
+  int n_threads = static_cast<int>(grp.f_end - grp.f_begin) * threads_per_feature;
+  bool idle     = false;
+  for (uint32_t i = 1; tid >= n_threads; ++i) {
+    if (i == bundle.n_groups) {
+      idle = true;  // the width is rounded up to a power of two
+      break;
+    }
+    tid -= n_threads;
+    grp       = f.q_groups[bundle.first_group + i];
+    n_threads = static_cast<int>(grp.f_end - grp.f_begin) * threads_per_feature;
+  }
+  const uint32_t group_at = grp.blob_off - bundle.blob_off;
+  const QFeatRec* rec     = reinterpret_cast<const QFeatRec*>(blob + group_at);
   __syncthreads();
   grid_release();
   grid_wait();  // the tables are part of the forest; rows and scratch may still be in use
   // while the tables arrive, ask the L2 for the rows of the CTA's first tile
   if (threadIdx.x < R) {
-    const int64_t row = static_cast<int64_t>(blockIdx.x) * R + threadIdx.x;
+    const int64_t row = static_cast<int64_t>(blockIdx.x) * tiles_par * R + threadIdx.x;
     if (row < p.n_rows)
       asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const T*>(p.X) + row * p.row_stride + grp.f_begin));
   }
   if (flags.arrived != nullptr && blockIdx.y == 0) {
-    const int64_t n_tiles = (p.n_rows + R - 1) / R;
-    for (int64_t t = blockIdx.x * 1024ll + threadIdx.x; t < n_tiles; t += gridDim.x * 1024ll)
+    for (int64_t t = blockIdx.x * 1024ll + threadIdx.x; t < n_tiles; t += step * 1024ll)
       flags.arrived[t] = 0;
   }
+  if (idle) return;
   if (!mbar_wait(bar, 0)) {
     if (threadIdx.x == 0) report_status(p.status, 4);
     return;
   }
   // the number of halvings is fixed per group: pick the unrolled body once
+  const uint32_t tables = blob_a + group_at;
   switch (grp.steps) {
-    case 0: quantise_rows<T, 0>(p, grp, Q, flags, R, blob_a, rec); break;
-    case 1: quantise_rows<T, 1>(p, grp, Q, flags, R, blob_a, rec); break;
-    case 2: quantise_rows<T, 2>(p, grp, Q, flags, R, blob_a, rec); break;
-    case 3: quantise_rows<T, 3>(p, grp, Q, flags, R, blob_a, rec); break;
-    case 4: quantise_rows<T, 4>(p, grp, Q, flags, R, blob_a, rec); break;
-    case 5: quantise_rows<T, 5>(p, grp, Q, flags, R, blob_a, rec); break;
-    default: quantise_rows<T, -1>(p, grp, Q, flags, R, blob_a, rec); break;
+    case 0: quantise_rows<T, 0>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
+    case 1: quantise_rows<T, 1>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
+    case 2: quantise_rows<T, 2>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
+    case 3: quantise_rows<T, 3>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
+    case 4: quantise_rows<T, 4>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
+    case 5: quantise_rows<T, 5>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
+    default: quantise_rows<T, -1>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
   }
 }
 
@@ -1035,24 +1062,29 @@ int launch_dense_q_kernel(const QLaunch& L, int mode, bool f64, std::string& err
   return launch_q_generic(L, mode, f64, err);
 }
 
-// CTAs per feature group of the rank pre-pass.  Every CTA loads the tables of one group (about 200 KB
-// of an SM's 48 bytes per cycle from L2) and then ranks its share of the group's tiles; the SMs take
-// the grid in waves of one CTA each.  Taken is the count with the least estimated time,
-//   waves x (start and tables + tiles of a CTA x time per tile),
-// a warp ranking 32 values in 17.4 SM cycles (measured on 1 M rows of 256 features).  With large
-// batches many short CTAs fill the last wave (64 groups on 148 SMs: 37 CTAs per group), with
-// 20,000 rows loading the tables twice on an SM costs more than it evens out.
-int quantise_ctas_per_group(const ForestView& f, int R, int sm_count, int64_t n_tiles)
+// CTAs per bundle of the rank pre-pass.  Every CTA loads the tables of one bundle of feature groups
+// (about 200 KB of an SM's 48 bytes per cycle from L2) and then ranks its share of the row tiles; the
+// SMs take the grid in waves of one CTA each.  Taken is the count with the least estimated time,
+//   waves x (start and tables + rounds of a CTA x time per round),
+// a warp ranking 32 values in kRankCycles SM cycles (measured on 1 M rows of 256 features).  With large
+// batches many short CTAs fill the last wave (64 bundles on 148 SMs: 37 CTAs each), with 20,000 rows
+// loading the tables twice on an SM costs more than it evens out.
+constexpr double kRankCycles = 14.0;
+int quantise_ctas_per_bundle(const ForestView& f, int R, int slots, int sm_count, int64_t n_tiles)
 {
-  const int n_groups   = std::max(1, f.q_n_groups);
+  const double bundles = f.q_n_bundles - 1 + static_cast<double>(f.q_last_features) / f.q_bundle_features;
   const double tables  = 3000.0 + static_cast<double>(f.q_max_blob_bytes) / 48.0;
-  const double per_tile = 17.4 * R * f.n_features / n_groups / 32.0 + 100.0;
+  int width = 1;
+  while (width < f.q_bundle_features) width *= 2;
+  const int par          = 1024 / width * slots / R;  // tiles that a CTA ranks at a time
+  const int64_t n_rounds = (n_tiles + par - 1) / par;
+  const double per_round = kRankCycles * R * par * f.q_bundle_features / 32.0 + 100.0;
   int best = 1;
   double best_cost = 1e300;
-  const int most = static_cast<int>(std::min<int64_t>(n_tiles, std::max(48, sm_count / n_groups)));
+  const int most = static_cast<int>(std::min<double>(n_rounds, std::max(48.0, sm_count / bundles)));
   for (int gx = 1; gx <= most; ++gx) {
-    const int waves   = (gx * n_groups + sm_count - 1) / sm_count;
-    const double cost = waves * (tables + static_cast<double>((n_tiles + gx - 1) / gx) * per_tile);
+    const int waves   = (static_cast<int>(std::ceil(gx * bundles)) + sm_count - 1) / sm_count;
+    const double cost = waves * (tables + static_cast<double>((n_rounds + gx - 1) / gx) * per_round);
     if (cost < best_cost * 0.995) {  // ties and near ties: fewer CTAs
       best_cost = cost;
       best      = gx;
@@ -1067,12 +1099,17 @@ int launch_quantise(const PredictParams& p, uint16_t* Q, const QFlags& flags, in
                     int sm_count, cudaStream_t stream, std::string& err)
 {
   const ForestView& f = p.f;
-  // shared memory: mbarrier and the largest group blob
+  // shared memory: mbarrier and the largest bundle of tables
   const size_t smem = 16 + static_cast<size_t>(f.q_max_blob_bytes);
-  const int gx      = quantise_ctas_per_group(f, R, sm_count, (p.n_rows + R - 1) / R);
-  const SplitLaunch l{dim3(gx, f.q_n_groups), 1024, smem, stream, 1, true};
-  return f64 ? launch_split(l, err, quantise_kernel<double>, p, Q, flags, R)
-             : launch_split(l, err, quantise_kernel<float>, p, Q, flags, R);
+  // Eight ranks per thread and store; four where tiles are small and so few that the CTAs have one
+  // round of them each: there the time of one thread counts.
+  const int64_t n_tiles = (p.n_rows + R - 1) / R;
+  const int slots       = R <= 128 && n_tiles * f.q_n_bundles <= sm_count ? 4 : 8;
+  const int gx          = quantise_ctas_per_bundle(f, R, slots, sm_count, n_tiles);
+  const int last        = (gx * f.q_last_features + f.q_bundle_features - 1) / f.q_bundle_features;
+  const SplitLaunch l{dim3(gx, f.q_n_bundles), 1024, smem, stream, 1, true};
+  return f64 ? launch_split(l, err, quantise_kernel<double>, p, Q, flags, R, slots, last)
+             : launch_split(l, err, quantise_kernel<float>, p, Q, flags, R, slots, last);
 }
 
 // Rank-quantised prediction: rows are processed in chunks of whole waves of tiles; for each
@@ -1118,7 +1155,7 @@ int launch_dense_q(const PredictParams& p, int mode, int chunk_size, int sm_coun
   const size_t q_bytes   = static_cast<size_t>(ch_tiles) * tile_b;
   const size_t sum_bytes =
     reduce ? align16(static_cast<size_t>(2 * sm_count) * f.n_outputs * R * es) : 0;
-  const int flag_words   = f.q_n_groups * 8;  // a byte per warp of the pre-pass
+  const int flag_words   = (f.n_features + 3) / 4;  // a byte per feature
   const size_t fl_bytes  = static_cast<size_t>(ch_tiles) * flag_words * 4;
   const size_t arr_bytes = reduce ? static_cast<size_t>(ch_tiles) * 4 : 0;
   const size_t need      = q_bytes + sum_bytes + fl_bytes + arr_bytes;

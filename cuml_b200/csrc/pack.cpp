@@ -392,6 +392,39 @@ struct Packer {
     return B2FIL_OK;
   }
 
+  // Consecutive feature groups that one CTA of the pre-pass takes together (see QBundle).
+  void bundle_groups()
+  {
+    out.q_bundles.clear();
+    out.view.q_max_blob_bytes = 0;
+    uint32_t widest           = 1;
+    for (size_t i = 0; i < out.q_groups.size();) {
+      QBundle b{};
+      b.first_group   = static_cast<uint32_t>(i);
+      b.blob_off      = out.q_groups[i].blob_off;
+      uint32_t n_feat = 0;
+      for (; i < out.q_groups.size(); ++i) {
+        const QGroup& g  = out.q_groups[i];
+        const uint32_t n = g.f_end - g.f_begin;
+        if (b.n_groups > 0 && (n_feat + n > kQMaxGroupFeatures ||
+                               b.blob_bytes + g.blob_bytes > kQGroupSmemBudget))
+          break;
+        n_feat += n;
+        b.blob_bytes += g.blob_bytes;
+        ++b.n_groups;
+      }
+      b.width = 1;
+      while (b.width < n_feat) b.width *= 2;
+      b.n_features              = n_feat;
+      widest                    = std::max(widest, n_feat);
+      out.view.q_max_blob_bytes = std::max<int64_t>(out.view.q_max_blob_bytes, b.blob_bytes);
+      out.q_bundles.push_back(b);
+    }
+    out.view.q_n_bundles       = static_cast<int32_t>(out.q_bundles.size());
+    out.view.q_bundle_features = static_cast<int32_t>(widest);
+    out.view.q_last_features   = static_cast<int32_t>(out.q_bundles.back().n_features);
+  }
+
   // ---- rank-quantised copy of a dense forest ----------------------------------------------------
   // Returns false (and leaves the forest unquantised) when a limit is exceeded.
   template <typename T>
@@ -558,10 +591,10 @@ struct Packer {
       }
       g.blob_bytes = static_cast<uint32_t>(blob.size());
       out.q_blob.insert(out.q_blob.end(), blob.begin(), blob.end());
-      out.view.q_max_blob_bytes = std::max<int64_t>(out.view.q_max_blob_bytes, g.blob_bytes);
       out.q_groups.push_back(g);
       f += n;
     }
+    bundle_groups();
     // 4. nodes: same heap layout as the dense blocks, 4 bytes per test node; in forests with
     //    categorical tests a node is 8 bytes {node, 32-bit category set}, so that one load brings
     //    both (a numerical node holds an empty set)
@@ -671,7 +704,6 @@ struct Packer {
     }
     out.view.q_has_cat     = has_cat ? 1 : 0;
     out.view.q_enabled     = 1;
-    out.view.q_n_groups    = static_cast<int32_t>(out.q_groups.size());
     out.view.q_tree_stride = qstride;
     out.view.q_leaf_bytes  = static_cast<int32_t>(lbytes);
     return true;
@@ -1137,6 +1169,7 @@ int pack_forest(const b2fil_forest_desc& desc, const b2fil_create_opts& opts,
       out.q_lut.clear();
       out.q_feats.clear();
       out.q_groups.clear();
+      out.q_bundles.clear();
       out.q_blob.clear();
       out.view.q_enabled        = 0;
       out.view.q_max_blob_bytes = 0;

@@ -34,3 +34,24 @@ def test_one_output_per_tree_at_every_alignment(n_trees, precision):
         for n in (11_001, 11_002, 11_003):
             _all_kinds(desc, random_rows(n, n, 9, "float64", nan_frac=0.02), precision,
                        "depth_first", storage)
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("n_features", [1, 2, 7, 28, 33, 61, 100])
+def test_rank_prepass_over_ragged_feature_groups(n_features, precision):
+    """Feature counts that make one wide group, narrow tails of several groups, and groups that are
+    ranked several tiles at a time; row tiles of every size, a partial last tile, NaN in some tiles
+    only, categories, thresholds that rows hit exactly, infinities."""
+    import numpy as np
+
+    desc = random_forest_desc(91, n_trees=61, n_features=n_features, max_depth=5, mixed_ops=True,
+                              categorical=n_features == 33, postproc="sigmoid")
+    thr = desc.threshold[desc.node_kind == 1]
+    for n, chunk in ((70, 1), (1000, 2), (1000, 4), (5001, 8), (12_007, 4), (12_007, 8)):
+        X = random_rows(n, n, n_features, np.float64, nan_frac=0.0,
+                        categories=22 if n_features == 33 else None)
+        X[: n // 3, 0] = np.resize(thr, n // 3)
+        X[n // 2, -1] = np.nan
+        X[-1, 0] = np.nan
+        X[1, 0], X[2, 0] = np.inf, -np.inf
+        _all_kinds(desc, X, precision, "depth_first", "dense", chunk_size=chunk)
