@@ -338,12 +338,12 @@ __device__ __forceinline__ uint32_t q_bucket(double x, double scale, double offs
 
 // GFC > 0 fixes the group size at compile time (table strides become immediates), GFC == 0 reads it
 // from the group.  `tid`: the thread's number among those of its group; `tiles_par`: tiles that the
-// CTA ranks at a time; it takes every `step`-th batch of them.
+// CTA ranks at a time; it takes batch `first` of them and every `step`-th one after.
 template <typename T, int STEPS, int NU, int GFC>
 __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGroup& grp,
                                                uint16_t* __restrict__ Q, const QFlags& flags, int R,
                                                uint32_t blob_a, const QFeatRec* rec, int tid,
-                                               int step, int tiles_par)
+                                               int first, int step, int tiles_par)
 {
   using TR               = Traits<T>;
   constexpr int CH       = 4;  // values ranked side by side
@@ -367,13 +367,15 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
   const bool any_cat     = __any_sync(0xffffffffu, mine.is_cat != 0);
   const uint32_t tile_elems = static_cast<uint32_t>(p.f.n_features) * R;  // ranks per tile
   const int n_rows       = static_cast<int>(p.n_rows);  // a chunk of the batch
-  const int n_tiles      = (n_rows + R - 1) / R;
+  const int rshift       = 31 - __clz(R);  // R is a power of two
+  const int n_tiles      = (n_rows + R - 1) >> rshift;
+  const int n_full       = n_rows >> rshift;  // without the partial one at the end
   const int stride       = step * tiles_par;  // tiles between two rounds of the CTA
   // slots s0 + j, j = 0..NU-1, hold rows b + (j >> 1) * pair + (j & 1) * odd (see q_slot)
   const int b            = static_cast<int>(q_row_of_slot(s0, R));
   const int pair         = R >= 64 ? 1 : 2;
   const int odd          = R >= 64 ? 32 : 1;
-  int base               = blockIdx.x * tiles_par;  // first tile of the round
+  int base               = first * tiles_par;  // first tile of the round
   const T* src  = static_cast<const T*>(p.X) +
                  (static_cast<int64_t>(base + sub) * R + b) * p.row_stride + grp.f_begin + i;
   uint16_t* dst = Q + static_cast<int64_t>(base + sub) * tile_elems + (grp.f_begin + i) * R + s0;
@@ -381,14 +383,14 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
   const int64_t advance  = static_cast<int64_t>(stride) * R * p.row_stride;
 
   T xs[NU];
-  // loads chunk c (slots s0 + c * CH ...) of the round that starts at tile `first`
-  auto fetch = [&](const T* at, int first, int c) {
-    if (first + tiles_par <= n_rows / R) {
+  // loads chunk c (slots s0 + c * CH ...) of the round that starts at `tile`
+  auto fetch = [&](const T* at, int tile, int c) {
+    if (tile + tiles_par <= n_full) {
 #pragma unroll
       for (int j = c * CH; j < c * CH + CH; ++j)
         xs[j] = TR::ldg_here(at + static_cast<uint32_t>((j >> 1) * pair + (j & 1) * odd) * rs);
     } else {
-      const int row = (first + sub) * R + b;
+      const int row = (tile + sub) * R + b;
 #pragma unroll
       for (int j = c * CH; j < c * CH + CH; ++j) {
         const int off = (j >> 1) * pair + (j & 1) * odd;
@@ -488,9 +490,10 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
       const int lanes = min(32, per_tile);
       if ((in_tile & (lanes - 1)) == 0 && live) {
         const uint32_t mask = lanes == 32 ? 0xffffffffu : ((1u << lanes) - 1u) << (tid & 31);
-        const int n         = max(1, lanes * GF / per_tile);  // bytes: the lanes' share of the group's
+        // bytes: the lanes' share of the group's, lanes * GF / per_tile = lanes * NU / R
+        const int n = per_tile < 32 ? GF : (32 * NU) >> rshift;
         uint8_t* at = flags.bytes + static_cast<int64_t>(base + sub) * ((p.f.n_features + 3) & ~3) +
-                      grp.f_begin + in_tile / lanes * n;
+                      grp.f_begin + (in_tile >> 5) * n;
         for (int k = 0; k < n; ++k) at[k] = (nan_lanes & mask) != 0u ? 1 : 0;
         if (grp.f_end == static_cast<uint32_t>(p.f.n_features) && in_tile == 0)
           for (uint32_t k = grp.f_end; k & 3u; ++k) at[k - grp.f_begin] = 0;  // the padding
@@ -504,37 +507,39 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
 template <typename T, int STEPS>
 __device__ __forceinline__ void quantise_rows(const PredictParams& p, const QGroup& grp,
                                               uint16_t* __restrict__ Q, const QFlags& flags, int R,
-                                              uint32_t blob_a, const QFeatRec* rec, int tid, int step,
-                                              int slots, int tiles_par)
+                                              uint32_t blob_a, const QFeatRec* rec, int tid, int first,
+                                              int step, int slots, int tiles_par)
 {
   // full-width groups on large tiles, the shape of big batches, get the group size baked in
   if (grp.f_end - grp.f_begin == 32 && STEPS >= 2 && slots == 8) {
-    quantise_tiles<T, STEPS, 8, 32>(p, grp, Q, flags, R, blob_a, rec, tid, step, tiles_par);
+    quantise_tiles<T, STEPS, 8, 32>(p, grp, Q, flags, R, blob_a, rec, tid, first, step, tiles_par);
   } else if (slots == 8) {
-    quantise_tiles<T, STEPS, 8, 0>(p, grp, Q, flags, R, blob_a, rec, tid, step, tiles_par);
+    quantise_tiles<T, STEPS, 8, 0>(p, grp, Q, flags, R, blob_a, rec, tid, first, step, tiles_par);
   } else {
-    quantise_tiles<T, STEPS, 4, 0>(p, grp, Q, flags, R, blob_a, rec, tid, step, tiles_par);
+    quantise_tiles<T, STEPS, 4, 0>(p, grp, Q, flags, R, blob_a, rec, tid, first, step, tiles_par);
   }
 }
 
 template <typename T>
 __global__ void __launch_bounds__(1024, 1)
 quantise_kernel(const __grid_constant__ PredictParams p, uint16_t* __restrict__ Q, const QFlags flags,
-                const int R, const int slots, const int last_ctas)
+                const int R, const int slots, const int ctas)
 {
   extern __shared__ __align__(128) unsigned char smem[];
   const ForestView& f   = p.f;
   const uint32_t bar    = smem_addr(smem);
   unsigned char* blob   = smem + 16;
   const uint32_t blob_a = smem_addr(blob);
-  const QBundle bundle  = f.q_bundles[blockIdx.y];
+  // `ctas` CTAs per bundle; the last one may have fewer features, and then takes what is left
+  const int which       = min(static_cast<int>(blockIdx.x) / ctas, f.q_n_bundles - 1);
+  const int first       = static_cast<int>(blockIdx.x) - which * ctas;
+  const int step        = which + 1 == f.q_n_bundles ? static_cast<int>(gridDim.x) - which * ctas : ctas;
+  const QBundle bundle  = f.q_bundles[which];
   const int64_t n_tiles = (p.n_rows + R - 1) / R;
   // every feature has 1024 / width threads and every thread `slots` slots of a tile
   const int threads_per_feature = 1024 / static_cast<int>(bundle.width);
   const int tiles_par           = threads_per_feature * slots / R;
-  // the last bundle may have fewer features, and then takes fewer CTAs
-  const int step = blockIdx.y + 1 == gridDim.y ? last_ctas : static_cast<int>(gridDim.x);
-  if (static_cast<int>(blockIdx.x) >= step || static_cast<int64_t>(blockIdx.x) * tiles_par >= n_tiles) return;
+  if (static_cast<int64_t>(first) * tiles_par >= n_tiles) return;
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     mbar_fence_init();
@@ -562,12 +567,12 @@ quantise_kernel(const __grid_constant__ PredictParams p, uint16_t* __restrict__ 
   grid_wait();  // the tables are part of the forest; rows and scratch may still be in use
   // while the tables arrive, ask the L2 for the rows of the CTA's first tile
   if (threadIdx.x < R) {
-    const int64_t row = static_cast<int64_t>(blockIdx.x) * tiles_par * R + threadIdx.x;
+    const int64_t row = static_cast<int64_t>(first) * tiles_par * R + threadIdx.x;
     if (row < p.n_rows)
       asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const T*>(p.X) + row * p.row_stride + grp.f_begin));
   }
-  if (flags.arrived != nullptr && blockIdx.y == 0) {
-    for (int64_t t = blockIdx.x * 1024ll + threadIdx.x; t < n_tiles; t += step * 1024ll)
+  if (flags.arrived != nullptr && which == 0) {
+    for (int64_t t = first * 1024ll + threadIdx.x; t < n_tiles; t += step * 1024ll)
       flags.arrived[t] = 0;
   }
   if (idle) return;
@@ -578,13 +583,13 @@ quantise_kernel(const __grid_constant__ PredictParams p, uint16_t* __restrict__ 
   // the number of halvings is fixed per group: pick the unrolled body once
   const uint32_t tables = blob_a + group_at;
   switch (grp.steps) {
-    case 0: quantise_rows<T, 0>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
-    case 1: quantise_rows<T, 1>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
-    case 2: quantise_rows<T, 2>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
-    case 3: quantise_rows<T, 3>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
-    case 4: quantise_rows<T, 4>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
-    case 5: quantise_rows<T, 5>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
-    default: quantise_rows<T, -1>(p, grp, Q, flags, R, tables, rec, tid, step, slots, tiles_par); break;
+    case 0: quantise_rows<T, 0>(p, grp, Q, flags, R, tables, rec, tid, first, step, slots, tiles_par); break;
+    case 1: quantise_rows<T, 1>(p, grp, Q, flags, R, tables, rec, tid, first, step, slots, tiles_par); break;
+    case 2: quantise_rows<T, 2>(p, grp, Q, flags, R, tables, rec, tid, first, step, slots, tiles_par); break;
+    case 3: quantise_rows<T, 3>(p, grp, Q, flags, R, tables, rec, tid, first, step, slots, tiles_par); break;
+    case 4: quantise_rows<T, 4>(p, grp, Q, flags, R, tables, rec, tid, first, step, slots, tiles_par); break;
+    case 5: quantise_rows<T, 5>(p, grp, Q, flags, R, tables, rec, tid, first, step, slots, tiles_par); break;
+    default: quantise_rows<T, -1>(p, grp, Q, flags, R, tables, rec, tid, first, step, slots, tiles_par); break;
   }
 }
 
@@ -1093,8 +1098,7 @@ int quantise_ctas_per_bundle(const ForestView& f, int R, int slots, int sm_count
   return best;
 }
 
-// Enqueue the rank pre-pass of p's rows.  The kernel may start while the one before it in the
-// stream is still running, unless that is a copy or memset.
+// Enqueue the rank pre-pass of p's rows.
 int launch_quantise(const PredictParams& p, uint16_t* Q, const QFlags& flags, int R, bool f64,
                     int sm_count, cudaStream_t stream, std::string& err)
 {
@@ -1107,9 +1111,15 @@ int launch_quantise(const PredictParams& p, uint16_t* Q, const QFlags& flags, in
   const int slots       = R <= 128 && n_tiles * f.q_n_bundles <= sm_count ? 4 : 8;
   const int gx          = quantise_ctas_per_bundle(f, R, slots, sm_count, n_tiles);
   const int last        = (gx * f.q_last_features + f.q_bundle_features - 1) / f.q_bundle_features;
-  const SplitLaunch l{dim3(gx, f.q_n_bundles), 1024, smem, stream, 1, true};
-  return f64 ? launch_split(l, err, quantise_kernel<double>, p, Q, flags, R, slots, last)
-             : launch_split(l, err, quantise_kernel<float>, p, Q, flags, R, slots, last);
+  // A kernel that overlaps the one before it inherits how that one divided the SM's memory, and the
+  // traversal leaves little of it to the L1.  Rows that do not start on 128-byte lines occupy two
+  // lines per load in flight, which then no longer fit (400,000 rows of 100 features: 139 us on a
+  // fresh division, 236 us on the inherited one); other loads do, and win 5 us of start-up.
+  const size_t row_b = static_cast<size_t>(p.row_stride) * (f64 ? 8 : 4);
+  const bool overlap = f.q_n_bundles == 1 || row_b % 128 == 0;
+  const SplitLaunch l{dim3(gx * (f.q_n_bundles - 1) + last), 1024, smem, stream, 1, overlap};
+  return f64 ? launch_split(l, err, quantise_kernel<double>, p, Q, flags, R, slots, gx)
+             : launch_split(l, err, quantise_kernel<float>, p, Q, flags, R, slots, gx);
 }
 
 // Rank-quantised prediction: rows are processed in chunks of whole waves of tiles; for each
