@@ -455,19 +455,22 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
         special     = special || cur[u] != cur[u] || cur[u + 1] != cur[u + 1];
       }
       if (__any_sync(0xffffffffu, special)) {
-#pragma unroll
-        for (int u = 0; u < CH; ++u) {
-          const T x     = cur[u];
-          uint32_t code = (two[u >> 1] >> (16 * (u & 1))) & 0xffffu;
+        if (any_cat) {
           // the code of a categorical value is the category itself (truncated value); negative and
           // huge values match no listed category
-          if (mine.is_cat)
-            code = (x >= T(0)) && (x < T(Q_NO_CATEGORY)) ? static_cast<uint32_t>(x) : Q_NO_CATEGORY;
-          if (x != x) {
-            code    = Q_NAN_CODE;
-            saw_nan = true;
+#pragma unroll
+          for (int u = 0; u < CH; ++u) {
+            const T x           = cur[u];
+            const uint32_t code = (x >= T(0)) && (x < T(Q_NO_CATEGORY)) ? static_cast<uint32_t>(x) : Q_NO_CATEGORY;
+            const uint32_t keep = (u & 1) ? 0xffffu : 0xffff0000u;
+            if (mine.is_cat) two[u >> 1] = (two[u >> 1] & keep) | (code << (16 * (u & 1)));
           }
-          two[u >> 1] = (u & 1) ? (two[u >> 1] & 0xffffu) | (code << 16) : (two[u >> 1] & 0xffff0000u) | code;
+        }
+#pragma unroll
+        for (int u = 0; u < CH; u += 2) {
+          const uint32_t nan = (cur[u] != cur[u] ? 0xffffu : 0u) | (cur[u + 1] != cur[u + 1] ? 0xffff0000u : 0u);
+          two[u >> 1] = (two[u >> 1] & ~nan) | (Q_NAN_CODE * 0x10001u & nan);
+          saw_nan |= nan != 0u;
         }
       }
       // the same chunk of the CTA's next round goes into the registers just read, so a whole round of
@@ -1113,10 +1116,12 @@ int launch_quantise(const PredictParams& p, uint16_t* Q, const QFlags& flags, in
   const int last        = (gx * f.q_last_features + f.q_bundle_features - 1) / f.q_bundle_features;
   // A kernel that overlaps the one before it inherits how that one divided the SM's memory, and the
   // traversal leaves little of it to the L1.  Rows that do not start on 128-byte lines occupy two
-  // lines per load in flight, which then no longer fit (400,000 rows of 100 features: 139 us on a
-  // fresh division, 236 us on the inherited one); other loads do, and win 5 us of start-up.
+  // lines per load in flight, which then no longer fit once they come from HBM (400,000 rows of 100
+  // features: 139 us on a fresh division, 236 us on the inherited one); other loads do, and win 5 us
+  // of start-up.
   const size_t row_b = static_cast<size_t>(p.row_stride) * (f64 ? 8 : 4);
-  const bool overlap = f.q_n_bundles == 1 || row_b % 128 == 0;
+  const bool overlap = f.q_n_bundles == 1 || row_b % 128 == 0 ||
+                       static_cast<size_t>(p.n_rows) * row_b <= size_t(64) << 20;
   const SplitLaunch l{dim3(gx * (f.q_n_bundles - 1) + last), 1024, smem, stream, 1, overlap};
   return f64 ? launch_split(l, err, quantise_kernel<double>, p, Q, flags, R, slots, gx)
              : launch_split(l, err, quantise_kernel<float>, p, Q, flags, R, slots, gx);
