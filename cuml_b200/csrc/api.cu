@@ -812,6 +812,8 @@ int b2fil_forest_create(const b2fil_forest_desc* desc, const b2fil_create_opts* 
       add_upload(list, pf.c_top_src, offsetof(ForestView, c_top_src));
     }
     if (pf.view.q_enabled) {
+      for (auto* image : {&pf.q_nodes, &pf.q_nodes_ids, &pf.q_nodes_nan})
+        split_category_sets(pf.view, *image);
       add_upload(list, pf.q_nodes, offsetof(ForestView, q_nodes));
       add_upload(list, pf.q_nodes_ids, offsetof(ForestView, q_nodes_ids));
       add_upload(list, pf.q_nodes_nan, offsetof(ForestView, q_nodes_nan));

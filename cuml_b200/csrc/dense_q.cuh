@@ -49,6 +49,30 @@ __device__ __forceinline__ uint2 lds_u32x2(uint32_t a)
   return v;
 }
 
+// A categorical node is recognisable by its rank field, the largest there is (0x3FFF, or 0x3FFE in the
+// image for doubled columns).  Only such nodes have a category set, in an array of its own behind the
+// nodes, and only lanes on such a node fetch it: in a forest with one categorical test in sixteen
+// that is less than half a shared-memory wavefront per visit, against one and more for nodes that
+// carry their set along (5000 depth-6 trees, 8 of 128 features categorical).
+template <uint32_t OFF>
+__device__ __forceinline__ uint32_t lds_if_categorical(uint32_t node, uint32_t a)
+{
+  // (the address register takes the set, so that a lane without one needs no other value for it)
+  asm volatile(
+    "{\n.reg .pred p;\nsetp.ge.s32 p, %1, 0x7FFC0000;\n@p ld.shared.u32 %0, [%0+%2];\n}"
+    : "+r"(a)
+    : "r"(node), "n"(OFF));
+  return a;
+}
+__device__ __forceinline__ uint32_t shift_if_categorical(uint32_t node, uint32_t d, uint32_t set, uint32_t code)
+{
+  static_assert(((Q_MAX_RANK_FIELD - 1u) << Q_RANK_SHIFT) == 0x7FFC0000u, "the constant below");
+  asm("{\n.reg .pred p;\nsetp.ge.s32 p, %1, 0x7FFC0000;\n@p shf.l.clamp.b32 %0, %0, %2, %3;\n}"
+      : "+r"(d)
+      : "r"(node), "r"(set), "r"(code));
+  return d;
+}
+
 // DEPTH > 0 fixes the tree depth at compile time (the level loop is fully unrolled); DEPTH == 0
 // reads it from the forest.  TOPC: the first two levels take their nodes from `top`.
 // PAIR: the walk for launch shapes that shared memory keeps small (few warps, few trees in
@@ -87,8 +111,9 @@ struct DenseQWalker {
                   "payloads outside the stages exist for fp32 scalar leaves without categorical tests");
     const ForestView& f    = p.f;
     const int D            = DEPTH > 0 ? DEPTH : f.dense_depth;
-    constexpr uint32_t QNB = CAT ? 8u : 4u;  // bytes per test node: {node, category set} or node
-    const uint32_t width_b = (1u << D) * QNB;
+    // bytes of a tree's test nodes, or (CAT) of its test nodes and the category sets behind them
+    const uint32_t width_b = (1u << D) * (CAT ? 8u : 4u);
+    const uint32_t sets_at = 4u << D;  // from a node to its category set
     // bytes between two trees of a stage
     const uint32_t tstride = LEAFG ? width_b : static_cast<uint32_t>(f.q_tree_stride);
     // bytes per leaf payload: the element size, except where vector leaves sit in the tree block
@@ -121,14 +146,14 @@ struct DenseQWalker {
         // slots past the end of the forest repeat the last live tree; results are dropped
         base[k] = base0 + static_cast<uint32_t>(FULL ? k : min(k, n_act - 1)) * tstride;
         idx[k]  = 1u;  // heap index of the root
-        a[k]    = base[k] + QNB;
+        a[k]    = base[k] + 4u;
       }
       // the NT walks are independent: all node loads are issued first, then all rank loads,
       // so that their shared-memory latencies overlap inside one warp.
       // test(): the rows' ranks against NT nodes; the sign bit of d[k] is the step to the right.
-      auto test = [&](const uint32_t(&node)[NT], const uint32_t(&bits)[CAT ? NT : 1], uint32_t(&d)[NT],
+      auto test = [&](const uint32_t(&node)[NT], const uint32_t(&at)[NT], uint32_t(&d)[NT],
                       auto is_top) {
-        uint32_t q[NT];
+        uint32_t q[NT], bits[NT];
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           uint32_t from = row_addr;
@@ -141,16 +166,20 @@ struct DenseQWalker {
         }
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
+          if (CAT)
+            bits[k] = lds_if_categorical<DEPTH ? 4u << DEPTH : 0u>(node[k], at[k] + (DEPTH ? 0u : sets_at));
+        }
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
           // rank j in the high half: x < T[j] <=> rank(x) <= j, so right <=> j - rank < 0
           d[k] = rank_diff(node[k], q[k]);
           if (CAT) {
-            // the code of a categorical value is its category and the node's set (fetched with
-            // the node; numerical nodes hold an empty one) is stored bit-reversed: the clamped
-            // funnel shift by the code moves the category's bit to the sign position and yields 0
-            // for every code of 32 and above (no category, NaN).  A categorical node carries the
-            // largest rank (its comparison never says "right"), so the two answers are simply
-            // ORed and the walk has no data-dependent branch.
-            d[k] |= __funnelshift_lc(0u, bits[k], q[k]);
+            // the code of a categorical value is its category and the node's set is stored
+            // bit-reversed: the clamped funnel shift by the code moves the category's bit to the sign
+            // position, and leaves d for every code of 32 and above (no category, NaN), which the
+            // large rank of a categorical node has made non-negative, or right for a missing value
+            // of a doubled column.  Predicated: the walk has no data-dependent branch.
+            d[k] = shift_if_categorical(node[k], d[k], bits[k], q[k]);
           }
           if (NANS) {
             // the missing-goes-right flag sits 15 bits below the sign.  (Both forms compute the
@@ -165,26 +194,17 @@ struct DenseQWalker {
         }
       };
       auto level = [&]() {
-        uint32_t node[NT], d[NT], bits[CAT ? NT : 1];
+        uint32_t node[NT], d[NT];
 #pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          if (CAT) {
-            const uint2 both = lds_u32x2(a[k]);
-            node[k]          = both.x;
-            bits[k]          = both.y;
-          } else {
-            node[k] = lds_u32(a[k]);
-          }
-        }
-        test(node, bits, d, std::false_type{});
+        for (int k = 0; k < NT; ++k) node[k] = lds_u32(a[k]);
+        test(node, a, d, std::false_type{});
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           // heap index 2i + right in one funnel shift: (i << 1) | (d >> 31)
           idx[k] = __funnelshift_l(d[k], idx[k], 1);
-          a[k]   = idx[k] * QNB + base[k];
+          a[k]   = idx[k] * 4u + base[k];
         }
       };
-      const uint32_t no_bits[1] = {0u};  // walks without categorical tests
       if constexpr (PAIR) {
         uint32_t node[NT], d[NT];
 #pragma unroll
@@ -196,7 +216,7 @@ struct DenseQWalker {
           uint2 pair[NT];
 #pragma unroll
           for (int k = 0; k < NT; ++k) pair[k] = lds_u32x2(base[k] + idx[k] * 8u);
-          test(node, reinterpret_cast<const uint32_t(&)[CAT ? NT : 1]>(no_bits), d, std::false_type{});
+          test(node, a, d, std::false_type{});
 #pragma unroll
           for (int k = 0; k < NT; ++k) {
             idx[k]  = __funnelshift_l(d[k], idx[k], 1);
@@ -220,13 +240,13 @@ struct DenseQWalker {
           n2[k]       = top->w[t + 1];
           n3[k]       = top->w[t + 2];
         }
-        test(n1, reinterpret_cast<const uint32_t(&)[CAT ? NT : 1]>(no_bits), d, std::true_type{});
+        test(n1, a, d, std::true_type{});
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           node[k] = static_cast<int32_t>(d[k]) < 0 ? n3[k] : n2[k];
           idx[k]  = __funnelshift_l(d[k], 1u, 1);
         }
-        test(node, reinterpret_cast<const uint32_t(&)[CAT ? NT : 1]>(no_bits), d, std::true_type{});
+        test(node, a, d, std::true_type{});
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           idx[k] = __funnelshift_l(d[k], idx[k], 1);

@@ -268,8 +268,8 @@ struct ForestView {
                                 // forest with few outputs sit in the tree blocks themselves
   int32_t q_any_default_left;   // 0: missing values go right in every test
   int64_t q_tree_stride;        // bytes between trees: 2^D * (node bytes + leaf bytes), 16-byte multiple
-  const void* q_nodes;          // [n_trees] blocks of [2^D nodes][2^D leaf payloads]; a node is a
-                                // uint32, or {uint32 node, uint32 category set} when q_has_cat
+  const void* q_nodes;          // [n_trees] blocks of [2^D nodes][2^D leaf payloads] of uint32 nodes,
+                                // with [2^D category sets] in between when q_has_cat
   const void* q_nodes_ids;      // same blocks with the leaf id (uint32) in every leaf payload slot:
                                 // what the traversal streams when it reports leaf ids
   const void* q_nodes_nan;      // q_nodes for tiles with missing values and doubled columns (see
@@ -345,6 +345,10 @@ inline uint32_t q_bucket_host(T x, T scale, T offset, uint32_t n_buckets)
 // Shared memory the quantisation kernel may spend on the tables of one feature group.
 constexpr uint32_t kQGroupSmemBudget = 208 * 1024;
 constexpr uint32_t kQMaxGroupFeatures = 32;
+
+// Before the upload: the tree blocks of a rank-quantised image with categorical tests change from
+// [2^D {node, category set}] to [2^D nodes][2^D category sets], which is what the kernels read.
+void split_category_sets(const ForestView& view, std::vector<uint8_t>& image);
 
 // Validate `desc`, normalise its tests and lay its nodes out.  Returns B2FIL_OK or an error code
 // with `err` set.  `dense_ok(depth, precision, n_features, n_outputs)` tells whether the dense

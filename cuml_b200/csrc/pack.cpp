@@ -1074,6 +1074,21 @@ struct Packer {
 
 }  // namespace
 
+void split_category_sets(const ForestView& v, std::vector<uint8_t>& image)
+{
+  if (!v.q_has_cat || image.empty()) return;
+  const size_t width = size_t(1) << v.dense_depth;
+  std::vector<uint32_t> split(2 * width);
+  for (int t = 0; t < v.n_trees; ++t) {
+    uint8_t* at = image.data() + static_cast<size_t>(v.q_tree_stride) * t;
+    for (size_t i = 0; i < width; ++i) {
+      std::memcpy(&split[i], at + i * 8, 4);
+      std::memcpy(&split[width + i], at + i * 8 + 4, 4);
+    }
+    std::memcpy(at, split.data(), width * 8);
+  }
+}
+
 int pack_forest(const b2fil_forest_desc& desc, const b2fil_create_opts& opts,
                 int (*dense_ok)(int, int, int, int), PackedForest& out, std::string& err)
 {
