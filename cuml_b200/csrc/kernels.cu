@@ -842,7 +842,9 @@ size_t q_node_only_stride(const ForestView& f, int mode)
 // Most trees a warp of the quantised kernel may walk side by side: the kernels that exist.
 int q_max_trees_in_flight(const ForestView& f, int mode)
 {
-  if (f.q_has_cat) return 4;
+  if (f.q_has_cat) {
+    return f.format == FMT_DENSE_F && mode == MODE_SCALAR && f.dense_depth >= 4 && f.dense_depth <= 8 ? 6 : 4;
+  }
   const bool specialised = f.format == FMT_DENSE_F && (mode == MODE_SCALAR || mode == MODE_VECTOR) &&
                            f.dense_depth >= 4 && f.dense_depth <= 10;
   return specialised ? 6 : 4;
@@ -1014,7 +1016,7 @@ int launch_dense_q_kernel(const QLaunch& L, int mode, bool f64, std::string& err
   rec.K               = L.c.sub_batches;
   if (f.q_has_cat) {
     // kernels_q_cat.cu: fp32 scalar leaves of depth 4..8 with four trees in flight are specialised
-    if (!f64 && mode == MODE_SCALAR && L.c.trees_in_flight == 4 && f.dense_depth >= 4 &&
+    if (!f64 && mode == MODE_SCALAR && L.c.trees_in_flight >= 4 && f.dense_depth >= 4 &&
         f.dense_depth <= 8)
       rec.depth = f.dense_depth;
     return launch_q_cat(L, mode, f64, err);

@@ -113,7 +113,7 @@ int launch_q_pair(const QLaunch& L, std::string& err);
 // fp32 scalar leaves of depth 9 and 10, two to four trees in flight, payloads left in global memory.
 int launch_q_leafg(const QLaunch& L, std::string& err);
 // Forests with categorical tests: every precision, output mode and depth; 1, 2 or 4 trees in
-// flight (depth-specialised bodies for fp32 scalar leaves of depth 4..8 with four trees).
+// flight (depth-specialised bodies for fp32 scalar leaves of depth 4..8 with four and six trees).
 int launch_q_cat(const QLaunch& L, int mode, bool f64, std::string& err);
 // Everything else: generic depth, every precision and output mode; 1, 2 or 4 trees in flight.
 int launch_q_generic(const QLaunch& L, int mode, bool f64, std::string& err);
