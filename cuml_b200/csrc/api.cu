@@ -779,6 +779,8 @@ int b2fil_forest_create(const b2fil_forest_desc* desc, const b2fil_create_opts* 
     int rc = pack_forest(*desc, *opts, dense_ok, pf, err);
     if (rc != B2FIL_OK) return set_error(rc, err);
 
+    if (pf.view.c_enabled && !build_blocks(pf)) pf.view.c_enabled = 0;
+
     std::unique_ptr<b2fil_forest> f(new b2fil_forest());
     f->device = opts->device_id;
     DeviceGuard guard(f->device);
@@ -803,13 +805,13 @@ int b2fil_forest_create(const b2fil_forest_desc* desc, const b2fil_create_opts* 
     add_upload(list, pf.leaf_vectors, offsetof(ForestView, leaf_vectors));
     add_upload(list, pf.out_scale, offsetof(ForestView, out_scale));
     add_upload(list, pf.out_bias, offsetof(ForestView, out_bias));
-    if (pf.view.c_enabled) {
-      add_upload(list, pf.c_nodes, offsetof(ForestView, c_nodes));
-      add_upload(list, pf.c_exact, offsetof(ForestView, c_exact));
-      add_upload(list, pf.c_leaf_payload, offsetof(ForestView, c_leaf_payload));
-      add_upload(list, pf.c_leaf_ids, offsetof(ForestView, c_leaf_ids));
-      add_upload(list, pf.c_top, offsetof(ForestView, c_top));
-      add_upload(list, pf.c_top_src, offsetof(ForestView, c_top_src));
+    if (f->view.c_enabled) {
+      add_upload(list, pf.b_blocks, offsetof(ForestView, c_blocks));
+      add_upload(list, pf.b_exact, offsetof(ForestView, c_exact));
+      add_upload(list, pf.b_leaf_payload, offsetof(ForestView, c_leaf_payload));
+      add_upload(list, pf.b_leaf_ids, offsetof(ForestView, c_leaf_ids));
+      add_upload(list, pf.b_top, offsetof(ForestView, c_top));
+      add_upload(list, pf.b_top_exact, offsetof(ForestView, c_top_exact));
     }
     if (pf.view.q_enabled) {
       for (auto* image : {&pf.q_nodes, &pf.q_nodes_ids, &pf.q_nodes_nan})

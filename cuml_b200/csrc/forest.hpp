@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -191,6 +192,24 @@ constexpr uint32_t CMETA_LOW27       = 0x07FFFFFFu;
 constexpr uint32_t C_EXIT_LEAF      = 0x80000000u;
 constexpr uint32_t C_NO_NODE        = 0xFFFFFFFFu;
 constexpr int kCMaxTopLevels        = 10;
+// What the kernel walks below the heaps is made from these arrays at upload (blocks.cpp): blocks of
+// 32 bytes, one sector, that hold a node, its two children and the heaviest of its grandchildren, so
+// that a fetch is good for two tests always and for a third one more often than not (the pairs of
+// depth-first neighbours that the 8-byte nodes allow were good for 1.35 on average, and the sectors
+// between L1 and L2 are what bounds the walk):
+//   words 0..3: values of root, left child, right child, grandchild
+//   words 4, 5: a 16-bit test each: feature | missing-goes-left | categorical, and three more bits
+//     root: is there a grandchild (else the fourth test is a filler), whose place it has: 0..3
+//     left and right child: which of the edges out of the block lead to a leaf (3 + 2 bits)
+//   word 6: first child block, word 7: first leaf.
+// The edges are numbered left to right, five with the grandchild and four without; the blocks that
+// the edges lead to are consecutive, and so are the leaves.  A leaf in a child's place stands on both
+// sides of a filler test, twice in the leaf arrays.  Exits of the heaps name a block or a leaf.
+constexpr uint32_t BLK_FEATURE      = 0x7FFu;
+constexpr uint32_t BLK_DEFAULT_LEFT = 0x800u;
+constexpr uint32_t BLK_CATEGORICAL  = 0x1000u;
+constexpr uint32_t BLK_FOURTH_SHIFT = 13;
+constexpr uint32_t BLK_HAS_FOURTH   = 0x8000u;
 struct CompactNode {  // 8 bytes
   uint32_t value;     // float threshold bits (fp64 forests: rounded down) | bitset | pool offset
   uint32_t meta;
@@ -286,12 +305,14 @@ struct ForestView {
   int32_t c_feat_bits;
   int32_t c_bottom_steps;       // most steps a walk takes below the heap
   int64_t c_top_stride;         // bytes between the heaps of two trees: 2^T * 16
-  const CompactNode* c_nodes;   // [n_internal, rounded up to even]: pairs are loaded together
-  const double* c_exact;        // [n_internal] exact thresholds (fp64 forests), else null
+  int32_t c_block_steps;        // most blocks on a walk
+  int32_t c_pad_;
+  const uint32_t* c_blocks;     // [n_blocks * 8]
+  const double* c_exact;        // [n_blocks * 4] exact thresholds (fp64 forests), else null
   const void* c_leaf_payload;   // [n_leaves] scalar in the forest precision or vector index
   const uint32_t* c_leaf_ids;   // [n_leaves] id of the leaf in the imported model
   const unsigned char* c_top;   // [n_trees] heaps
-  const uint32_t* c_top_src;    // [n_trees << T] internal node behind every heap node (fp64), C_NO_NODE = padding
+  const double* c_top_exact;    // [n_trees << T] exact thresholds of the heap nodes (fp64), -inf = padding
 };
 
 // Host-side result of packing, before upload.
@@ -329,6 +350,13 @@ struct PackedForest {
   std::vector<uint32_t> c_leaf_ids;
   std::vector<uint8_t> c_top;
   std::vector<uint32_t> c_top_src;
+  // blocks of the compact image, filled by build_blocks()
+  std::vector<uint32_t> b_blocks;
+  std::vector<double> b_exact;
+  std::vector<uint8_t> b_leaf_payload;
+  std::vector<uint32_t> b_leaf_ids;
+  std::vector<uint8_t> b_top;
+  std::vector<double> b_top_exact;
 };
 
 // Bucket of a value in a feature's table; the same expression runs on the device
@@ -345,6 +373,9 @@ inline uint32_t q_bucket_host(T x, T scale, T offset, uint32_t n_buckets)
 // Shared memory the quantisation kernel may spend on the tables of one feature group.
 constexpr uint32_t kQGroupSmemBudget = 208 * 1024;
 constexpr uint32_t kQMaxGroupFeatures = 32;
+
+// Before the upload: the blocks of a forest with a compact image.  False when a field does not fit.
+bool build_blocks(PackedForest& pf);
 
 // Before the upload: the tree blocks of a rank-quantised image with categorical tests change from
 // [2^D {node, category set}] to [2^D nodes][2^D category sets], which is what the kernels read.

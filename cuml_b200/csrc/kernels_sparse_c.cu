@@ -8,12 +8,10 @@
 //      ring of shared-memory stages (bulk copies from the L2-resident heap array; one stage =
 //      the heaps of G * NT trees): T steps without a global fetch, then one exit {k, L} that names
 //      the internal node to continue at and the leaves before it, or the leaf reached;
-//   2. below the heap the walk follows the compact nodes in global memory: 8-byte internal
-//      nodes, first child adjacent, (k, L) bookkeeping for the leaf number, nodes fetched as
-//      aligned 16-byte pairs so that a step from an even node to its first child needs no fetch.
-//      A step is straight-line code: the NT tests, then per walk compact_step, which moves
-//      (k, L) and ends in the predicated fetch for the next step; only a test that the float
-//      compare leaves open (missing value, fp64 tie) takes a branch.
+//   2. below the heap the walk goes from block to block in global memory: 32 bytes, one sector, with
+//      a node, its two children and one grandchild (forest.hpp).  The tests of a block are
+//      straight-line code and end in the predicated fetch of the next one; only a test that the
+//      float compare leaves open (missing value, fp64 tie) takes a branch.
 // A stage is released as soon as the warp has left the heaps, before it starts on part 2, so the
 // next batch of heaps arrives while the warps wait for their node fetches.
 // The row tile holds floats also for fp64 forests: every value is rounded DOWN to float when the
@@ -40,22 +38,20 @@ __device__ __forceinline__ void lds_node(uint32_t a, uint32_t& value, uint32_t& 
   asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(value), "=r"(meta) : "r"(a));
 }
 
-// One aligned 16-byte fetch = nodes 2m and 2m + 1, issued only where `wanted`; the registers keep
-// their contents otherwise.  A predicated instruction rather than a branch: the walks of a warp
-// want their fetches at different steps, and a branch per fetch costs more issue slots than the
-// fetch.  L2-only (.cg): the fetches of a warp go to 32 unrelated lines and nothing is reused, so
-// the L1 should only track the misses in flight (measured 4 to 8 % faster than the read-only
-// path; L2 eviction hints measured slower).
-__device__ __forceinline__ void ld_compact_pair_if(bool wanted, const void* ptr, uint32_t& x,
-                                                   uint32_t& y, uint32_t& z, uint32_t& w)
+// One block, issued only where `wanted`; the registers keep their contents otherwise.  A predicated
+// instruction rather than a branch: the walks of a warp want their fetches at different steps, and a
+// branch per fetch costs more issue slots than the fetch.  L2-only (.cg): the fetches of a warp go to
+// 32 unrelated lines and nothing is reused, so the L1 should only track the misses in flight (measured
+// 4 to 8 % faster than the read-only path; L2 eviction hints measured slower).
+__device__ __forceinline__ void ld_block_if(bool wanted, const uint32_t* ptr, uint32_t (&w)[8])
 {
   asm volatile(
     "{\n\t"
     ".reg .pred want;\n\t"
-    "setp.ne.u32 want, %5, 0;\n\t"
-    "@want ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];\n\t"
+    "setp.ne.u32 want, %9, 0;\n\t"
+    "@want ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
     "}"
-    : "+r"(x), "+r"(y), "+r"(z), "+r"(w)
+    : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "+r"(w[6]), "+r"(w[7])
     : "l"(ptr), "r"(static_cast<uint32_t>(wanted)));
 }
 
@@ -70,30 +66,26 @@ __device__ __forceinline__ bool test_is_open(float xl, float lo)
   return xl != xl;
 }
 
-// Exact form of an fp64 test that the floats left open.  `k` is the internal node whose exact
-// threshold settles it (C_NO_NODE: none, heap padding: the row goes right).
-__device__ __noinline__ bool compact_exact_left(const double* row_values, const double* exact,
-                                                uint32_t k, uint32_t feat)
+// Exact form of an fp64 test that the floats left open; `exact` points to its threshold.
+__device__ __noinline__ bool compact_exact_left(const double* row_values, const double* exact, uint32_t feat)
 {
-  if (k == C_NO_NODE) return false;
   // rows past the end of the batch (no values) were staged as zeros
   const double x = row_values != nullptr ? __ldg(row_values + feat) : 0.0;
-  return x < __ldg(exact + k);
+  return x < __ldg(exact);
 }
 
 // Settle an open test off the common path and rewrite (xl, lo) so that the plain compare
 // xl < lo gives the answer.
-template <typename T, typename ExactIndex>
-__device__ __forceinline__ void settle_open_test(float& xl, float& lo, uint32_t meta, uint32_t feat,
-                                                 const double* row_values, const double* exact,
-                                                 ExactIndex exact_index)
+template <typename T, typename Exact>
+__device__ __forceinline__ void settle_open_test(float& xl, float& lo, bool default_left, uint32_t feat,
+                                                 const double* row_values, Exact exact)
 {
   if (!test_is_open<T>(xl, lo)) return;
   bool left = false;  // fp32 forests: xl == lo is x == threshold, which goes right
   if (xl != xl) {
-    left = (meta & META_DEFAULT_LEFT) != 0u;
+    left = default_left;
   } else if constexpr (sizeof(T) == 8) {
-    left = compact_exact_left(row_values, exact, exact_index(), feat);
+    left = compact_exact_left(row_values, exact(), feat);
   }
   lo = 0.f;
   xl = left ? -1.f : 1.f;
@@ -107,55 +99,6 @@ __device__ __forceinline__ void settle_categorical_test(float& xl, float& lo, ui
   lo               = 0.f;
   xl               = right ? 1.f : -1.f;
 }
-
-// One step of a walk below the heap, after its test operands (xl, lo) are known.  State: k = the
-// node the walk is on (bit 31 set once it has reached its leaf), L = leaves before the walk's
-// position, {x, y, z, w} = the aligned pair of nodes that holds node k.  The step takes the
-// branch, moves (k, L), and fetches the pair of the new node when that is a different pair: a
-// first child reached from an even node is the neighbour already held.  Predicate logic all the
-// way, no branch; written in PTX because the C++ form of the same step compiled to 2.5 times the
-// instructions (flags kept as integers and re-tested), and issue slots are what the walk is
-// short of.
-__device__ __forceinline__ void compact_step(uint32_t& k, uint32_t& L, uint32_t& x, uint32_t& y,
-                                             uint32_t& z, uint32_t& w, float xl, float lo,
-                                             uint32_t meta, int off_shift, const void* nodes)
-{
-  asm volatile(
-    "{\n\t"
-    ".reg .pred lt, sw, second, leaf, live, ls, go, want;\n\t"
-    ".reg .u32 t, off, hop, kn;\n\t"
-    ".reg .u64 a;\n\t"
-    "setp.lt.f32 lt, %6, %7;\n\t"
-    "and.b32 t, %8, 0x08000000;\n\t"  // CMETA_SWAPPED
-    "setp.ne.u32 sw, t, 0;\n\t"
-    "xor.pred second, lt, sw;\n\t"
-    "not.pred second, second;\n\t"    // second child = (left == swapped)
-    "shl.b32 off, %8, 5;\n\t"
-    "shr.u32 off, off, %9;\n\t"
-    "selp.u32 t, 0x10000000, 0x20000000, second;\n\t"  // CMETA_SECOND_LEAF, CMETA_FIRST_LEAF
-    "and.b32 t, t, %8;\n\t"
-    "setp.ne.u32 leaf, t, 0;\n\t"
-    "setp.ge.s32 live, %0, 0;\n\t"
-    "and.pred ls, live, second;\n\t"
-    "@ls add.u32 %1, %1, off;\n\t"    // the second child skips the leaves of the first
-    "selp.u32 hop, off, 1, second;\n\t"
-    "and.pred go, live, !leaf;\n\t"
-    "add.u32 kn, %0, hop;\n\t"
-    "xor.b32 t, kn, %0;\n\t"
-    "setp.gt.u32 want, t, 1;\n\t"     // another pair
-    "and.pred want, want, go;\n\t"
-    "@!go or.b32 %0, %0, 0x80000000;\n\t"
-    "@go mov.u32 %0, kn;\n\t"
-    "and.b32 t, kn, 0x7ffffffe;\n\t"
-    "mad.wide.u32 a, t, 8, %10;\n\t"
-    "@want ld.global.cg.v4.u32 {%2, %3, %4, %5}, [a];\n\t"
-    "}"
-    : "+r"(k), "+r"(L), "+r"(x), "+r"(y), "+r"(z), "+r"(w)
-    : "f"(xl), "f"(lo), "r"(meta), "r"(off_shift), "l"(nodes));
-}
-static_assert(CMETA_SWAPPED == 0x08000000u && CMETA_SECOND_LEAF == 0x10000000u &&
-                CMETA_FIRST_LEAF == 0x20000000u && C_EXIT_LEAF == 0x80000000u,
-              "compact_step spells these constants out");
 
 // Stage rows [row0, row0 + R) feature-major as floats (fp64 inputs rounded down).  A warp reads 32
 // consecutive features of one row and scatters them to 32 different banks.  Rows past the end of
@@ -218,8 +161,6 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
   const int TL        = f.c_top_levels;
   const uint32_t heap_n     = 1u << TL;
   const uint32_t top_stride = static_cast<uint32_t>(f.c_top_stride);
-  const int fb              = f.c_feat_bits;
-  const uint32_t feat_mask  = (1u << fb) - 1u;
 
   const uint32_t stride_b    = (R + 1) * 4u;  // the tile holds floats whatever the forest precision
   const size_t tile_bytes    = align16(static_cast<size_t>(F) * stride_b);
@@ -285,7 +226,6 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
   const int r             = (warp % rw) * 32 + lane;
   T* acc_group            = acc + static_cast<size_t>(g) * NC * R;
   const uint32_t row_addr = tile + r * 4u;
-  const CompactNode* __restrict__ nodes = f.c_nodes;
   RingPos pos;
   bool ok = true;
   grid_wait();
@@ -321,7 +261,7 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
       if (ok) ok = mbar_wait(bars + 8u * s, pos.phase);
       const int first = b * per_batch + g * NT;
       const int n_act = ok ? min(NT, f.n_trees - first) : 0;
-      uint32_t k[NT], L[NT];  // bit 31 of k: the walk has reached its leaf, L is its number
+      uint32_t k[NT];  // the block a walk is on, or, with bit 31, the leaf it has reached
       if (n_act > 0) {
         // part 1: the heaps in shared memory
         uint32_t base[NT], h[NT];
@@ -349,10 +289,10 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
           if (any_open) {
 #pragma unroll
             for (int kk = 0; kk < NT; ++kk) {
-              settle_open_test<T>(xl[kk], lo[kk], meta[kk], meta[kk] & CMETA_LOW27, row_values(),
-                                  f.c_exact, [&]() {
+              settle_open_test<T>(xl[kk], lo[kk], (meta[kk] & META_DEFAULT_LEFT) != 0u,
+                                  meta[kk] & CMETA_LOW27, row_values(), [&]() {
                                     const size_t tree = static_cast<size_t>(first + min(kk, n_act - 1));
-                                    return __ldg(f.c_top_src + tree * heap_n + h[kk]);
+                                    return f.c_top_exact + tree * heap_n + h[kk];
                                   });
             }
           }
@@ -362,11 +302,7 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
 #pragma unroll
         for (int kk = 0; kk < NT; ++kk) {
           // the exits follow the 2^T node slots: exit e sits at 8 * (2^T + e) = 8 * h
-          uint32_t ek, eL;
-          lds_node(base[kk] + h[kk] * 8u, ek, eL);
-          const bool done = (ek & C_EXIT_LEAF) != 0u;
-          k[kk]           = ek;                              // an exit that is a leaf carries bit 31
-          L[kk]           = done ? (ek & ~C_EXIT_LEAF) : eL;  // the leaf itself, or leaves before k
+          k[kk] = lds_u32(base[kk] + h[kk] * 8u);
         }
       }
       // the heaps of this batch are no longer needed: let the producer refill the stage
@@ -374,57 +310,79 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
       if (lane == 0) mbar_arrive(bars + 8u * (kMaxStages + s));
       pos.advance(S);
       if (n_act > 0) {
-        // part 2: compact nodes in global memory
-        // Nodes come in aligned pairs {2m, 2m + 1} and a walk holds the pair of its node.  The
-        // first child of node k is node k + 1, so a walk that sits on an even node and goes to its
-        // first child already holds the next node and skips the fetch: lanes that skip touch no
-        // cache line.  A step is straight-line code: the operands of the NT tests, one rarely
-        // taken branch for tests that the floats leave open, then NT times compact_step, which
-        // ends in the (predicated) fetch for the next step.
-        uint32_t pair[NT][4];
-        const uint2* node_ptr = reinterpret_cast<const uint2*>(nodes);
+        // part 2: blocks in global memory.  All lanes of the warp do the three tests of the block
+        // they are on, without a branch: root, the child it leads to, and the grandchild (whose
+        // operands do not depend on the others) where the walk comes past it.
+        uint32_t w[NT][8];
+        const uint32_t* blocks = f.c_blocks;
 #pragma unroll
         for (int kk = 0; kk < NT; ++kk) {
-          // a walk that ended in the heap keeps a node that no value ties with
-          pair[kk][0] = pair[kk][2] = 0x00800001u;
-          pair[kk][1] = pair[kk][3] = 0u;
-          ld_compact_pair_if(static_cast<int32_t>(k[kk]) >= 0, node_ptr + (k[kk] & 0x7ffffffeu),
-                             pair[kk][0], pair[kk][1], pair[kk][2], pair[kk][3]);
+          // a walk that ended in the heap keeps a block whose tests no value leaves open
+          w[kk][0] = w[kk][1] = w[kk][2] = w[kk][3] = 0x00800001u;
+          w[kk][4] = w[kk][5] = w[kk][6] = w[kk][7] = 0u;
+          ld_block_if(static_cast<int32_t>(k[kk]) >= 0, blocks + static_cast<size_t>(k[kk] & ~C_EXIT_LEAF) * 8,
+                      w[kk]);
         }
-        const int off_shift = 5 + fb;  // the offset sits between the five flag bits and the feature
-        for (int step = 0; step < f.c_bottom_steps; ++step) {
-          uint32_t value[NT], meta[NT];
+        // the row's value and the node's for test number `slot(kk)` = test word `half(kk)`
+        auto run_tests = [&](auto value, auto half, auto slot, bool (&right)[NT]) {
           float xl[NT], lo[NT];
           bool any_open = false;
 #pragma unroll
           for (int kk = 0; kk < NT; ++kk) {
-            const bool odd = (k[kk] & 1u) != 0u;
-            value[kk]      = odd ? pair[kk][2] : pair[kk][0];
-            meta[kk]       = odd ? pair[kk][3] : pair[kk][1];
-            xl[kk]         = Traits<float>::ld_real((meta[kk] & feat_mask) * stride_b + row_addr);
-            lo[kk]         = __uint_as_float(value[kk]);
-            if (CAT && (meta[kk] & META_CATEGORICAL))
-              settle_categorical_test(xl[kk], lo[kk], value[kk], meta[kk], f);
+            xl[kk] = Traits<float>::ld_real((half(kk) & BLK_FEATURE) * stride_b + row_addr);
+            lo[kk] = __uint_as_float(value(kk));
+          }
+#pragma unroll
+          for (int kk = 0; kk < NT; ++kk) {
+            if (CAT && (half(kk) & BLK_CATEGORICAL))
+              settle_categorical_test(xl[kk], lo[kk], value(kk),
+                                      META_CATEGORICAL | ((half(kk) & BLK_DEFAULT_LEFT) ? META_DEFAULT_LEFT : 0u), f);
             any_open |= test_is_open<T>(xl[kk], lo[kk]);
           }
           if (any_open) {
 #pragma unroll
             for (int kk = 0; kk < NT; ++kk) {
-              // (a finished walk repeats its last test: nothing to settle)
+              // (a finished walk repeats its last tests: nothing to settle)
               if (static_cast<int32_t>(k[kk]) >= 0)
-                settle_open_test<T>(xl[kk], lo[kk], meta[kk], meta[kk] & feat_mask, row_values(),
-                                    f.c_exact, [&]() { return k[kk]; });
+                settle_open_test<T>(xl[kk], lo[kk], (half(kk) & BLK_DEFAULT_LEFT) != 0u,
+                                    half(kk) & BLK_FEATURE, row_values(),
+                                    [&]() { return f.c_exact + static_cast<size_t>(k[kk]) * 4 + slot(kk); });
             }
           }
 #pragma unroll
-          for (int kk = 0; kk < NT; ++kk)
-            compact_step(k[kk], L[kk], pair[kk][0], pair[kk][1], pair[kk][2], pair[kk][3], xl[kk],
-                         lo[kk], meta[kk], off_shift, node_ptr);
-          uint32_t all = k[0];
+          for (int kk = 0; kk < NT; ++kk) right[kk] = !(xl[kk] < lo[kk]);
+        };
+        for (int step = 0; step < f.c_block_steps; ++step) {
+          bool r0[NT], r1[NT], r2[NT];
+          run_tests([&](int kk) { return w[kk][0]; }, [&](int kk) { return w[kk][4]; },
+                    [](int) { return 0; }, r0);
+          run_tests([&](int kk) { return w[kk][3]; }, [&](int kk) { return w[kk][5] >> 16; },
+                    [](int) { return 3; }, r2);
+          run_tests([&](int kk) { return r0[kk] ? w[kk][2] : w[kk][1]; },
+                    [&](int kk) { return r0[kk] ? w[kk][5] : w[kk][4] >> 16; },
+                    [&](int kk) { return r0[kk] ? 2 : 1; }, r1);
+          bool walking = false;
 #pragma unroll
-          for (int kk = 1; kk < NT; ++kk) all &= k[kk];
-          if (!__any_sync(0xffffffffu, static_cast<int32_t>(all) >= 0)) break;
+          for (int kk = 0; kk < NT; ++kk) {
+            const uint32_t pos    = (r0[kk] ? 2u : 0u) + (r1[kk] ? 1u : 0u);
+            const bool has        = (w[kk][4] & BLK_HAS_FOURTH) != 0u;
+            const uint32_t fourth = has ? (w[kk][4] >> BLK_FOURTH_SHIFT) & 3u : 4u;
+            const uint32_t edge   = pos + ((pos > fourth || (pos == fourth && r2[kk])) ? 1u : 0u);
+            const uint32_t mask   = (w[kk][4] >> 29) | ((w[kk][5] >> 10) & 0x18u);  // edges to leaves
+            const uint32_t before = __popc(mask & ~(0xffffffffu << edge));
+            const bool leaf       = ((mask >> edge) & 1u) != 0u;
+            const uint32_t next   = leaf ? (w[kk][7] + before) | C_EXIT_LEAF : w[kk][6] + edge - before;
+            const bool live       = static_cast<int32_t>(k[kk]) >= 0;
+            if (live) k[kk] = next;
+            const bool go = live && !leaf;
+            ld_block_if(go, blocks + static_cast<size_t>(next & ~C_EXIT_LEAF) * 8, w[kk]);
+            walking |= go;
+          }
+          if (!__any_sync(0xffffffffu, walking)) break;
         }
+        uint32_t L[NT];
+#pragma unroll
+        for (int kk = 0; kk < NT; ++kk) L[kk] = k[kk] & ~C_EXIT_LEAF;
         // the leaves: payload (or id) from the leaf arrays
         if (MODE == MODE_LEAFID) {
           uint32_t id[NT];
