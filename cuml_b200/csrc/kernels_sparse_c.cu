@@ -6,8 +6,8 @@
 // a time.  Every walk has two parts:
 //   1. the top T levels of the tree are a complete heap that a producer warp streams through a
 //      ring of shared-memory stages (bulk copies from the L2-resident heap array; one stage =
-//      the heaps of G * NT trees): T steps without a global fetch, then one exit {k, L} that names
-//      the internal node to continue at and the leaves before it, or the leaf reached;
+//      the heaps of G * NT trees): T steps without a global fetch, then one exit that names the
+//      block to continue at or the leaf reached;
 //   2. below the heap the walk goes from block to block in global memory: 32 bytes, one sector, with
 //      a node, its two children and one grandchild (forest.hpp).  The tests of a block are
 //      straight-line code and end in the predicated fetch of the next one; only a test that the
@@ -30,8 +30,11 @@
 namespace b2fil {
 namespace {
 
-constexpr int kCompactThreads    = 800;   // 24 consumer warps + 1 producer warp (72 registers)
-constexpr int kCompactThreadsBig = 1024;  // 31 consumer warps + 1 producer warp (64 registers)
+// 23 consumer warps and a producer: 80 registers a thread.  A walk holds a block (8 registers) and four
+// of them are in flight; with the 64 registers that 31 consumer warps leave, the blocks spill (200
+// trees of depth 20, 300,000 fp64 rows: 28 warps 2100 us, 20 warps 1694 us, 16 warps 1864 us).
+constexpr int kCompactWarps   = 23;
+constexpr int kCompactThreads = (kCompactWarps + 1) * 32;
 
 __device__ __forceinline__ void lds_node(uint32_t a, uint32_t& value, uint32_t& meta)
 {
@@ -67,7 +70,7 @@ __device__ __forceinline__ bool test_is_open(float xl, float lo)
 }
 
 // Exact form of an fp64 test that the floats left open; `exact` points to its threshold.
-__device__ __noinline__ bool compact_exact_left(const double* row_values, const double* exact, uint32_t feat)
+__device__ __forceinline__ bool compact_exact_left(const double* row_values, const double* exact, uint32_t feat)
 {
   // rows past the end of the batch (no values) were staged as zeros
   const double x = row_values != nullptr ? __ldg(row_values + feat) : 0.0;
@@ -142,8 +145,8 @@ __device__ __forceinline__ void stage_rows_as_float(const PredictParams& p, uint
 }
 
 // Shared memory: [mbarriers 256 B][row tile][accumulators][16 B][S stages of G * NT heaps].
-template <typename T, bool CAT, int MODE, int NT, int MAXT>
-__global__ void __launch_bounds__(MAXT, 1)
+template <typename T, bool CAT, int MODE, int NT>
+__global__ void __launch_bounds__(kCompactThreads, 1)
 sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, const int G, const int S,
                       const int n_splits)
 {
@@ -353,24 +356,35 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
           for (int kk = 0; kk < NT; ++kk) right[kk] = !(xl[kk] < lo[kk]);
         };
         for (int step = 0; step < f.c_block_steps; ++step) {
-          bool r0[NT], r1[NT], r2[NT];
-          run_tests([&](int kk) { return w[kk][0]; }, [&](int kk) { return w[kk][4]; },
-                    [](int) { return 0; }, r0);
+          bool right[NT];
+          // edges to leaves (5 bits), place of the grandchild << 8, its answer << 12, root's << 13
+          uint32_t facts[NT], value[NT], half[NT];
           run_tests([&](int kk) { return w[kk][3]; }, [&](int kk) { return w[kk][5] >> 16; },
-                    [](int) { return 3; }, r2);
-          run_tests([&](int kk) { return r0[kk] ? w[kk][2] : w[kk][1]; },
-                    [&](int kk) { return r0[kk] ? w[kk][5] : w[kk][4] >> 16; },
-                    [&](int kk) { return r0[kk] ? 2 : 1; }, r1);
+                    [](int) { return 3; }, right);
+#pragma unroll
+          for (int kk = 0; kk < NT; ++kk) {
+            facts[kk] = (w[kk][4] >> 29) | ((w[kk][5] >> 10) & 0x18u) | (right[kk] ? 0x1000u : 0u) |
+                        ((w[kk][4] & BLK_HAS_FOURTH) ? (w[kk][4] >> (BLK_FOURTH_SHIFT - 8)) & 0x300u : 0x400u);
+          }
+          run_tests([&](int kk) { return w[kk][0]; }, [&](int kk) { return w[kk][4]; },
+                    [](int) { return 0; }, right);
+#pragma unroll
+          for (int kk = 0; kk < NT; ++kk) {
+            value[kk] = right[kk] ? w[kk][2] : w[kk][1];
+            half[kk]  = right[kk] ? w[kk][5] : w[kk][4] >> 16;
+            facts[kk] |= right[kk] ? 0x2000u : 0u;
+          }
+          run_tests([&](int kk) { return value[kk]; }, [&](int kk) { return half[kk]; },
+                    [&](int kk) { return (facts[kk] & 0x2000u) ? 2 : 1; }, right);
           bool walking = false;
 #pragma unroll
           for (int kk = 0; kk < NT; ++kk) {
-            const uint32_t pos    = (r0[kk] ? 2u : 0u) + (r1[kk] ? 1u : 0u);
-            const bool has        = (w[kk][4] & BLK_HAS_FOURTH) != 0u;
-            const uint32_t fourth = has ? (w[kk][4] >> BLK_FOURTH_SHIFT) & 3u : 4u;
-            const uint32_t edge   = pos + ((pos > fourth || (pos == fourth && r2[kk])) ? 1u : 0u);
-            const uint32_t mask   = (w[kk][4] >> 29) | ((w[kk][5] >> 10) & 0x18u);  // edges to leaves
-            const uint32_t before = __popc(mask & ~(0xffffffffu << edge));
-            const bool leaf       = ((mask >> edge) & 1u) != 0u;
+            const uint32_t pos    = ((facts[kk] >> 12) & 2u) + (right[kk] ? 1u : 0u);
+            const uint32_t fourth = (facts[kk] >> 8) & 7u;
+            // past the grandchild's place, or at it and to its right
+            const uint32_t edge   = pos + ((2u * pos + ((facts[kk] >> 12) & 1u) > 2u * fourth) ? 1u : 0u);
+            const uint32_t before = __popc(facts[kk] & 0x1fu & ~(0xffffffffu << edge));
+            const bool leaf       = ((facts[kk] >> edge) & 1u) != 0u;
             const uint32_t next   = leaf ? (w[kk][7] + before) | C_EXIT_LEAF : w[kk][6] + edge - before;
             const bool live       = static_cast<int32_t>(k[kk]) >= 0;
             if (live) k[kk] = next;
@@ -486,9 +500,7 @@ size_t compact_smem(const ForestView& f, size_t es, bool reduce, int R, int G, i
 template <typename T, bool CAT, int MODE>
 int launch_mode(const PredictParams& p, const CompactCfg& c, cudaStream_t stream, std::string& err)
 {
-  auto k = c.threads > kCompactThreads
-             ? sparse_compact_kernel<T, CAT, MODE, kCompactTreesInFlight, kCompactThreadsBig>
-             : sparse_compact_kernel<T, CAT, MODE, kCompactTreesInFlight, kCompactThreads>;
+  auto k = sparse_compact_kernel<T, CAT, MODE, kCompactTreesInFlight>;
   const SplitLaunch l{dim3(c.grid * c.splits), c.threads, c.smem_bytes, stream,
                       MODE <= MODE_VECTOR ? c.splits : 1, c.splits > 1};
   return launch_split(l, err, k, p, c.rows_per_tile, c.tree_groups, c.stages, c.splits);
@@ -526,7 +538,7 @@ bool compact_config(const ForestView& f, bool reduce, int rows_per_tile, int64_t
       want_splits = c;
     }
     const int n_quads     = (f.n_trees + kCompactTreesInFlight - 1) / kCompactTreesInFlight;
-    int G                 = std::max(1, std::min(31, (n_quads + want_splits - 1) / want_splits));
+    int G                 = std::max(1, std::min(kCompactWarps, (n_quads + want_splits - 1) / want_splits));
     for (; G >= 1; --G) {
       const size_t b = compact_smem(f, es, reduce, 32, G, kCompactTreesInFlight, 1);
       if (b > kMaxSmemBytes) continue;
@@ -541,7 +553,7 @@ bool compact_config(const ForestView& f, bool reduce, int rows_per_tile, int64_t
   }
   if (const int R = tuning_value("compact_R", 0), G = tuning_value("compact_G", 0),
       S = tuning_value("compact_S", 0);
-      R >= 32 && (R & (R - 1)) == 0 && R <= 128 && G >= 1 && (R / 32) * G <= 31 && S >= 1 &&
+      R >= 32 && (R & (R - 1)) == 0 && R <= 128 && G >= 1 && (R / 32) * G <= kCompactWarps && S >= 1 &&
       S <= kMaxStages) {  // tuning aid: forced shape
     const size_t b = compact_smem(f, es, reduce, R, G, kCompactTreesInFlight, S);
     if (b <= kMaxSmemBytes) {
@@ -553,12 +565,12 @@ bool compact_config(const ForestView& f, bool reduce, int rows_per_tile, int64_t
   }
   // Shared memory left unused becomes L1, which is what keeps the node fetches in flight: shapes
   // that stay under 160 KiB are preferred (measured: the same kernel runs twice as fast at
-  // 110 KiB as at 216 KiB).  Within a limit: as many warps as fit (up to 31 consumer warps; above
-  // 24 the 1024-thread build with 64 registers runs), then a second stage.
+  // 110 KiB as at 216 KiB).  Within a limit: as many warps as there are registers for, then a second
+  // stage.
   for (const size_t limit : {size_t(160) * 1024, kMaxSmemBytes}) {
     for (int R = rows_per_tile; R >= 32; R /= 2) {
       const int rw = R / 32;
-      for (int G = std::min(31 / rw, std::max(1, (f.n_trees + kCompactTreesInFlight - 1) /
+      for (int G = std::min(kCompactWarps / rw, std::max(1, (f.n_trees + kCompactTreesInFlight - 1) /
                                                     kCompactTreesInFlight));
            G >= 1; --G) {
         for (int S = 2; S >= 1; --S) {
