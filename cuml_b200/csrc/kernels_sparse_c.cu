@@ -103,42 +103,56 @@ __device__ __forceinline__ void settle_categorical_test(float& xl, float& lo, ui
   xl               = right ? 1.f : -1.f;
 }
 
-// Stage rows [row0, row0 + R) feature-major as floats (fp64 inputs rounded down).  A warp reads 32
-// consecutive features of one row and scatters them to 32 different banks.  Rows past the end of
-// the batch become zeros.  fp32 rows are asynchronous copies, fp64 rows pass through registers
-// eight loads at a time: with one load and one store in turn every 32 values cost a memory latency.
+// Stage rows [row0, row0 + R) feature-major as floats (fp64 inputs rounded down), R floats per feature,
+// so that the 32 rows of a warp are 32 banks whatever feature each lane asks for.  (With a padded
+// stride the lanes' different features shifted them over each other: three wavefronts per test operand,
+// more than half of the shared-memory traffic of the walk.)  For stores without conflicts the lanes of a
+// warp take 32 rows and, where rows start on 16-byte boundaries, 16 bytes of each; four such loads
+// are in flight together.  Rows past the end of the batch become zeros.
 template <typename T>
 __device__ __forceinline__ void stage_rows_as_float(const PredictParams& p, uint32_t tile, int R,
                                                     int64_t row0, int warp, int lane, int n_warps)
 {
-  if constexpr (sizeof(T) == 4) {
-    stage_rows_async<T>(p, tile, R, row0, warp, lane, n_warps);
-    cp_async_wait_all();
-  } else {
-    const int F             = p.f.n_features;
-    const uint32_t stride_b = (R + 1) * 4u;
-    const T* X              = static_cast<const T*>(p.X);
-    constexpr int U         = 8;
-    int rr = warp, cb = 0;  // next row of the warp, next run of 32 features
-    while (rr < R) {
-      T v[U];
-      uint32_t dst[U];  // 0: nothing to store (the tile does not start at address 0)
+  constexpr int V  = 16 / sizeof(T);  // values of a load
+  constexpr int U  = 4;
+  const int F      = p.f.n_features;
+  const int rw     = R >> 5;
+  const int wshift = 31 - __clz(rw);
+  const int items  = (F + V - 1) / V * rw;
+  const T* X       = static_cast<const T*>(p.X);
+  const bool wide  = ((reinterpret_cast<uintptr_t>(X) | (p.row_stride * sizeof(T))) & 15u) == 0;
+  for (int item = warp; item < items; item += U * n_warps) {
+    T v[U][V];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int c       = cb + lane;
-        const bool have   = rr < R && c < F;
-        const int64_t row = row0 + rr;
-        dst[u]            = have ? tile + c * stride_b + rr * 4u : 0u;
-        v[u]              = (have && row < p.n_rows) ? __ldg(X + row * p.row_stride + c) : T(0);
-        cb += 32;
-        if (cb >= F) {
-          cb = 0;
-          rr += n_warps;
-        }
+    for (int u = 0; u < U; ++u) {
+      const int it      = item + u * n_warps;
+      const int c       = (it >> wshift) * V;
+      const int64_t row = row0 + (it & (rw - 1)) * 32 + lane;
+      const bool live   = it < items && row < p.n_rows;
+      const T* at       = X + row * p.row_stride + c;
+      if (wide && c + V <= F) {
+        uint4 raw = make_uint4(0u, 0u, 0u, 0u);
+        if (live) raw = __ldg(reinterpret_cast<const uint4*>(at));
+        memcpy(v[u], &raw, 16);
+      } else {
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[u][k] = live && c + k < F ? __ldg(at + k) : T(0);
       }
+    }
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (dst[u] != 0u) Traits<float>::st_real(dst[u], __double2float_rd(v[u]));
+    for (int u = 0; u < U; ++u) {
+      const int it = item + u * n_warps;
+      const int c  = (it >> wshift) * V;
+      const int r  = (it & (rw - 1)) * 32 + lane;
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        float x;
+        if constexpr (sizeof(T) == 8) {
+          x = __double2float_rd(v[u][k]);
+        } else {
+          x = v[u][k];
+        }
+        if (it < items && c + k < F) Traits<float>::st_real(tile + ((c + k) * R + r) * 4u, x);
       }
     }
   }
@@ -165,7 +179,7 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
   const uint32_t heap_n     = 1u << TL;
   const uint32_t top_stride = static_cast<uint32_t>(f.c_top_stride);
 
-  const uint32_t stride_b    = (R + 1) * 4u;  // the tile holds floats whatever the forest precision
+  const uint32_t stride_b    = R * 4u;  // the tile holds floats whatever the forest precision
   const size_t tile_bytes    = align16(static_cast<size_t>(F) * stride_b);
   const size_t acc_bytes     = (MODE <= MODE_VECTOR) ? align16(static_cast<size_t>(G) * NC * R * TR::ES) : 0;
   unsigned char* tile_ptr    = smem + kBarBytes;
@@ -490,7 +504,7 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
 size_t compact_smem(const ForestView& f, size_t es, bool reduce, int R, int G, int NT, int S)
 {
   size_t b = kBarBytes;
-  b += align16(static_cast<size_t>(f.n_features) * (R + 1) * 4);  // the row tile holds floats
+  b += align16(static_cast<size_t>(f.n_features) * R * 4);  // the row tile holds floats
   if (reduce) b += align16(static_cast<size_t>(G) * f.n_outputs * R * es);
   b += 16;
   b += static_cast<size_t>(S) * G * NT * static_cast<size_t>(f.c_top_stride);
