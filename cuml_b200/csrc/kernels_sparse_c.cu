@@ -539,31 +539,41 @@ bool compact_config(const ForestView& f, bool reduce, int rows_per_tile, int64_t
 {
   if (!f.c_enabled) return false;
   const size_t es = f.format == FMT_SPARSE_16D ? 8 : 4;
-  // Small batches (fewer row tiles than half the SMs): one CTA per tile would walk the whole
-  // forest batch after batch, which is what bounds their latency.  The tree batches are split
-  // over CTAs instead (tiles x splits fills the SMs once; reduced outputs: the CTAs of a cluster)
-  // with few tree groups per CTA, so that there are enough batches to split.
-  const int64_t small_tiles = (n_rows + 31) / 32;
-  if (may_split && small_tiles * 2 <= sm_count && tuning_value("compact_R", 0) == 0) {
-    int want_splits = static_cast<int>(sm_count / small_tiles);
-    if (reduce) {
-      int c = kMaxCluster;
-      while (c > want_splits) c /= 2;
-      want_splits = c;
+  // Batches of up to two rounds of 128-row tiles: what counts is how many tree batches an SM walks one
+  // after the other.  The tree batches of a tile are split over CTAs (reduced outputs: a cluster) where
+  // SMs would stay idle, and tile and groups are taken with the least estimated time,
+  //   rounds of CTAs x (3 us + tree batches of a CTA x (6 us + 0.15 us per warp)),
+  // a tree batch being a chain of dependent fetches whose length hardly depends on its width (100
+  // trees of depth 18 on 10,000 rows: 128-row tiles of five groups 51 us, 64-row tiles, which take two
+  // rounds, 59 us).  More than 160 KiB of shared memory cost a quarter (the L1 keeps the fetches in
+  // flight), and large clusters that need most of the chip wait for the launch before them.
+  if (may_split && n_rows <= static_cast<int64_t>(256) * sm_count && tuning_value("compact_R", 0) == 0) {
+    const int n_quads = (f.n_trees + kCompactTreesInFlight - 1) / kCompactTreesInFlight;
+    double best       = 1e300;
+    for (int R = 32; R <= 128; R *= 2) {
+      const int rw        = R / 32;
+      const int64_t tiles = (n_rows + R - 1) / R;
+      int most            = std::min(kCompactWarps / rw, n_quads);
+      for (const size_t limit : {kMaxSmemBytes, size_t(160) * 1024}) {
+        while (most > 0 && compact_smem(f, es, reduce, R, most, kCompactTreesInFlight, 1) > limit) --most;
+        if (most == 0) break;
+        for (int C = 1; C <= (reduce ? kMaxCluster : 32); ++C) {
+          const int G         = std::min(most, (n_quads + C - 1) / C);
+          const int n_batches = (n_quads + G - 1) / G;
+          if (C > n_batches) break;
+          const double rounds = std::ceil(static_cast<double>(tiles * C) / cluster_ctas(sm_count, reduce ? C : 1));
+          const size_t smem   = compact_smem(f, es, reduce, R, G, kCompactTreesInFlight, 1);
+          const double walk   = (6.0 + 0.15 * rw * G) * (smem > size_t(160) * 1024 ? 1.25 : 1.0);
+          const double wait   = reduce && C > 4 && tiles * C > sm_count / 2 ? 2.0 : 0.0;
+          const double cost   = rounds * (3.0 + wait + (n_batches + C - 1) / C * walk);
+          if (cost < best) {
+            best = cost;
+            cfg  = CompactCfg{R, G, 1, smem, (rw * G + 1) * 32, static_cast<int>(tiles), C};
+          }
+        }
+      }
     }
-    const int n_quads     = (f.n_trees + kCompactTreesInFlight - 1) / kCompactTreesInFlight;
-    int G                 = std::max(1, std::min(kCompactWarps, (n_quads + want_splits - 1) / want_splits));
-    for (; G >= 1; --G) {
-      const size_t b = compact_smem(f, es, reduce, 32, G, kCompactTreesInFlight, 1);
-      if (b > kMaxSmemBytes) continue;
-      const int per_batch = G * kCompactTreesInFlight;
-      const int n_batches = (f.n_trees + per_batch - 1) / per_batch;
-      int splits          = std::max(1, std::min(n_batches, want_splits));
-      if (reduce)  // whole clusters at once, or fewer CTAs per cluster
-        while (splits > 1 && cluster_ctas(sm_count, splits) < small_tiles * splits) --splits;
-      cfg = CompactCfg{32, G, 1, b, (G + 1) * 32, static_cast<int>(small_tiles), splits};
-      return true;
-    }
+    if (best < 1e300) return true;
   }
   if (const int R = tuning_value("compact_R", 0), G = tuning_value("compact_G", 0),
       S = tuning_value("compact_S", 0);

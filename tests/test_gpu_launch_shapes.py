@@ -55,3 +55,20 @@ def test_rank_prepass_over_ragged_feature_groups(n_features, precision):
         X[-1, 0] = np.nan
         X[1, 0], X[2, 0] = np.inf, -np.inf
         _all_kinds(desc, X, precision, "depth_first", "dense", chunk_size=chunk)
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("n_trees,n_features", [(3, 5), (61, 9), (190, 40)])
+def test_deep_trees_at_batch_sizes_where_the_launch_shape_changes(n_trees, n_features, precision):
+    """Blocks of four nodes below the heaps: trees deep enough for several blocks on a walk, values
+    that hit thresholds (open tests), unaligned rows, and row counts around the edges of tiles,
+    clusters and rounds of CTAs."""
+    import numpy as np
+
+    desc = random_forest_desc(93, n_trees=n_trees, n_features=n_features, max_depth=15, p_leaf=0.2,
+                              mixed_ops=True)
+    thr = desc.threshold[desc.node_kind == 1]
+    for n in (1, 129, 1025, 4750, 9473, 19_001):
+        X = random_rows(n, n, n_features, np.float64, nan_frac=0.02)
+        X[::3, 0] = np.resize(thr, len(X[::3]))
+        _all_kinds(desc, X, precision, "depth_first", "sparse")
