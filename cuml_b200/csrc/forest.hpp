@@ -79,10 +79,11 @@ struct SparseNode16D {  // fp64
 // stride between features and adds the row's address.
 // Categorical features (every test on them is categorical, every listed category below 32) keep
 // their place in the same scheme: the "rank" of a value is its category (Q_NO_CATEGORY when it is
-// negative, fractional-truncated out of range or too large), and in such forests every node is
-// 8 bytes {node, 32-bit category set} (a numerical node holds an empty set), fetched with one
-// load; a set bit sends the row right.  (A categorical node is recognisable by j = Q_MAX_RANK_FIELD; the walk does not need
-// to know, and the low half of every node stays a clean feature * 4 for the address arithmetic.)  The sets are stored bit-reversed (category c in bit 31 - c) and a categorical node
+// negative, fractional-truncated out of range or too large), and in such forests every node has
+// a 32-bit category set (8 bytes {node, set} in the packed host image; before the upload
+// split_category_sets moves the sets of a tree behind its nodes); a set bit sends the row right.  A
+// categorical node is recognisable by j = Q_MAX_RANK_FIELD, and the walk loads the set only there;
+// the low half of every node stays a clean feature * 4 for the address arithmetic.  The sets are stored bit-reversed (category c in bit 31 - c) and a categorical node
 // carries the largest rank, so its rank comparison always says "left" and the walk can simply OR
 // the two answers: sign(node - (code << 17)) | sign(set << code).
 // Row tiles that hold missing values are walked with a second image of the nodes where room allows
