@@ -131,18 +131,6 @@ __device__ __forceinline__ void consumer_sync(int n_threads)
   asm volatile("bar.sync 1, %0;" ::"r"(n_threads) : "memory");
 }
 
-// Asynchronous copy of one 4- or 8-byte element global -> shared memory; zeros where !live.
-template <uint32_t BYTES>
-__device__ __forceinline__ void cp_async(uint32_t dst, const void* src, bool live)
-{
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(BYTES),
-               "r"(live ? BYTES : 0u)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all()
-{
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
 // Thread-block clusters: barrier over the live threads of all CTAs, and a read of another CTA's
 // shared memory (`a`: the address the datum has in this CTA).
 __device__ __forceinline__ void cluster_arrive()
@@ -334,48 +322,80 @@ __device__ __forceinline__ bool goes_right(typename Traits<T>::Val v, uint32_t m
 // shared pieces of both kernels: row-tile staging, accumulation of a leaf, epilogue
 // ---------------------------------------------------------------------------------------------
 
-// Stage rows [row0, row0+R) feature-major.  A warp reads 32 consecutive features of one row
-// (one 128-byte line for fp32) and scatters them to 32 different banks.  Rows past the end of the
-// batch are filled with zeros.  Returns true when this thread saw a NaN.
-template <typename T>
-__device__ __forceinline__ bool stage_rows(const PredictParams& p, uint32_t tile, int R,
-                                           int64_t row0, int warp, int lane, int n_warps)
+// The tile of stage_rows, V neighbouring values of one row per lane and item, U items in flight.  No
+// branch per load: dead lanes and items past the end read the tile's first row (one address for all of
+// them), and only the stores look at them (with a branch around every load the smallest predictions took 0.3 to
+// 0.8 us longer, up to a tenth).
+template <typename T, typename OUT, bool WIDE>
+__device__ __forceinline__ bool stage_items(const PredictParams& p, uint32_t tile, int R, int64_t row0,
+                                            int warp, int lane, int n_warps)
 {
-  const int F             = p.f.n_features;
-  const uint32_t stride_b = (R + 1) * Traits<T>::ES;
-  const T* X              = static_cast<const T*>(p.X);
-  bool saw_nan            = false;
-  for (int rr = warp; rr < R; rr += n_warps) {
-    const int64_t row = row0 + rr;
-    const bool live   = row < p.n_rows;
-    const T* src      = X + row * p.row_stride;
-    for (int c = lane; c < F; c += 32) {
-      const T v = live ? __ldg(src + c) : T(0);
-      saw_nan |= (v != v);
-      Traits<T>::st_real(tile + c * stride_b + rr * Traits<T>::ES, v);
+  constexpr int V       = 16 / sizeof(T);
+  constexpr int U       = 4;
+  constexpr uint32_t ES = sizeof(OUT);
+  const int F           = p.f.n_features;
+  const int rw          = R >> 5;
+  const int wshift      = 31 - __clz(rw);
+  const int items       = (F + V - 1) / V * rw;
+  const T* X            = static_cast<const T*>(p.X) + row0 * p.row_stride;
+  const int n_live      = static_cast<int>(min(static_cast<int64_t>(R), p.n_rows - row0));
+  bool saw_nan          = false;
+  for (int item = warp; item < items; item += U * n_warps) {
+    T v[U][V];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int it    = item + u * n_warps;
+      const int r     = (it & (rw - 1)) * 32 + lane;
+      const int c     = (min(it, items - 1) >> wshift) * V;
+      const bool live = it < items && r < n_live;
+      const T* at     = X + static_cast<int64_t>(live ? r : 0) * p.row_stride;
+      if constexpr (WIDE) {
+        const uint4 raw = __ldg(reinterpret_cast<const uint4*>(at + c));
+        memcpy(v[u], &raw, 16);
+      } else {
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[u][k] = __ldg(at + min(c + k, F - 1));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int it = item + u * n_warps;
+      const int r  = (it & (rw - 1)) * 32 + lane;
+      const int c  = (it >> wshift) * V;
+      if (it >= items) break;
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const T x = r < n_live ? v[u][k] : T(0);
+        saw_nan |= x != x;
+        OUT y;
+        if constexpr (sizeof(T) > sizeof(OUT)) {
+          y = __double2float_rd(x);
+        } else {
+          y = x;
+        }
+        if (WIDE || c + k < F) Traits<OUT>::st_real(tile + ((c + k) * R + r) * ES, y);
+      }
     }
   }
   return saw_nan;
 }
 
-// The same for small batches, where what counts is the time until the tile is there: every element
-// is an asynchronous copy of its own, so all of them are in flight together and no register waits
-// (loads and stores in turn cost one memory latency per row and 32 features: 5 of the 12 us of a
-// 1,000-row prediction).  NaN is not looked for; the caller walks as if there were some.
-template <typename T>
-__device__ __forceinline__ void stage_rows_async(const PredictParams& p, uint32_t tile, int R,
-                                                 int64_t row0, int warp, int lane, int n_warps)
+// Stage rows [row0, row0 + R) feature-major, R elements per feature, so that the 32 rows of a warp are
+// 32 banks whatever feature each lane asks for.  (With a padded stride the lanes' different features
+// shifted them over each other: three wavefronts per test operand, more than half of the
+// shared-memory traffic of the sparse walk; dense fp32 walk, 500 trees of depth 8 x 200,000 rows
+// without ranks: 652 -> 523 us.)  For stores without conflicts the lanes of a warp take 32 rows and 16
+// bytes of each, in one load where rows start on 16-byte boundaries.  OUT is T, or float for doubles
+// that are rounded down.  Rows past the end of the batch become zeros.  Returns true when this thread
+// saw a NaN.
+template <typename T, typename OUT>
+__device__ __forceinline__ bool stage_rows(const PredictParams& p, uint32_t tile, int R,
+                                           int64_t row0, int warp, int lane, int n_warps)
 {
-  const int F             = p.f.n_features;
-  const uint32_t stride_b = (R + 1) * Traits<T>::ES;
-  const T* X              = static_cast<const T*>(p.X);
-  for (int rr = warp; rr < R; rr += n_warps) {
-    const int64_t row = row0 + rr;
-    const bool live   = row < p.n_rows;
-    const T* src      = X + (live ? row : row0) * p.row_stride;
-    for (int c = lane; c < F; c += 32)
-      cp_async<Traits<T>::ES>(tile + c * stride_b + rr * Traits<T>::ES, src + c, live);
-  }
+  const bool wide = ((reinterpret_cast<uintptr_t>(p.X) | (p.row_stride * sizeof(T)) |
+                      (p.f.n_features * sizeof(T))) & 15u) == 0;
+  return wide ? stage_items<T, OUT, true>(p, tile, R, row0, warp, lane, n_warps)
+              : stage_items<T, OUT, false>(p, tile, R, row0, warp, lane, n_warps);
 }
 
 template <typename T>

@@ -1,7 +1,7 @@
 // Prediction kernels for sm_100a.
 //
 // Work decomposition (both storages): a CTA owns a tile of R consecutive rows, staged once in
-// shared memory feature-major (`tile[f][r]`, row stride R+1 elements) so that the 32 lanes of a
+// shared memory feature-major (`tile[f][r]`) so that the 32 lanes of a
 // warp - 32 different rows - always read 32 different banks whatever feature each lane needs.
 // Warps are organised as (R/32 row sets) x (G tree groups): every warp walks its 32 rows through
 // the trees of its group, NT trees at a time for instruction-level parallelism, and keeps its
@@ -157,16 +157,16 @@ struct DenseWalker {
   }
 };
 
-// small: a small batch.  With n_splits > 1 the trees of a row tile are split over n_splits CTAs,
-// each of which streams and walks only its share.  Reduced outputs launch those CTAs as a cluster and
-// meet in its distributed shared memory (finish_cluster_rows); per-tree outputs need no meeting.
+// With n_splits > 1 (small batches) the trees of a row tile are split over n_splits CTAs, each of
+// which streams and walks only its share.  Reduced outputs launch those CTAs as a cluster and meet
+// in its distributed shared memory (finish_cluster_rows); per-tree outputs need no meeting.
 // What bounds such a launch is latency: launch, tile, trees, walk, sum, one after the other.  So
 // the barriers are set up and the trees requested before grid_wait(), while the kernel before
-// this one may still be running, and the row tile arrives by asynchronous copies.
+// this one may still be running.
 template <typename T, bool CAT, int MODE, int NT>
 __global__ void __launch_bounds__(544, 1)
 dense_kernel(const __grid_constant__ PredictParams p, const int R, const int G, const int S,
-             const int n_splits, const bool small)
+             const int n_splits)
 {
   using TR = Traits<T>;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -179,7 +179,7 @@ dense_kernel(const __grid_constant__ PredictParams p, const int R, const int G, 
   const int warp      = threadIdx.x >> 5;
   const int lane      = threadIdx.x & 31;
 
-  const uint32_t stride_b   = (R + 1) * TR::ES;
+  const uint32_t stride_b   = R * TR::ES;
   const size_t tile_bytes   = align16(static_cast<size_t>(F) * stride_b);
   const size_t acc_bytes    = (MODE <= MODE_VECTOR) ? align16(static_cast<size_t>(G) * NC * R * TR::ES) : 0;
   unsigned char* tile_ptr   = smem + kBarBytes;
@@ -246,17 +246,11 @@ dense_kernel(const __grid_constant__ PredictParams p, const int R, const int G, 
   grid_wait();
   for (int64_t t = blockIdx.x / n_splits; t < n_tiles; t += tile_step) {
     const int64_t row0 = t * R;
-    bool saw_nan       = true;
-    if (small) {
-      stage_rows_async<T>(p, tile, R, row0, warp, lane, n_cw);
-    } else {
-      saw_nan = stage_rows<T>(p, tile, R, row0, warp, lane, n_cw);
-    }
+    const bool saw_nan = stage_rows<T, T>(p, tile, R, row0, warp, lane, n_cw);
     if (MODE <= MODE_VECTOR) {
       for (int i = threadIdx.x; i < G * NC * R; i += n_ct) acc[i] = T(0);
     }
     if (__any_sync(0xffffffffu, saw_nan) && lane == 0) flags[0] = 1;
-    if (small) cp_async_wait_all();
     consumer_sync(n_ct);
     const bool nans = flags[0] != 0;
     Running<T> run{T(0), 0, {}};
@@ -676,7 +670,7 @@ sparse_kernel(const PredictParams p, const int R, const int G, const int rows_in
   const bool dfs      = f.layout == B2FIL_LAYOUT_DEPTH_FIRST;
   const int fb        = f.feat_bits;
 
-  const uint32_t stride_b = (R + 1) * TR::ES;
+  const uint32_t stride_b = R * TR::ES;
   const size_t tile_bytes = rows_in_smem ? align16(static_cast<size_t>(F) * stride_b) : 0;
   T* acc                  = reinterpret_cast<T*>(smem + tile_bytes);
   T* acc_group            = acc + static_cast<size_t>(g) * NC * R;
@@ -689,7 +683,7 @@ sparse_kernel(const PredictParams p, const int R, const int G, const int rows_in
   for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const int64_t row0 = t * R;
     const int64_t row  = row0 + r;
-    if (rows_in_smem) stage_rows<T>(p, tile, R, row0, warp, lane, n_warps);
+    if (rows_in_smem) stage_rows<T, T>(p, tile, R, row0, warp, lane, n_warps);
     if (MODE <= MODE_VECTOR) {
       for (int i = threadIdx.x; i < G * NC * R; i += n_warps * 32) acc[i] = T(0);
     }
@@ -759,7 +753,7 @@ size_t dense_smem(int depth, int precision, int F, int NC, bool reduce, int R, i
 {
   const size_t es = precision == B2FIL_F32 ? 4 : 8;
   size_t b        = kBarBytes;
-  b += align16(static_cast<size_t>(F) * (R + 1) * es);
+  b += align16(static_cast<size_t>(F) * R * es);
   if (reduce) b += align16(static_cast<size_t>(G) * NC * R * es);
   b += 16;
   b += static_cast<size_t>(S) * G * NT * dense_tree_stride(depth, precision);
@@ -780,7 +774,7 @@ int launch_dense_mode(const PredictParams& p, const DenseCfg& c, const SplitLaun
                       std::string& err)
 {
   auto k = c.trees_in_flight == 2 ? dense_kernel<T, CAT, MODE, 2> : dense_kernel<T, CAT, MODE, 1>;
-  return launch_split(l, err, k, p, c.rows_per_tile, c.tree_groups, c.stages, n_splits, l.overlap);
+  return launch_split(l, err, k, p, c.rows_per_tile, c.tree_groups, c.stages, n_splits);
 }
 
 template <typename T, bool CAT>
@@ -1351,9 +1345,10 @@ double rank_path_us(const ForestView& f, int mode, int64_t n_rows, int sm_count)
 // `fixed` is what every CTA spends on starting, meeting and finishing, `rows` and `trees` the time
 // to bring the row tile and the CTA's trees in at the 48 bytes per cycle an SM gets from L2, `walk`
 // the steps of its tree batches, each bound by the latency of two dependent shared-memory loads
-// or by the wavefronts of all its warps (5.6 per warp and step in fp32, 9 in fp64).  Checked
-// against all shapes of four forests (100 depth-6 to 1000 depth-8 trees; 1,000 and 4,000 rows): it
-// picked the fastest each time (5.5 / 7.1 / 17.1 / 36.1 us).
+// or by the wavefronts of all its warps (4 per warp and step in fp32, 7 in fp64: a little above the
+// 3.7 and 6.1 of large batches, at which fp64 took shapes a quarter slower).  Of 13 forests from 1 to
+// 18,000 rows, 5.6 sent 300 depth-6 trees x 5,000 rows to the rank path (17.7 us, now 14.6) and
+// 400 depth-9 trees x 2,500 rows (20.6, now 18.4).
 struct SplitShape {
   DenseCfg c;
   int n_splits;
@@ -1366,7 +1361,7 @@ bool pick_split_shape(const ForestView& f, int mode, int precision, int64_t n_ro
   const bool reduce   = mode <= MODE_VECTOR;
   const double es     = precision == B2FIL_F32 ? 4 : 8;
   const double stride = static_cast<double>(dense_tree_stride(f.dense_depth, precision));
-  const double wave_w = (precision == B2FIL_F32 ? 5.6 : 9.0) * (f.has_categorical ? 2.0 : 1.0);
+  const double wave_w = (precision == B2FIL_F32 ? 4.0 : 7.0) * (f.has_categorical ? 2.0 : 1.0);
   const double leaf_w = mode == MODE_SCALAR ? 4.0 : (mode == MODE_VECTOR ? 32.0 : 64.0);
   const int depth     = std::max(1, f.dense_depth);
   double best_cost    = 1e300;
@@ -1565,7 +1560,7 @@ int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStr
     int rows_in_smem = 1;
     for (;;) {
       acc_b  = reduce ? align16(static_cast<size_t>(G) * f.n_outputs * R * es) : 0;
-      tile_b = align16(static_cast<size_t>(f.n_features) * (R + 1) * es);
+      tile_b = align16(static_cast<size_t>(f.n_features) * R * es);
       if (acc_b + tile_b <= kMaxSmemBytes) break;
       if (R > 32) {
         R /= 2;

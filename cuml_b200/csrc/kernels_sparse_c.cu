@@ -103,61 +103,6 @@ __device__ __forceinline__ void settle_categorical_test(float& xl, float& lo, ui
   xl               = right ? 1.f : -1.f;
 }
 
-// Stage rows [row0, row0 + R) feature-major as floats (fp64 inputs rounded down), R floats per feature,
-// so that the 32 rows of a warp are 32 banks whatever feature each lane asks for.  (With a padded
-// stride the lanes' different features shifted them over each other: three wavefronts per test operand,
-// more than half of the shared-memory traffic of the walk.)  For stores without conflicts the lanes of a
-// warp take 32 rows and, where rows start on 16-byte boundaries, 16 bytes of each; four such loads
-// are in flight together.  Rows past the end of the batch become zeros.
-template <typename T>
-__device__ __forceinline__ void stage_rows_as_float(const PredictParams& p, uint32_t tile, int R,
-                                                    int64_t row0, int warp, int lane, int n_warps)
-{
-  constexpr int V  = 16 / sizeof(T);  // values of a load
-  constexpr int U  = 4;
-  const int F      = p.f.n_features;
-  const int rw     = R >> 5;
-  const int wshift = 31 - __clz(rw);
-  const int items  = (F + V - 1) / V * rw;
-  const T* X       = static_cast<const T*>(p.X);
-  const bool wide  = ((reinterpret_cast<uintptr_t>(X) | (p.row_stride * sizeof(T))) & 15u) == 0;
-  for (int item = warp; item < items; item += U * n_warps) {
-    T v[U][V];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int it      = item + u * n_warps;
-      const int c       = (it >> wshift) * V;
-      const int64_t row = row0 + (it & (rw - 1)) * 32 + lane;
-      const bool live   = it < items && row < p.n_rows;
-      const T* at       = X + row * p.row_stride + c;
-      if (wide && c + V <= F) {
-        uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-        if (live) raw = __ldg(reinterpret_cast<const uint4*>(at));
-        memcpy(v[u], &raw, 16);
-      } else {
-#pragma unroll
-        for (int k = 0; k < V; ++k) v[u][k] = live && c + k < F ? __ldg(at + k) : T(0);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int it = item + u * n_warps;
-      const int c  = (it >> wshift) * V;
-      const int r  = (it & (rw - 1)) * 32 + lane;
-#pragma unroll
-      for (int k = 0; k < V; ++k) {
-        float x;
-        if constexpr (sizeof(T) == 8) {
-          x = __double2float_rd(v[u][k]);
-        } else {
-          x = v[u][k];
-        }
-        if (it < items && c + k < F) Traits<float>::st_real(tile + ((c + k) * R + r) * 4u, x);
-      }
-    }
-  }
-}
-
 // Shared memory: [mbarriers 256 B][row tile][accumulators][16 B][S stages of G * NT heaps].
 template <typename T, bool CAT, int MODE, int NT>
 __global__ void __launch_bounds__(kCompactThreads, 1)
@@ -249,7 +194,7 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
   for (int64_t t = tile0; t < n_tiles; t += tile_step) {
     const int64_t row0 = t * R;
     const int64_t row  = row0 + r;
-    stage_rows_as_float<T>(p, tile, R, row0, warp, lane, n_cw);
+    stage_rows<T, float>(p, tile, R, row0, warp, lane, n_cw);
     if (MODE <= MODE_VECTOR) {
       for (int i = threadIdx.x; i < G * NC * R; i += n_ct) acc[i] = T(0);
     }
