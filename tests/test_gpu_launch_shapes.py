@@ -72,3 +72,18 @@ def test_deep_trees_at_batch_sizes_where_the_launch_shape_changes(n_trees, n_fea
         X = random_rows(n, n, n_features, np.float64, nan_frac=0.02)
         X[::3, 0] = np.resize(thr, len(X[::3]))
         _all_kinds(desc, X, precision, "depth_first", "sparse")
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("n_features", [1, 3, 4, 6, 50, 132])
+def test_row_tiles_of_every_alignment(n_features, precision):
+    """Rows that start on 16-byte boundaries and rows that do not, fewer columns than one load and
+    more than the warps of a CTA bring at once, full and partial tiles, and one missing value in the
+    batch, in its last row and column: the kernels that stage rows themselves must see it."""
+    desc = random_forest_desc(93, n_trees=33, n_features=n_features, max_depth=7)
+    for storage, kw in (("dense", dict(quantize_rows=False)), ("sparse", {}),
+                        ("sparse", dict(compact_nodes=False))):
+        for n in (1, 31, 33, 600, 30_001):
+            X = random_rows(n, n, n_features, "float64", nan_frac=0.0)
+            X[-1, -1] = float("nan")
+            _all_kinds(desc, X, precision, "depth_first", storage, **kw)
