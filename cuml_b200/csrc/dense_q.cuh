@@ -125,6 +125,7 @@ struct DenseQWalker {
     const uint32_t mine    = static_cast<uint32_t>(g * NT) * tstride;  // this warp's trees in a sub-batch
     const uint32_t sub_b   = static_cast<uint32_t>(per_sub) * tstride;
     bool ok                = true;
+    uint32_t seen          = 0u;  // what release_stage() cannot tell from the sums, folded
 
     // LEAFG: payloads requested by the previous sub-batch, not yet added
     uint32_t pend[NT] = {};
@@ -269,6 +270,7 @@ struct DenseQWalker {
         for (int k = 0; k < NT; ++k) {
           const uint32_t slot = idx[k] - (1u << D);
           const int tree      = first + (FULL ? k : min(k, n_act - 1));
+          seen ^= slot;
           pend[k] = __ldg(reinterpret_cast<const uint32_t*>(
             image + static_cast<size_t>(tree) * static_cast<size_t>(f.q_tree_stride) + slot * 4u));
         }
@@ -372,6 +374,7 @@ struct DenseQWalker {
               continue;
             }
             const typename TR::Val payload = TR::ld_val(leaf_a);
+            if (MODE == MODE_VECTOR) seen ^= TR::low32(payload);
             if (MODE == MODE_SCALAR && CAT && same_class) {
               run.sum += TR::as_real(payload);
             } else {
@@ -399,8 +402,11 @@ struct DenseQWalker {
           }
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bars + 8u * (kMaxStages + s));
+      // (payloads that were stored to global memory or to the accumulators have been read)
+      bool read = seen != 0xffffffffu;
+      if ((MODE == MODE_SCALAR && !LEAFG) || (MODE == MODE_VECTOR && inline_vec))
+        read = sums_known<T, MODE>(run);
+      release_stage(bars + 8u * (kMaxStages + s), lane, read, p.zero);
       pos.advance(S);
     }
     if constexpr (LEAFG) take_pending();

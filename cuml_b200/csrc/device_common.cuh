@@ -89,6 +89,20 @@ __device__ __forceinline__ void report_status(int32_t* status, int32_t code)
 {
   *reinterpret_cast<volatile int32_t*>(status) = code;
 }
+// A warp gives a stage of the ring back to the producer.  The arrival does not wait for shared-memory
+// loads that the warp has issued, and the bulk copy that refills the stage does not queue behind
+// them as another warp's store would: a load that is held up (the walk of deep forests fills the
+// load pipe with fetches from HBM) then reads the next batch.  200 trees of depth 20 in fp64, 200,000
+// rows: one prediction in twelve had a few leaves of the wrong tree.  So the arrival depends on what was
+// read: `read` is any condition on the last values that this lane has loaded from the stage (all
+// loads before them fed their addresses), the vote needs it from every lane, and the arrival's
+// address needs the vote, by way of a zero that only the host knows to be one.
+__device__ __forceinline__ void release_stage(uint32_t bar, int lane, bool read, uint32_t zero)
+{
+  const uint32_t all = __ballot_sync(0xffffffffu, read);
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bar + (all & zero));
+}
 // Position in a ring of S stages: the stage index and the parity of its current use, advanced
 // without a division.
 struct RingPos {
@@ -623,6 +637,17 @@ __device__ __forceinline__ void store_quads(V* out, int64_t width, int64_t row, 
   if (first + 1 < n_rows) at[width] = v1;
   if (first + 2 < n_rows) at[2 * width] = v2;
   if (first + 3 < n_rows) at[3 * width] = v3;
+}
+
+// A condition on the running sums for release_stage(): a reduced walk adds every leaf it reads to them.
+template <typename T, int MODE>
+__device__ __forceinline__ bool sums_known(const Running<T>& run)
+{
+  if (MODE == MODE_SCALAR) return run.sum == run.sum;
+  bool b = true;
+#pragma unroll
+  for (int c = 0; c < kRegClasses; ++c) b = b && run.v[c] == run.v[c];
+  return b;
 }
 
 // Add a thread's running sums to its accumulators in shared memory (end of a row tile), or store

@@ -109,6 +109,7 @@ struct DenseWalker {
     const uint32_t width_b = (1u << D) * TR::NB;  // bytes of the node array of one tree
     const int per_batch    = G * NT;
     bool ok                = true;
+    uint32_t seen          = 0u;  // the payloads read, folded
     for (int batch = t_begin; batch < t_end; batch += per_batch) {
       const uint32_t s = pos.stage;
       if (ok) ok = mbar_wait(bars + 8u * s, pos.phase);
@@ -142,6 +143,7 @@ struct DenseWalker {
             if (k < n_act) {
               const uint32_t slot = (a[k] - base[k]) / TR::NB - (1u << D);
               const typename TR::Val payload = TR::ld_val(base[k] + width_b + slot * TR::ES);
+              seen ^= TR::low32(payload);
               take_leaf<T, MODE>(p, first + k, payload,
                                  (static_cast<uint32_t>(first + k) << D) + slot, acc_group, R, r,
                                  row, run);
@@ -149,8 +151,9 @@ struct DenseWalker {
           }
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bars + 8u * (kMaxStages + s));
+      // (scalar leaves: their sum will do; the others are folded on the way)
+      release_stage(bars + 8u * (kMaxStages + s), lane,
+                    MODE == MODE_SCALAR ? sums_known<T, MODE>(run) : seen != 0xffffffffu, p.zero);
       pos.advance(S);
     }
     return ok;

@@ -23,6 +23,7 @@ struct PredictParams {
   // HOST memory, never read on the device: three top nodes per tree of the rank-quantised copy
   // (PackedForest::q_top), or null; the launch code copies them into a kernel parameter
   const uint32_t* q_top;
+  uint32_t zero;       // always 0, which the compiler must not know (see release_stage)
 };
 
 // Shape of one dense launch.

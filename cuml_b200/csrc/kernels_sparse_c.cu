@@ -268,8 +268,12 @@ sparse_compact_kernel(const __grid_constant__ PredictParams p, const int R, cons
         }
       }
       // the heaps of this batch are no longer needed: let the producer refill the stage
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bars + 8u * (kMaxStages + s));
+      uint32_t exits = 0u;
+      if (n_act > 0) {
+#pragma unroll
+        for (int kk = 0; kk < NT; ++kk) exits ^= k[kk];
+      }
+      release_stage(bars + 8u * (kMaxStages + s), lane, exits != 0xffffffffu, p.zero);
       pos.advance(S);
       if (n_act > 0) {
         // part 2: blocks in global memory.  All lanes of the warp do the three tests of the block

@@ -87,3 +87,28 @@ def test_row_tiles_of_every_alignment(n_features, precision):
             X = random_rows(n, n, n_features, "float64", nan_frac=0.0)
             X[-1, -1] = float("nan")
             _all_kinds(desc, X, precision, "depth_first", storage, **kw)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_deep_forest_beyond_the_caches_repeats_itself(dtype):
+    """Leaf ids of a forest whose nodes come from HBM, predicted again and again, against the kernel
+    that stages no trees: the loads of a heap are held up behind node fetches for longer than it takes
+    to refill the heap's stage, so a stage that is given back before they have arrived shows here (one
+    call in sixty of this fp64 forest)."""
+    import torch
+
+    from cuml_b200.fil import ForestInference
+    from perf import cases
+
+    case = dict(cases.BASE, forest="regressor", trees=200, depth=20, leaves=60_000, features=64,
+                dtype=dtype, rows=200_000, call="apply")
+    g = torch.Generator(device="cuda:0")
+    g.manual_seed(5)
+    desc = cases._bagged_forest(case, g, "cuda:0")
+    X = cases._rows(case, g, "cuda:0")
+    kw = dict(precision="double" if dtype == "float64" else "single", storage="sparse")
+    want = ForestInference.load_from_treelite_model(desc, compact_nodes=False, **kw).apply(X)
+    fi = ForestInference.load_from_treelite_model(desc, **kw)
+    assert fi.describe()["compact_image"] == 1
+    differing = [int((fi.apply(X) != want).sum()) for _ in range(400)]
+    assert max(differing) == 0, f"{sum(d > 0 for d in differing)} of 400 calls, up to {max(differing)} ids"
