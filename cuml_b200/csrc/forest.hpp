@@ -375,6 +375,15 @@ inline uint32_t q_bucket_host(T x, T scale, T offset, uint32_t n_buckets)
 constexpr uint32_t kQGroupSmemBudget = 208 * 1024;
 constexpr uint32_t kQMaxGroupFeatures = 32;
 
+// Rows of a tile for a caller's chunk_size > 0 (units of 32 rows): rounded down to a power of two, which
+// is what every kernel's tile arithmetic needs, and at most `most`, itself a power of two.
+inline int chunk_rows(int chunk_size, int most)
+{
+  int rows = 32;
+  while (rows < most && rows / 16 <= chunk_size) rows *= 2;
+  return rows;
+}
+
 // Before the upload: the blocks of a forest with a compact image.  False when a field does not fit.
 bool build_blocks(PackedForest& pf);
 

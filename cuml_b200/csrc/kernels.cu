@@ -871,7 +871,7 @@ bool dense_q_config(size_t qstride, int max_nt, int precision, int F, int NC, bo
 {
   int want = 256;
   if (chunk_size > 0) {
-    want = std::min(256, std::max(32, 32 * chunk_size));
+    want = chunk_rows(chunk_size, 256);
   } else {
     // tiles are cut between CTAs, so their number need not fill the SMs; larger ones stream the
     // forest less often.  Smaller ones serve forests with few visits per row, which have too few
@@ -1253,7 +1253,7 @@ int fixed_scratch_address(int device, void** out, std::string& err)
 
 int pick_rows_per_tile(int64_t n_rows, int chunk_size, int sm_count)
 {
-  if (chunk_size > 0) return std::min(128, std::max(32, 32 * chunk_size));
+  if (chunk_size > 0) return chunk_rows(chunk_size, 128);
   // keep every SM busy before growing the tile
   if (n_rows >= static_cast<int64_t>(128) * sm_count) return 128;
   if (n_rows >= static_cast<int64_t>(64) * sm_count) return 64;

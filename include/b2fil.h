@@ -255,7 +255,8 @@ int64_t b2fil_output_elems_per_row(const b2fil_forest* f, int infer_kind);
 /* Batched prediction, device buffers.  X_dev: row-major (n_rows, n_features) of the forest's
  * precision with `row_stride` elements between rows; out_dev: n_rows *
  * b2fil_output_elems_per_row() elements (precision type; uint32 for LEAF_ID, int32 for CLASS).
- * chunk_size 0 = the forest's default.  `threshold` is the binary decision threshold of
+ * chunk_size 0 = the forest's default; positive values ask for row tiles of 32 * chunk_size rows and are
+ * rounded down to a power of two.  `threshold` is the binary decision threshold of
  * B2FIL_INFER_CLASS for one-output classifiers.  Enqueues on cuda_stream (NULL = default stream)
  * of the forest's device and does not synchronise.  Two cases take stream-ordered scratch from a
  * memory pool owned by the forest (cached between calls): forests whose b2fil_info reports

@@ -315,6 +315,8 @@ int64_t walk_compact(const PackedForest& pf, const T* X, int64_t n_rows, int64_t
 extern "C" {
 const char* pack_check_error() { return g_err.c_str(); }
 
+int pack_check_chunk_rows(int chunk_size, int most) { return chunk_rows(chunk_size, most); }
+
 // Packs `desc` and walks n_rows rows.  ids: leaf id per (row, tree); payload: scalar leaf value
 // (or vector index) per (row, tree).  info[0..5] = format, storage, dense_depth, node_bytes,
 // n_nodes_packed, feat_bits; info[6] = 1 when a rank-quantised copy was built, info[7] = number of

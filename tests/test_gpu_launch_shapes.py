@@ -112,3 +112,29 @@ def test_deep_forest_beyond_the_caches_repeats_itself(dtype):
     assert fi.describe()["compact_image"] == 1
     differing = [int((fi.apply(X) != want).sum()) for _ in range(400)]
     assert max(differing) == 0, f"{sum(d > 0 for d in differing)} of 400 calls, up to {max(differing)} ids"
+
+
+@pytest.mark.parametrize("kw", [dict(storage="dense", quantize_rows=False), dict(storage="dense"),
+                                dict(storage="sparse"), dict(storage="sparse", compact_nodes=False)])
+def test_any_chunk_size_of_the_c_interface(kw):
+    """The C interface takes every chunk_size (the Python layer only powers of two): row tiles are
+    rounded down to a power of two, and results do not depend on them."""
+    import numpy as np
+    import torch
+
+    from cuml_b200.fil import ForestInference, _lib
+    from cuml_b200.fil._desc import INFER_LEAF_ID
+    from oracle import oracle
+
+    desc = random_forest_desc(94, n_trees=40, n_features=18, max_depth=7)
+    X = random_rows(5, 20_001, 18, np.float32, nan_frac=0.02)
+    want = oracle.predict(desc, X, INFER_LEAF_ID, "single")
+    Xd = torch.as_tensor(X, device="cuda:0")
+    fi = ForestInference.load_from_treelite_model(desc, **kw)
+    for n in (97, 20_001):
+        for chunk in (3, 5, 6, 7, 9, 2**26, 2**31 - 1):
+            out = torch.full((n, 40), -1, dtype=torch.int32, device="cuda:0")
+            _lib.check(_lib.load().b2fil_predict(
+                fi.forest.handle, INFER_LEAF_ID, Xd.data_ptr(), n, 18, out.data_ptr(), chunk, 0.5,
+                torch.cuda.current_stream().cuda_stream))
+            assert np.array_equal(out.cpu().numpy().astype(np.uint32), want[:n]), (n, chunk)

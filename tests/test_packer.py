@@ -291,3 +291,11 @@ def test_heap_levels_of_the_compact_image_follow_the_row_tile(pack_check):
         levels[n_features] = int(info[14])
     assert levels[24] == 8
     assert 1 <= levels[1000] < 8
+
+
+def test_row_tiles_of_any_chunk_size_are_powers_of_two(pack_check):
+    """The kernels index a row tile with shifts and masks; the C ABI takes any chunk_size."""
+    for most in (128, 256):
+        for chunk in (*range(1, 40), 2**26, 2**26 + 1, 2**31 - 1):
+            want = 32 << (min(chunk, most // 32).bit_length() - 1)
+            assert pack_check.pack_check_chunk_rows(chunk, most) == want, (chunk, most)
