@@ -70,10 +70,15 @@ __global__ void bounded_wait_selftest_kernel(int32_t* status, const uint32_t tri
 // Bound by the link (45 of its 55 GB/s from 4 MB on): four 16-byte loads in flight per thread and a
 // thread for every 64 bytes, as long as the SMs hold them, cover its 1.5 us.
 __global__ void __launch_bounds__(256)
-fetch_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, const uint32_t n)
+fetch_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, const uint32_t n,
+             const uint32_t tail_words)
 {
   grid_release();
   grid_wait();  // the kernel before this one may still be reading what dst held
+  // (the source may be the caller's own array: not a word behind its end is read)
+  if (blockIdx.x == 0 && threadIdx.x < tail_words)
+    reinterpret_cast<uint32_t*>(dst + n)[threadIdx.x] =
+      __ldcs(reinterpret_cast<const uint32_t*>(src + n) + threadIdx.x);
   const uint32_t step = gridDim.x * 256u;
   for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < n; i += 4u * step) {
     uint4 v[4];
@@ -1699,11 +1704,11 @@ int launch_predict_fixed_scratch(const PredictParams& p, int chunk_size, int sm_
 int launch_fetch(void* dst, const void* src_mapped, size_t bytes, int sm_count, cudaStream_t stream,
                  std::string& err)
 {
-  const uint32_t n   = static_cast<uint32_t>((bytes + 15) / 16);
+  const uint32_t n   = static_cast<uint32_t>(bytes / 16);
   const int blocks   = static_cast<int>(std::min<uint32_t>((n + 1023) / 1024, sm_count * 8u));
   const SplitLaunch l{dim3(std::max(1, blocks)), 256, 0, stream, 1, true};
   return launch_split(l, err, fetch_kernel, static_cast<uint4*>(dst),
-                      static_cast<const uint4*>(src_mapped), n);
+                      static_cast<const uint4*>(src_mapped), n, static_cast<uint32_t>(bytes % 16 / 4));
 }
 
 std::string last_launch_variant()

@@ -70,8 +70,8 @@ int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStr
 int launch_predict_fixed_scratch(const PredictParams& p, int chunk_size, int sm_count, int device,
                                  cudaStream_t stream, std::string& err, int64_t* launches);
 
-// Enqueue a kernel that copies `bytes` bytes from mapped host memory to the device.  Both addresses are
-// 16-byte aligned, and both buffers may be read / written up to the next multiple of 16.
+// Enqueue a kernel that copies `bytes` bytes, a multiple of 4, from mapped host memory to the device.  Both
+// addresses are 16-byte aligned.
 int launch_fetch(void* dst, const void* src_mapped, size_t bytes, int sm_count, cudaStream_t stream,
                  std::string& err);
 

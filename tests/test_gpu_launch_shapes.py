@@ -138,3 +138,19 @@ def test_any_chunk_size_of_the_c_interface(kw):
                 fi.forest.handle, INFER_LEAF_ID, Xd.data_ptr(), n, 18, out.data_ptr(), chunk, 0.5,
                 torch.cuda.current_stream().cuda_stream))
             assert np.array_equal(out.cpu().numpy().astype(np.uint32), want[:n]), (n, chunk)
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+def test_pinned_inputs_of_every_length_are_fetched_to_their_end(precision):
+    """Pinned rows that a kernel fetches from the caller's array itself: lengths that are no multiple of
+    the 16 bytes of a load, the last values counting."""
+    import torch
+
+    for n_features in (1, 3, 5, 7, 8):
+        desc = random_forest_desc(95, n_trees=12, n_features=n_features, max_depth=6)
+        for n in (16_385 // (4 * n_features) + 1, 1001 * 8 // n_features + 13, 30_003):
+            X = random_rows(n, n, n_features, "float64", nan_frac=0.02)
+            dt = torch.float32 if precision == "single" else torch.float64
+            pinned = torch.empty(X.shape, dtype=dt, pin_memory=True)
+            pinned.copy_(torch.from_numpy(X))
+            _all_kinds(desc, pinned.numpy(), precision, "depth_first", "auto", host=True)
