@@ -58,23 +58,63 @@ def _nvcc() -> str:
     return exe
 
 
-def up_to_date() -> bool:
-    if not os.path.exists(LIB):
+def _newer(target: str, deps: list) -> bool:
+    if not os.path.exists(target):
         return False
-    me = os.path.abspath(__file__)
+    t = os.path.getmtime(target)
+    return all((not os.path.exists(d)) or os.path.getmtime(d) <= t for d in deps)
 
-    def newer(target, deps):
-        t = os.path.getmtime(target)
-        return all((not os.path.exists(d)) or os.path.getmtime(d) <= t for d in deps)
 
+def _lib_up_to_date() -> bool:
+    deps = [os.path.join(SRC, s) for s in SOURCES + HEADERS] + [os.path.abspath(__file__)]
+    return _newer(LIB, deps)
+
+
+def _torch_module_settled() -> bool:
+    """Built, not needed, or tried and failed (the log of a failed try is kept as <module>.failed)."""
     module = torch_module_path()
-    if module and not (os.path.exists(module) and newer(module, [TORCH_SOURCE, me])):
-        return False
-    return newer(LIB, [os.path.join(SRC, s) for s in SOURCES + HEADERS] + [me])
+    deps = [TORCH_SOURCE, os.path.abspath(__file__)]
+    return module is None or _newer(module, deps) or _newer(module + ".failed", deps)
+
+
+def up_to_date() -> bool:
+    return _lib_up_to_date() and _torch_module_settled()
+
+
+def _build_torch_module() -> str:
+    """Compile the torch module and return the log.  Not an error when that fails: device calls then go
+    through ctypes, a few microseconds slower."""
+    module = torch_module_path()
+    failed = module + ".failed"
+    try:
+        cmd = _torch_command(module + ".tmp")
+        proc = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        text, ok = " ".join(cmd) + "\n" + proc.stdout, proc.returncode == 0
+    except (OSError, RuntimeError, AttributeError) as e:  # no compiler, no CUDA headers, no torch
+        text, ok = f"torch call path: {e!r}\n", False
+    if ok:
+        os.replace(module + ".tmp", module)
+        if os.path.exists(failed):
+            os.remove(failed)
+    else:
+        with open(failed, "w") as fh:
+            fh.write(text)
+        if os.path.exists(module):
+            os.remove(module)  # older than its source
+        sys.stderr.write(f"{text}\nthe torch call path could not be built; device calls go through ctypes\n")
+    return text
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and up_to_date():
+        return LIB
+    if force or not _torch_module_settled():
+        os.makedirs(LIB_DIR, exist_ok=True)
+        if torch_module_path():
+            log = _build_torch_module()
+            if verbose:
+                print(log)
+    if not force and _lib_up_to_date():
         return LIB
     if not all(os.path.exists(os.path.join(SRC, s)) for s in SOURCES):
         raise RuntimeError("kernel sources missing; cannot build libb2fil.so")
@@ -91,11 +131,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
         cmd = base + ["-c", os.path.join(SRC, src), "-o", obj]
         out = open(obj + ".log", "w+")  # a file, not a pipe: nothing blocks while others run
         jobs.append((cmd, obj, subprocess.Popen(cmd, stdout=out, stderr=subprocess.STDOUT), out))
-    module = torch_module_path()
-    if module:
-        cmd = _torch_command(module)
-        out = open(os.path.join(obj_dir, "torch_call.log"), "w+")
-        jobs.append((cmd, None, subprocess.Popen(cmd, stdout=out, stderr=subprocess.STDOUT), out))
     log, failed = [], False
     for cmd, obj, proc, out in jobs:
         proc.wait()
@@ -105,7 +140,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         failed |= proc.returncode != 0
     if not failed:
         cmd = [_nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", LIB]
-        cmd += [obj for _, obj, _, _ in jobs if obj]
+        cmd += [obj for _, obj, _, _ in jobs]
         proc = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
         log.append(" ".join(cmd) + "\n" + proc.stdout)
         failed = proc.returncode != 0

@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes as C
 import time
+import warnings
 from typing import Optional
 
 import numpy as np
@@ -42,7 +43,7 @@ class _Forest:
         info = CInfo()
         _lib.check(_lib.load().b2fil_forest_info(self.handle, C.byref(info)))
         self.info = info
-        self._device_call = None
+        self._device_call = None  # False: not available
 
     @classmethod
     def create(cls, desc: ForestDesc, precision: int, layout: int, storage: int,
@@ -66,11 +67,19 @@ class _Forest:
         return np.float32 if self.info.precision == F32 else np.float64
 
     def device_call(self):
-        """The compiled call path of this forest for torch tensors (created on first use)."""
+        """The compiled call path of this forest for torch tensors (created on first use), or False
+        where it was not built for the installed torch: the same calls then go through ctypes."""
         if self._device_call is None:
+            try:
+                module = _lib.torch_module()
+            except (ImportError, OSError) as e:
+                warnings.warn(f"device calls take a few microseconds longer than they need: {e}",
+                              RuntimeWarning, stacklevel=2)
+                self._device_call = False
+                return False
             i = self.info
             predict = C.cast(_lib.load().b2fil_predict, C.c_void_p).value
-            self._device_call = _lib.torch_module().DeviceCall(
+            self._device_call = module.DeviceCall(
                 predict, self.handle.value, i.n_features, i.n_trees, i.n_outputs, i.device_id,
                 i.precision != F32, i.leaf_vector_len > 1)
         return self._device_call
@@ -276,7 +285,7 @@ class ForestInference:
             raise ValueError("chunk_size must be a positive power of two")
         # CUDA tensors that need no conversion: one native call (None: not such a call)
         call = f._device_call
-        if call is not None and self.output_type != "numpy":
+        if call and self.output_type != "numpy":
             out = call(X, preds, kind, cs, threshold)
             if out is not None:
                 if type(out) is int:

@@ -87,3 +87,39 @@ def test_product_never_imports_the_oracle():
                 text = open(os.path.join(dirpath, fn)).read()
                 assert "fil_oracle" not in text and "import oracle" not in text, fn
                 assert "from oracle" not in text, fn
+
+
+def test_without_the_compiled_torch_path_device_calls_go_through_ctypes(monkeypatch):
+    """The module for the installed torch may be missing (another torch, no compiler): a forest then
+    says so once, and the ctypes path serves its calls."""
+    from cuml_b200.fil.forest_inference import _Forest
+
+    def missing():
+        raise ImportError("b2fil_torch-9.9.so is missing")
+
+    monkeypatch.setattr(_lib, "torch_module", missing)
+    f = _Forest.__new__(_Forest)
+    f.handle, f.info, f._device_call = C.c_void_p(), CInfo(), None
+    with pytest.warns(RuntimeWarning, match="b2fil_torch"):
+        assert f.device_call() is False
+    assert f.device_call() is False
+
+
+def test_torch_path_that_does_not_compile_leaves_the_library_alone(monkeypatch, tmp_path, capfd):
+    import sys
+
+    from cuml_b200 import build
+
+    if build.torch_module_path() is None:
+        pytest.skip("no torch")
+    monkeypatch.setattr(build, "LIB_DIR", str(tmp_path))
+    assert not build._torch_module_settled()
+    built = []
+    monkeypatch.setattr(build, "_lib_up_to_date", lambda: True)
+    monkeypatch.setattr(build, "_torch_command",
+                        lambda out: built.append(out) or [sys.executable, "-c", "import sys; sys.exit(3)"])
+    assert build.build() == build.LIB and len(built) == 1
+    assert "ctypes" in capfd.readouterr().err
+    # not tried again until its source changes or a build is forced
+    assert build.up_to_date() and build.build() == build.LIB and len(built) == 1
+    assert not os.path.exists(build.torch_module_path())
