@@ -1410,12 +1410,13 @@ bool pick_split_shape(const ForestView& f, int mode, int precision, int64_t n_ro
 }
 
 // The same from a small per-thread table of recent answers: the search takes a few microseconds,
-// and a serving loop asks for the same few shapes again and again.
+// and a serving loop asks for the same few shapes again and again.  The key is all that
+// pick_split_shape() looks at.
 bool split_shape(const ForestView& f, int mode, int precision, int64_t n_rows, int rows_per_tile,
                  int sm_count, SplitShape& out)
 {
   struct Entry {
-    int32_t depth, precision, mode, n_features, n_outputs, n_trees, rows_per_tile, sm_count;
+    int32_t depth, precision, mode, n_features, n_outputs, n_trees, has_categorical, rows_per_tile, sm_count;
     int64_t n_rows;
     bool found;
     SplitShape shape;
@@ -1425,7 +1426,8 @@ bool split_shape(const ForestView& f, int mode, int precision, int64_t n_rows, i
   for (const Entry& e : table) {
     if (e.n_rows == n_rows && e.depth == f.dense_depth && e.precision == precision &&
         e.mode == mode && e.n_features == f.n_features && e.n_outputs == f.n_outputs &&
-        e.n_trees == f.n_trees && e.rows_per_tile == rows_per_tile && e.sm_count == sm_count) {
+        e.n_trees == f.n_trees && e.has_categorical == f.has_categorical &&
+        e.rows_per_tile == rows_per_tile && e.sm_count == sm_count) {
       out = e.shape;
       return e.found;
     }
@@ -1433,7 +1435,7 @@ bool split_shape(const ForestView& f, int mode, int precision, int64_t n_rows, i
   Entry& e = table[next];
   next     = (next + 1) % 8;
   e        = Entry{f.dense_depth, precision, mode, f.n_features, f.n_outputs, f.n_trees,
-                   rows_per_tile, sm_count, n_rows, false, {}};
+                   f.has_categorical, rows_per_tile, sm_count, n_rows, false, {}};
   e.found  = pick_split_shape(f, mode, precision, n_rows, rows_per_tile, sm_count, e.shape);
   out      = e.shape;
   return e.found;

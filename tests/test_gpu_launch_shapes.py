@@ -154,3 +154,31 @@ def test_pinned_inputs_of_every_length_are_fetched_to_their_end(precision):
             pinned = torch.empty(X.shape, dtype=dt, pin_memory=True)
             pinned.copy_(torch.from_numpy(X))
             _all_kinds(desc, pinned.numpy(), precision, "depth_first", "auto", host=True)
+
+
+def test_launch_shape_does_not_depend_on_what_ran_before():
+    """A plain and a categorical forest of the same size, predicted in both orders by fresh threads
+    (each has its own table of recent launch shapes): the same kernels and shapes every time."""
+    import threading
+
+    import torch
+
+    from cuml_b200.fil import ForestInference, _lib, synthetic_complete_forest
+
+    plain, cat = (ForestInference.load_from_treelite_model(
+        synthetic_complete_forest(300, 6, 40, 7, n_categorical=c, n_categories=20)) for c in (0, 8))
+    seen = {}
+    for n in (64, 700, 3000, 6000, 12_000):
+        X = torch.zeros((n, 40), device="cuda:0")
+        for order in ((plain, cat), (cat, plain)):
+            def run():
+                for fi in order:
+                    fi.predict_proba(X)
+                    seen.setdefault((n, fi is cat), set()).add(_lib.last_variant().replace(",CAT", ""))
+
+            t = threading.Thread(target=run)
+            t.start()
+            t.join()
+    assert all(len(v) == 1 for v in seen.values()), seen
+    # (the sizes are such that the two have shapes of their own)
+    assert any(seen[n, False] != seen[n, True] for n in (64, 700, 3000, 6000, 12_000)), seen
