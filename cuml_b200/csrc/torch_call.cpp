@@ -11,6 +11,7 @@
 
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/b2fil.h"
@@ -65,9 +66,12 @@ bool out_spec(const DeviceCall* c, int64_t kind, int64_t n, OutSpec& s)
 }
 
 // X, preds (tensor or None), kind, chunk_size, threshold.  Returns the output tensor, None when
-// the call is not one of the common ones, or the library's error code as an int.
+// the call is not one of the common ones, or the library's error code as an int.  Any of torch's
+// functions may throw (a tensor subclass answers even size() in Python): the macros turn what they
+// throw into the Python exception.
 PyObject* device_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject*)
 {
+  HANDLE_TH_ERRORS
   const DeviceCall* c = reinterpret_cast<const DeviceCall*>(self);
   if (PyVectorcall_NARGS(nargsf) != 5) {
     PyErr_SetString(PyExc_TypeError, "DeviceCall takes X, preds, kind, chunk_size, threshold");
@@ -87,34 +91,32 @@ PyObject* device_call(PyObject* self, PyObject* const* args, size_t nargsf, PyOb
   OutSpec s;
   if (!out_spec(c, kind, n, s)) Py_RETURN_NONE;
   const at::IntArrayRef dims(s.dims, s.ndim);
-  try {
-    at::TensorBase made;
-    const bool given = args[1] != Py_None;
-    if (given) {
-      if (!THPVariable_Check(args[1])) Py_RETURN_NONE;
-      const at::Tensor& out = THPVariable_Unpack(args[1]);
-      if (out.sizes() != dims || out.scalar_type() != s.dtype || !out.is_cuda() ||
-          !out.is_contiguous())
-        Py_RETURN_NONE;
-      made = out;
-    } else {
-      made = at::detail::empty_cuda(dims, s.dtype, X.device(), std::nullopt);
-    }
-    void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(c->device)).stream();
-    int rc;
-    Py_BEGIN_ALLOW_THREADS;
-    rc = c->predict(c->forest, static_cast<int>(kind), X.const_data_ptr(), n, X.stride(0),
-                    made.mutable_data_ptr(), static_cast<int>(chunk), thr, stream);
-    Py_END_ALLOW_THREADS;
-    if (rc != B2FIL_OK) return PyLong_FromLong(rc);
-    if (given) return Py_NewRef(args[1]);
-    return THPVariable_Wrap(std::move(made));
-  } catch (const c10::OutOfMemoryError& e) {
-    Py_RETURN_NONE;  // the Python path repeats the allocation and raises torch's own error
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
+  const void* from      = X.const_data_ptr();
+  const int64_t stride  = X.stride(0);
+  at::TensorBase made;
+  const bool given = args[1] != Py_None;
+  if (given) {
+    if (!THPVariable_Check(args[1])) Py_RETURN_NONE;
+    const at::Tensor& out = THPVariable_Unpack(args[1]);
+    if (out.sizes() != dims || out.scalar_type() != s.dtype || !out.is_cuda() ||
+        !out.is_contiguous())
+      Py_RETURN_NONE;
+    made = out;
+  } else {
+    made = at::detail::empty_cuda(dims, s.dtype, X.device(), std::nullopt);
   }
+  void* to     = made.mutable_data_ptr();
+  void* stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(c->device)).stream();
+  int rc;
+  // (nothing in here throws: the lock has to come back)
+  Py_BEGIN_ALLOW_THREADS;
+  rc = c->predict(c->forest, static_cast<int>(kind), from, n, stride, to, static_cast<int>(chunk), thr,
+                  stream);
+  Py_END_ALLOW_THREADS;
+  if (rc != B2FIL_OK) return PyLong_FromLong(rc);
+  if (given) return Py_NewRef(args[1]);
+  return THPVariable_Wrap(std::move(made));
+  END_HANDLE_TH_ERRORS
 }
 
 // DeviceCall(predict_address, forest_address, n_features, n_trees, n_outputs, device, f64, vector)

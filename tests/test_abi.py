@@ -123,3 +123,35 @@ def test_torch_path_that_does_not_compile_leaves_the_library_alone(monkeypatch, 
     # not tried again until its source changes or a build is forced
     assert build.up_to_date() and build.build() == build.LIB and len(built) == 1
     assert not os.path.exists(build.torch_module_path())
+
+
+_ODD_TENSOR = """
+import torch
+from cuml_b200.fil import _lib
+
+class Odd(torch.Tensor):  # says it is a CUDA tensor and raises when asked for its sizes
+    @staticmethod
+    def __new__(cls):
+        return torch.Tensor._make_wrapper_subclass(
+            cls, (3, 4), strides=(4, 1), dtype=torch.float32, device="cuda:0",
+            dispatch_sizes_strides_policy="sizes")
+
+    @classmethod
+    def __torch_dispatch__(cls, func, types, args=(), kwargs=None):
+        raise ValueError("no sizes here")
+
+call = _lib.torch_module().DeviceCall(1, 1, 4, 3, 1, 0, False, False)
+try:
+    call(Odd(), None, 0, 0, 0.5)
+except ValueError as e:
+    print("raised:", e)
+"""
+
+
+def test_device_call_raises_what_a_tensor_raises(lib):
+    """Errors of torch's C++ side come out as Python exceptions; they used to end the process."""
+    import subprocess
+    import sys
+
+    r = subprocess.run([sys.executable, "-c", _ODD_TENSOR], cwd=ROOT, capture_output=True, text=True)
+    assert r.returncode == 0 and "raised: no sizes here" in r.stdout, r.stderr[-500:]

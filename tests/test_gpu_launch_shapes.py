@@ -182,3 +182,21 @@ def test_launch_shape_does_not_depend_on_what_ran_before():
     assert all(len(v) == 1 for v in seen.values()), seen
     # (the sizes are such that the two have shapes of their own)
     assert any(seen[n, False] != seen[n, True] for n in (64, 700, 3000, 6000, 12_000)), seen
+
+
+def test_tensor_without_memory_is_an_error():
+    """A fake CUDA tensor has shapes and no data: every call with it raises, the first one (ctypes)
+    and later ones (compiled call path), and the forest goes on predicting."""
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from cuml_b200.fil import ForestInference, synthetic_complete_forest
+
+    fi = ForestInference.load_from_treelite_model(synthetic_complete_forest(20, 4, 6, 1))
+    X = torch.zeros((7, 6), device="cuda:0")
+    with FakeTensorMode():
+        fake = torch.empty((7, 6), device="cuda:0")
+    for _ in range(3):
+        with pytest.raises(RuntimeError):
+            fi.apply(fake)
+        assert fi.apply(X).shape == (7, 20)
