@@ -96,11 +96,12 @@ __device__ __forceinline__ void report_status(int32_t* status, int32_t code)
 // rows: one prediction in twelve had a few leaves of the wrong tree.  So the arrival depends on what was
 // read: `read` is any condition on the last values that this lane has loaded from the stage (all
 // loads before them fed their addresses), the vote needs it from every lane, and the arrival's
-// address needs the vote, by way of a zero that only the host knows to be one.
+// address needs the vote, by way of a zero that only the host knows to be one.  The vote is the
+// warp's meeting as well; a __syncwarp() beside it is not needed, nothing being written to the stage
+// (1.5 M rows of the headline forest: 3.99 ms without the dependency, 4.00 with it, 4.02 with both).
 __device__ __forceinline__ void release_stage(uint32_t bar, int lane, bool read, uint32_t zero)
 {
   const uint32_t all = __ballot_sync(0xffffffffu, read);
-  __syncwarp();
   if (lane == 0) mbar_arrive(bar + (all & zero));
 }
 // Position in a ring of S stages: the stage index and the parity of its current use, advanced
