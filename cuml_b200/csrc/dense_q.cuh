@@ -601,12 +601,18 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
       if (tpos.stage == 0) tprimed = true;
       return true;
     };
+    // LEAFG: a stage is one copy per tree (a dozen to 28 of them), which the lanes issue side by side.
+    // One lane needs 0.2 to 0.3 us for them, and a batch of trees is walked in 1.3 to 1.8 us (2000 trees
+    // of depth 9 x 500,000 rows of 440 features 4.70 -> 4.02 ms; depth 10, 512 features 5.80 -> 5.48).
+    // Otherwise lane 0 does everything.
+    const bool issues = LEAFG || lane == 0;
     grid_wait();
     bool going = seg.live();
     if (lane == 0 && going) going = request_tile(seg.tile);
+    if (LEAFG) going = __shfl_sync(0xffffffffu, going, 0);
     for (; seg.live(); seg.next()) {
       const bool nan_image = q.nan_columns && has_nan(seg.tile);
-      if (lane != 0 || !going) continue;
+      if (!issues || !going) continue;
       const unsigned char* src = static_cast<const unsigned char*>(nan_image ? f.q_nodes_nan : image);
       const bool more = seg.more();
       const int end   = seg.end();
@@ -614,18 +620,21 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
       const int ask_at = q.tile_bufs == 2 ? min(end, seg.begin + S) - 1 : end - 1;
       for (int b = seg.begin; b < end && going; ++b) {
         const uint32_t s = pos.stage;
-        if (primed && !mbar_wait(bars + 8u * (kMaxStages + s), pos.phase ^ 1u)) {
-          report_status(p.status, 1);
+        bool free = !primed || mbar_wait(bars + 8u * (kMaxStages + s), pos.phase ^ 1u);
+        if (LEAFG) free = __all_sync(0xffffffffu, free);
+        if (!free) {
+          if (lane == 0) report_status(p.status, 1);
           going = false;
           break;
         }
         const int first      = b * per_batch;
         const int count      = min(per_batch, f.n_trees - first);
         const uint32_t bytes = count * tstride;
-        mbar_expect_tx(bars + 8u * s, bytes);
+        if (lane == 0) mbar_expect_tx(bars + 8u * s, bytes);
         if (LEAFG) {
-          // one copy per tree: the node half of its block
-          for (int i = 0; i < count; ++i)
+          __syncwarp();
+          // the node half of every tree's block
+          for (int i = lane; i < count; i += 32)
             bulk_copy_g2s(stages + s * stage_bytes + i * tstride,
                           src + static_cast<size_t>(first + i) * gstride, tstride, bars + 8u * s);
         } else {
@@ -634,7 +643,10 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
         }
         pos.advance(S);
         if (pos.stage == 0) primed = true;
-        if (more && b == ask_at) going = request_tile(seg.tile + 1);
+        if (more && b == ask_at) {
+          if (lane == 0) going = request_tile(seg.tile + 1);
+          if (LEAFG) going = __shfl_sync(0xffffffffu, going, 0);
+        }
       }
     }
     return;
