@@ -570,11 +570,13 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
   grid_release();
   QSegments seg(n_tiles, n_batches, !REDUCE || q.partial != nullptr);
 
-  // does the tile hold a missing value?  (asked by whole warps)
+  // Does the tile hold a missing value?  (asked by whole warps)  Read past the L1: the pre-pass may have
+  // written the flags while this kernel was already on the SM, next to the traversal of the call
+  // before it, which read the flags of its own rows at the same addresses.
   auto has_nan = [&](int t) {
     uint32_t bits = 0;
     for (int i = lane; i < q.flag_words; i += 32)
-      bits |= __ldg(q.flags + static_cast<int64_t>(t) * q.flag_words + i);
+      bits |= __ldcg(q.flags + static_cast<int64_t>(t) * q.flag_words + i);
     return __any_sync(0xffffffffu, bits != 0u);
   };
 

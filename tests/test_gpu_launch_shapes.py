@@ -200,3 +200,24 @@ def test_tensor_without_memory_is_an_error():
         with pytest.raises(RuntimeError):
             fi.apply(fake)
         assert fi.apply(X).shape == (7, 20)
+
+
+def test_missing_values_come_and_go_between_overlapped_calls():
+    """Batches with and without missing values in turn, never waited for: kernels of neighbouring calls
+    share SMs (small forests leave room) and scratch addresses, and every call has to see its own flags."""
+    import torch
+
+    from cuml_b200.fil import ForestInference
+
+    desc = random_forest_desc(96, n_trees=150, n_features=10, max_depth=4, postproc="sigmoid")
+    fi = ForestInference.load_from_treelite_model(desc, storage="dense")
+    g = torch.Generator(device="cuda:0")
+    g.manual_seed(1)
+    X = [torch.randn((60_000, 10), generator=g, device="cuda:0") for _ in range(2)]
+    X[1][torch.rand(X[1].shape, generator=g, device="cuda:0") < 0.1] = float("nan")
+    want = [fi.apply(x) for x in X]
+    proba = [fi.predict_proba(x) for x in X]
+    torch.cuda.synchronize()
+    got = [(fi.apply(X[i % 2]), fi.predict_proba(X[i % 2])) for i in range(40)]
+    for i, (ids, p) in enumerate(got):
+        assert torch.equal(ids, want[i % 2]) and torch.equal(p, proba[i % 2]), i
