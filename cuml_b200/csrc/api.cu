@@ -185,6 +185,100 @@ void release_scratch_pool(int device)
   }
 }
 
+// Pinned host memory through which predictions on host arrays pass.  It belongs to the process, and a
+// call takes what it needs and gives it back when its work is done: pinning takes a millisecond and
+// more, which the first call of every model paid when each had its own.  Kept for later calls: 64 MiB,
+// or more if that much was in use at one time; every forest that is freed brings it back to 64 MiB, the
+// last one to nothing.  Sizes are rounded up, so that batches that grow a little find their buffer.
+struct PinnedBuf {
+  void* ptr    = nullptr;
+  size_t bytes = 0;
+};
+class PinnedPool {
+ public:
+  static PinnedPool& get()
+  {
+    static PinnedPool* pool = new PinnedPool;
+    return *pool;
+  }
+  // A buffer of at least `bytes`, in place of the one in `b`.
+  cudaError_t take(size_t bytes, PinnedBuf& b)
+  {
+    if (b.bytes >= bytes) return cudaSuccess;
+    give(b);
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      size_t best = free_.size();
+      for (size_t i = 0; i < free_.size(); ++i)
+        if (free_[i].bytes >= bytes && (best == free_.size() || free_[i].bytes < free_[best].bytes)) best = i;
+      if (best < free_.size()) {
+        b            = free_[best];
+        free_[best]  = free_.back();
+        free_.pop_back();
+        kept_ -= b.bytes;
+        used_ += b.bytes;
+        most_used_ = std::max(most_used_, used_);
+        return cudaSuccess;
+      }
+    }
+    const size_t size   = pinned_size(bytes);
+    void* ptr           = nullptr;
+    const cudaError_t e = cudaHostAlloc(&ptr, size, cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e != cudaSuccess) return e;
+    b = PinnedBuf{ptr, size};
+    std::lock_guard<std::mutex> lock(mu_);
+    used_ += size;
+    most_used_ = std::max(most_used_, used_);
+    return cudaSuccess;
+  }
+  // Nothing on the GPU uses the buffer any more.
+  void give(PinnedBuf& b)
+  {
+    if (!b.ptr) return;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      used_ -= b.bytes;
+      if (users_ > 0 && kept_ + b.bytes <= std::max(kKeep, most_used_)) {
+        free_.push_back(b);
+        kept_ += b.bytes;
+        b = PinnedBuf{};
+      }
+    }
+    if (b.ptr) cudaFreeHost(b.ptr);
+    b = PinnedBuf{};
+  }
+  void add_user()
+  {
+    std::lock_guard<std::mutex> lock(mu_);
+    ++users_;
+  }
+  void drop_user()
+  {
+    std::vector<PinnedBuf> gone;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      --users_;
+      most_used_         = used_;
+      const size_t limit = users_ > 0 ? kKeep : 0;
+      // the largest first: what is left serves most calls
+      std::sort(free_.begin(), free_.end(), [](const PinnedBuf& x, const PinnedBuf& y) { return x.bytes < y.bytes; });
+      while (kept_ > limit && !free_.empty()) {
+        kept_ -= free_.back().bytes;
+        gone.push_back(free_.back());
+        free_.pop_back();
+      }
+    }
+    for (PinnedBuf& b : gone) cudaFreeHost(b.ptr);
+  }
+
+ private:
+  static constexpr size_t kKeep = size_t(64) << 20;
+  std::mutex mu_;
+  std::vector<PinnedBuf> free_;
+  size_t kept_ = 0, used_ = 0, most_used_ = 0;
+  int users_ = 0;
+};
+
 // Status words live in pinned host memory, so that the host reads one without a copy (12 us per
 // call).  A page of them serves a thousand forests; pages are kept.
 std::mutex g_status_mu;
@@ -214,24 +308,18 @@ void release_status_word(int32_t* word)
 // One slot of the host-buffer pipeline: device staging buffers and the stream that orders them.
 struct HostSlot {
   cudaStream_t stream = nullptr;
-  void* x             = nullptr;
+  void* x             = nullptr;  // rows and results on the device, from the scratch pool
   void* out           = nullptr;
   size_t x_bytes      = 0;
   size_t out_bytes    = 0;
-  cudaEvent_t ev[3]   = {nullptr, nullptr, nullptr};  // sharded prediction: begin, kernels done, gathered
-  void* pin_out        = nullptr;  // results for pageable arrays pass through here
-  size_t pin_out_bytes = 0;
-  int64_t pending_r0   = -1;  // rows whose results sit in pin_out, not yet handed to the caller
-  int64_t pending_n    = 0;
+  // sharded prediction: results on their way to the first device (memory of its own, which peers may
+  // read), and the events begin, kernels done, gathered
+  void* shard_out        = nullptr;
+  size_t shard_out_bytes = 0;
+  cudaEvent_t ev[3]      = {nullptr, nullptr, nullptr};
 };
 
-// One piece of pinned memory through which pageable inputs pass.
-struct StageChunk {
-  void* ptr        = nullptr;
-  size_t bytes     = 0;
-  cudaEvent_t free = nullptr;  // its last copy to the device is done
-};
-constexpr int kStageChunks = 4;
+constexpr int kStageChunks = 4;  // pieces of pinned memory through which pageable inputs pass
 
 struct b2fil_forest {
   ForestView view{};
@@ -260,24 +348,28 @@ struct b2fil_forest {
   int32_t clone_direct     = -1;  // 1: that replication went over a direct peer path
   std::mutex host_mu;  // serialises the calls that use the slots below
   HostSlot slots[kMaxHostSlots];
-  StageChunk chunks[kStageChunks];
+  cudaEvent_t chunk_free[kStageChunks] = {};  // the last copy from that piece of pinned memory is done
   ~b2fil_forest()
   {
     DeviceGuard g(device);
-    if (arena) cudaFree(arena);
-    if (status) release_status_word(status);
-    if (pool) release_scratch_pool(device);
-    for (auto& c : chunks) {
-      if (c.ptr) cudaFreeHost(c.ptr);
-      if (c.free) cudaEventDestroy(c.free);
-    }
     for (auto& s : slots) {
-      if (s.x) cudaFree(s.x);
-      if (s.out) cudaFree(s.out);
-      if (s.stream) cudaStreamDestroy(s.stream);
+      if (s.x) cudaFreeAsync(s.x, s.stream);
+      if (s.out) cudaFreeAsync(s.out, s.stream);
+      if (s.shard_out) cudaFree(s.shard_out);
+      if (s.stream) {
+        cudaStreamSynchronize(s.stream);
+        cudaStreamDestroy(s.stream);
+      }
       for (auto& e : s.ev)
         if (e) cudaEventDestroy(e);
-      if (s.pin_out) cudaFreeHost(s.pin_out);
+    }
+    for (auto& e : chunk_free)
+      if (e) cudaEventDestroy(e);
+    if (arena) cudaFree(arena);
+    if (status) release_status_word(status);
+    if (pool) {
+      release_scratch_pool(device);
+      PinnedPool::get().drop_user();
     }
   }
 };
@@ -334,6 +426,7 @@ int init_device_state(b2fil_forest* f)
   f->sm_count = sms;
   B2FIL_CUDA(acquire_status_word(&f->status));
   B2FIL_CUDA(acquire_scratch_pool(f->device, &f->pool));
+  PinnedPool::get().add_user();
   return B2FIL_OK;
 }
 
@@ -395,24 +488,41 @@ int enqueue(const b2fil_forest* f, int kind, const void* X, int64_t n_rows, int6
   return B2FIL_OK;
 }
 
-int ensure_slot(HostSlot& s, size_t x_bytes, size_t out_bytes)
+// Make a slot's device buffer hold `want` bytes.  Stream-ordered: batches that grow do not stall the
+// device, and grow the buffer by half at least.
+int grow_buffer(const b2fil_forest* f, HostSlot& s, void** buf, size_t* have, size_t want)
+{
+  if (*have >= want) return B2FIL_OK;
+  size_t size = std::max(want, *have + *have / 2);
+  if (*buf) B2FIL_CUDA(cudaFreeAsync(*buf, s.stream));
+  *buf          = nullptr;
+  *have         = 0;
+  cudaError_t e = cudaMallocFromPoolAsync(buf, size, f->pool, s.stream);
+  if (e == cudaErrorMemoryAllocation && size > want) {
+    cudaGetLastError();
+    size = want;
+    e    = cudaMallocFromPoolAsync(buf, size, f->pool, s.stream);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *buf = nullptr;
+    return set_error(e == cudaErrorMemoryAllocation ? B2FIL_ERR_NO_MEMORY : B2FIL_ERR_CUDA,
+                     std::string("device staging buffer: ") + cudaGetErrorString(e));
+  }
+  *have = size;
+  return B2FIL_OK;
+}
+int ensure_stream(HostSlot& s)
 {
   if (!s.stream) B2FIL_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
-  if (s.x_bytes < x_bytes) {
-    if (s.x) cudaFree(s.x);
-    s.x = nullptr;
-    s.x_bytes = 0;
-    B2FIL_CUDA(cudaMalloc(&s.x, x_bytes));
-    s.x_bytes = x_bytes;
-  }
-  if (s.out_bytes < out_bytes) {
-    if (s.out) cudaFree(s.out);
-    s.out = nullptr;
-    s.out_bytes = 0;
-    B2FIL_CUDA(cudaMalloc(&s.out, out_bytes));
-    s.out_bytes = out_bytes;
-  }
   return B2FIL_OK;
+}
+int ensure_slot(const b2fil_forest* f, HostSlot& s, size_t x_bytes, size_t out_bytes)
+{
+  int rc = ensure_stream(s);
+  if (rc == B2FIL_OK) rc = grow_buffer(f, s, &s.x, &s.x_bytes, x_bytes);
+  if (rc == B2FIL_OK) rc = grow_buffer(f, s, &s.out, &s.out_bytes, out_bytes);
+  return rc;
 }
 
 // Read and clear the status word.  The caller has already waited for the work it cares about.
@@ -447,19 +557,12 @@ bool is_pageable(const void* p, void** mapped)
   return a.type == cudaMemoryTypeUnregistered;
 }
 
-int ensure_pinned(void** buf, size_t* have, size_t want)
+int ensure_pinned(PinnedBuf& b, size_t want)
 {
-  if (*have >= want) return B2FIL_OK;
-  if (*buf) cudaFreeHost(*buf);
-  *buf  = nullptr;
-  *have = 0;
-  const cudaError_t e = cudaHostAlloc(buf, want, cudaHostAllocDefault);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return set_error(B2FIL_ERR_NO_MEMORY, std::string("pinned staging buffer: ") + cudaGetErrorString(e));
-  }
-  *have = want;
-  return B2FIL_OK;
+  const cudaError_t e = PinnedPool::get().take(want, b);
+  if (e == cudaSuccess) return B2FIL_OK;
+  cudaGetLastError();
+  return set_error(B2FIL_ERR_NO_MEMORY, std::string("pinned staging buffer: ") + cudaGetErrorString(e));
 }
 
 // Copy `n_rows` rows of `row_bytes` bytes (source rows `src_stride` bytes apart) into a dense
@@ -512,6 +615,16 @@ class HostPrediction {
     in_pinned_  = !is_pageable(X, &in_mapped_);
     out_pinned_ = !is_pageable(out, &out_mapped_);
   }
+  HostPrediction(const HostPrediction&) = delete;
+  ~HostPrediction()
+  {
+    // also after an error: work already enqueued still uses the caller's arrays and the staging
+    if (!drained_)
+      for (HostSlot& s : f_->slots)
+        if (s.stream) cudaStreamSynchronize(s.stream);
+    for (PinnedBuf& b : chunk_) PinnedPool::get().give(b);
+    for (Result& r : result_) PinnedPool::get().give(r.pinned);
+  }
 
   int run()
   {
@@ -523,14 +636,9 @@ class HostPrediction {
     } else {
       rc = blocks();
     }
-    // also after an error: work already enqueued still uses the caller's arrays and the staging
-    for (HostSlot& s : f_->slots) {
-      if (!s.stream) continue;
-      const int drained = rc == B2FIL_OK ? flush(s) : (cudaStreamSynchronize(s.stream), B2FIL_OK);
-      if (rc == B2FIL_OK) rc = drained;
-      s.pending_r0 = -1;
-    }
+    for (int i = 0; i < kMaxHostSlots && rc == B2FIL_OK; ++i) rc = flush(i);
     if (rc != B2FIL_OK) return rc;
+    drained_       = true;
     int32_t status = 0;
     return read_status_word(f_, &status);
   }
@@ -546,33 +654,34 @@ class HostPrediction {
 
   int in_place()
   {
-    HostSlot& s   = f_->slots[0];
-    StageChunk& c = f_->chunks[0];
-    int rc        = ensure_slot(s, 0, 0);
-    if (rc == B2FIL_OK) rc = ensure_chunk(c, kInPlaceIn);
-    if (rc == B2FIL_OK) rc = ensure_pinned(&s.pin_out, &s.pin_out_bytes, kInPlaceOut);
+    HostSlot& s  = f_->slots[0];
+    PinnedBuf& c = chunk_[0];
+    Result& r    = result_[0];
+    int rc       = ensure_stream(s);
+    if (rc == B2FIL_OK) rc = ensure_pinned(c, kInPlaceIn);
+    if (rc == B2FIL_OK) rc = ensure_pinned(r.pinned, kInPlaceOut);
     if (rc != B2FIL_OK) return rc;
     copy_rows(static_cast<char*>(c.ptr), x_, n_rows_, in_row_b_, in_stride_);
-    rc = enqueue(f_, kind_, c.ptr, n_rows_, f_->view.n_features, s.pin_out, chunk_size_, threshold_,
+    rc = enqueue(f_, kind_, c.ptr, n_rows_, f_->view.n_features, r.pinned.ptr, chunk_size_, threshold_,
                  s.stream);
-    s.pending_r0 = 0;
-    s.pending_n  = n_rows_;
+    r.row0 = 0;
+    r.rows = n_rows_;
     return rc;
   }
 
   int short_call()
   {
     HostSlot& s       = f_->slots[0];
-    StageChunk& c     = f_->chunks[0];
+    PinnedBuf& c      = chunk_[0];
+    Result& r         = result_[0];
     const bool direct = in_mapped_ != nullptr && in_stride_ == in_row_b_ &&
                         reinterpret_cast<uintptr_t>(in_mapped_) % 16 == 0;
     // results without a copy: consecutive ones, not a store of its own per row and tree
     const bool write  = out_bytes_ <= (per_tree() ? kPerTreeOut : kShortOut);
-    int rc            = ensure_slot(s, (in_bytes_ + 15) / 16 * 16, write ? 0 : out_bytes_);
-    if (rc == B2FIL_OK && !direct) rc = ensure_chunk(c, (in_bytes_ + 15) / 16 * 16);
+    int rc            = ensure_slot(f_, s, in_bytes_, write ? 0 : out_bytes_);
+    if (rc == B2FIL_OK && !direct) rc = ensure_pinned(c, in_bytes_);
     const bool to_pin = write ? out_mapped_ == nullptr : !out_pinned_;
-    if (rc == B2FIL_OK && to_pin)
-      rc = ensure_pinned(&s.pin_out, &s.pin_out_bytes, std::max(out_bytes_, kShortOut));
+    if (rc == B2FIL_OK && to_pin) rc = ensure_pinned(r.pinned, out_bytes_);
     if (rc != B2FIL_OK) return rc;
     std::string err;
     if (direct) {
@@ -581,13 +690,13 @@ class HostPrediction {
       rc = stage_and_fetch(static_cast<char*>(c.ptr), static_cast<char*>(s.x), s.stream, err);
     }
     if (rc != B2FIL_OK) return set_error(rc, err);
-    void* to = to_pin ? s.pin_out : (write ? out_mapped_ : static_cast<void*>(out_));
+    void* to = to_pin ? r.pinned.ptr : (write ? out_mapped_ : static_cast<void*>(out_));
     rc = enqueue(f_, kind_, s.x, n_rows_, f_->view.n_features, write ? to : s.out, chunk_size_,
                  threshold_, s.stream);
     if (rc != B2FIL_OK) return rc;
     if (!write) B2FIL_CUDA(cudaMemcpyAsync(to, s.out, out_bytes_, cudaMemcpyDeviceToHost, s.stream));
-    s.pending_r0 = 0;
-    s.pending_n  = to_pin ? n_rows_ : 0;
+    r.row0 = 0;
+    r.rows = to_pin ? n_rows_ : 0;
     return B2FIL_OK;
   }
 
@@ -653,28 +762,28 @@ class HostPrediction {
     block_rows              = std::min(block_rows, n_rows_);
     const int n_slots       = static_cast<int>(std::min<int64_t>(pipe.slots, (n_rows_ + block_rows - 1) / block_rows));
     for (int i = 0; i < n_slots; ++i) {
-      HostSlot& s = f_->slots[i];
-      int rc      = ensure_slot(s, static_cast<size_t>(block_rows) * in_row_b_,
-                                static_cast<size_t>(block_rows) * out_row_b_);
+      int rc = ensure_slot(f_, f_->slots[i], static_cast<size_t>(block_rows) * in_row_b_,
+                           static_cast<size_t>(block_rows) * out_row_b_);
       if (rc == B2FIL_OK && !out_pinned_)
-        rc = ensure_pinned(&s.pin_out, &s.pin_out_bytes, static_cast<size_t>(block_rows) * out_row_b_);
+        rc = ensure_pinned(result_[i].pinned, static_cast<size_t>(block_rows) * out_row_b_);
       if (rc != B2FIL_OK) return rc;
     }
     int which = 0;
     for (int64_t r0 = 0; r0 < n_rows_; r0 += block_rows, which = (which + 1) % n_slots) {
       HostSlot& s     = f_->slots[which];
+      Result& r       = result_[which];
       const int64_t n = std::min(block_rows, n_rows_ - r0);
       // stream order makes the slot's previous block finish before its device buffers are reused
-      int rc = flush(s);
+      int rc = flush(which);
       if (rc == B2FIL_OK) rc = in_pinned_ ? send(s, r0, n) : send_staged(s, r0, n);
       if (rc == B2FIL_OK)
         rc = enqueue(f_, kind_, s.x, n, f_->view.n_features, s.out, chunk_size_, threshold_, s.stream);
       if (rc != B2FIL_OK) return rc;
-      void* to = out_pinned_ ? out_ + static_cast<size_t>(r0) * out_row_b_ : static_cast<char*>(s.pin_out);
+      void* to = out_pinned_ ? out_ + static_cast<size_t>(r0) * out_row_b_ : static_cast<char*>(r.pinned.ptr);
       B2FIL_CUDA(cudaMemcpyAsync(to, s.out, static_cast<size_t>(n) * out_row_b_,
                                  cudaMemcpyDeviceToHost, s.stream));
-      s.pending_r0 = r0;
-      s.pending_n  = out_pinned_ ? 0 : n;
+      r.row0 = r0;
+      r.rows = out_pinned_ ? 0 : n;
     }
     return B2FIL_OK;
   }
@@ -701,37 +810,40 @@ class HostPrediction {
       next_size_        = size * 2;
       m = std::min(std::max<int64_t>(1, static_cast<int64_t>(size / in_row_b_)), n - b);
       const size_t bytes = static_cast<size_t>(m) * in_row_b_;
-      StageChunk& c      = f_->chunks[next_chunk_];
+      PinnedBuf& c       = chunk_[next_chunk_];
+      cudaEvent_t& free  = f_->chunk_free[next_chunk_];
       next_chunk_        = (next_chunk_ + 1) % kStageChunks;
-      int rc             = ensure_chunk(c, std::max(bytes, kChunkMax));
+      if (!free) B2FIL_CUDA(cudaEventCreateWithFlags(&free, cudaEventDisableTiming));
+      B2FIL_CUDA(cudaEventSynchronize(free));  // its last copy, in this call or one before
+      const int rc = ensure_pinned(c, std::max(bytes, kChunkMax));
       if (rc != B2FIL_OK) return rc;
-      B2FIL_CUDA(cudaEventSynchronize(c.free));
       copy_rows(static_cast<char*>(c.ptr), x_ + static_cast<size_t>(r0 + b) * in_stride_, m,
                 in_row_b_, in_stride_);
       B2FIL_CUDA(cudaMemcpyAsync(static_cast<char*>(s.x) + static_cast<size_t>(b) * in_row_b_, c.ptr,
                                  bytes, cudaMemcpyHostToDevice, s.stream));
-      B2FIL_CUDA(cudaEventRecord(c.free, s.stream));
+      B2FIL_CUDA(cudaEventRecord(free, s.stream));
     }
     return B2FIL_OK;
   }
   // Wait for a slot and hand its results to the caller.
-  int flush(HostSlot& s)
+  int flush(int slot)
   {
-    if (s.pending_r0 < 0) return B2FIL_OK;
-    B2FIL_CUDA(cudaStreamSynchronize(s.stream));
-    if (s.pending_n > 0)
-      copy_rows(out_ + static_cast<size_t>(s.pending_r0) * out_row_b_,
-                static_cast<const char*>(s.pin_out), s.pending_n, out_row_b_, out_row_b_);
-    s.pending_r0 = -1;
+    Result& r = result_[slot];
+    if (r.row0 < 0) return B2FIL_OK;
+    B2FIL_CUDA(cudaStreamSynchronize(f_->slots[slot].stream));
+    if (r.rows > 0)
+      copy_rows(out_ + static_cast<size_t>(r.row0) * out_row_b_, static_cast<const char*>(r.pinned.ptr),
+                r.rows, out_row_b_, out_row_b_);
+    r.row0 = -1;
     return B2FIL_OK;
   }
-  int ensure_chunk(StageChunk& c, size_t bytes)
-  {
-    if (!c.free) B2FIL_CUDA(cudaEventCreateWithFlags(&c.free, cudaEventDisableTiming));
-    if (c.bytes >= bytes) return B2FIL_OK;
-    B2FIL_CUDA(cudaEventSynchronize(c.free));  // the old memory may still be on its way
-    return ensure_pinned(&c.ptr, &c.bytes, bytes);
-  }
+
+  // Results of a slot's block that are still on their way to the caller; those for pageable arrays pass
+  // through pinned memory.
+  struct Result {
+    PinnedBuf pinned;
+    int64_t row0 = -1, rows = 0;
+  };
 
   b2fil_forest* f_;
   int kind_;
@@ -743,6 +855,9 @@ class HostPrediction {
   size_t in_row_b_, in_stride_, out_row_b_, in_bytes_, out_bytes_;
   bool in_pinned_, out_pinned_;
   void *in_mapped_ = nullptr, *out_mapped_ = nullptr;
+  PinnedBuf chunk_[kStageChunks];
+  Result result_[kMaxHostSlots];
+  bool drained_   = false;
   int next_chunk_ = 0;
   size_t next_size_ = size_t(1) << 20;  // bytes of the next staged chunk
 };
@@ -1090,7 +1205,18 @@ int b2fil_predict_sharded(b2fil_forest* const* forests, int n_devices, int infer
     row_off += n;
     if (n == 0) continue;
     const bool local = f->device == f0->device;
-    int rc = ensure_slot(s, 0, local ? 0 : static_cast<size_t>(n) * out_row_b);
+    int rc = ensure_stream(s);
+    if (const size_t want = static_cast<size_t>(n) * out_row_b; rc == B2FIL_OK && !local && s.shard_out_bytes < want) {
+      if (s.shard_out) cudaFree(s.shard_out);
+      s.shard_out       = nullptr;
+      s.shard_out_bytes = 0;
+      const cudaError_t e = cudaMalloc(&s.shard_out, want);
+      if (e != cudaSuccess) {
+        rc = cuda_error("cudaMalloc", e);
+      } else {
+        s.shard_out_bytes = want;
+      }
+    }
     for (auto& ev : s.ev) {
       if (rc == B2FIL_OK && !ev && cudaEventCreate(&ev) != cudaSuccess)
         rc = set_error(B2FIL_ERR_CUDA, "cudaEventCreate failed");
@@ -1101,11 +1227,11 @@ int b2fil_predict_sharded(b2fil_forest* const* forests, int n_devices, int infer
     }
     fed.push_back(i);
     cudaEventRecord(s.ev[0], s.stream);
-    rc = enqueue(f, infer_kind, X_shards[i], n, row_stride, local ? static_cast<void*>(dst0) : s.out,
+    rc = enqueue(f, infer_kind, X_shards[i], n, row_stride, local ? static_cast<void*>(dst0) : s.shard_out,
                  chunk_size, threshold, s.stream);
     cudaEventRecord(s.ev[1], s.stream);
     if (rc == B2FIL_OK && !local) {
-      const cudaError_t e = cudaMemcpyPeerAsync(dst0, f0->device, s.out, f->device,
+      const cudaError_t e = cudaMemcpyPeerAsync(dst0, f0->device, s.shard_out, f->device,
                                                 static_cast<size_t>(n) * out_row_b, s.stream);
       if (e != cudaSuccess) rc = cuda_error("cudaMemcpyPeerAsync", e);
     }

@@ -21,6 +21,17 @@
 
 namespace b2fil {
 
+// Size of a pinned buffer for `bytes`: the next power of two up to a megabyte, then the next of four steps
+// to the next power of two.
+inline size_t pinned_size(size_t bytes)
+{
+  size_t power = size_t(64) << 10;
+  while (power < bytes) power *= 2;
+  if (power <= (size_t(1) << 20)) return power;
+  const size_t step = power / 8;  // a quarter of the power of two below
+  return (bytes + step - 1) / step * step;
+}
+
 class CopyPool {
  public:
   // The process-wide pool with `threads` threads, the caller's included (first call decides).
