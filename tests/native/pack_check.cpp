@@ -1,7 +1,8 @@
 // Test-only host walker over a PACKED forest (the arrays the kernels read), used by the CPU test
-// suite to check the packer without a GPU: it links cuml_b200/csrc/pack.cpp directly, packs a
-// description and follows the packed nodes with the same index arithmetic as the kernels
-// (heap addressing for dense storage, child offsets and bit fields for sparse storage).
+// suite to check the packer without a GPU: it links cuml_b200/csrc/pack.cpp and blocks.cpp directly,
+// packs a description, makes the images that are uploaded from it and follows them with the same index
+// arithmetic as the kernels (heap addressing for dense storage, child offsets and bit fields for
+// sparse storage, blocks of four nodes below the heaps).
 // It is not part of libb2fil.so.
 #include <algorithm>
 #include <cmath>
@@ -118,6 +119,47 @@ void walk(const PackedForest& pf, const T* X, int64_t n_rows, int64_t stride, ui
     }
   }
 }
+// Walk the images of the rank-quantised copy as they are uploaded (category sets behind the nodes of a
+// tree), the way dense_q_kernel does: the plain image with a comparison per missing value, and the
+// image for doubled columns, whose second half holds the codes with Q_NAN_LEFT_BIT on missing values.
+int64_t walk_uploaded_ranks(const PackedForest& pf, const std::vector<uint16_t>& q, int64_t r,
+                            const std::vector<uint8_t>& plain, const std::vector<uint8_t>& doubled,
+                            const uint32_t* ids)
+{
+  const ForestView& v = pf.view;
+  const int D = v.dense_depth, F = v.n_features;
+  std::vector<uint32_t> codes(q.begin(), q.end());
+  for (int f = 0; f < F; ++f) codes.push_back(q[f] == Q_NAN_CODE ? q[f] | Q_NAN_LEFT_BIT : q[f]);
+  int64_t bad = 0;
+  for (int image = 0; image < 2; ++image) {
+    const std::vector<uint8_t>& nodes = image == 0 ? plain : doubled;
+    if (nodes.empty()) continue;
+    for (int p = 0; p < v.n_trees; ++p) {
+      const uint8_t* t = nodes.data() + static_cast<size_t>(v.q_tree_stride) * p;
+      uint32_t i       = 1;
+      for (int l = 0; l < D; ++l) {
+        uint32_t node, set = 0;
+        std::memcpy(&node, t + i * 4u, 4);
+        const uint32_t feature = (node & Q_FEATURE_FIELD) >> Q_FEATURE_SHIFT;
+        if (feature >= (image == 0 ? static_cast<uint32_t>(F) : 2u * F)) return bad + 1;
+        const uint32_t code = codes[feature];
+        uint32_t d          = node - (code << Q_RANK_SHIFT);
+        if (v.q_has_cat && static_cast<int32_t>(node) >= 0x7FFC0000) {  // categorical
+          std::memcpy(&set, t + (size_t(4) << D) + i * 4u, 4);
+          const uint32_t n = std::min(code, 32u);  // the clamped funnel shift
+          if (n > 0) d = n < 32 ? set << n | d >> (32 - n) : d;
+          else d = set;
+        }
+        // (a forest without default-left tests and categories is walked without looking for NaN)
+        if (image == 0 && code == Q_NAN_CODE && (v.q_any_default_left || v.q_has_cat)) d = node << 15;
+        i = 2 * i + (d >> 31);
+      }
+      const uint32_t id = pf.leaf_ids[(static_cast<size_t>(p) << D) + (i - (1u << D))];
+      if (id != ids[r * v.n_trees + pf.tree_orig[p]]) ++bad;
+    }
+  }
+  return bad;
+}
 // Walk the rank-quantised copy of a dense forest the way quantise_kernel + dense_q_kernel do:
 // rank through the bucket table, then one signed subtraction per test.  Returns the number of
 // (row, tree) pairs whose leaf differs from `ids`.
@@ -129,6 +171,9 @@ int64_t walk_quantised(const PackedForest& pf, const T* X, int64_t n_rows, int64
   const int D         = v.dense_depth;
   const int F         = v.n_features;
   std::vector<uint16_t> q(F);
+  std::vector<uint8_t> plain = pf.q_nodes, doubled = pf.q_nodes_nan;
+  split_category_sets(v, plain);
+  split_category_sets(v, doubled);
   int64_t bad = 0;
   for (int64_t r = 0; r < n_rows; ++r) {
     const T* row = X + r * stride;
@@ -162,6 +207,7 @@ int64_t walk_quantised(const PackedForest& pf, const T* X, int64_t n_rows, int64
         q[f] = static_cast<uint16_t>(pos);
       }
     }
+    bad += walk_uploaded_ranks(pf, q, r, plain, doubled, ids);
     for (int p = 0; p < v.n_trees; ++p) {
       const uint8_t* t = pf.q_nodes.data() + static_cast<size_t>(v.q_tree_stride) * p;
       const size_t qnb = pf.view.q_has_cat ? 8 : 4;  // {node, category set} or node alone
@@ -208,95 +254,78 @@ int64_t walk_quantised(const PackedForest& pf, const T* X, int64_t n_rows, int64
   }
   return bad;
 }
-// Walk the compact image of a sparse forest the way the fast sparse kernel does: T steps through
-// the tree's heap, leave through an exit, then (k, L) steps over the 8-byte internal nodes; fp64
-// tests look the exact threshold up only when the float bound leaves the answer open.  Returns
-// the number of (row, tree) pairs whose leaf id or payload differs from the primary walk, and
-// counts the exact look-ups in *n_exact.
+// Walk the compact image of a sparse forest the way sparse_compact_kernel does: T steps through the
+// tree's heap, out through an exit, then from block to block; rows are floats rounded down, and a test
+// that they leave open in an fp64 forest reads the exact threshold.  Returns the number of (row, tree)
+// pairs whose leaf id or payload differs from the primary walk, and counts the exact look-ups in
+// *n_exact.
 template <typename T>
-int64_t walk_compact(const PackedForest& pf, const T* X, int64_t n_rows, int64_t stride,
-                     const uint32_t* ids, const double* payload, int64_t* n_exact)
+int64_t walk_blocks(const PackedForest& pf, const T* X, int64_t n_rows, int64_t stride,
+                    const uint32_t* ids, const double* payload, int64_t* n_exact)
 {
-  const ForestView& v = pf.view;
-  using V             = typename std::conditional<sizeof(T) == 4, uint32_t, uint64_t>::type;
-  const int TL        = v.c_top_levels;
-  const size_t heap_n = size_t(1) << TL;
-  const int fb        = v.c_feat_bits;
-  int64_t bad         = 0;
-  auto test = [&](uint32_t value, uint32_t meta, T x, uint32_t k) -> bool {
-    if (meta & META_CATEGORICAL) return goes_right<T, V>(static_cast<V>(value), meta, x, pf);
-    bool left;
-    if (sizeof(T) == 4) {
-      float thr;
-      std::memcpy(&thr, &value, 4);
-      left = x < static_cast<T>(thr);
-    } else {
-      float lo;
-      std::memcpy(&lo, &value, 4);
-      left = static_cast<double>(x) < static_cast<double>(lo);
-      if (!left && k != C_NO_NODE) {
-        // x rounded down to float
-        float xf = static_cast<float>(x);
-        if (static_cast<double>(xf) > static_cast<double>(x))
-          xf = std::nextafter(xf, -std::numeric_limits<float>::infinity());
-        if (xf == lo) {
-          ++*n_exact;
-          left = static_cast<double>(x) < pf.c_exact[k];
-        }
-      }
+  const ForestView& v   = pf.view;
+  using V               = typename std::conditional<sizeof(T) == 4, uint32_t, uint64_t>::type;
+  const int TL          = v.c_top_levels;
+  const size_t heap_n   = size_t(1) << TL;
+  const size_t n_blocks = pf.b_blocks.size() / 8, n_leaves = pf.b_leaf_ids.size();
+  int64_t bad           = 0;
+  // does the row go right?  `exact` is called for its threshold when the floats leave the test open
+  auto test = [&](uint32_t value, bool default_left, bool categorical, T x, auto exact) -> bool {
+    float xl = static_cast<float>(x);
+    if (static_cast<T>(xl) > x) xl = std::nextafter(xl, -std::numeric_limits<float>::infinity());
+    if (categorical) {
+      const uint32_t meta = META_CATEGORICAL | (default_left ? META_DEFAULT_LEFT : 0u);
+      return goes_right<float, uint32_t>(value, meta, xl, pf);
     }
-    if (x != x) left = (meta & META_DEFAULT_LEFT) != 0;
-    return !left;
+    float lo;
+    std::memcpy(&lo, &value, 4);
+    if (xl != xl) return !default_left;
+    if (sizeof(T) == 8 && xl == lo) {
+      ++*n_exact;
+      return !(static_cast<double>(x) < exact());
+    }
+    return !(xl < lo);
   };
   for (int64_t r = 0; r < n_rows; ++r) {
     const T* row = X + r * stride;
     for (int p = 0; p < v.n_trees; ++p) {
-      const uint8_t* top = pf.c_top.data() + static_cast<size_t>(v.c_top_stride) * p;
+      const uint8_t* top = pf.b_top.data() + static_cast<size_t>(v.c_top_stride) * p;
       uint32_t h         = 1;
       for (int l = 0; l < TL; ++l) {
         uint32_t value, meta;
         std::memcpy(&value, top + h * 8, 4);
         std::memcpy(&meta, top + h * 8 + 4, 4);
-        const uint32_t feat = meta & CMETA_LOW27;
-        const uint32_t src  = pf.c_top_src.empty() ? C_NO_NODE : pf.c_top_src[p * heap_n + h];
-        h = 2 * h + (test(value, meta, row[feat], src) ? 1 : 0);
+        h = 2 * h + (test(value, (meta & META_DEFAULT_LEFT) != 0, (meta & META_CATEGORICAL) != 0,
+                          row[meta & CMETA_LOW27], [&] { return pf.b_top_exact[p * heap_n + h]; })
+                       ? 1 : 0);
       }
-      uint32_t exit[2];
-      std::memcpy(exit, top + size_t(h) * 8, 8);  // exit e follows the 2^T node slots
-      uint32_t leaf;
-      if (exit[0] & C_EXIT_LEAF) {
-        leaf = exit[0] & ~C_EXIT_LEAF;
-      } else {
-        uint32_t k = exit[0], L = exit[1];
-        if (L != pf.c_leaves_before[k]) ++bad;
-        int steps  = 0;
-        for (;;) {
-          if (++steps > v.c_bottom_steps) {
-            ++bad;  // the kernel's loop bound would have cut this walk short
-          }
-          const uint32_t value = pf.c_nodes[size_t(k) * 2], meta = pf.c_nodes[size_t(k) * 2 + 1];
-          const uint32_t feat  = meta & ((1u << fb) - 1u);
-          const uint32_t off   = (meta & CMETA_LOW27) >> fb;
-          const bool right     = test(value, meta, row[feat], k);
-          // the first child (adjacent) is the left one unless the node says otherwise
-          const bool second    = right != ((meta & CMETA_SWAPPED) != 0);
-          bool at_leaf;
-          if (second) {
-            at_leaf = (meta & CMETA_SECOND_LEAF) != 0;
-            L += off;
-            k += off;
-          } else {
-            at_leaf = (meta & CMETA_FIRST_LEAF) != 0;
-            k += 1;
-          }
-          if (at_leaf) break;
-        }
-        leaf = L;
+      uint32_t k;
+      std::memcpy(&k, top + size_t(h) * 8, 4);  // exit e follows the 2^T node slots
+      for (int step = 0; !(k & C_EXIT_LEAF); ++step) {
+        // the kernel's loop bound, and its arrays
+        if (step >= v.c_block_steps || k >= n_blocks) return bad + 1;
+        const uint32_t* w = pf.b_blocks.data() + size_t(k) * 8;
+        auto go = [&](uint32_t value, uint32_t half, int slot) {
+          return test(value, (half & BLK_DEFAULT_LEFT) != 0, (half & BLK_CATEGORICAL) != 0,
+                      row[half & BLK_FEATURE], [&] { return pf.b_exact[size_t(k) * 4 + slot]; });
+        };
+        const bool last      = go(w[3], w[5] >> 16, 3);
+        const bool root      = go(w[0], w[4], 0);
+        const bool child     = root ? go(w[2], w[5], 2) : go(w[1], w[4] >> 16, 1);
+        const uint32_t leafs = (w[4] >> 29) | ((w[5] >> 10) & 0x18u);
+        const uint32_t fourth = (w[4] & BLK_HAS_FOURTH) ? (w[4] >> BLK_FOURTH_SHIFT) & 3u : 4u;
+        const uint32_t pos    = 2u * root + child;
+        const uint32_t edge   = pos + (2u * pos + last > 2u * fourth ? 1u : 0u);
+        uint32_t before       = 0;
+        for (uint32_t e = 0; e < edge; ++e) before += (leafs >> e) & 1u;
+        k = ((leafs >> edge) & 1u) ? (w[7] + before) | C_EXIT_LEAF : w[6] + edge - before;
       }
+      const uint32_t leaf = k & ~C_EXIT_LEAF;
+      if (leaf >= n_leaves) return bad + 1;
       const int orig = pf.tree_orig[p];
-      if (pf.c_leaf_ids[leaf] != ids[r * v.n_trees + orig]) ++bad;
+      if (pf.b_leaf_ids[leaf] != ids[r * v.n_trees + orig]) ++bad;
       V pay;
-      std::memcpy(&pay, pf.c_leaf_payload.data() + size_t(leaf) * sizeof(V), sizeof(V));
+      std::memcpy(&pay, pf.b_leaf_payload.data() + size_t(leaf) * sizeof(V), sizeof(V));
       double got;
       if (v.leaf_vector_len > 1) {
         got = static_cast<double>(static_cast<uint32_t>(pay));
@@ -346,6 +375,7 @@ int pack_check(const b2fil_forest_desc* desc, const b2fil_create_opts* opts, con
     info[10] = std::max<int64_t>(info[10], g.blob_bytes);
   }
   if (!pf.q_groups.empty()) info[11] = pf.q_groups[0].f_end - pf.q_groups[0].f_begin;
+  if (pf.view.c_enabled && !build_blocks(pf)) pf.view.c_enabled = 0;  // as b2fil_forest_create does
   info[12] = pf.view.c_enabled;
   info[13] = info[15] = 0;
   info[14] = pf.view.c_enabled ? pf.view.c_top_levels : 0;
@@ -355,14 +385,14 @@ int pack_check(const b2fil_forest_desc* desc, const b2fil_create_opts* opts, con
       if (pf.view.q_enabled)
         info[7] = walk_quantised<float>(pf, static_cast<const float*>(X), n_rows, stride, ids);
       if (pf.view.c_enabled)
-        info[13] = walk_compact<float>(pf, static_cast<const float*>(X), n_rows, stride, ids,
+        info[13] = walk_blocks<float>(pf, static_cast<const float*>(X), n_rows, stride, ids,
                                        payload, &info[15]);
     } else {
       walk<double>(pf, static_cast<const double*>(X), n_rows, stride, ids, payload);
       if (pf.view.q_enabled)
         info[7] = walk_quantised<double>(pf, static_cast<const double*>(X), n_rows, stride, ids);
       if (pf.view.c_enabled)
-        info[13] = walk_compact<double>(pf, static_cast<const double*>(X), n_rows, stride, ids,
+        info[13] = walk_blocks<double>(pf, static_cast<const double*>(X), n_rows, stride, ids,
                                         payload, &info[15]);
     }
   }

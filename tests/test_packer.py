@@ -299,3 +299,36 @@ def test_row_tiles_of_any_chunk_size_are_powers_of_two(pack_check):
         for chunk in (*range(1, 40), 2**26, 2**26 + 1, 2**31 - 1):
             want = 32 << (min(chunk, most // 32).bit_length() - 1)
             assert pack_check.pack_check_chunk_rows(chunk, most) == want, (chunk, most)
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("kw", [dict(mixed_ops=True), dict(categorical=True, mixed_ops=True),
+                                dict(categorical=True, big_categories=True), dict(n_outputs=3, vector=True)])
+def test_blocks_below_the_heaps(pack_check, kw, precision):
+    """Trees far deeper than their heaps, so that walks go from block to block: every shape of a block
+    (leaves among the children, no grandchild, grandchildren in each place), values on thresholds."""
+    desc = random_forest_desc(30, n_trees=13, n_features=9, max_depth=15, p_leaf=0.2, **kw)
+    X = random_rows(31, 600, 9, np.float64, nan_frac=0.05,
+                    categories=75 if kw.get("big_categories") else 22 if "categorical" in kw else None)
+    thr = desc.threshold[desc.node_kind == 1]
+    X[::3, 0] = np.resize(thr, len(X[::3]))
+    X[1, :], X[2, :] = np.inf, -np.inf
+    info = _check(pack_check, desc, X, precision, "depth_first", "sparse")
+    assert info[12] == 1 and info[14] < 14
+    if precision == "double":
+        assert info[15] > 0
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("kw", [dict(mixed_ops=True), dict(n_categorical=3)])
+def test_images_for_missing_values(pack_check, kw, precision):
+    """Rank images as they are uploaded: missing values by comparison and by doubled columns, category
+    sets behind the nodes, and a forest whose missing values all go right."""
+    if "n_categorical" in kw:
+        desc = synthetic_complete_forest(30, 5, 12, seed=3, n_categories=32, **kw)
+    else:
+        desc = random_forest_desc(33, n_trees=30, n_features=12, max_depth=6, **kw)
+    X = random_rows(34, 500, 12, np.float64, nan_frac=0.2, categories=35)
+    assert _check(pack_check, desc, X, precision, "depth_first", "dense")[6] == 1
+    desc.default_left = np.zeros_like(desc.default_left)
+    assert _check(pack_check, desc, X, precision, "depth_first", "dense")[6] == 1
