@@ -144,14 +144,15 @@ namespace {
 // forests on it: creating and first growing a pool costs milliseconds, which every newly loaded
 // model would otherwise pay.  It keeps what was freed for the next call (a pool of its own leaves
 // the settings of the device's default pool alone) and is destroyed with the last forest.
+// What a freed forest needed beyond the others' largest prediction goes back to the device.
 struct ScratchPool {
   cudaMemPool_t pool = nullptr;
-  int users          = 0;
+  std::vector<const std::atomic<int64_t>*> users;  // most scratch that a prediction of each has taken
 };
 std::mutex g_pool_mu;
 std::map<int, ScratchPool> g_pools;
 
-cudaError_t acquire_scratch_pool(int device, cudaMemPool_t* out)
+cudaError_t acquire_scratch_pool(int device, const std::atomic<int64_t>* peak, cudaMemPool_t* out)
 {
   std::lock_guard<std::mutex> lock(g_pool_mu);
   ScratchPool& s = g_pools[device];
@@ -171,18 +172,24 @@ cudaError_t acquire_scratch_pool(int device, cudaMemPool_t* out)
       return e;
     }
   }
-  ++s.users;
+  s.users.push_back(peak);
   *out = s.pool;
   return cudaSuccess;
 }
-void release_scratch_pool(int device)
+void release_scratch_pool(int device, const std::atomic<int64_t>* peak)
 {
   std::lock_guard<std::mutex> lock(g_pool_mu);
   ScratchPool& s = g_pools[device];
-  if (--s.users == 0) {
+  s.users.erase(std::remove(s.users.begin(), s.users.end(), peak), s.users.end());
+  if (s.users.empty()) {
     cudaMemPoolDestroy(s.pool);
     s.pool = nullptr;
+    return;
   }
+  // (up to 64 MiB are not worth the milliseconds of taking them again)
+  int64_t most = int64_t(64) << 20;
+  for (const auto* u : s.users) most = std::max(most, u->load());
+  cudaMemPoolTrimTo(s.pool, static_cast<size_t>(most));
 }
 
 // Pinned host memory through which predictions on host arrays pass.  It belongs to the process, and a
@@ -368,7 +375,7 @@ struct b2fil_forest {
     if (arena) cudaFree(arena);
     if (status) release_status_word(status);
     if (pool) {
-      release_scratch_pool(device);
+      release_scratch_pool(device, &scratch_peak);
       PinnedPool::get().drop_user();
     }
   }
@@ -425,7 +432,7 @@ int init_device_state(b2fil_forest* f)
   B2FIL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, f->device));
   f->sm_count = sms;
   B2FIL_CUDA(acquire_status_word(&f->status));
-  B2FIL_CUDA(acquire_scratch_pool(f->device, &f->pool));
+  B2FIL_CUDA(acquire_scratch_pool(f->device, &f->scratch_peak, &f->pool));
   PinnedPool::get().add_user();
   return B2FIL_OK;
 }

@@ -103,3 +103,24 @@ def test_threads_share_the_staging_memory():
     for t in threads:
         t.join()
     assert not errors, errors[:2]
+
+
+def test_scratch_of_a_freed_model_goes_back_to_the_device():
+    """The scratch pool of a device outlives its models: freeing one that needed much returns what the
+    others do not need."""
+    import torch
+
+    desc, small = _model(6, n_trees=200)
+    x = torch.zeros((20_000, 6), device="cuda:0")
+    small.predict_proba(x)
+    wide, big = _model(200, n_trees=200)
+    X = torch.zeros((1_000_000, 200), device="cuda:0")
+    big.predict_proba(X)
+    torch.cuda.synchronize()
+    scratch = big.describe()["scratch_pool_bytes"]
+    assert scratch > 100 << 20
+    before = torch.cuda.mem_get_info()[0]
+    big.forest.close()
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] - before > scratch * 0.8
+    assert torch.equal(small.predict_proba(x), small.predict_proba(x))
