@@ -162,13 +162,11 @@ constexpr int kQInlineClasses = 4;
 
 // ---- compact image of a sparse forest -----------------------------------------------------------
 // Deep, ragged forests are bound by the chain of dependent node fetches from L2 / HBM.  Sparse
-// forests whose fields fit therefore carry a second image built for exactly that:
+// forests whose fields fit therefore carry a second image built for exactly that.  The packer writes
+// it node by node; what the kernel reads below the heaps are blocks made from it (further down).
 //  * internal nodes only, 8 bytes each {value, meta}, in depth-first order per tree, the child
-//    with the larger subtree first (rows are more likely to go where the training data went), so
-//    the node array is half the size of an array that also holds the leaves and a quarter of the
-//    16-byte fp64 array: it stays in L2.  The first child of node k is node k + 1: an aligned
-//    16-byte load brings a node and its neighbour, and half of the steps to a first child need no
-//    fetch at all;
+//    with the larger subtree first (rows are more likely to go where the training data went);
+//    the first child of node k is node k + 1;
 //  * leaves live in their own arrays (payload, id), numbered in the same depth-first order.  A
 //    walk carries the pair (k, L) = (internal node, number of leaves that precede it); with
 //    `off` = 1 + internal nodes of the first child's subtree,
@@ -180,12 +178,12 @@ constexpr int kQInlineClasses = 4;
 //  * fp64 forests keep `value` = the largest float <= threshold, and the kernel stages rows as
 //    floats rounded down: xl < value proves x < threshold, xl > value proves x > threshold, and
 //    only when xl == value the row's double and the exact threshold (`c_exact`) are read (one in
-//    2^24 visits on continuous data), so 8-byte nodes and 4-byte row values decide every fp64
-//    test exactly;
+//    2^24 visits on continuous data), so 4-byte values decide every fp64 test exactly;
 //  * the top `c_top_levels` levels of every tree are also stored as a complete heap
-//    [2^T nodes {value, feature | flags}][2^T exits {k, L}], which the kernel streams through
+//    [2^T nodes {value, feature | flags}][2^T exits], which the kernel streams through
 //    shared memory: a walk starts with T steps that cost no global fetch and leaves the heap
-//    through an exit = the pair (k, L) to continue at, or the leaf reached (bit 31 of k).
+//    through an exit: the node to continue at (in the uploaded heaps its block), or the leaf reached
+//    (bit 31).
 constexpr uint32_t CMETA_FIRST_LEAF  = 0x20000000u;
 constexpr uint32_t CMETA_SECOND_LEAF = 0x10000000u;
 constexpr uint32_t CMETA_SWAPPED     = 0x08000000u;  // the first (adjacent) child is the right child
@@ -219,12 +217,14 @@ struct CompactNode {  // 8 bytes
 // depth-20 forest: the walk below the heap is bound by how many dependent fetches an SM keeps in
 // flight (warps x walks per warp, and the L1 that tracks the misses: it shrinks as shared memory
 // grows), so heap levels are only worth their shared memory while they do not cost warps.  Eight
-// levels (4 KB per tree) with 28 warps on 128-row tiles were the best trade (9.5e7 rows/s; six
-// levels 8.9e7, nine levels - room for 12 warps only - 5.8e7).
+// levels (4 KB per tree) on 128-row tiles were the best trade when 8-byte nodes were walked by 28
+// warps (9.5e7 rows/s; six levels 8.9e7, nine levels - room for 12 warps only - 5.8e7); the walk over
+// blocks, with 20 warps, kept them.
 constexpr int kCDefaultTopLevels = 8;
 // With many features the row tile leaves little room: the heaps then get fewer levels, so that
-// 24 warps still fit under the 160 KiB that the launch code prefers (one warp per CTA next to
-// eight-level heaps ran a 1024-feature forest at 3.7e7 rows/s).
+// 24 warps would still fit under the 160 KiB that the launch code prefers (one warp per CTA next to
+// eight-level heaps ran a 1024-feature forest at 3.7e7 rows/s).  On the safe side of what is launched:
+// 20 warps on 128-row tiles, 23 at most, and a tile without the padding word per feature.
 inline int compact_pick_top_levels(int elem_bytes, int n_features, int n_outputs, int max_depth)
 {
   const size_t hard = 218 * 1024, soft = 160 * 1024;
@@ -304,10 +304,8 @@ struct ForestView {
   int32_t c_enabled;
   int32_t c_top_levels;         // T
   int32_t c_feat_bits;
-  int32_t c_bottom_steps;       // most steps a walk takes below the heap
-  int64_t c_top_stride;         // bytes between the heaps of two trees: 2^T * 16
   int32_t c_block_steps;        // most blocks on a walk
-  int32_t c_pad_;
+  int64_t c_top_stride;         // bytes between the heaps of two trees: 2^T * 16
   const uint32_t* c_blocks;     // [n_blocks * 8]
   const double* c_exact;        // [n_blocks * 4] exact thresholds (fp64 forests), else null
   const void* c_leaf_payload;   // [n_leaves] scalar in the forest precision or vector index

@@ -94,7 +94,7 @@ fetch_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, const uint3
 // ---------------------------------------------------------------------------------------------
 // DENSE kernel
 // ---------------------------------------------------------------------------------------------
-// Shared memory: [mbarriers 128 B][row tile][accumulators][flags 16 B][S tree stages].
+// Shared memory: [mbarriers 256 B][row tile][accumulators][flags 16 B][S tree stages].
 template <typename T, bool CAT, int MODE, int NT>
 struct DenseWalker {
   using TR = Traits<T>;
@@ -1545,7 +1545,7 @@ int launch_predict(const PredictParams& p, int chunk_size, int sm_count, cudaStr
   } else if (CompactCfg cc; compact_config(f, reduce, pick_rows_per_tile(p.n_rows, chunk_size, sm_count),
                                           p.n_rows, sm_count, chunk_size <= 0, cc)) {
     // deep / ragged forests with a compact image: heaps of the top levels through shared memory,
-    // 8-byte internal nodes below
+    // blocks of four nodes below
     LaunchRecord& rec = g_last_launch;
     rec               = LaunchRecord{};
     rec.kernel        = "sparse_compact_kernel";
@@ -1677,8 +1677,8 @@ int launch_predict_fixed_scratch(const PredictParams& p, int chunk_size, int sm_
   if (rc != B2FIL_OK) return rc;
   uint16_t* Q    = reinterpret_cast<uint16_t*>(base);
   int32_t* flags = reinterpret_cast<int32_t*>(static_cast<unsigned char*>(base) + q_bytes);
-  // the array keeps what the previous call left in it: the NaN flags of the tiles are
-  // accumulated with atomicOr and must start at zero (the ranks themselves are fully rewritten)
+  // the array keeps what the previous call left in it: the NaN flags of the tiles are only ever set
+  // and must start at zero (the ranks themselves are fully rewritten)
   cudaError_t e = cudaMemsetAsync(flags, 0, static_cast<size_t>(n_tiles) * 4, stream);
   if (e != cudaSuccess) {
     err = std::string("cudaMemsetAsync: ") + cudaGetErrorString(e);

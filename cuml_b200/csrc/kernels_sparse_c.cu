@@ -32,7 +32,9 @@ namespace {
 
 // 23 consumer warps and a producer: 80 registers a thread.  A walk holds a block (8 registers) and four
 // of them are in flight; with the 64 registers that 31 consumer warps leave, the blocks spill (200
-// trees of depth 20, 300,000 fp64 rows: 28 warps 2100 us, 20 warps 1694 us, 16 warps 1864 us).
+// trees of depth 20, 300,000 fp64 rows: 28 warps 2100 us, 20 warps 1694 us, 16 warps 1864 us).  At 80
+// some words still spill: 60 bytes in fp64 and 24 in fp32 for sums of scalar leaves, 8 and none for leaf
+// ids; sums of leaf vectors and categorical tests more.
 constexpr int kCompactWarps   = 23;
 constexpr int kCompactThreads = (kCompactWarps + 1) * 32;
 

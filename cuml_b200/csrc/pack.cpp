@@ -1055,7 +1055,6 @@ struct Packer {
     out.view.c_enabled      = 1;
     out.view.c_top_levels   = T;
     out.view.c_feat_bits    = fb;
-    out.view.c_bottom_steps = std::max(0, maxd - T);
     out.view.c_top_stride   = static_cast<int64_t>(top_bytes);
   }
 

@@ -103,7 +103,8 @@ class ForestInference:
     Parameters mirror `cuml.fil.ForestInference`:
 
     layout : 'depth_first' | 'breadth_first' | 'layered' - node order of sparse storage.
-    default_chunk_size : rows-per-CTA knob (1 -> 32 rows, 2 -> 64, >= 4 -> 128); None = automatic.
+    default_chunk_size : rows-per-CTA knob (1 -> 32 rows, 2 -> 64, 4 -> 128, on ranks 8 -> 256; more as
+        the largest); None = automatic.
     align_bytes : pad every tree of a sparse forest to a multiple of this many bytes.
     precision : 'single' | 'double' | 'native' (the model's own threshold type).
     is_classifier : whether `predict` returns classes and `predict_proba` is available.
@@ -112,8 +113,8 @@ class ForestInference:
     quantize_rows : dense forests (categorical splits only with categories below 32) predict on
         16-bit per-feature ranks of the inputs (exact: rank(x) <= j  <=>  x < threshold_j); False
         keeps the raw values.
-    compact_nodes : sparse forests also get a compact image (8-byte internal nodes in depth-first
-        order, leaves apart, the top levels of every tree as a heap that the kernel keeps in
+    compact_nodes : sparse forests also get a compact image (blocks of four tests that one fetch
+        brings, leaves apart, the top levels of every tree as a heap that the kernel keeps in
         shared memory) whenever their fields fit; False keeps only the plain node array.
     device_id : CUDA device that holds the forest.
     output_type : 'input' (same kind of array as X), 'numpy' or 'torch'.

@@ -142,7 +142,7 @@ typedef struct b2fil_create_opts {
                                  actually does is reported by b2fil_info.row_quantization, where
                                  1 means "on".                                                    */
   int32_t compact_image;      /* REQUEST, sparse storage: 0 = automatic (forests whose fields fit
-                                 also get the compact image - 8-byte internal nodes, leaves apart,
+                                 also get the compact image - blocks of four tests, leaves apart,
                                  top levels of every tree as a heap for shared memory - that the
                                  fast sparse kernel reads), 1 = never, 100 + T = automatic with at
                                  most T heap levels (tuning aid).  b2fil_info.compact_image says
@@ -258,10 +258,10 @@ int64_t b2fil_output_elems_per_row(const b2fil_forest* f, int infer_kind);
  * chunk_size 0 = the forest's default; positive values ask for row tiles of 32 * chunk_size rows and are
  * rounded down to a power of two.  `threshold` is the binary decision threshold of
  * B2FIL_INFER_CLASS for one-output classifiers.  Enqueues on cuda_stream (NULL = default stream)
- * of the forest's device and does not synchronise.  Two cases take stream-ordered scratch from a
- * memory pool owned by the forest (cached between calls): forests whose b2fil_info reports
- * row_quantization = 1 keep the 16-bit rank image of the batch there, and small batches of dense forests (fewer 128-row
- * tiles than half the SMs) keep the partial sums of the CTAs that share the forest there.
+ * of the forest's device and does not synchronise.  Forests whose b2fil_info reports
+ * row_quantization = 1 take stream-ordered scratch (the 16-bit rank image of the batch and the sums of row
+ * tiles that CTAs share) from a memory pool that the forests of a device share and that keeps it between
+ * calls; batches small enough for the kernel without ranks, and other forests, take none.
  * Replaces forest_model.predict(...) (cpp/tests/sg/rf_test.cu:268-275). */
 int b2fil_predict(const b2fil_forest* f, int infer_kind, const void* X_dev, int64_t n_rows,
                   int64_t row_stride, void* out_dev, int chunk_size, double threshold,

@@ -309,8 +309,8 @@ def test_row_stride_and_host_buffers():
 
 def test_pageable_host_arrays_take_the_staged_pipeline(lib):
     """An ordinary NumPy array of several hundred MB: the library gathers row blocks into its own
-    pinned staging buffers with a few host threads (three slots, 64 MiB blocks, so slots are
-    reused) instead of leaving the staging to the driver.  Leaf ids must equal the device path bit
+    pinned staging buffers with a few host threads (four slots and about eight blocks, so slots
+    are reused) instead of leaving the staging to the driver.  Leaf ids must equal the device path bit
     for bit and scores within the parity tolerance (row blocks choose their own tile shapes, and
     with them the order of the sums); a strided input through the C ABI as well."""
     import ctypes as C
@@ -319,7 +319,7 @@ def test_pageable_host_arrays_take_the_staged_pipeline(lib):
     desc = synthetic_complete_forest(60, 6, 256, seed=12)
     fi = ForestInference.load_from_treelite_model(desc)
     rng = np.random.default_rng(13)
-    n = 330_000  # 338 MB of fp32 rows: six blocks
+    n = 330_000  # 338 MB of fp32 rows: eight blocks
     X = rng.standard_normal((n, 256), dtype=np.float32)
     X[::1000, 7] = np.nan
     want = fi.predict_proba(torch.as_tensor(X, device="cuda:0")).cpu().numpy()
