@@ -221,3 +221,32 @@ def test_missing_values_come_and_go_between_overlapped_calls():
     got = [(fi.apply(X[i % 2]), fi.predict_proba(X[i % 2])) for i in range(40)]
     for i, (ids, p) in enumerate(got):
         assert torch.equal(ids, want[i % 2]) and torch.equal(p, proba[i % 2]), i
+
+
+def test_the_variants_that_these_tests_are_about_are_launched():
+    """Trees split over a cluster, row tiles with doubled columns, two row-tile buffers: at the shapes that
+    the tests above take them to run at."""
+    import numpy as np
+    import torch
+
+    from cuml_b200.fil import ForestInference, _lib, synthetic_complete_forest
+    from cuml_b200.fil._desc import INFER_DEFAULT, INFER_LEAF_ID
+    from oracle import oracle
+
+    small = random_forest_desc(90, max_depth=6, n_trees=130, n_features=9)
+    for storage, kernel in (("dense", "dense_kernel"), ("sparse", "sparse_compact_kernel")):
+        fi = ForestInference.load_from_treelite_model(small, storage=storage)
+        fi._run(torch.zeros((481, 9), device="cuda:0"), INFER_DEFAULT, None)
+        assert kernel in _lib.last_variant() and "forest_splits=" in _lib.last_variant()
+    desc = synthetic_complete_forest(300, 6, 60, 11)
+    assert desc.default_left.any()
+    fi = ForestInference.load_from_treelite_model(desc)
+    X = random_rows(9, 60_001, 60, np.float32, nan_frac=0.03)
+    x = torch.as_tensor(X, device="cuda:0")
+    p = fi.predict_proba(x).cpu().numpy()
+    assert "nan_columns" in _lib.last_variant() and "tiles=2" in _lib.last_variant()
+    np.testing.assert_allclose(p[:, 1:], oracle.predict(desc, X, INFER_DEFAULT, "single"), rtol=1e-5,
+                               atol=1e-6)
+    assert np.array_equal(fi.apply(x).cpu().numpy().astype(np.uint32),
+                          oracle.predict(desc, X, INFER_LEAF_ID, "single"))
+    assert "nan_columns" not in _lib.last_variant()
