@@ -56,7 +56,8 @@ def pack_check():
     blocks = os.path.join(ROOT, "cuml_b200", "csrc", "blocks.cpp")
     deps = [src, pack, blocks, os.path.join(ROOT, "cuml_b200", "csrc", "forest.hpp")]
     if not os.path.exists(so) or any(os.path.getmtime(d) > os.path.getmtime(so) for d in deps):
-        subprocess.check_call(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-o", so, src, pack, blocks])
+        subprocess.check_call(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-pthread", "-o", so, src, pack,
+                               blocks])
     lib = C.CDLL(so)
     lib.pack_check.restype = C.c_int
     lib.pack_check.argtypes = [C.POINTER(CForestDesc), C.POINTER(CCreateOpts), C.c_void_p,

@@ -332,3 +332,13 @@ def test_images_for_missing_values(pack_check, kw, precision):
     assert _check(pack_check, desc, X, precision, "depth_first", "dense")[6] == 1
     desc.default_left = np.zeros_like(desc.default_left)
     assert _check(pack_check, desc, X, precision, "depth_first", "dense")[6] == 1
+
+
+def test_blocks_of_a_forest_that_several_threads_cut(pack_check):
+    """More than a hundred thousand nodes: the trees are cut by several threads and put one behind the
+    other."""
+    desc = random_forest_desc(6, n_trees=31, max_depth=14, p_leaf=0.1, categorical=True)
+    X = random_rows(35, 60, desc.n_features, np.float64, nan_frac=0.05, categories=22)
+    for precision in ("single", "double"):
+        info = _check(pack_check, desc, X, precision, "depth_first", "sparse")
+        assert info[12] == 1 and info[4] > 200_000
