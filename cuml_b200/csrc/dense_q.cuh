@@ -402,11 +402,15 @@ struct DenseQWalker {
           }
         }
       }
-      // (payloads that were stored to global memory or to the accumulators have been read)
-      bool read = seen != 0xffffffffu;
-      if ((MODE == MODE_SCALAR && !LEAFG) || (MODE == MODE_VECTOR && inline_vec))
-        read = sums_known<T, MODE>(run);
-      release_stage(bars + 8u * (kMaxStages + s), lane, read, p.zero);
+      const uint32_t empty = bars + 8u * (kMaxStages + s);
+      if (MODE >= MODE_PERTREE) {
+        release_stored_stage(empty, lane);
+      } else {
+        bool read = seen != 0xffffffffu;
+        if ((MODE == MODE_SCALAR && !LEAFG) || (MODE == MODE_VECTOR && inline_vec))
+          read = sums_known<T, MODE>(run);
+        release_stage(empty, lane, read, p.zero);
+      }
       pos.advance(S);
     }
     if constexpr (LEAFG) take_pending();

@@ -104,6 +104,14 @@ __device__ __forceinline__ void release_stage(uint32_t bar, int lane, bool read,
   const uint32_t all = __ballot_sync(0xffffffffu, read);
   if (lane == 0) mbar_arrive(bar + (all & zero));
 }
+// The same where everything that was read has been stored to global memory (one output per row and tree):
+// a store leaves the warp with its data, and __syncwarp() keeps the stores before the arrival.  (The
+// vote costs leaf ids of 300 trees x 100,003 rows about half a percent.)
+__device__ __forceinline__ void release_stored_stage(uint32_t bar, int lane)
+{
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bar);
+}
 // Position in a ring of S stages: the stage index and the parity of its current use, advanced
 // without a division.
 struct RingPos {

@@ -148,7 +148,7 @@ struct DenseWalker {
             if (k < n_act) {
               const uint32_t slot = (a[k] - base[k]) / TR::NB - (1u << D);
               const typename TR::Val payload = TR::ld_val(base[k] + width_b + slot * TR::ES);
-              seen ^= TR::low32(payload);
+              if (MODE == MODE_VECTOR) seen ^= TR::low32(payload);
               take_leaf<T, MODE>(p, first + k, payload,
                                  (static_cast<uint32_t>(first + k) << D) + slot, acc_group, R, r,
                                  row, run);
@@ -156,9 +156,14 @@ struct DenseWalker {
           }
         }
       }
-      // (scalar leaves: their sum will do; the others are folded on the way)
-      release_stage(bars + 8u * (kMaxStages + s), lane,
-                    MODE == MODE_SCALAR ? sums_known<T, MODE>(run) : seen != 0xffffffffu, p.zero);
+      const uint32_t empty = bars + 8u * (kMaxStages + s);
+      if (MODE >= MODE_PERTREE) {
+        release_stored_stage(empty, lane);
+      } else {
+        // (scalar leaves: their sum will do; the indices of vector leaves are folded on the way)
+        release_stage(empty, lane, MODE == MODE_SCALAR ? sums_known<T, MODE>(run) : seen != 0xffffffffu,
+                      p.zero);
+      }
       pos.advance(S);
     }
     return ok;
