@@ -51,10 +51,10 @@ ROWS_PER_GPU = 10_000_000
 BYTES_PER_ROW = N_FEATURES * 4 + 2 * 4
 WORKLOAD = "gbdt_1000x_depth8_256f_fp32_sigmoid_10M_rows"
 # dram__bytes_read.sum + dram__bytes_write.sum per row of the two kernels of a prediction, from
-# the ncu captures of a 1 M-row case summarised under profiles/ (quantise 1560 B + dense_q 525 B;
+# the ncu captures of a 1 M-row chunk summarised under profiles/ (quantise 1542 B + dense_q 527 B;
 # the rank image of a chunk is larger than L2 and goes through HBM); traffic grows in proportion to
 # the rows, so it is scaled to the batch
-NCU_TRAFFIC_BYTES_PER_ROW = 2085
+NCU_TRAFFIC_BYTES_PER_ROW = 2069
 NCU_TRAFFIC_KERNELS = "quantise_kernel<float> + dense_q_top_kernel<float,scalar,NT=6,DEPTH=8>"
 
 
