@@ -316,8 +316,13 @@ __device__ __forceinline__ void for_each_constant(F&& f, std::integer_sequence<i
 // pulls into shared memory with a single bulk copy.  Groups or tiles too small to occupy the CTA's
 // threads that way are ranked several tiles at a time.  Nothing is exchanged between threads, so the
 // tile loop has no barrier.
-// Bound by issue slots: 46 instructions per 32 values in the first version, of which the search
-// (table entry, four halvings) is 17.  So values are ranked where they were loaded (the next tile's
+// The stores of a warp go to 32 different lines, one wavefront of the L1's data pipe each, whatever their
+// width: with 16 bytes per lane and store (NU = 8) they were 4 of the 14 wavefronts that 32 values cost, and that
+// pipe was busy 80 % of the time.  Sixteen ranks leave as one 32-byte store, a whole sector (NU = 16).  With
+// that and one halving less (better bucket grids) 1.5 M rows of 256 features are ranked in 590 us instead of
+// 750, 200,000 rows of 512 features in 330 instead of 380.
+// Next come the issue slots: 46 instructions per 32 values in the first version, of which the search
+// (table entry, four halvings) was 17.  So values are ranked where they were loaded (the next tile's
 // load follows in the same registers), the conversion to a bucket saturates instead of clamping,
 // ranks are made relative two at a time, and NaN and categories are fixed up off the common path.
 // Shared memory: [mbarrier 16 B][blobs].
@@ -389,33 +394,35 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
   const uint32_t rs      = static_cast<uint32_t>(p.row_stride);  // below 2^22: offsets inside a tile fit 32 bits
   const int64_t advance  = static_cast<int64_t>(stride) * R * p.row_stride;
 
-  T xs[NU];
+  // Up to eight values per thread are in flight (more did not fit the registers: 16 spilled).
+  constexpr int CHUNKS = NU / CH, AHEAD = CHUNKS < 2 ? CHUNKS : 2;
+  T xs[AHEAD * CH];
   // loads chunk c (slots s0 + c * CH ...) of the round that starts at `tile`
   auto fetch = [&](const T* at, int tile, int c) {
+    T* to = xs + c % AHEAD * CH;
     if (tile + tiles_par <= n_full) {
 #pragma unroll
       for (int j = c * CH; j < c * CH + CH; ++j)
-        xs[j] = TR::ldg_here(at + static_cast<uint32_t>((j >> 1) * pair + (j & 1) * odd) * rs);
+        to[j - c * CH] = TR::ldg_here(at + static_cast<uint32_t>((j >> 1) * pair + (j & 1) * odd) * rs);
     } else {
       const int row = (tile + sub) * R + b;
 #pragma unroll
       for (int j = c * CH; j < c * CH + CH; ++j) {
-        const int off = (j >> 1) * pair + (j & 1) * odd;
-        xs[j] = row + off < n_rows ? TR::ldg_here(at + static_cast<uint32_t>(off) * rs) : T(0);
+        const int off  = (j >> 1) * pair + (j & 1) * odd;
+        to[j - c * CH] = row + off < n_rows ? TR::ldg_here(at + static_cast<uint32_t>(off) * rs) : T(0);
       }
     }
   };
   if (base < n_tiles) {
 #pragma unroll
-    for (int c = 0; c < NU / CH; ++c) fetch(src, base, c);
+    for (int c = 0; c < AHEAD; ++c) fetch(src, base, c);
   }
   for (; base < n_tiles; base += stride) {
-    src += advance;
     uint32_t packed[NU / 2];
     bool saw_nan = false;
 #pragma unroll
-    for (int c = 0; c < NU / CH; ++c) {
-      const T* cur = xs + c * CH;
+    for (int c = 0; c < CHUNKS; ++c) {
+      const T* cur = xs + c % AHEAD * CH;
       // rank of the CH values, step by step across all of them so that the dependent
       // shared-memory lookups of different values overlap.  A NaN walks the same code (bucket 0,
       // every comparison false) and is replaced by Q_NAN_CODE at the end; so does a categorical
@@ -480,14 +487,24 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
           saw_nan |= nan != 0u;
         }
       }
-      // the same chunk of the CTA's next round goes into the registers just read, so a whole round of
-      // loads per thread stays in flight (an additional L2 prefetch further ahead measured slower)
-      if (base + stride < n_tiles) fetch(src, base + stride, c);
+      // the chunk after next, of this round or the CTA's next one, goes into the registers just read
+      // (an additional L2 prefetch further ahead measured slower)
+      if (c + AHEAD < CHUNKS) {
+        fetch(src, base, c + AHEAD);
+      } else if (base + stride < n_tiles) {
+        if (c + AHEAD == CHUNKS) src += advance;
+        fetch(src, base + stride, c + AHEAD - CHUNKS);
+      }
     }
     const bool live = base + sub < n_tiles;
     // Q[tile][feature][slot]: the thread's NU consecutive slots of its feature in one store
     if (live) {
-      if constexpr (NU == 8) {
+      if constexpr (NU == 16) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(packed[0]),
+                     "r"(packed[1]), "r"(packed[2]), "r"(packed[3]), "r"(packed[NU > 8 ? 4 : 0]),
+                     "r"(packed[NU > 8 ? 5 : 0]), "r"(packed[NU > 8 ? 6 : 0]), "r"(packed[NU > 8 ? 7 : 0])
+                     : "memory");
+      } else if constexpr (NU == 8) {
         *reinterpret_cast<uint4*>(dst) = make_uint4(packed[0], packed[1], packed[NU > 4 ? 2 : 0], packed[NU > 4 ? 3 : 0]);
       } else {
         *reinterpret_cast<uint2*>(dst) = make_uint2(packed[0], packed[1]);
@@ -520,6 +537,16 @@ __device__ __forceinline__ void quantise_rows(const PredictParams& p, const QGro
                                               uint32_t blob_a, const QFeatRec* rec, int tid, int first,
                                               int step, int slots, int tiles_par)
 {
+  if constexpr (sizeof(T) == 4) {
+    if (slots == 16) {
+      if (grp.f_end - grp.f_begin == 32 && STEPS >= 2) {
+        quantise_tiles<T, STEPS, 16, 32>(p, grp, Q, flags, R, blob_a, rec, tid, first, step, tiles_par);
+      } else {
+        quantise_tiles<T, STEPS, 16, 0>(p, grp, Q, flags, R, blob_a, rec, tid, first, step, tiles_par);
+      }
+      return;
+    }
+  }
   // full-width groups on large tiles, the shape of big batches, get the group size baked in
   if (grp.f_end - grp.f_begin == 32 && STEPS >= 2 && slots == 8) {
     quantise_tiles<T, STEPS, 8, 32>(p, grp, Q, flags, R, blob_a, rec, tid, first, step, tiles_par);
@@ -1086,7 +1113,7 @@ int launch_dense_q_kernel(const QLaunch& L, int mode, bool f64, std::string& err
 // a warp ranking 32 values in kRankCycles SM cycles (measured on 1 M rows of 256 features).  With large
 // batches many short CTAs fill the last wave (64 bundles on 148 SMs: 37 CTAs each), with 20,000 rows
 // loading the tables twice on an SM costs more than it evens out.
-constexpr double kRankCycles = 14.0;
+constexpr double kRankCycles = 14.0, kRankCycles16 = 11.0;  // (sixteen ranks per thread and store)
 int quantise_ctas_per_bundle(const ForestView& f, int R, int slots, int sm_count, int64_t n_tiles)
 {
   const double bundles = f.q_n_bundles - 1 + static_cast<double>(f.q_last_features) / f.q_bundle_features;
@@ -1095,7 +1122,7 @@ int quantise_ctas_per_bundle(const ForestView& f, int R, int slots, int sm_count
   while (width < f.q_bundle_features) width *= 2;
   const int par          = 1024 / width * slots / R;  // tiles that a CTA ranks at a time
   const int64_t n_rounds = (n_tiles + par - 1) / par;
-  const double per_round = kRankCycles * R * par * f.q_bundle_features / 32.0 + 100.0;
+  const double per_round = (slots == 16 ? kRankCycles16 : kRankCycles) * R * par * f.q_bundle_features / 32.0 + 100.0;
   int best = 1;
   double best_cost = 1e300;
   const int most = static_cast<int>(std::min<double>(n_rounds, std::max(48.0, sm_count / bundles)));
@@ -1118,9 +1145,14 @@ int launch_quantise(const PredictParams& p, uint16_t* Q, const QFlags& flags, in
   // shared memory: mbarrier and the largest bundle of tables
   const size_t smem = 16 + static_cast<size_t>(f.q_max_blob_bytes);
   // Eight ranks per thread and store; four where tiles are small and so few that the CTAs have one
-  // round of them each: there the time of one thread counts.
+  // round of them each: there the time of one thread counts.  Sixteen where a CTA has some rounds of so many
+  // (from 256 rows and 32 features per SM on) and all features are in groups of 32: whole calls of 13 forests
+  // with 32 to 512 features took 0.87 to 0.99 of the time with eight from there on, 1.0 to 1.1 below, and with a
+  // narrow group at the end (its CTAs rank 8 or 16 tiles at a time) 0.93 to 1.08.
   const int64_t n_tiles = (p.n_rows + R - 1) / R;
-  const int slots       = R <= 128 && n_tiles * f.q_n_bundles <= sm_count ? 4 : 8;
+  const bool sixteen    = !f64 && f.n_features % 32 == 0 && f.q_bundle_features == 32 &&
+                       f.q_last_features == 32 && p.n_rows * f.q_n_bundles >= int64_t(256) * sm_count;
+  const int slots       = R <= 128 && n_tiles * f.q_n_bundles <= sm_count ? 4 : (sixteen ? 16 : 8);
   const int gx          = quantise_ctas_per_bundle(f, R, slots, sm_count, n_tiles);
   const int last        = (gx * f.q_last_features + f.q_bundle_features - 1) / f.q_bundle_features;
   // A kernel that overlaps the one before it inherits how that one divided the SM's memory, and the

@@ -57,6 +57,26 @@ def test_rank_prepass_over_ragged_feature_groups(n_features, precision):
         _all_kinds(desc, X, precision, "depth_first", "dense", chunk_size=chunk)
 
 
+@pytest.mark.parametrize("n_features,max_depth", [(32, 5), (96, 8)])
+def test_rank_prepass_with_sixteen_ranks_per_thread(n_features, max_depth):
+    """Batches large enough for it (256 rows and 32 features per SM, groups of 32 only): row tiles of every
+    size, which are ranked 1 to 16 at a time, a partial last tile, few and many halvings, NaN in some tiles
+    only, thresholds that rows hit exactly, infinities."""
+    import numpy as np
+
+    desc = random_forest_desc(97, n_trees=61, n_features=n_features, max_depth=max_depth, mixed_ops=True,
+                              postproc="sigmoid")
+    thr = desc.threshold[desc.node_kind == 1]
+    n = 38_145
+    X = random_rows(n, n, n_features, np.float64, nan_frac=0.0)
+    X[: n // 3, 0] = np.resize(thr, n // 3)
+    X[n // 2, -1] = np.nan
+    X[-1, 0] = np.nan
+    X[1, 0], X[2, 0] = np.inf, -np.inf
+    for chunk in (1, 2, 4, 8, None):
+        _all_kinds(desc, X, "single", "depth_first", "dense", chunk_size=chunk)
+
+
 @pytest.mark.parametrize("precision", ["single", "double"])
 @pytest.mark.parametrize("n_trees,n_features", [(3, 5), (61, 9), (190, 40)])
 def test_deep_trees_at_batch_sizes_where_the_launch_shape_changes(n_trees, n_features, precision):

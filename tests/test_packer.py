@@ -224,6 +224,25 @@ def test_rank_tables_feature_groups(pack_check):
         assert info[10] <= 208 * 1024
 
 
+@pytest.mark.parametrize("op", [OP_LT, OP_LE])
+@pytest.mark.parametrize("precision", ["single", "double"])
+def test_bucket_grids_that_spare_a_halving(pack_check, op, precision):
+    """Hundreds of thresholds per feature, so that other bucket grids are tried: rows on the thresholds, next
+    to them, far outside of the grid, infinite and missing, with the halvings that 24 grids leave (in
+    fp32 the plain grid needs one more)."""
+    desc = synthetic_complete_forest(130, 8, 32, seed=5, op=op)
+    dt = np.float32 if precision == "single" else np.float64
+    thr = desc.threshold[desc.node_kind == 1].astype(dt)
+    X = random_rows(9, 1200, 32, dt)
+    X[:300] = np.resize(thr, (300, 32))
+    X[300:600] = np.nextafter(X[:300], dt(np.inf))
+    X[600:900] = np.nextafter(X[:300], dt(-np.inf))
+    X[900:903] = np.array([[np.inf], [-np.inf], [np.nan]])
+    X[903:905] = np.array([[1e30], [-1e30]])
+    info = _check(pack_check, desc, X, precision, "depth_first", "dense")
+    assert info[9] == 3, info[9]
+
+
 def test_rank_quantisation_threshold_limit(pack_check):
     """A feature with more distinct thresholds than a rank can number keeps the forest on the
     plain dense path."""
