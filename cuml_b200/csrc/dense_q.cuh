@@ -17,24 +17,78 @@ namespace {
 // The row tile arrives with one bulk copy per tile (the pre-pass already stored it feature-major),
 // where there is room for two while the tile before it is being walked (forests whose trees last
 // only a few microseconds per tile spend a fifth of them waiting for it otherwise);
-// tree batches stream through the stage ring exactly as in dense_kernel.  A node is 4 bytes
-// (rank j << 17 | default-right << 16 | feature << 2 | categorical) and a test is one signed
-// subtraction.
+// tree batches stream through the stage ring exactly as in dense_kernel.  A node is 4 bytes, a test one
+// half-precision compare, a step one predicated addition (forest.hpp).
 constexpr int NAN_NONE = 0, NAN_TESTED = 1, NAN_COLUMNS = 2;
 
 constexpr int kBarTileFull  = 2 * kMaxStages;      // mbarrier slots after the stage ring: two each
 constexpr int kBarTileEmpty = 2 * kMaxStages + 2;
 
-// node - (q << 17) in one multiply-add: the sign of (j - rank) lands in bit 31.
-__device__ __forceinline__ uint32_t rank_diff(uint32_t node, uint32_t q)
+// A test and the step behind it: the walk at `a` goes on to the right, `inc` bytes further in its level, when
+// the row's rank q is above the node's threshold.  NANS: the tile may hold missing values and its columns
+// are not doubled.  A visit is five instructions (node, address of the rank, rank, compare, addition)
+// instead of six in heap order with signed subtractions (multiply-add, funnel shift, address): the
+// headline forest executes 1.76e9 warp instructions per million rows instead of 2.14e9 at the same 5.9e8
+// shared-memory wavefronts, and the traversal takes 2.17 ms instead of 2.24.
+template <bool CAT, bool NANS>
+__device__ __forceinline__ void walk_step(uint32_t& a, uint32_t node, uint32_t q, uint32_t set, uint32_t inc)
 {
-  static_assert(Q_RANK_SHIFT == 17, "the multiplier below is -(1 << Q_RANK_SHIFT)");
-  uint32_t d;
-  asm("mad.lo.u32 %0, %1, 0xFFFE0000, %2;" : "=r"(d) : "r"(q), "r"(node));
-  return d;
+  static_assert(Q_WALK_CATEGORICAL == 0x7BFFu && Q_TILE_NAN == 0x7C00u, "the constants below");
+  if constexpr (!CAT && !NANS) {
+    asm("{\n.reg .pred p;\n.reg .b16 l, h, j, r, z;\n"
+        "mov.b32 {l, h}, %1;\nabs.f16 j, h;\nmov.b32 {r, z}, %2;\n"
+        "setp.gt.f16 p, r, j;\n@p add.u32 %0, %0, %3;\n}"
+        : "+r"(a)
+        : "r"(node), "r"(q), "r"(inc));
+  } else if constexpr (!CAT) {
+    asm("{\n.reg .pred p, m;\n.reg .b16 l, h, j, r, z;\n"
+        "mov.b32 {l, h}, %1;\nabs.f16 j, h;\nmov.b32 {r, z}, %2;\n"
+        "setp.lt.s32 m, %1, 0;\nsetp.eq.and.u32 m, %2, 0x7C00, m;\n"
+        "setp.gt.and.f16 p, r, j, !m;\n@p add.u32 %0, %0, %3;\n}"
+        : "+r"(a)
+        : "r"(node), "r"(q), "r"(inc));
+  } else {
+    // The code of a categorical value is its category and the node's set is stored bit-reversed: the shift by
+    // the code moves the category's bit to the sign position, and nothing but zeros for codes of 32 and
+    // above (no category, missing).  No code but a missing value is above the node's threshold.
+    // Predicated: the walk has no data-dependent branch.
+    const uint32_t before = a;
+    asm("{\n.reg .pred p;\n.reg .b16 l, h, j, r, z;\n.reg .b32 t;\n"
+        "mov.b32 {l, h}, %1;\nabs.f16 j, h;\nmov.b32 {r, z}, %2;\n"
+        "setp.gt.f16 p, r, j;\nshl.b32 t, %3, %2;\nsetp.lt.or.s32 p, t, 0, p;\n"
+        "@p add.u32 %0, %0, %4;\n}"
+        : "+r"(a)
+        : "r"(node), "r"(q), "r"(set), "r"(inc));
+    if (NANS) {
+      // missing values go left: the sign of a numerical node, the lowest bit of a categorical one's threshold
+      const bool cat = static_cast<int32_t>(node) >= 0x7BFE0000;
+      if (q == Q_TILE_NAN && (cat ? (node & 0x10000u) == 0u : static_cast<int32_t>(node) < 0)) a = before;
+    }
+  }
+}
+// The same at the root, where both children are at hand: returns the one that the row goes to.
+template <bool NANS>
+__device__ __forceinline__ uint32_t root_step(uint32_t& a, uint32_t node, uint32_t q, uint32_t left, uint32_t right)
+{
+  uint32_t next;
+  if constexpr (!NANS) {
+    asm("{\n.reg .pred p;\n.reg .b16 l, h, j, r, z;\n"
+        "mov.b32 {l, h}, %2;\nabs.f16 j, h;\nmov.b32 {r, z}, %3;\n"
+        "setp.gt.f16 p, r, j;\nselp.b32 %1, %5, %4, p;\n@p add.u32 %0, %0, 4;\n}"
+        : "+r"(a), "=r"(next)
+        : "r"(node), "r"(q), "r"(left), "r"(right));
+  } else {
+    asm("{\n.reg .pred p, m;\n.reg .b16 l, h, j, r, z;\n"
+        "mov.b32 {l, h}, %2;\nabs.f16 j, h;\nmov.b32 {r, z}, %3;\n"
+        "setp.lt.s32 m, %2, 0;\nsetp.eq.and.u32 m, %3, 0x7C00, m;\n"
+        "setp.gt.and.f16 p, r, j, !m;\nselp.b32 %1, %5, %4, p;\n@p add.u32 %0, %0, 4;\n}"
+        : "+r"(a), "=r"(next)
+        : "r"(node), "r"(q), "r"(left), "r"(right));
+  }
+  return next;
 }
 
-// The three top nodes (heap words 1..3) of every tree, passed to the kernel by value: kernel
+// The three top nodes (words 1..3) of every tree, passed to the kernel by value: kernel
 // parameters live in the constant bank, so the first two levels of every walk read their nodes
 // through the constant cache and spend no shared-memory bandwidth, the resource that bounds the
 // traversal (a warp reads the same tree in all lanes, so each lookup is one constant access).
@@ -49,42 +103,36 @@ __device__ __forceinline__ uint2 lds_u32x2(uint32_t a)
   return v;
 }
 
-// A categorical node is recognisable by its rank field, the largest there is (0x3FFF, or 0x3FFE in the
-// image for doubled columns).  Only such nodes have a category set, in an array of its own behind the
-// nodes, and only lanes on such a node fetch it: in a forest with one categorical test in sixteen
-// that is less than half a shared-memory wavefront per visit, against one and more for nodes that
-// carry their set along (5000 depth-6 trees, 8 of 128 features categorical).
+// A categorical node is recognisable by its threshold, above that of every other.  Only such nodes have a
+// category set, in an array of its own behind the nodes, and only lanes on such a node fetch it: in a forest
+// with one categorical test in sixteen that is less than half a shared-memory wavefront per visit, against
+// one and more for nodes that carry their set along (5000 depth-6 trees, 8 of 128 features categorical).
+// (An empty set elsewhere: a predicate that lived until the test made them spill.)
 template <uint32_t OFF>
 __device__ __forceinline__ uint32_t lds_if_categorical(uint32_t node, uint32_t a)
 {
-  // (the address register takes the set, so that a lane without one needs no other value for it)
-  asm volatile(
-    "{\n.reg .pred p;\nsetp.ge.s32 p, %1, 0x7FFC0000;\n@p ld.shared.u32 %0, [%0+%2];\n}"
-    : "+r"(a)
-    : "r"(node), "n"(OFF));
-  return a;
-}
-__device__ __forceinline__ uint32_t shift_if_categorical(uint32_t node, uint32_t d, uint32_t set, uint32_t code)
-{
-  static_assert(((Q_MAX_RANK_FIELD - 1u) << Q_RANK_SHIFT) == 0x7FFC0000u, "the constant below");
-  asm("{\n.reg .pred p;\nsetp.ge.s32 p, %1, 0x7FFC0000;\n@p shf.l.clamp.b32 %0, %0, %2, %3;\n}"
-      : "+r"(d)
-      : "r"(node), "r"(set), "r"(code));
-  return d;
+  uint32_t set = 0u;
+  asm volatile("{\n.reg .pred p;\nsetp.ge.s32 p, %1, 0x7BFE0000;\n@p ld.shared.u32 %0, [%2+%3];\n}"
+               : "+r"(set)
+               : "r"(node), "r"(a), "n"(OFF));
+  return set;
 }
 
 // DEPTH > 0 fixes the tree depth at compile time (the level loop is fully unrolled); DEPTH == 0
 // reads it from the forest.  TOPC: the first two levels take their nodes from `top`.
 // PAIR: the walk for launch shapes that shared memory keeps small (few warps, few trees in
 // flight), where the latency of one step, not the shared-memory pipe, is the limit: both children
-// of the current node (heap words 2i and 2i + 1, one aligned 8-byte load) are requested together
+// of the current node are requested together
 // with the row's rank, before the test is decided, so the next node is already there when the
 // test is known; a step costs one shared-memory latency instead of two, and one more wavefront.
 // LEAFG: the stages hold only the test nodes of the trees and a walk fetches its leaf payload from
 // the forest image in global memory (L2).  Deep trees are half payloads (4 KB of 8 KB at depth
 // 10); where shared memory next to the row tile holds only a dozen whole trees, leaving the
 // payloads out doubles the walks in flight, which is what such shapes are bound by.  The payload
-// fetch of a sub-batch is consumed one sub-batch later, behind the next walk.
+// fetch of a sub-batch is consumed one sub-batch later, behind the next walk.  Nodes and payloads are
+// arrays of their own: a stage is one copy (a copy per tree was 20 us slower with 2000 trees of depth 10 on
+// 200,000 rows), and the payloads of ways that part late are neighbours (180 us: in the order of the
+// blocks, whose last steps are the longest, every row fetched another sector).
 template <typename T, int MODE, int NT, int DEPTH, bool CAT, bool TOPC, bool PAIR = false,
           bool LEAFG = false>
 struct DenseQWalker {
@@ -112,10 +160,13 @@ struct DenseQWalker {
     const ForestView& f    = p.f;
     const int D            = DEPTH > 0 ? DEPTH : f.dense_depth;
     // bytes of a tree's test nodes, or (CAT) of its test nodes and the category sets behind them
-    const uint32_t width_b = (1u << D) * (CAT ? 8u : 4u);
-    const uint32_t sets_at = 4u << D;  // from a node to its category set
+    const uint32_t sets_at   = 4u * walk_sets_at(D);         // from a node to its category set
+    const uint32_t leaves_at = 4u * walk_leaves_at(D, CAT);  // from the start of a tree to its payloads
     // bytes between two trees of a stage
-    const uint32_t tstride = LEAFG ? width_b : static_cast<uint32_t>(f.q_tree_stride);
+    constexpr uint32_t kStride = LEAFG ? walk_nodes_stride(DEPTH)
+                                       : static_cast<uint32_t>(walk_tree_stride(DEPTH, CAT, TR::ES));
+    constexpr bool known_stride = MODE == MODE_SCALAR && DEPTH > 0;
+    const uint32_t tstride      = known_stride ? kStride : static_cast<uint32_t>(f.q_tree_stride);
     // bytes per leaf payload: the element size, except where vector leaves sit in the tree block
     const uint32_t lbytes  = MODE == MODE_SCALAR ? TR::ES : static_cast<uint32_t>(f.q_leaf_bytes);
     const bool inline_vec  = MODE != MODE_SCALAR && lbytes > TR::ES;
@@ -124,6 +175,24 @@ struct DenseQWalker {
     const int per_batch    = per_sub * K;
     const uint32_t mine    = static_cast<uint32_t>(g * NT) * tstride;  // this warp's trees in a sub-batch
     const uint32_t sub_b   = static_cast<uint32_t>(per_sub) * tstride;
+    // bytes from the start of a tree to a level, and of a step to the right on it (`lvl` is a number, or, where
+    // DEPTH is a constant, a constant)
+    auto level_at = [&](auto lvl) {
+      if constexpr (std::is_same_v<decltype(lvl), int>) {
+        return 4u * walk_level_at(D, lvl);
+      } else {
+        constexpr uint32_t at = 4u * walk_level_at(DEPTH, decltype(lvl)::value);
+        return at;
+      }
+    };
+    auto step_bytes = [&](auto lvl) {
+      if constexpr (std::is_same_v<decltype(lvl), int>) {
+        return 4u * walk_step_words(D, lvl);
+      } else {
+        constexpr uint32_t step = 4u * walk_step_words(DEPTH, decltype(lvl)::value);
+        return step;
+      }
+    };
     bool ok                = true;
     uint32_t seen          = 0u;  // what release_stage() cannot tell from the sums, folded
 
@@ -141,88 +210,83 @@ struct DenseQWalker {
     // the compiler drop every per-slot guard.
     auto sub_batch = [&](auto full_tag, uint32_t base0, int first, int n_act) {
       constexpr bool FULL = decltype(full_tag)::value;
-      uint32_t base[NT], idx[NT], a[NT];
+      // Where the size of a tree is a constant its slot is part of the loads' immediate offsets (headline
+      // forest, 1.5 M rows: 3980 -> 3945 us in heap order).
+      constexpr uint32_t TS = FULL && known_stride ? kStride : 0u;
+      using Each = std::make_integer_sequence<int, NT>;
+      // slots past the end of the forest repeat the last live tree; results are dropped
+      auto slot = [&](int k) { return static_cast<uint32_t>(FULL ? k : min(k, n_act - 1)) * tstride; };
+      uint32_t a[NT];  // start of the tree's block (the first one's, TS > 0) + 4 * place in the level
 #pragma unroll
-      for (int k = 0; k < NT; ++k) {
-        // slots past the end of the forest repeat the last live tree; results are dropped
-        base[k] = base0 + static_cast<uint32_t>(FULL ? k : min(k, n_act - 1)) * tstride;
-        idx[k]  = 1u;  // heap index of the root
-        a[k]    = base[k] + 4u;
-      }
+      for (int k = 0; k < NT; ++k) a[k] = TS ? base0 : base0 + slot(k);
       // the NT walks are independent: all node loads are issued first, then all rank loads,
       // so that their shared-memory latencies overlap inside one warp.
-      // test(): the rows' ranks against NT nodes; the sign bit of d[k] is the step to the right.
-      auto test = [&](const uint32_t(&node)[NT], const uint32_t(&at)[NT], uint32_t(&d)[NT],
-                      auto is_top) {
-        uint32_t q[NT], bits[NT];
+      // step(): the rows' ranks against NT nodes of level `lvl` (a constant where DEPTH is).
+      auto step = [&](const uint32_t(&node)[NT], auto lvl, auto from_param, auto&& move) {
+        constexpr bool PARAM = decltype(from_param)::value;
+        uint32_t q[NT], set[NT];
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           uint32_t from = row_addr;
-          if (decltype(is_top)::value && MISSING == NAN_COLUMNS && !(node[k] & Q_DEFAULT_RIGHT))
-            from += copy_off;
+          // (top nodes from the parameter block exist once and pick the column by their direction)
+          if (PARAM && MISSING == NAN_COLUMNS && static_cast<int32_t>(node[k]) < 0) from += copy_off;
           // the low half of a node is feature * 4: one dot-product instruction (low half x byte 0
           // of fstride, high half x byte 1 = 0) turns it into the address of the row's rank of
           // that feature
           q[k] = lds_u16(__dp2a_lo(node[k], fstride, from));
         }
+        if constexpr (CAT && DEPTH > 0) {
+          for_each_constant(
+            [&](auto kc) {
+              constexpr int k = decltype(kc)::value, L = decltype(lvl)::value;
+              set[k] = lds_if_categorical<k * TS + 4u * walk_level_at(DEPTH, L) + 4u * walk_sets_at(DEPTH)>(node[k], a[k]);
+            },
+            Each{});
+        } else {
 #pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          if (CAT)
-            bits[k] = lds_if_categorical<DEPTH ? 4u << DEPTH : 0u>(node[k], at[k] + (DEPTH ? 0u : sets_at));
+          for (int k = 0; k < NT; ++k)
+            set[k] = CAT ? lds_if_categorical<0>(node[k], a[k] + level_at(lvl) + sets_at) : 0u;
         }
 #pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          // rank j in the high half: x < T[j] <=> rank(x) <= j, so right <=> j - rank < 0
-          d[k] = rank_diff(node[k], q[k]);
-          if (CAT) {
-            // the code of a categorical value is its category and the node's set is stored
-            // bit-reversed: the clamped funnel shift by the code moves the category's bit to the sign
-            // position, and leaves d for every code of 32 and above (no category, NaN), which the
-            // large rank of a categorical node has made non-negative, or right for a missing value
-            // of a doubled column.  Predicated: the walk has no data-dependent branch.
-            d[k] = shift_if_categorical(node[k], d[k], bits[k], q[k]);
-          }
-          if (NANS) {
-            // the missing-goes-right flag sits 15 bits below the sign.  (Both forms compute the
-            // same; each kernel family keeps the one it was measured fastest with: the two walks
-            // of a kernel share its register allocation.)
-            if (CAT) {
-              if (q[k] == Q_NAN_CODE) d[k] = node[k] << 15;
-            } else {
-              if (q[k] == Q_NAN_CODE) d[k] = (node[k] & Q_DEFAULT_RIGHT) ? 0x80000000u : 0u;
-            }
-          }
-        }
+        for (int k = 0; k < NT; ++k) move(k, node[k], q[k], set[k]);
       };
-      auto level = [&]() {
-        uint32_t node[NT], d[NT];
+      auto level = [&](auto lvl) {
+        uint32_t node[NT];
+        if constexpr (DEPTH > 0) {
+          for_each_constant(
+            [&](auto kc) {
+              constexpr int k = decltype(kc)::value, L = decltype(lvl)::value;
+              node[k] = lds_u32_at<k * TS + 4u * walk_level_at(DEPTH, L)>(a[k]);
+            },
+            Each{});
+        } else {
 #pragma unroll
-        for (int k = 0; k < NT; ++k) node[k] = lds_u32(a[k]);
-        test(node, a, d, std::false_type{});
-#pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          // heap index 2i + right in one funnel shift: (i << 1) | (d >> 31)
-          idx[k] = __funnelshift_l(d[k], idx[k], 1);
-          a[k]   = idx[k] * 4u + base[k];
+          for (int k = 0; k < NT; ++k) node[k] = lds_u32(a[k] + level_at(lvl));
         }
+        step(node, lvl, std::false_type{}, [&](int k, uint32_t n, uint32_t q, uint32_t set) {
+          walk_step<CAT, NANS>(a[k], n, q, set, step_bytes(lvl));
+        });
       };
       if constexpr (PAIR) {
-        uint32_t node[NT], d[NT];
+        uint32_t node[NT];
 #pragma unroll
-        for (int k = 0; k < NT; ++k) node[k] = lds_u32(a[k]);  // the root
+        for (int k = 0; k < NT; ++k) node[k] = lds_u32(a[k] + 4u);  // the root
 #pragma unroll 2
         for (int lvl = 0; lvl < D; ++lvl) {
-          // children of node i are heap words 2i and 2i + 1; below the last level these are the
-          // two leaf payloads (4-byte payloads continue the heap)
-          uint2 pair[NT];
-#pragma unroll
-          for (int k = 0; k < NT; ++k) pair[k] = lds_u32x2(base[k] + idx[k] * 8u);
-          test(node, a, d, std::false_type{});
+          // both children; below the last level these are the two leaf payloads (4-byte payloads go on
+          // behind the nodes)
+          const uint32_t inc = step_bytes(lvl), at = lvl + 1 < D ? level_at(lvl + 1) : leaves_at;
+          uint32_t left[NT], right[NT];
 #pragma unroll
           for (int k = 0; k < NT; ++k) {
-            idx[k]  = __funnelshift_l(d[k], idx[k], 1);
-            node[k] = static_cast<int32_t>(d[k]) < 0 ? pair[k].y : pair[k].x;
+            left[k]  = lds_u32(a[k] + at);
+            right[k] = lds_u32(a[k] + at + inc);
           }
+          step(node, lvl, std::false_type{}, [&](int k, uint32_t n, uint32_t q, uint32_t) {
+            const uint32_t before = a[k];
+            walk_step<false, NANS>(a[k], n, q, 0u, inc);
+            node[k] = a[k] != before ? right[k] : left[k];
+          });
         }
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
@@ -231,9 +295,9 @@ struct DenseQWalker {
         }
         return;
       }
-      if (TOPC) {
+      if constexpr (TOPC) {
         // root and children from the constant bank: the same words in every lane
-        uint32_t n1[NT], n2[NT], n3[NT], node[NT], d[NT];
+        uint32_t n1[NT], n2[NT], n3[NT], node[NT];
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           const int t = 3 * (first + (FULL ? k : min(k, n_act - 1)));
@@ -241,38 +305,48 @@ struct DenseQWalker {
           n2[k]       = top->w[t + 1];
           n3[k]       = top->w[t + 2];
         }
-        test(n1, a, d, std::true_type{});
-#pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          node[k] = static_cast<int32_t>(d[k]) < 0 ? n3[k] : n2[k];
-          idx[k]  = __funnelshift_l(d[k], 1u, 1);
-        }
-        test(node, a, d, std::true_type{});
-#pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          idx[k] = __funnelshift_l(d[k], idx[k], 1);
-          a[k]   = idx[k] * 4u + base[k];
-        }
+        step(n1, std::integral_constant<int, 0>{}, std::true_type{},
+             [&](int k, uint32_t n, uint32_t q, uint32_t) { node[k] = root_step<NANS>(a[k], n, q, n2[k], n3[k]); });
+        step(node, std::integral_constant<int, 1>{}, std::true_type{},
+             [&](int k, uint32_t n, uint32_t q, uint32_t) { walk_step<false, NANS>(a[k], n, q, 0u, 8u); });
       }
-      if (DEPTH > 0) {
+      uint32_t at_far[LEAFG ? NT : 1];  // LEAFG: where the walks were on level kWalkFarLevel
+      if constexpr (DEPTH > 0) {
+        constexpr int SKIP = TOPC ? 2 : 0;
+        for_each_constant(
+          [&](auto lc) {
+            constexpr int L = decltype(lc)::value + SKIP;
+            if constexpr (LEAFG && L == kWalkFarLevel) {
 #pragma unroll
-        for (int lvl = TOPC ? 2 : 0; lvl < DEPTH; ++lvl) level();
+              for (int k = 0; k < NT; ++k) at_far[k] = a[k];
+            }
+            level(std::integral_constant<int, L>{});
+          },
+          std::make_integer_sequence<int, DEPTH - SKIP>{});
       } else {
 #pragma unroll 4
-        for (int lvl = 0; lvl < D; ++lvl) level();
+        for (int lvl = 0; lvl < D; ++lvl) level(lvl);
       }
+      // place of the leaf * 4 in tree k, and the address of its payload
+      auto place4  = [&](int k) { return a[k] - (TS ? base0 : base0 + slot(k)); };
+      auto leaf_at = [&](int k) {
+        return lbytes == 4u ? a[k] + k * TS + leaves_at : base0 + slot(k) + leaves_at + (place4(k) >> 2) * lbytes;
+      };
       if constexpr (LEAFG) {
         // add the payloads that the previous sub-batch requested (they arrived during this
         // walk), then request this sub-batch's; nothing touches them until the next one is done
         take_pending();
-        const unsigned char* image = static_cast<const unsigned char*>(f.q_nodes) + width_b;
+        const unsigned char* far = static_cast<const unsigned char*>(f.q_far_leaves);
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
-          const uint32_t slot = idx[k] - (1u << D);
-          const int tree      = first + (FULL ? k : min(k, n_act - 1));
-          seen ^= slot;
+          // the steps from that level on are multiples of its own, 129 words, whose number is found by a shift
+          static_assert(4u * walk_step_words(DEPTH, kWalkFarLevel) == 516u, "the shift below");
+          const uint32_t start = TS ? base0 : base0 + slot(k);
+          const uint32_t at    = ((at_far[k] - start) << (DEPTH - kWalkFarLevel)) + ((a[k] - at_far[k]) >> 9) * 4u;
+          const int tree       = first + (FULL ? k : min(k, n_act - 1));
+          seen ^= at;
           pend[k] = __ldg(reinterpret_cast<const uint32_t*>(
-            image + static_cast<size_t>(tree) * static_cast<size_t>(f.q_tree_stride) + slot * 4u));
+            far + static_cast<size_t>(tree) * (4u * walk_level_words(DEPTH, DEPTH)) + at));
         }
         pend_first = first;
         pend_n     = FULL ? NT : n_act;
@@ -294,13 +368,8 @@ struct DenseQWalker {
         // four lanes at a time (store_quads): scalar 4-byte stores at a stride of a whole output
         // row cost one sector request each and bound these predictions otherwise.
         typename TR::Val val[NT];
-        uint32_t leaf_at[NT];
 #pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          const uint32_t slot = idx[k] - (1u << D);
-          leaf_at[k]          = base[k] + width_b + slot * lbytes;
-          val[k]              = TR::ld_val(leaf_at[k]);
-        }
+        for (int k = 0; k < NT; ++k) val[k] = TR::ld_val(leaf_at(k));
         const bool scalar_out = MODE == MODE_LEAFID || f.leaf_vector_len <= 1;
         const bool quad = FULL && NT == 4 && scalar_out && f.q_trees_in_order != 0;
         using Out = std::conditional_t<MODE == MODE_LEAFID, uint32_t, typename TR::Val>;
@@ -337,7 +406,7 @@ struct DenseQWalker {
                 if (row < p.n_rows) {
                   const int orig = __ldg(f.tree_orig + first + k);
                   T* out = static_cast<T*>(p.out) + (row * f.n_trees + orig) * f.n_outputs;
-                  for (int c = 0; c < f.n_outputs; ++c) out[c] = TR::ld_real(leaf_at[k] + c * TR::ES);
+                  for (int c = 0; c < f.n_outputs; ++c) out[c] = TR::ld_real(leaf_at(k) + c * TR::ES);
                 }
               } else {
                 take_leaf<T, MODE>(p, first + k, val[k], 0u, acc_group, R, r, row, run);
@@ -350,7 +419,7 @@ struct DenseQWalker {
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           if (FULL || k < n_act) {
-            const uint2 v = lds_u32x2(base[k] + width_b + (idx[k] - (1u << D)) * 8u);
+            const uint2 v = lds_u32x2(base0 + slot(k) + leaves_at + place4(k) * 2u);
             run.v[0] += static_cast<T>(__uint_as_float(v.x));
             run.v[1] += static_cast<T>(__uint_as_float(v.y));
           }
@@ -359,12 +428,7 @@ struct DenseQWalker {
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           if (FULL || k < n_act) {
-            // the leaf payloads follow the 2^D node words: for 4-byte payloads the heap
-            // address of leaf slot j is exactly the address the walk ended on
-            const uint32_t slot   = idx[k] - (1u << D);
-            const uint32_t leaf_a = (MODE == MODE_SCALAR && TR::ES == 4 && !CAT)
-                                      ? a[k]
-                                      : base[k] + width_b + slot * lbytes;
+            const uint32_t leaf_a = leaf_at(k);
             if (MODE == MODE_VECTOR && inline_vec) {
               // the leaf's vector sits in the tree block: one sum per output, in registers
 #pragma unroll
@@ -549,9 +613,8 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
   const uint32_t bars        = smem_addr(smem);
   const uint32_t tile        = smem_addr(tile_ptr);
   const uint32_t stages      = smem_addr(stage_ptr);
-  const uint32_t gstride     = static_cast<uint32_t>(f.q_tree_stride);  // trees in the forest image
-  // trees in a stage: whole, or (LEAFG) only their 2^depth test nodes
-  const uint32_t tstride     = LEAFG ? (4u << (DEPTH > 0 ? DEPTH : f.dense_depth)) : gstride;
+  // trees in the image and in a stage: whole, or (LEAFG) only their test nodes
+  const uint32_t tstride     = LEAFG ? walk_nodes_stride(DEPTH) : static_cast<uint32_t>(f.q_tree_stride);
   const int per_batch        = G * NT * K;
   const uint32_t stage_bytes = per_batch * tstride;
   const int n_batches        = (f.n_trees + per_batch - 1) / per_batch;
@@ -587,7 +650,8 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
   if (warp == n_cw) {
     // ---- producer: row tiles, and the tree batches of each of them -----------------------------
     // predictions that report leaves stream the image whose payload slots hold the leaf ids
-    const void* image         = MODE == MODE_LEAFID ? f.q_nodes_ids : f.q_nodes;
+    const void* image         = LEAFG ? f.q_far_nodes : (MODE == MODE_LEAFID ? f.q_nodes_ids : f.q_nodes);
+    const void* image_nan     = LEAFG ? f.q_far_nodes_nan : f.q_nodes_nan;
     const unsigned char* qsrc = reinterpret_cast<const unsigned char*>(q.Q);
     RingPos pos;
     bool primed = false;  // every stage has been filled once
@@ -607,52 +671,31 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
       if (tpos.stage == 0) tprimed = true;
       return true;
     };
-    // LEAFG: a stage is one copy per tree (a dozen to 28 of them), which the lanes issue side by side.
-    // One lane needs 0.2 to 0.3 us for them, and a batch of trees is walked in 1.3 to 1.8 us (2000 trees
-    // of depth 9 x 500,000 rows of 440 features 4.70 -> 4.02 ms; depth 10, 512 features 5.80 -> 5.48).
-    // Otherwise lane 0 does everything.
-    const bool issues = LEAFG || lane == 0;
     grid_wait();
     bool going = seg.live();
     if (lane == 0 && going) going = request_tile(seg.tile);
-    if (LEAFG) going = __shfl_sync(0xffffffffu, going, 0);
     for (; seg.live(); seg.next()) {
       const bool nan_image = q.nan_columns && has_nan(seg.tile);
-      if (!issues || !going) continue;
-      const unsigned char* src = static_cast<const unsigned char*>(nan_image ? f.q_nodes_nan : image);
+      if (lane != 0 || !going) continue;
+      const unsigned char* src = static_cast<const unsigned char*>(nan_image ? image_nan : image);
       const bool more = seg.more();
       const int end   = seg.end();
       // with two buffers the next tile is requested once the ring is full of this tile's trees
       const int ask_at = q.tile_bufs == 2 ? min(end, seg.begin + S) - 1 : end - 1;
       for (int b = seg.begin; b < end && going; ++b) {
         const uint32_t s = pos.stage;
-        bool free = !primed || mbar_wait(bars + 8u * (kMaxStages + s), pos.phase ^ 1u);
-        if (LEAFG) free = __all_sync(0xffffffffu, free);
-        if (!free) {
-          if (lane == 0) report_status(p.status, 1);
+        if (primed && !mbar_wait(bars + 8u * (kMaxStages + s), pos.phase ^ 1u)) {
+          report_status(p.status, 1);
           going = false;
           break;
         }
         const int first      = b * per_batch;
-        const int count      = min(per_batch, f.n_trees - first);
-        const uint32_t bytes = count * tstride;
-        if (lane == 0) mbar_expect_tx(bars + 8u * s, bytes);
-        if (LEAFG) {
-          __syncwarp();
-          // the node half of every tree's block
-          for (int i = lane; i < count; i += 32)
-            bulk_copy_g2s(stages + s * stage_bytes + i * tstride,
-                          src + static_cast<size_t>(first + i) * gstride, tstride, bars + 8u * s);
-        } else {
-          bulk_copy_g2s(stages + s * stage_bytes, src + static_cast<size_t>(first) * gstride, bytes,
-                        bars + 8u * s);
-        }
+        const uint32_t bytes = min(per_batch, f.n_trees - first) * tstride;
+        mbar_expect_tx(bars + 8u * s, bytes);
+        bulk_copy_g2s(stages + s * stage_bytes, src + static_cast<size_t>(first) * tstride, bytes, bars + 8u * s);
         pos.advance(S);
         if (pos.stage == 0) primed = true;
-        if (more && b == ask_at) {
-          if (lane == 0) going = request_tile(seg.tile + 1);
-          if (LEAFG) going = __shfl_sync(0xffffffffu, going, 0);
-        }
+        if (more && b == ask_at) going = request_tile(seg.tile + 1);
       }
     }
     return;
@@ -682,14 +725,14 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
     Running<T> run{T(0), 0, {}};
     const uint32_t at_tile = tpos.stage * tile_room;
     if (nans && q.nan_columns) {
-      // the second set of columns: the NaN code moves from "right" to "left"
+      // the second set of columns: missing values move from "right" to "left"
       for (uint32_t i = threadIdx.x * 16u; i < tile_bytes; i += n_ct * 16u) {
         uint4* from = reinterpret_cast<uint4*>(tile_ptr + at_tile + i);
         uint4 v     = *from;
         uint32_t* w = &v.x;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          w[k] |= __vcmpeq2(w[k], Q_NAN_CODE * 0x10001u) & Q_NAN_LEFT_BIT * 0x10001u;
+          w[k] |= __vcmpeq2(w[k], Q_TILE_NAN * 0x10001u) & Q_TILE_NAN_LEFT * 0x10001u;
         *reinterpret_cast<uint4*>(tile_ptr + at_tile + tile_bytes + i) = v;
       }
       consumer_sync(n_ct);
@@ -751,12 +794,20 @@ dense_q_pair_kernel(const __grid_constant__ PredictParams p, const __grid_consta
   dense_q_body<float, MODE_SCALAR, NT, 0, false, false, true>(p, q, nullptr);
 }
 
-// Same kernel with the leaf payloads left in global memory (see DenseQWalker).
+// Same kernel with the leaf payloads left in global memory (see DenseQWalker), and the same with the top nodes
+// in the parameter block.
 template <int NT, int DEPTH>
 __global__ void __launch_bounds__(1024, 1)
 dense_q_leafg_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q)
 {
   dense_q_body<float, MODE_SCALAR, NT, DEPTH, false, false, false, true>(p, q, nullptr);
+}
+template <int NT, int DEPTH>
+__global__ void __launch_bounds__(1024, 1)
+dense_q_leafg_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q,
+                     const __grid_constant__ QTop top)
+{
+  dense_q_body<float, MODE_SCALAR, NT, DEPTH, false, true, false, true>(p, q, &top);
 }
 
 // Same kernel with the top nodes of every tree in the parameter block.
@@ -768,14 +819,19 @@ dense_q_top_kernel(const __grid_constant__ PredictParams p, const __grid_constan
   dense_q_body<T, MODE, NT, DEPTH, false, true>(p, q, &top);
 }
 
+// The three top nodes of every tree, which travel in the parameter block.
+inline const QTop& top_nodes(const QLaunch& L)
+{
+  static thread_local QTop top;
+  std::memcpy(top.w, L.p.q_top, static_cast<size_t>(L.p.f.n_trees) * 3 * sizeof(uint32_t));
+  return top;
+}
+
 // Launch one instantiation of dense_q_top_kernel.
 template <typename T, int MODE, int NT, int DEPTH>
 int launch_q_top(const QLaunch& L, std::string& err)
 {
-  // the three top nodes of every tree travel in the parameter block
-  static thread_local QTop top;
-  std::memcpy(top.w, L.p.q_top, static_cast<size_t>(L.p.f.n_trees) * 3 * sizeof(uint32_t));
-  return launch_split(L.shape(), err, dense_q_top_kernel<T, MODE, NT, DEPTH>, L.p, L.q, top);
+  return launch_split(L.shape(), err, dense_q_top_kernel<T, MODE, NT, DEPTH>, L.p, L.q, top_nodes(L));
 }
 template <typename T, int MODE, int NT>
 int launch_q_top_depth(const QLaunch& L, std::string& err)

@@ -26,8 +26,8 @@ namespace {
 #define B2FIL_SPIN_NS 256  // sleep between two tries of a bounded mbarrier wait
 #endif
 constexpr uint32_t kSpinLimit = 1u << 22;  // tries of a bounded mbarrier wait
-constexpr int kBarBytes       = 256;       // room for the mbarriers at the start of shared memory
-constexpr int kMaxStages      = 8;
+constexpr int kBarBytes       = 192;       // room for the mbarriers at the start of shared memory
+constexpr int kMaxStages      = 8;         // (two for each stage, four more in the traversal over ranks)
 
 // ---------------------------------------------------------------------------------------------
 // shared-memory and mbarrier primitives (inline PTX)
@@ -147,6 +147,20 @@ __device__ __forceinline__ uint32_t lds_u16(uint32_t a)
   uint32_t v;  // a 16-bit load into a 32-bit register zero-extends
   asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(a));
   return v;
+}
+template <uint32_t OFF>
+__device__ __forceinline__ uint32_t lds_u32_at(uint32_t a)  // [a + OFF], OFF an immediate
+{
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(OFF));
+  return v;
+}
+// Calls f(std::integral_constant<int, K>) for K = 0, 1, ...: a loop whose counter is a constant
+// expression inside the body.
+template <typename F, int... Ks>
+__device__ __forceinline__ void for_each_constant(F&& f, std::integer_sequence<int, Ks...>)
+{
+  (f(std::integral_constant<int, Ks>{}), ...);
 }
 // Barrier among the consumer threads only (the producer warp never joins it).
 __device__ __forceinline__ void consumer_sync(int n_threads)

@@ -297,14 +297,6 @@ dense_kernel(const __grid_constant__ PredictParams p, const int R, const int G, 
 // ---------------------------------------------------------------------------------------------
 // RANK QUANTISATION of rows (pre-pass of the quantised dense kernel)
 // ---------------------------------------------------------------------------------------------
-// Calls f(std::integral_constant<int, K>) for K = 0, 1, ...: a loop whose counter is a constant
-// expression inside the body.
-template <typename F, int... Ks>
-__device__ __forceinline__ void for_each_constant(F&& f, std::integer_sequence<int, Ks...>)
-{
-  (f(std::integral_constant<int, Ks>{}), ...);
-}
-
 // One CTA owns a bundle of feature groups (usually one group of 32 features; a narrow tail is several
 // groups, dealt to its warps): the groups' blobs (feature records, bucket tables, sorted thresholds,
 // both tables interleaved across the group's features) arrive in shared memory with one bulk copy,
@@ -425,7 +417,7 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
       const T* cur = xs + c % AHEAD * CH;
       // rank of the CH values, step by step across all of them so that the dependent
       // shared-memory lookups of different values overlap.  A NaN walks the same code (bucket 0,
-      // every comparison false) and is replaced by Q_NAN_CODE at the end; so does a categorical
+      // every comparison false) and is replaced by Q_TILE_NAN at the end; so does a categorical
       // value (its feature has empty tables), replaced by its category.
       uint32_t a[CH];  // address of the threshold below the current window
 #pragma unroll
@@ -483,7 +475,7 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
 #pragma unroll
         for (int u = 0; u < CH; u += 2) {
           const uint32_t nan = (cur[u] != cur[u] ? 0xffffu : 0u) | (cur[u + 1] != cur[u + 1] ? 0xffff0000u : 0u);
-          two[u >> 1] = (two[u >> 1] & ~nan) | (Q_NAN_CODE * 0x10001u & nan);
+          two[u >> 1] = (two[u >> 1] & ~nan) | (Q_TILE_NAN * 0x10001u & nan);
           saw_nan |= nan != 0u;
         }
       }
@@ -868,9 +860,8 @@ size_t dense_q_smem(size_t qstride, int precision, int F, int NC, bool reduce, i
 // (dense_q_leafg_kernel: fp32 scalar leaves, no categorical tests, depth 9 or 10), else 0.
 size_t q_node_only_stride(const ForestView& f, int mode)
 {
-  const bool ok = f.format == FMT_DENSE_F && mode == MODE_SCALAR && !f.q_has_cat &&
-                  (f.dense_depth == 9 || f.dense_depth == 10);
-  return ok ? (size_t(4) << f.dense_depth) : 0;
+  const bool ok = mode == MODE_SCALAR && f.q_far_leaves != nullptr;
+  return ok ? walk_nodes_stride(f.dense_depth) : 0;
 }
 
 // Most trees a warp of the quantised kernel may walk side by side: the kernels that exist.
@@ -1099,9 +1090,13 @@ int launch_dense_q_kernel(const QLaunch& L, int mode, bool f64, std::string& err
     rec.depth = f.dense_depth;
     return launch_q_plain4(L, err);
   }
-  if (specialised && f.dense_depth >= 9 && (L.c.trees_in_flight == 2 || L.c.trees_in_flight == 3)) {
+  if (specialised && f.dense_depth >= 9 && L.c.trees_in_flight == 3) {
     rec.depth = f.dense_depth;
-    return launch_q_plain23(L, err);
+    return launch_q_plain3(L, err);
+  }
+  if (unrolled && L.c.trees_in_flight <= 2) {
+    rec.depth = f.dense_depth;
+    return launch_q_narrow(L, mode, err);
   }
   return launch_q_generic(L, mode, f64, err);
 }
@@ -1485,7 +1480,7 @@ int dense_ok(int depth, int precision, int n_features, int n_outputs)
   // else the traversal over rank-quantised rows alone, if a 32-row tile of ranks and two stages
   // of one tree fit (a tree counted at its largest: 8-byte test nodes, four inline outputs)
   const size_t es      = precision == B2FIL_F32 ? 4 : 8;
-  const size_t qstride = (size_t(8) + 4 * es) << depth;
+  const size_t qstride = walk_tree_stride(depth, true, 4 * es);
   if (dense_q_smem(qstride, precision, n_features, n_outputs, true, 32, 1, 1, 2, 1) <= kMaxSmemBytes &&
       n_features < (1 << 14))
     return 2;

@@ -7,7 +7,12 @@ namespace {
 template <int NT, int DEPTH>
 int launch_leafg(const QLaunch& L, std::string& err)
 {
-  auto k = dense_q_leafg_kernel<NT, DEPTH>;
+  // (the parameter block costs a launch 2.5 us)
+  if (L.p.q_top != nullptr && L.p.n_rows * L.p.f.n_trees * DEPTH > int64_t(200) << 20) {
+    void (*k)(const PredictParams, const QArgs, const QTop) = dense_q_leafg_kernel<NT, DEPTH>;
+    return launch_split(L.shape(), err, k, L.p, L.q, top_nodes(L));
+  }
+  void (*k)(const PredictParams, const QArgs) = dense_q_leafg_kernel<NT, DEPTH>;
   return launch_split(L.shape(), err, k, L.p, L.q);
 }
 
