@@ -92,9 +92,13 @@ __device__ __forceinline__ uint32_t root_step(uint32_t& a, uint32_t node, uint32
 // parameters live in the constant bank, so the first two levels of every walk read their nodes
 // through the constant cache and spend no shared-memory bandwidth, the resource that bounds the
 // traversal (a warp reads the same tree in all lanes, so each lookup is one constant access).
+// In two sizes: 24 KB of parameters make a launch 1 to 2 us longer than four.
+template <int TREES>
 struct QTop {
-  uint32_t w[3 * kQTopTrees];
+  uint32_t w[3 * TREES];
 };
+constexpr int kQTopFew = 320;
+static_assert(kQTopFew < kQTopTrees, "two sizes");
 
 __device__ __forceinline__ uint2 lds_u32x2(uint32_t a)
 {
@@ -148,7 +152,7 @@ struct DenseQWalker {
                                               uint32_t stages, uint32_t stage_bytes,
                                               uint32_t row_addr, uint32_t stride_b, T* acc_group,
                                               int R, RingPos& pos, Running<T>& run,
-                                              const QTop* top, int b_begin, int b_end,
+                                              const uint32_t* top, int b_begin, int b_end,
                                               uint32_t copy_off)
   {
     constexpr bool NANS = MISSING == NAN_TESTED;
@@ -301,9 +305,9 @@ struct DenseQWalker {
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           const int t = 3 * (first + (FULL ? k : min(k, n_act - 1)));
-          n1[k]       = top->w[t];
-          n2[k]       = top->w[t + 1];
-          n3[k]       = top->w[t + 2];
+          n1[k]       = top[t];
+          n2[k]       = top[t + 1];
+          n3[k]       = top[t + 2];
         }
         step(n1, std::integral_constant<int, 0>{}, std::true_type{},
              [&](int k, uint32_t n, uint32_t q, uint32_t) { node[k] = root_step<NANS>(a[k], n, q, n2[k], n3[k]); });
@@ -583,7 +587,7 @@ __device__ __forceinline__ void finish_shared_tile(const PredictParams& p, const
 template <typename T, int MODE, int NT, int DEPTH, bool CAT, bool TOPC, bool PAIR = false,
           bool LEAFG = false>
 __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs& q,
-                                             const QTop* top)
+                                             const uint32_t* top)
 {
   using TR = Traits<T>;
   using Walker = DenseQWalker<T, MODE, NT, DEPTH, CAT, TOPC, PAIR, LEAFG>;
@@ -802,27 +806,28 @@ dense_q_leafg_kernel(const __grid_constant__ PredictParams p, const __grid_const
 {
   dense_q_body<float, MODE_SCALAR, NT, DEPTH, false, false, false, true>(p, q, nullptr);
 }
-template <int NT, int DEPTH>
+template <int NT, int DEPTH, int TREES>
 __global__ void __launch_bounds__(1024, 1)
 dense_q_leafg_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q,
-                     const __grid_constant__ QTop top)
+                     const __grid_constant__ QTop<TREES> top)
 {
-  dense_q_body<float, MODE_SCALAR, NT, DEPTH, false, true, false, true>(p, q, &top);
+  dense_q_body<float, MODE_SCALAR, NT, DEPTH, false, true, false, true>(p, q, top.w);
 }
 
 // Same kernel with the top nodes of every tree in the parameter block.
-template <typename T, int MODE, int NT, int DEPTH>
+template <typename T, int MODE, int NT, int DEPTH, int TREES>
 __global__ void __launch_bounds__(NT > 4 ? 800 : 1024, 1)
 dense_q_top_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q,
-                   const __grid_constant__ QTop top)
+                   const __grid_constant__ QTop<TREES> top)
 {
-  dense_q_body<T, MODE, NT, DEPTH, false, true>(p, q, &top);
+  dense_q_body<T, MODE, NT, DEPTH, false, true>(p, q, top.w);
 }
 
 // The three top nodes of every tree, which travel in the parameter block.
-inline const QTop& top_nodes(const QLaunch& L)
+template <int TREES>
+const QTop<TREES>& top_nodes(const QLaunch& L)
 {
-  static thread_local QTop top;
+  static thread_local QTop<TREES> top;
   std::memcpy(top.w, L.p.q_top, static_cast<size_t>(L.p.f.n_trees) * 3 * sizeof(uint32_t));
   return top;
 }
@@ -831,7 +836,11 @@ inline const QTop& top_nodes(const QLaunch& L)
 template <typename T, int MODE, int NT, int DEPTH>
 int launch_q_top(const QLaunch& L, std::string& err)
 {
-  return launch_split(L.shape(), err, dense_q_top_kernel<T, MODE, NT, DEPTH>, L.p, L.q, top_nodes(L));
+  if (L.p.f.n_trees <= kQTopFew)
+    return launch_split(L.shape(), err, dense_q_top_kernel<T, MODE, NT, DEPTH, kQTopFew>, L.p, L.q,
+                        top_nodes<kQTopFew>(L));
+  return launch_split(L.shape(), err, dense_q_top_kernel<T, MODE, NT, DEPTH, kQTopTrees>, L.p, L.q,
+                      top_nodes<kQTopTrees>(L));
 }
 template <typename T, int MODE, int NT>
 int launch_q_top_depth(const QLaunch& L, std::string& err)

@@ -7,11 +7,12 @@ namespace {
 template <int NT, int DEPTH>
 int launch_leafg(const QLaunch& L, std::string& err)
 {
-  // (the parameter block costs a launch 2.5 us)
-  if (L.p.q_top != nullptr && L.p.n_rows * L.p.f.n_trees * DEPTH > int64_t(200) << 20) {
-    void (*k)(const PredictParams, const QArgs, const QTop) = dense_q_leafg_kernel<NT, DEPTH>;
-    return launch_split(L.shape(), err, k, L.p, L.q, top_nodes(L));
-  }
+  if (L.p.q_top != nullptr && L.p.f.n_trees <= kQTopFew)
+    return launch_split(L.shape(), err, dense_q_leafg_kernel<NT, DEPTH, kQTopFew>, L.p, L.q, top_nodes<kQTopFew>(L));
+  // (the launch of the large parameter block takes what it saves in calls of less than about 100 us)
+  if (L.p.q_top != nullptr && L.p.n_rows * L.p.f.n_trees * DEPTH > int64_t(200) << 20)
+    return launch_split(L.shape(), err, dense_q_leafg_kernel<NT, DEPTH, kQTopTrees>, L.p, L.q,
+                        top_nodes<kQTopTrees>(L));
   void (*k)(const PredictParams, const QArgs) = dense_q_leafg_kernel<NT, DEPTH>;
   return launch_split(L.shape(), err, k, L.p, L.q);
 }
