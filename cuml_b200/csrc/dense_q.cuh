@@ -18,11 +18,21 @@ namespace {
 // where there is room for two while the tile before it is being walked (forests whose trees last
 // only a few microseconds per tile spend a fifth of them waiting for it otherwise);
 // tree batches stream through the stage ring exactly as in dense_kernel.  A node is 4 bytes, a test one
-// half-precision compare, a step one predicated addition (forest.hpp).
+// half-precision compare and a step one predicated addition (forest.hpp), or, in forests with categorical
+// tests, one signed subtraction and a funnel shift.
 constexpr int NAN_NONE = 0, NAN_TESTED = 1, NAN_COLUMNS = 2;
 
 constexpr int kBarTileFull  = 2 * kMaxStages;      // mbarrier slots after the stage ring: two each
 constexpr int kBarTileEmpty = 2 * kMaxStages + 2;
+
+// node - (q << 17) in one multiply-add: the sign of (j - rank) lands in bit 31.
+__device__ __forceinline__ uint32_t rank_diff(uint32_t node, uint32_t q)
+{
+  static_assert(Q_RANK_SHIFT == 17, "the multiplier below is -(1 << Q_RANK_SHIFT)");
+  uint32_t d;
+  asm("mad.lo.u32 %0, %1, 0xFFFE0000, %2;" : "=r"(d) : "r"(q), "r"(node));
+  return d;
+}
 
 // A test and the step behind it: the walk at `a` goes on to the right, `inc` bytes further in its level, when
 // the row's rank q is above the node's threshold.  NANS: the tile may hold missing values and its columns
@@ -30,40 +40,23 @@ constexpr int kBarTileEmpty = 2 * kMaxStages + 2;
 // instead of six in heap order with signed subtractions (multiply-add, funnel shift, address): the
 // headline forest executes 1.76e9 warp instructions per million rows instead of 2.14e9 at the same 5.9e8
 // shared-memory wavefronts, and the traversal takes 2.17 ms instead of 2.24.
-template <bool CAT, bool NANS>
-__device__ __forceinline__ void walk_step(uint32_t& a, uint32_t node, uint32_t q, uint32_t set, uint32_t inc)
+template <bool NANS>
+__device__ __forceinline__ void walk_step(uint32_t& a, uint32_t node, uint32_t q, uint32_t inc)
 {
-  static_assert(Q_WALK_CATEGORICAL == 0x7BFFu && Q_TILE_NAN == 0x7C00u, "the constants below");
-  if constexpr (!CAT && !NANS) {
+  static_assert(Q_NAN_CODE == 0x3FFFu, "the constant below");
+  if constexpr (!NANS) {
     asm("{\n.reg .pred p;\n.reg .b16 l, h, j, r, z;\n"
         "mov.b32 {l, h}, %1;\nabs.f16 j, h;\nmov.b32 {r, z}, %2;\n"
         "setp.gt.f16 p, r, j;\n@p add.u32 %0, %0, %3;\n}"
         : "+r"(a)
         : "r"(node), "r"(q), "r"(inc));
-  } else if constexpr (!CAT) {
+  } else {
     asm("{\n.reg .pred p, m;\n.reg .b16 l, h, j, r, z;\n"
         "mov.b32 {l, h}, %1;\nabs.f16 j, h;\nmov.b32 {r, z}, %2;\n"
-        "setp.lt.s32 m, %1, 0;\nsetp.eq.and.u32 m, %2, 0x7C00, m;\n"
+        "setp.lt.s32 m, %1, 0;\nsetp.eq.and.u32 m, %2, 0x3FFF, m;\n"
         "setp.gt.and.f16 p, r, j, !m;\n@p add.u32 %0, %0, %3;\n}"
         : "+r"(a)
         : "r"(node), "r"(q), "r"(inc));
-  } else {
-    // The code of a categorical value is its category and the node's set is stored bit-reversed: the shift by
-    // the code moves the category's bit to the sign position, and nothing but zeros for codes of 32 and
-    // above (no category, missing).  No code but a missing value is above the node's threshold.
-    // Predicated: the walk has no data-dependent branch.
-    const uint32_t before = a;
-    asm("{\n.reg .pred p;\n.reg .b16 l, h, j, r, z;\n.reg .b32 t;\n"
-        "mov.b32 {l, h}, %1;\nabs.f16 j, h;\nmov.b32 {r, z}, %2;\n"
-        "setp.gt.f16 p, r, j;\nshl.b32 t, %3, %2;\nsetp.lt.or.s32 p, t, 0, p;\n"
-        "@p add.u32 %0, %0, %4;\n}"
-        : "+r"(a)
-        : "r"(node), "r"(q), "r"(set), "r"(inc));
-    if (NANS) {
-      // missing values go left: the sign of a numerical node, the lowest bit of a categorical one's threshold
-      const bool cat = static_cast<int32_t>(node) >= 0x7BFE0000;
-      if (q == Q_TILE_NAN && (cat ? (node & 0x10000u) == 0u : static_cast<int32_t>(node) < 0)) a = before;
-    }
   }
 }
 // The same at the root, where both children are at hand: returns the one that the row goes to.
@@ -80,7 +73,7 @@ __device__ __forceinline__ uint32_t root_step(uint32_t& a, uint32_t node, uint32
   } else {
     asm("{\n.reg .pred p, m;\n.reg .b16 l, h, j, r, z;\n"
         "mov.b32 {l, h}, %2;\nabs.f16 j, h;\nmov.b32 {r, z}, %3;\n"
-        "setp.lt.s32 m, %2, 0;\nsetp.eq.and.u32 m, %3, 0x7C00, m;\n"
+        "setp.lt.s32 m, %2, 0;\nsetp.eq.and.u32 m, %3, 0x3FFF, m;\n"
         "setp.gt.and.f16 p, r, j, !m;\nselp.b32 %1, %5, %4, p;\n@p add.u32 %0, %0, 4;\n}"
         : "+r"(a), "=r"(next)
         : "r"(node), "r"(q), "r"(left), "r"(right));
@@ -107,19 +100,28 @@ __device__ __forceinline__ uint2 lds_u32x2(uint32_t a)
   return v;
 }
 
-// A categorical node is recognisable by its threshold, above that of every other.  Only such nodes have a
-// category set, in an array of its own behind the nodes, and only lanes on such a node fetch it: in a forest
-// with one categorical test in sixteen that is less than half a shared-memory wavefront per visit, against
-// one and more for nodes that carry their set along (5000 depth-6 trees, 8 of 128 features categorical).
-// (An empty set elsewhere: a predicate that lived until the test made them spill.)
+// A categorical node is recognisable by its rank field, the largest there is (0x3FFF, or 0x3FFE in the
+// image for doubled columns).  Only such nodes have a category set, in an array of its own behind the
+// nodes, and only lanes on such a node fetch it: in a forest with one categorical test in sixteen
+// that is less than half a shared-memory wavefront per visit, against one and more for nodes that
+// carry their set along (5000 depth-6 trees, 8 of 128 features categorical).
 template <uint32_t OFF>
 __device__ __forceinline__ uint32_t lds_if_categorical(uint32_t node, uint32_t a)
 {
-  uint32_t set = 0u;
-  asm volatile("{\n.reg .pred p;\nsetp.ge.s32 p, %1, 0x7BFE0000;\n@p ld.shared.u32 %0, [%2+%3];\n}"
-               : "+r"(set)
-               : "r"(node), "r"(a), "n"(OFF));
-  return set;
+  // (the address register takes the set, so that a lane without one needs no other value for it)
+  asm volatile(
+    "{\n.reg .pred p;\nsetp.ge.s32 p, %1, 0x7FFC0000;\n@p ld.shared.u32 %0, [%0+%2];\n}"
+    : "+r"(a)
+    : "r"(node), "n"(OFF));
+  return a;
+}
+__device__ __forceinline__ uint32_t shift_if_categorical(uint32_t node, uint32_t d, uint32_t set, uint32_t code)
+{
+  static_assert(((Q_MAX_RANK_FIELD - 1u) << Q_RANK_SHIFT) == 0x7FFC0000u, "the constant below");
+  asm("{\n.reg .pred p;\nsetp.ge.s32 p, %1, 0x7FFC0000;\n@p shf.l.clamp.b32 %0, %0, %2, %3;\n}"
+      : "+r"(d)
+      : "r"(node), "r"(set), "r"(code));
+  return d;
 }
 
 // DEPTH > 0 fixes the tree depth at compile time (the level loop is fully unrolled); DEPTH == 0
@@ -137,8 +139,7 @@ __device__ __forceinline__ uint32_t lds_if_categorical(uint32_t node, uint32_t a
 // arrays of their own: a stage is one copy (a copy per tree was 20 us slower with 2000 trees of depth 10 on
 // 200,000 rows), and the payloads of ways that part late are neighbours (180 us: in the order of the
 // blocks, whose last steps are the longest, every row fetched another sector).
-template <typename T, int MODE, int NT, int DEPTH, bool CAT, bool TOPC, bool PAIR = false,
-          bool LEAFG = false>
+template <typename T, int MODE, int NT, int DEPTH, bool TOPC, bool PAIR = false, bool LEAFG = false>
 struct DenseQWalker {
   using TR = Traits<T>;
   // Walk the warp's 32 rows through all trees.  A stage of the ring holds K sub-batches of G * NT
@@ -156,19 +157,17 @@ struct DenseQWalker {
                                               uint32_t copy_off)
   {
     constexpr bool NANS = MISSING == NAN_TESTED;
-    static_assert(!TOPC || (DEPTH >= 2 && !CAT), "top nodes need two plain levels");
-    static_assert(!PAIR || (!CAT && !TOPC && MODE == MODE_SCALAR && sizeof(T) == 4),
+    static_assert(!TOPC || DEPTH >= 2, "top nodes need two levels");
+    static_assert(!PAIR || (!TOPC && MODE == MODE_SCALAR && sizeof(T) == 4),
                   "the child-pair walk exists for fp32 scalar leaves without categorical tests");
-    static_assert(!LEAFG || (!CAT && !PAIR && MODE == MODE_SCALAR && sizeof(T) == 4),
+    static_assert(!LEAFG || (!PAIR && MODE == MODE_SCALAR && sizeof(T) == 4),
                   "payloads outside the stages exist for fp32 scalar leaves without categorical tests");
     const ForestView& f    = p.f;
     const int D            = DEPTH > 0 ? DEPTH : f.dense_depth;
-    // bytes of a tree's test nodes, or (CAT) of its test nodes and the category sets behind them
-    const uint32_t sets_at   = 4u * walk_sets_at(D);         // from a node to its category set
-    const uint32_t leaves_at = 4u * walk_leaves_at(D, CAT);  // from the start of a tree to its payloads
+    const uint32_t leaves_at = 4u * walk_leaves_at(D);  // from the start of a tree to its payloads
     // bytes between two trees of a stage
     constexpr uint32_t kStride = LEAFG ? walk_nodes_stride(DEPTH)
-                                       : static_cast<uint32_t>(walk_tree_stride(DEPTH, CAT, TR::ES));
+                                       : static_cast<uint32_t>(walk_tree_stride(DEPTH, TR::ES));
     constexpr bool known_stride = MODE == MODE_SCALAR && DEPTH > 0;
     const uint32_t tstride      = known_stride ? kStride : static_cast<uint32_t>(f.q_tree_stride);
     // bytes per leaf payload: the element size, except where vector leaves sit in the tree block
@@ -226,9 +225,9 @@ struct DenseQWalker {
       // the NT walks are independent: all node loads are issued first, then all rank loads,
       // so that their shared-memory latencies overlap inside one warp.
       // step(): the rows' ranks against NT nodes of level `lvl` (a constant where DEPTH is).
-      auto step = [&](const uint32_t(&node)[NT], auto lvl, auto from_param, auto&& move) {
+      auto step = [&](const uint32_t(&node)[NT], auto from_param, auto&& move) {
         constexpr bool PARAM = decltype(from_param)::value;
-        uint32_t q[NT], set[NT];
+        uint32_t q[NT];
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           uint32_t from = row_addr;
@@ -239,20 +238,8 @@ struct DenseQWalker {
           // that feature
           q[k] = lds_u16(__dp2a_lo(node[k], fstride, from));
         }
-        if constexpr (CAT && DEPTH > 0) {
-          for_each_constant(
-            [&](auto kc) {
-              constexpr int k = decltype(kc)::value, L = decltype(lvl)::value;
-              set[k] = lds_if_categorical<k * TS + 4u * walk_level_at(DEPTH, L) + 4u * walk_sets_at(DEPTH)>(node[k], a[k]);
-            },
-            Each{});
-        } else {
 #pragma unroll
-          for (int k = 0; k < NT; ++k)
-            set[k] = CAT ? lds_if_categorical<0>(node[k], a[k] + level_at(lvl) + sets_at) : 0u;
-        }
-#pragma unroll
-        for (int k = 0; k < NT; ++k) move(k, node[k], q[k], set[k]);
+        for (int k = 0; k < NT; ++k) move(k, node[k], q[k]);
       };
       auto level = [&](auto lvl) {
         uint32_t node[NT];
@@ -267,8 +254,8 @@ struct DenseQWalker {
 #pragma unroll
           for (int k = 0; k < NT; ++k) node[k] = lds_u32(a[k] + level_at(lvl));
         }
-        step(node, lvl, std::false_type{}, [&](int k, uint32_t n, uint32_t q, uint32_t set) {
-          walk_step<CAT, NANS>(a[k], n, q, set, step_bytes(lvl));
+        step(node, std::false_type{}, [&](int k, uint32_t n, uint32_t q) {
+          walk_step<NANS>(a[k], n, q, step_bytes(lvl));
         });
       };
       if constexpr (PAIR) {
@@ -286,9 +273,9 @@ struct DenseQWalker {
             left[k]  = lds_u32(a[k] + at);
             right[k] = lds_u32(a[k] + at + inc);
           }
-          step(node, lvl, std::false_type{}, [&](int k, uint32_t n, uint32_t q, uint32_t) {
+          step(node, std::false_type{}, [&](int k, uint32_t n, uint32_t q) {
             const uint32_t before = a[k];
-            walk_step<false, NANS>(a[k], n, q, 0u, inc);
+            walk_step<NANS>(a[k], n, q, inc);
             node[k] = a[k] != before ? right[k] : left[k];
           });
         }
@@ -309,10 +296,9 @@ struct DenseQWalker {
           n2[k]       = top[t + 1];
           n3[k]       = top[t + 2];
         }
-        step(n1, std::integral_constant<int, 0>{}, std::true_type{},
-             [&](int k, uint32_t n, uint32_t q, uint32_t) { node[k] = root_step<NANS>(a[k], n, q, n2[k], n3[k]); });
-        step(node, std::integral_constant<int, 1>{}, std::true_type{},
-             [&](int k, uint32_t n, uint32_t q, uint32_t) { walk_step<false, NANS>(a[k], n, q, 0u, 8u); });
+        step(n1, std::true_type{},
+             [&](int k, uint32_t n, uint32_t q) { node[k] = root_step<NANS>(a[k], n, q, n2[k], n3[k]); });
+        step(node, std::true_type{}, [&](int k, uint32_t n, uint32_t q) { walk_step<NANS>(a[k], n, q, 8u); });
       }
       uint32_t at_far[LEAFG ? NT : 1];  // LEAFG: where the walks were on level kWalkFarLevel
       if constexpr (DEPTH > 0) {
@@ -356,14 +342,6 @@ struct DenseQWalker {
         pend_n     = FULL ? NT : n_act;
         return;
       }
-      // scalar leaves of a multi-class forest: trees are stored class by class, so when the
-      // first and the last tree of the sub-batch feed the class of the running sum, all do
-      bool same_class = false;
-      if (MODE == MODE_SCALAR && CAT) {
-        same_class = f.n_outputs == 1 ||
-                     (__ldg(f.tree_class + first) == run.cls &&
-                      __ldg(f.tree_class + first + n_act - 1) == run.cls);
-      }
       if (MODE >= MODE_PERTREE) {
         // One output per (row, tree).  The payload slot holds what is reported: the leaf value,
         // or the leaf id when the CTA streams the image made for that (MODE_LEAFID).  With four
@@ -375,27 +353,29 @@ struct DenseQWalker {
 #pragma unroll
         for (int k = 0; k < NT; ++k) val[k] = TR::ld_val(leaf_at(k));
         const bool scalar_out = MODE == MODE_LEAFID || f.leaf_vector_len <= 1;
-        const bool quad = FULL && NT == 4 && scalar_out && f.q_trees_in_order != 0;
+        const bool quad = FULL && NT % 4 == 0 && scalar_out && f.q_trees_in_order != 0;
         using Out = std::conditional_t<MODE == MODE_LEAFID, uint32_t, typename TR::Val>;
         Out* out  = static_cast<Out*>(p.out);
         if (quad && (f.n_trees & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0) {
           if (row < p.n_rows) {
             Out* dst = out + row * f.n_trees + first;
-            if constexpr (sizeof(Out) == 4) {
-              *reinterpret_cast<uint4*>(dst) =
-                make_uint4(TR::low32(val[0]), TR::low32(val[NT > 1 ? 1 : 0]),
-                           TR::low32(val[NT > 2 ? 2 : 0]), TR::low32(val[NT > 3 ? 3 : 0]));
-            } else {
-              *reinterpret_cast<ulonglong2*>(dst) =
-                make_ulonglong2(val[0], val[NT > 1 ? 1 : 0]);
-              *reinterpret_cast<ulonglong2*>(dst + 2) =
-                make_ulonglong2(val[NT > 2 ? 2 : 0], val[NT > 3 ? 3 : 0]);
+#pragma unroll
+            for (int k = 0; k + 3 < NT; k += 4) {
+              if constexpr (sizeof(Out) == 4) {
+                *reinterpret_cast<uint4*>(dst + k) = make_uint4(TR::low32(val[k]), TR::low32(val[k + 1]),
+                                                                TR::low32(val[k + 2]), TR::low32(val[k + 3]));
+              } else {
+                *reinterpret_cast<ulonglong2*>(dst + k)     = make_ulonglong2(val[k], val[k + 1]);
+                *reinterpret_cast<ulonglong2*>(dst + k + 2) = make_ulonglong2(val[k + 2], val[k + 3]);
+              }
             }
           }
         } else if (quad) {
-          store_quads<Out>(out, f.n_trees, row, p.n_rows, first, static_cast<Out>(val[0]),
-                           static_cast<Out>(val[NT > 1 ? 1 : 0]), static_cast<Out>(val[NT > 2 ? 2 : 0]),
-                           static_cast<Out>(val[NT > 3 ? 3 : 0]));
+#pragma unroll
+          for (int k = 0; k + 3 < NT; k += 4)
+            store_quads<Out>(out, f.n_trees, row, p.n_rows, first + k, static_cast<Out>(val[k]),
+                             static_cast<Out>(val[k + 1]), static_cast<Out>(val[k + 2]),
+                             static_cast<Out>(val[k + 3]));
         } else {
 #pragma unroll
           for (int k = 0; k < NT; ++k) {
@@ -443,11 +423,7 @@ struct DenseQWalker {
             }
             const typename TR::Val payload = TR::ld_val(leaf_a);
             if (MODE == MODE_VECTOR) seen ^= TR::low32(payload);
-            if (MODE == MODE_SCALAR && CAT && same_class) {
-              run.sum += TR::as_real(payload);
-            } else {
-              take_leaf<T, MODE>(p, first + k, payload, 0u, acc_group, R, r, row, run);
-            }
+            take_leaf<T, MODE>(p, first + k, payload, 0u, acc_group, R, r, row, run);
           }
         }
       }
@@ -482,6 +458,239 @@ struct DenseQWalker {
       pos.advance(S);
     }
     if constexpr (LEAFG) take_pending();
+    return ok;
+  }
+};
+
+// The walk of forests with categorical tests, over the images in heap order: words 2i and 2i + 1 of a tree's block
+// are the children of word i, a test is one signed subtraction whose sign goes into the heap index with one
+// funnel shift.  A category set takes part in that sum by a shift; with compares and predicates it took as many
+// instructions in walking order, and a longer way from the rank to the next node (5000 depth-6 trees, 150,000
+// rows: 1894 us against 1871).
+template <typename T, int MODE, int NT, int DEPTH>
+struct HeapWalker {
+  using TR = Traits<T>;
+  // Walk the warp's 32 rows through all trees.  A stage of the ring holds K sub-batches of G * NT
+  // trees; the warp waits once per stage and walks its NT trees of every sub-batch.
+  // MISSING: see DenseQWalker.
+  template <int MISSING>
+  static __device__ __forceinline__ bool walk(const PredictParams& p, int G, int S, int K, int g,
+                                              int r, int64_t row, int lane, uint32_t bars,
+                                              uint32_t stages, uint32_t stage_bytes,
+                                              uint32_t row_addr, uint32_t stride_b, T* acc_group,
+                                              int R, RingPos& pos, Running<T>& run, int b_begin,
+                                              int b_end)
+  {
+    constexpr bool NANS = MISSING == NAN_TESTED;
+    const ForestView& f    = p.f;
+    const int D            = DEPTH > 0 ? DEPTH : f.dense_depth;
+    // bytes of a tree's test nodes and the category sets behind them
+    const uint32_t width_b = 8u << D;
+    const uint32_t sets_at = 4u << D;  // from a node to its category set
+    // bytes between two trees of a stage
+    const uint32_t tstride = static_cast<uint32_t>(f.q_tree_stride);
+    // bytes per leaf payload: the element size, except where vector leaves sit in the tree block
+    const uint32_t lbytes  = MODE == MODE_SCALAR ? TR::ES : static_cast<uint32_t>(f.q_leaf_bytes);
+    const bool inline_vec  = MODE != MODE_SCALAR && lbytes > TR::ES;
+    const uint32_t fstride = stride_b >> Q_FEATURE_SHIFT;  // R / 2 <= 128: fits a byte
+    const int per_sub      = G * NT;
+    const int per_batch    = per_sub * K;
+    const uint32_t mine    = static_cast<uint32_t>(g * NT) * tstride;  // this warp's trees in a sub-batch
+    const uint32_t sub_b   = static_cast<uint32_t>(per_sub) * tstride;
+    bool ok                = true;
+    uint32_t seen          = 0u;  // what release_stage() cannot tell from the sums, folded
+
+    // One sub-batch: NT trees side by side.  FULL means all NT slots hold live trees, which lets
+    // the compiler drop every per-slot guard.
+    auto sub_batch = [&](auto full_tag, uint32_t base0, int first, int n_act) {
+      constexpr bool FULL = decltype(full_tag)::value;
+      uint32_t base[NT], idx[NT], a[NT];
+#pragma unroll
+      for (int k = 0; k < NT; ++k) {
+        // slots past the end of the forest repeat the last live tree; results are dropped
+        base[k] = base0 + static_cast<uint32_t>(FULL ? k : min(k, n_act - 1)) * tstride;
+        idx[k]  = 1u;  // heap index of the root
+        a[k]    = base[k] + 4u;
+      }
+      // the NT walks are independent: all node loads are issued first, then all rank loads,
+      // so that their shared-memory latencies overlap inside one warp.
+      // test(): the rows' ranks against NT nodes; the sign bit of d[k] is the step to the right.
+      auto test = [&](const uint32_t(&node)[NT], const uint32_t(&at)[NT], uint32_t(&d)[NT]) {
+        uint32_t q[NT], bits[NT];
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          // the low half of a node is feature * 4: one dot-product instruction (low half x byte 0
+          // of fstride, high half x byte 1 = 0) turns it into the address of the row's rank of
+          // that feature
+          q[k] = lds_u16(__dp2a_lo(node[k], fstride, row_addr));
+        }
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          bits[k] = lds_if_categorical<DEPTH ? 4u << DEPTH : 0u>(node[k], at[k] + (DEPTH ? 0u : sets_at));
+        }
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          // rank j in the high half: x < T[j] <=> rank(x) <= j, so right <=> j - rank < 0
+          d[k] = rank_diff(node[k], q[k]);
+          // the code of a categorical value is its category and the node's set is stored
+          // bit-reversed: the clamped funnel shift by the code moves the category's bit to the sign
+          // position, and leaves d for every code of 32 and above (no category, NaN), which the
+          // large rank of a categorical node has made non-negative, or right for a missing value
+          // of a doubled column.  Predicated: the walk has no data-dependent branch.
+          d[k] = shift_if_categorical(node[k], d[k], bits[k], q[k]);
+          // the missing-goes-right flag sits 15 bits below the sign
+          if (NANS && q[k] == Q_NAN_CODE) d[k] = node[k] << 15;
+        }
+      };
+      auto level = [&]() {
+        uint32_t node[NT], d[NT];
+#pragma unroll
+        for (int k = 0; k < NT; ++k) node[k] = lds_u32(a[k]);
+        test(node, a, d);
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          // heap index 2i + right in one funnel shift: (i << 1) | (d >> 31)
+          idx[k] = __funnelshift_l(d[k], idx[k], 1);
+          a[k]   = idx[k] * 4u + base[k];
+        }
+      };
+      if (DEPTH > 0) {
+#pragma unroll
+        for (int lvl = 0; lvl < DEPTH; ++lvl) level();
+      } else {
+#pragma unroll 4
+        for (int lvl = 0; lvl < D; ++lvl) level();
+      }
+      // scalar leaves of a multi-class forest: trees are stored class by class, so when the
+      // first and the last tree of the sub-batch feed the class of the running sum, all do
+      bool same_class = false;
+      if (MODE == MODE_SCALAR) {
+        same_class = f.n_outputs == 1 ||
+                     (__ldg(f.tree_class + first) == run.cls &&
+                      __ldg(f.tree_class + first + n_act - 1) == run.cls);
+      }
+      if (MODE >= MODE_PERTREE) {
+        // One output per (row, tree).  The payload slot holds what is reported: the leaf value,
+        // or the leaf id when the CTA streams the image made for that (MODE_LEAFID).  With four
+        // live trees that are also the caller's trees first..first+3, a row's four outputs are
+        // contiguous and leave as 16-byte stores, or, where the rows are not aligned for that,
+        // four lanes at a time (store_quads): scalar 4-byte stores at a stride of a whole output
+        // row cost one sector request each and bound these predictions otherwise.
+        typename TR::Val val[NT];
+        uint32_t leaf_at[NT];
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          const uint32_t slot = idx[k] - (1u << D);
+          leaf_at[k]          = base[k] + width_b + slot * lbytes;
+          val[k]              = TR::ld_val(leaf_at[k]);
+        }
+        const bool scalar_out = MODE == MODE_LEAFID || f.leaf_vector_len <= 1;
+        const bool quad = FULL && NT == 4 && scalar_out && f.q_trees_in_order != 0;
+        using Out = std::conditional_t<MODE == MODE_LEAFID, uint32_t, typename TR::Val>;
+        Out* out  = static_cast<Out*>(p.out);
+        if (quad && (f.n_trees & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0) {
+          if (row < p.n_rows) {
+            Out* dst = out + row * f.n_trees + first;
+            if constexpr (sizeof(Out) == 4) {
+              *reinterpret_cast<uint4*>(dst) =
+                make_uint4(TR::low32(val[0]), TR::low32(val[NT > 1 ? 1 : 0]),
+                           TR::low32(val[NT > 2 ? 2 : 0]), TR::low32(val[NT > 3 ? 3 : 0]));
+            } else {
+              *reinterpret_cast<ulonglong2*>(dst) =
+                make_ulonglong2(val[0], val[NT > 1 ? 1 : 0]);
+              *reinterpret_cast<ulonglong2*>(dst + 2) =
+                make_ulonglong2(val[NT > 2 ? 2 : 0], val[NT > 3 ? 3 : 0]);
+            }
+          }
+        } else if (quad) {
+          store_quads<Out>(out, f.n_trees, row, p.n_rows, first, static_cast<Out>(val[0]),
+                           static_cast<Out>(val[NT > 1 ? 1 : 0]), static_cast<Out>(val[NT > 2 ? 2 : 0]),
+                           static_cast<Out>(val[NT > 3 ? 3 : 0]));
+        } else {
+#pragma unroll
+          for (int k = 0; k < NT; ++k) {
+            if (FULL || k < n_act) {
+              if (MODE == MODE_LEAFID) {
+                if (row < p.n_rows) {
+                  const int orig = __ldg(f.tree_orig + first + k);
+                  static_cast<uint32_t*>(p.out)[row * f.n_trees + orig] = TR::low32(val[k]);
+                }
+              } else if (inline_vec) {
+                // per-tree outputs of vector leaves that sit in the tree block
+                if (row < p.n_rows) {
+                  const int orig = __ldg(f.tree_orig + first + k);
+                  T* out = static_cast<T*>(p.out) + (row * f.n_trees + orig) * f.n_outputs;
+                  for (int c = 0; c < f.n_outputs; ++c) out[c] = TR::ld_real(leaf_at[k] + c * TR::ES);
+                }
+              } else {
+                take_leaf<T, MODE>(p, first + k, val[k], 0u, acc_group, R, r, row, run);
+              }
+            }
+          }
+        }
+      } else if (MODE == MODE_VECTOR && inline_vec && f.n_outputs == 2 && sizeof(T) == 4) {
+        // two classes, the common random-forest classifier: one 8-byte load per leaf
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          if (FULL || k < n_act) {
+            const uint2 v = lds_u32x2(base[k] + width_b + (idx[k] - (1u << D)) * 8u);
+            run.v[0] += static_cast<T>(__uint_as_float(v.x));
+            run.v[1] += static_cast<T>(__uint_as_float(v.y));
+          }
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          if (FULL || k < n_act) {
+            const uint32_t leaf_a = base[k] + width_b + (idx[k] - (1u << D)) * lbytes;
+            if (MODE == MODE_VECTOR && inline_vec) {
+              // the leaf's vector sits in the tree block: one sum per output, in registers
+#pragma unroll
+              for (int c = 0; c < kRegClasses; ++c) {
+                if (c < f.n_outputs) run.v[c] += TR::ld_real(leaf_a + c * TR::ES);
+              }
+              continue;
+            }
+            const typename TR::Val payload = TR::ld_val(leaf_a);
+            if (MODE == MODE_VECTOR) seen ^= TR::low32(payload);
+            if (MODE == MODE_SCALAR && same_class) {
+              run.sum += TR::as_real(payload);
+            } else {
+              take_leaf<T, MODE>(p, first + k, payload, 0u, acc_group, R, r, row, run);
+            }
+          }
+        }
+      }
+    };
+
+    for (int b = b_begin; b < b_end; ++b) {
+      const uint32_t s = pos.stage;
+      if (ok) ok = mbar_wait(bars + 8u * s, pos.phase);
+      if (ok) {
+        uint32_t base0 = stages + s * stage_bytes + mine;
+        int first      = b * per_batch + g * NT;  // first tree of this warp inside the stage
+        for (int kk = 0; kk < K; ++kk, base0 += sub_b, first += per_sub) {
+          const int n_act = f.n_trees - first;
+          if (n_act >= NT) {
+            sub_batch(std::true_type{}, base0, first, NT);
+          } else if (n_act > 0) {
+            sub_batch(std::false_type{}, base0, first, n_act);
+          } else {
+            break;
+          }
+        }
+      }
+      const uint32_t empty = bars + 8u * (kMaxStages + s);
+      if (MODE >= MODE_PERTREE) {
+        release_stored_stage(empty, lane);
+      } else {
+        bool read = seen != 0xffffffffu;
+        if (MODE == MODE_SCALAR || (MODE == MODE_VECTOR && inline_vec))
+          read = sums_known<T, MODE>(run);
+        release_stage(empty, lane, read, p.zero);
+      }
+      pos.advance(S);
+    }
     return ok;
   }
 };
@@ -590,7 +799,6 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
                                              const uint32_t* top)
 {
   using TR = Traits<T>;
-  using Walker = DenseQWalker<T, MODE, NT, DEPTH, CAT, TOPC, PAIR, LEAFG>;
   extern __shared__ __align__(128) unsigned char smem[];
   const ForestView& f = p.f;
   const int R         = q.R;
@@ -609,7 +817,7 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
   const uint32_t stride_b    = R * 2u;  // bytes between features in the tile
   const uint32_t tile_bytes  = static_cast<uint32_t>(F) * stride_b;  // multiple of 64
   const uint32_t acc_bytes   = REDUCE ? static_cast<uint32_t>(align16(static_cast<size_t>(G) * NC * R * TR::ES)) : 0u;
-  unsigned char* tile_ptr    = smem + kBarBytes;
+  unsigned char* tile_ptr    = smem + kQBarBytes;
   const uint32_t tile_room   = tile_bytes * (q.nan_columns ? 2u : 1u);  // per buffer
   unsigned char* acc_ptr     = tile_ptr + q.tile_bufs * tile_room;
   volatile int* last_flag    = reinterpret_cast<volatile int*>(acc_ptr + q.acc_bufs * acc_bytes);
@@ -736,7 +944,7 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
         uint32_t* w = &v.x;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          w[k] |= __vcmpeq2(w[k], Q_TILE_NAN * 0x10001u) & Q_TILE_NAN_LEFT * 0x10001u;
+          w[k] |= __vcmpeq2(w[k], Q_NAN_CODE * 0x10001u) & Q_NAN_LEFT_BIT * 0x10001u;
         *reinterpret_cast<uint4*>(tile_ptr + at_tile + tile_bytes + i) = v;
       }
       consumer_sync(n_ct);
@@ -744,9 +952,15 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
     if (ok) {
       const uint32_t row_addr = row_slot + at_tile;
       auto go = [&](auto missing) {
-        return Walker::template walk<decltype(missing)::value>(
-          p, G, S, K, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b, acc_group,
-          R, pos, run, top, seg.begin, seg.end(), tile_bytes);
+        if constexpr (CAT) {
+          return HeapWalker<T, MODE, NT, DEPTH>::template walk<decltype(missing)::value>(
+            p, G, S, K, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b, acc_group, R,
+            pos, run, seg.begin, seg.end());
+        } else {
+          return DenseQWalker<T, MODE, NT, DEPTH, TOPC, PAIR, LEAFG>::template walk<decltype(missing)::value>(
+            p, G, S, K, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b, acc_group, R,
+            pos, run, top, seg.begin, seg.end(), tile_bytes);
+        }
       };
       if (nans && !q.nan_columns) {
         ok = go(std::integral_constant<int, NAN_TESTED>{});

@@ -26,8 +26,9 @@ namespace {
 #define B2FIL_SPIN_NS 256  // sleep between two tries of a bounded mbarrier wait
 #endif
 constexpr uint32_t kSpinLimit = 1u << 22;  // tries of a bounded mbarrier wait
-constexpr int kBarBytes       = 192;       // room for the mbarriers at the start of shared memory
-constexpr int kMaxStages      = 8;         // (two for each stage, four more in the traversal over ranks)
+constexpr int kBarBytes       = 256;       // room for the mbarriers at the start of shared memory
+constexpr int kQBarBytes      = 192;       // the same in the traversal over ranks, to which the last bytes matter
+constexpr int kMaxStages      = 8;
 
 // ---------------------------------------------------------------------------------------------
 // shared-memory and mbarrier primitives (inline PTX)

@@ -158,13 +158,12 @@ constexpr uint32_t Q_DEFAULT_RIGHT = 0x10000u;  // missing values go right (stor
 constexpr uint32_t Q_RANK_SHIFT    = 17;
 constexpr uint32_t Q_NEVER_LEFT    = 0x7FFFu;  // j of a test that no value passes
 constexpr uint32_t Q_MAX_RANK_FIELD = 0x3FFFu;  // j of a test that every code passes (categorical nodes)
-// What the kernels read is this image in walking order (walk_order() before the upload):
+// Without categorical tests the kernels read this image in walking order (walk_order() before the upload):
 //     bits 31..16: a half-precision float, the bits of j, whose sign says that missing values go left
-//                  (categorical nodes: Q_WALK_CATEGORICAL, or one less where missing values go left)
 //     bits 15..2: feature                    bits 1..0: zero
 // Ranks below 0x4000 are the bits of small positive floats in the same order, so one half-precision compare
 // takes both operands from the halves of the words they were loaded in: right <=> rank > |j|.  A missing
-// value is +infinity (right of everything), or -infinity in the copies of columns.
+// value, 0x3FFF, is above every j, and in the copies of columns 0x7FFF, not a number, above none.
 // The nodes of a level are together, and their places in it grow with the way: a step to the right on level l
 // adds walk_step_words() to the place and a step to the left nothing, one predicated addition, and the
 // level itself is the constant offset of the load.  (In heap order, 2 i + right, a step took two more
@@ -173,7 +172,7 @@ constexpr uint32_t Q_MAX_RANK_FIELD = 0x3FFFu;  // j of a test that every code p
 // forest: 21 wavefronts per 32 rows and tree against 18 in heap order and this way).  So there is a hole
 // behind every 32 words.  Trees of depth 9 and more, of which a stage holds few, make do with less holes:
 // steps of 32, 65, 129, 258, ... (at depth 10, 0.7 % more bytes and a wavefront more than heap order,
-// against 2.9 %).  Leaf payloads and category sets are in the same order.
+// against 2.9 %).  Leaf payloads are in the same order.
 B2FIL_HD inline constexpr bool walk_tight(int depth) { return depth >= 9; }
 B2FIL_HD inline constexpr uint32_t walk_step_words(int depth, int level)
 {
@@ -193,25 +192,18 @@ B2FIL_HD inline constexpr uint32_t walk_level_at(int depth, int level)
   if (walk_tight(depth)) return level < 7 ? 1u << level : (129u << (level - 7)) - 1u;
   return level < 6 ? 1u << level : (33u << (level - 5)) - 2u;
 }
-// Words from a node to its category set, and first word of the payloads (8-byte ones are loaded at once).
-B2FIL_HD inline constexpr uint32_t walk_sets_at(int depth) { return walk_level_at(depth, depth); }
-B2FIL_HD inline constexpr uint32_t walk_leaves_at(int depth, bool has_cat)
-{
-  return has_cat ? 2u * walk_sets_at(depth) : (walk_sets_at(depth) + 1u) & ~1u;
-}
+// First word of the payloads (8-byte ones are loaded at once).
+B2FIL_HD inline constexpr uint32_t walk_leaves_at(int depth) { return (walk_level_at(depth, depth) + 1u) & ~1u; }
 // Payloads that stay in global memory (depth 9 and 10, four bytes each) are in an order of their own, in which
 // the ways that part on this level or later end next to each other: rows that are together deep in a tree
 // then fetch the same sector.  Index: place on this level << (depth - level) | the later ways, first one lowest.
 constexpr int kWalkFarLevel = 7;
 // Bytes from one tree to the next, and of its nodes alone.
-B2FIL_HD inline constexpr size_t walk_tree_stride(int depth, bool has_cat, size_t leaf_bytes)
+B2FIL_HD inline constexpr size_t walk_tree_stride(int depth, size_t leaf_bytes)
 {
-  return (4u * walk_leaves_at(depth, has_cat) + walk_level_words(depth, depth) * leaf_bytes + 15) / 16 * 16;
+  return (4u * walk_leaves_at(depth) + walk_level_words(depth, depth) * leaf_bytes + 15) / 16 * 16;
 }
-B2FIL_HD inline constexpr uint32_t walk_nodes_stride(int depth) { return (4u * walk_sets_at(depth) + 15u) / 16u * 16u; }
-constexpr uint32_t Q_TILE_NAN         = 0x7C00u;
-constexpr uint32_t Q_TILE_NAN_LEFT    = 0x8000u;  // set in the missing values of the second set of columns
-constexpr uint32_t Q_WALK_CATEGORICAL = 0x7BFFu;  // the largest finite float: no code is above it
+B2FIL_HD inline constexpr uint32_t walk_nodes_stride(int depth) { return (4u * walk_level_at(depth, depth) + 15u) / 16u * 16u; }
 // Forests of at most this many trees, at least two levels deep and without categorical tests also
 // keep the three top nodes of every tree on the host: the traversal kernel takes them as a launch
 // parameter and reads them through the constant cache instead of shared memory.
@@ -453,8 +445,8 @@ bool build_blocks(PackedForest& pf);
 // [2^D {node, category set}] to [2^D nodes][2^D category sets], which is what the kernels read.
 void split_category_sets(const ForestView& view, std::vector<uint8_t>& image);
 
-// After that: heap order and ranks << 17 become what the kernels walk (see above), trees of walk_tree_stride()
-// bytes.  `doubled`: the image for doubled columns.
+// Before the upload of an image without categorical tests: heap order and ranks << 17 become what the kernels
+// walk (see above), trees of walk_tree_stride() bytes.  `doubled`: the image for doubled columns.
 void walk_order(const ForestView& view, bool doubled, std::vector<uint8_t>& image);
 // The payloads of such an image in the order for global memory, level_words(depth) of four bytes per tree.
 std::vector<uint32_t> far_leaves(const ForestView& view, const std::vector<uint8_t>& image);

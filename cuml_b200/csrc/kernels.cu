@@ -417,7 +417,7 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
       const T* cur = xs + c % AHEAD * CH;
       // rank of the CH values, step by step across all of them so that the dependent
       // shared-memory lookups of different values overlap.  A NaN walks the same code (bucket 0,
-      // every comparison false) and is replaced by Q_TILE_NAN at the end; so does a categorical
+      // every comparison false) and is replaced by Q_NAN_CODE at the end; so does a categorical
       // value (its feature has empty tables), replaced by its category.
       uint32_t a[CH];  // address of the threshold below the current window
 #pragma unroll
@@ -475,7 +475,7 @@ __device__ __forceinline__ void quantise_tiles(const PredictParams& p, const QGr
 #pragma unroll
         for (int u = 0; u < CH; u += 2) {
           const uint32_t nan = (cur[u] != cur[u] ? 0xffffu : 0u) | (cur[u + 1] != cur[u + 1] ? 0xffff0000u : 0u);
-          two[u >> 1] = (two[u >> 1] & ~nan) | (Q_TILE_NAN * 0x10001u & nan);
+          two[u >> 1] = (two[u >> 1] & ~nan) | (Q_NAN_CODE * 0x10001u & nan);
           saw_nan |= nan != 0u;
         }
       }
@@ -848,7 +848,7 @@ size_t dense_q_smem(size_t qstride, int precision, int F, int NC, bool reduce, i
                     int S, int K, int tile_bufs = 1, int acc_bufs = 1, int columns = 1)
 {
   const size_t es = precision == B2FIL_F32 ? 4 : 8;
-  size_t b        = kBarBytes;
+  size_t b        = kQBarBytes;
   b += static_cast<size_t>(tile_bufs) * columns * F * R * 2;
   if (reduce) b += acc_bufs * align16(static_cast<size_t>(G) * NC * R * es);
   b += 16;
@@ -865,14 +865,16 @@ size_t q_node_only_stride(const ForestView& f, int mode)
 }
 
 // Most trees a warp of the quantised kernel may walk side by side: the kernels that exist.
-int q_max_trees_in_flight(const ForestView& f, int mode)
+int q_max_trees_in_flight(const ForestView& f, int mode, bool has_top)
 {
   if (f.q_has_cat) {
     return f.format == FMT_DENSE_F && mode == MODE_SCALAR && f.dense_depth >= 4 && f.dense_depth <= 8 ? 6 : 4;
   }
   const bool specialised = f.format == FMT_DENSE_F && (mode == MODE_SCALAR || mode == MODE_VECTOR) &&
                            f.dense_depth >= 4 && f.dense_depth <= 10;
-  return specialised ? 6 : 4;
+  const bool outputs = f.format == FMT_DENSE_F && mode >= MODE_PERTREE && has_top && f.dense_depth >= 4 &&
+                       f.dense_depth <= 10;
+  return specialised ? 6 : (outputs ? 8 : 4);
 }
 
 // Can tiles with missing values be walked with doubled columns?
@@ -933,7 +935,7 @@ bool dense_q_config(size_t qstride, int max_nt, int precision, int F, int NC, bo
     const int R = forced.R, G = forced.G, NT = forced.NT, S = forced.S, K = forced.K;
     if (R >= 32 && R % 32 == 0 &&
         R <= 256 && (R & (R - 1)) == 0 && G >= 1 && (R / 32) * G <= 31 &&
-        (NT == 1 || NT == 2 || NT == 4 || (NT == 6 && (R / 32) * G <= 24) ||
+        (NT == 1 || NT == 2 || NT == 4 || ((NT == 6 || NT == 8) && (R / 32) * G <= 24) ||
          (NT == 3 && max_nt == 6 && depth_hint >= 9)) && S >= 2 &&
         S <= kMaxStages && K >= 1 && NT <= max_nt) {
       const bool leafg = node_stride > 0 && tuning_value("q_leafg", 0) == 1 && NT >= 2 && NT <= 4;
@@ -954,9 +956,12 @@ bool dense_q_config(size_t qstride, int max_nt, int precision, int F, int NC, bo
     // trees 7.2e7 rows/s, 5 groups x 1 tree 6.3e7).  Ties go to more warps.
     int best_g = 0, best_nt = 0;
     // a CTA holds at most 32 warps and one of them is the producer
+    // (eight trees: from a tile per SM and 1000 visits per row on; below, 100 trees of depth 8 x 150,000 rows took
+    // 66 us instead of 59, 300 of depth 6 x 20,000 25.4 instead of 24.2)
+    const bool eight = n_rows >= static_cast<int64_t>(256) * sm_count && visits_per_row >= 1000;
     for (int G = std::min(8, 31 / rw); G >= 1; --G) {
-      for (int NT = max_nt; NT >= 1; NT = NT == 6 ? 4 : NT / 2) {
-        // the six-tree kernels are built for at most 24 consumer warps (80 registers a thread)
+      for (int NT = max_nt == 8 && !eight ? 4 : max_nt; NT >= 1; NT = NT == 6 ? 4 : NT / 2) {
+        // the kernels for six and eight trees are built for at most 24 consumer warps (80 registers a thread)
         if (NT > 4 && rw * G > 24) continue;
         if (dense_q_smem(qstride, precision, F, NC, reduce, R, G, NT, 2, 1) > kMaxSmemBytes) continue;
         if (G * NT > best_g * best_nt) {
@@ -993,13 +998,17 @@ bool dense_q_config(size_t qstride, int max_nt, int precision, int F, int NC, bo
     // Two stages already hide the bulk copies (measured: S = 2 and S = 3 run alike), so a second
     // row tile and room for doubled columns come first - the tile where the trees of a row last only
     // a few microseconds -, and a second set of accumulators takes what is left.
+    // One output per row and tree, eight trees at a time: the stores need the L1, and what shared memory leaves
+    // of it is more use than a second row tile or longer stages (leaf ids of 300 depth-6 trees, 100,003 rows:
+    // 109 us with both, 101 without).
+    const bool lean       = best_nt == 8;
     const bool tile_first = visits_per_row < 4000;
     for (int pass = 0; pass < 4; ++pass) {
       const int tiles   = (pass == 0 || pass == (tile_first ? 1 : 2)) ? 2 : 1;
       const int columns = (pass == 0 || pass == (tile_first ? 2 : 1)) ? 2 : 1;
-      if (columns == 2 && !nan_image) continue;
-      for (int K = 2; K >= 1; K /= 2) {
-        for (int S = 3; S >= 2; --S) {
+      if ((columns == 2 && !nan_image) || (tiles == 2 && lean)) continue;
+      for (int K = lean ? 1 : 2; K >= 1; K /= 2) {
+        for (int S = lean ? 2 : 3; S >= 2; --S) {
           for (int accs = reduce ? 2 : 1; accs >= 1; --accs) {
             const size_t b = dense_q_smem(stride, precision, F, NC, reduce, R, best_g, best_nt, S,
                                           K, tiles, accs, columns);
@@ -1062,7 +1071,7 @@ int launch_dense_q_kernel(const QLaunch& L, int mode, bool f64, std::string& err
   }
   const bool unrolled = !f64 && f.dense_depth >= 4 && f.dense_depth <= 10;
   const bool has_top  = L.p.q_top != nullptr && f.n_trees <= kQTopTrees;
-  if (unrolled && mode >= MODE_PERTREE && has_top && L.c.trees_in_flight == 4) {
+  if (unrolled && mode >= MODE_PERTREE && has_top && (L.c.trees_in_flight == 4 || L.c.trees_in_flight == 8)) {
     rec.depth  = f.dense_depth;
     rec.kernel = "dense_q_top_kernel";
     return launch_q_top_out(L, mode, err);
@@ -1174,7 +1183,7 @@ int launch_dense_q(const PredictParams& p, int mode, int chunk_size, int sm_coun
   const int precision = f.format == FMT_DENSE_F ? B2FIL_F32 : B2FIL_F64;
   const bool reduce   = mode <= MODE_VECTOR;
   DenseCfg c;
-  if (!dense_q_config(static_cast<size_t>(f.q_tree_stride), q_max_trees_in_flight(f, mode), precision,
+  if (!dense_q_config(static_cast<size_t>(f.q_tree_stride), q_max_trees_in_flight(f, mode, p.q_top != nullptr), precision,
                       f.n_features, f.n_outputs, reduce, p.n_rows, chunk_size, sm_count, c,
                       f.dense_depth, q_node_only_stride(f, mode),
                       static_cast<int64_t>(f.n_trees) * f.dense_depth, has_nan_image(f, mode))) {
@@ -1480,7 +1489,8 @@ int dense_ok(int depth, int precision, int n_features, int n_outputs)
   // else the traversal over rank-quantised rows alone, if a 32-row tile of ranks and two stages
   // of one tree fit (a tree counted at its largest: 8-byte test nodes, four inline outputs)
   const size_t es      = precision == B2FIL_F32 ? 4 : 8;
-  const size_t qstride = walk_tree_stride(depth, true, 4 * es);
+  // (and, with fewer outputs, the holes of the walking order still fit into that)
+  const size_t qstride = std::max((size_t(8) + 4 * es) << depth, walk_tree_stride(depth, 4 * es));
   if (dense_q_smem(qstride, precision, n_features, n_outputs, true, 32, 1, 1, 2, 1) <= kMaxSmemBytes &&
       n_features < (1 << 14))
     return 2;
@@ -1683,7 +1693,7 @@ int launch_predict_fixed_scratch(const PredictParams& p, int chunk_size, int sm_
   }
   const int precision = f.format == FMT_DENSE_F ? B2FIL_F32 : B2FIL_F64;
   DenseCfg c;
-  if (!dense_q_config(static_cast<size_t>(f.q_tree_stride), q_max_trees_in_flight(f, mode), precision,
+  if (!dense_q_config(static_cast<size_t>(f.q_tree_stride), q_max_trees_in_flight(f, mode, p.q_top != nullptr), precision,
                       f.n_features, f.n_outputs, mode <= MODE_VECTOR, p.n_rows, chunk_size,
                       sm_count, c, f.dense_depth, q_node_only_stride(f, mode),
                       static_cast<int64_t>(f.n_trees) * f.dense_depth, has_nan_image(f, mode))) {

@@ -1158,14 +1158,13 @@ void split_category_sets(const ForestView& v, std::vector<uint8_t>& image)
 
 void walk_order(const ForestView& v, bool doubled, std::vector<uint8_t>& image)
 {
-  if (image.empty()) return;
+  if (image.empty() || v.q_has_cat) return;
   const int D           = v.dense_depth;
   const size_t width    = size_t(1) << D;
   const size_t lbytes   = static_cast<size_t>(v.q_leaf_bytes);
-  const size_t leaves   = width * (v.q_has_cat ? 8 : 4);  // of a tree in heap order
-  const size_t sets_to  = size_t(4) * walk_sets_at(D);
-  const size_t leaf_to  = size_t(4) * walk_leaves_at(D, v.q_has_cat != 0);
-  const size_t stride   = walk_tree_stride(D, v.q_has_cat != 0, lbytes);
+  const size_t leaves   = width * 4;  // of a tree in heap order
+  const size_t leaf_to  = size_t(4) * walk_leaves_at(D);
+  const size_t stride   = walk_tree_stride(D, lbytes);
   const uint32_t copies = doubled ? static_cast<uint32_t>(v.n_features) : 0u;  // first copy of a column
   std::vector<uint8_t> out(stride * static_cast<size_t>(v.n_trees), 0);
   struct Place {
@@ -1185,18 +1184,15 @@ void walk_order(const ForestView& v, bool doubled, std::vector<uint8_t>& image)
         uint32_t feature = (node & Q_FEATURE_FIELD) >> Q_FEATURE_SHIFT;
         if (feature >= copies && copies > 0) feature -= copies;
         bool left          = (node & Q_DEFAULT_RIGHT) == 0u;  // where missing values go
-        const bool cat     = v.q_has_cat && (j == Q_MAX_RANK_FIELD || j == Q_MAX_RANK_FIELD - 1u);
         const bool swapped = j == Q_NEVER_LEFT;
         if (swapped) {  // never left = always left of exchanged children; every code passes 0x3FFE
           j    = Q_MAX_RANK;
           left = !left;
         }
-        const uint32_t half = cat ? Q_WALK_CATEGORICAL - (left ? 1u : 0u) : (j | (left ? 0x8000u : 0u));
         if (left) feature += copies;
-        const uint32_t word = half << 16 | feature << Q_FEATURE_SHIFT;
+        const uint32_t word = (j | (left ? 0x8000u : 0u)) << 16 | feature << Q_FEATURE_SHIFT;
         const size_t at     = (walk_level_at(D, l) + p.at) * 4;
         std::memcpy(to + at, &word, 4);
-        if (v.q_has_cat) std::memcpy(to + sets_to + at, from + width * 4 + p.heap * 4, 4);
         next.push_back({2 * p.heap + (swapped ? 1u : 0u), p.at});
         next.push_back({2 * p.heap + (swapped ? 0u : 1u), p.at + walk_step_words(D, l)});
       }
@@ -1212,7 +1208,7 @@ std::vector<uint32_t> far_leaves(const ForestView& v, const std::vector<uint8_t>
 {
   const int D         = v.dense_depth;
   const uint32_t n    = walk_level_words(D, D);
-  const size_t stride = walk_tree_stride(D, v.q_has_cat != 0, 4);
+  const size_t stride = walk_tree_stride(D, 4);
   std::vector<uint32_t> out(static_cast<size_t>(n) * v.n_trees, 0u);
   for (uint32_t way = 0; way < 1u << D; ++way) {  // bit l: right on level l
     uint32_t place = 0, far = 0;
@@ -1223,7 +1219,7 @@ std::vector<uint32_t> far_leaves(const ForestView& v, const std::vector<uint8_t>
     far |= way >> kWalkFarLevel;
     for (int t = 0; t < v.n_trees; ++t)
       std::memcpy(&out[static_cast<size_t>(t) * n + far],
-                  image.data() + stride * t + 4u * (walk_leaves_at(D, v.q_has_cat != 0) + place), 4);
+                  image.data() + stride * t + 4u * (walk_leaves_at(D) + place), 4);
   }
   return out;
 }
@@ -1231,8 +1227,8 @@ std::vector<uint32_t> far_leaves(const ForestView& v, const std::vector<uint8_t>
 std::vector<uint8_t> far_nodes(const ForestView& v, const std::vector<uint8_t>& image)
 {
   if (image.empty()) return {};
-  const size_t n      = walk_nodes_stride(v.dense_depth), used = size_t(4) * walk_sets_at(v.dense_depth);
-  const size_t stride = walk_tree_stride(v.dense_depth, v.q_has_cat != 0, 4);
+  const size_t n      = walk_nodes_stride(v.dense_depth), used = size_t(4) * walk_level_at(v.dense_depth, v.dense_depth);
+  const size_t stride = walk_tree_stride(v.dense_depth, 4);
   std::vector<uint8_t> out(n * v.n_trees, 0);
   for (int t = 0; t < v.n_trees; ++t) std::memcpy(out.data() + n * t, image.data() + stride * t, used);
   return out;

@@ -31,47 +31,38 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
 {
   PackedForest pf;
   std::string err;
-  if (pack_forest(*desc, *opts, yes, pf, err) != B2FIL_OK || !pf.view.q_enabled) return -1;
+  if (pack_forest(*desc, *opts, yes, pf, err) != B2FIL_OK || !pf.view.q_enabled || pf.view.q_has_cat) return -1;
   const ForestView& v = pf.view;
   const int D = v.dense_depth, F = v.n_features;
-  const size_t width = size_t(1) << D, leaves = width * (v.q_has_cat ? 8 : 4);
-  const size_t to     = size_t(4) * walk_leaves_at(D, v.q_has_cat != 0);
-  const size_t stride = walk_tree_stride(D, v.q_has_cat != 0, static_cast<size_t>(v.q_leaf_bytes));
+  const size_t width = size_t(1) << D, leaves = width * 4;
+  const size_t to     = size_t(4) * walk_leaves_at(D);
+  const size_t stride = walk_tree_stride(D, static_cast<size_t>(v.q_leaf_bytes));
   std::mt19937 rng(seed);
   int64_t bad = 0;
   for (int image = 0; image < 3; ++image) {
     std::vector<uint8_t> heap = image == 0 ? pf.q_nodes : (image == 1 ? pf.q_nodes_ids : pf.q_nodes_nan);
     if (heap.empty()) continue;
     const bool doubled = image == 2;
-    split_category_sets(v, heap);
     std::vector<uint8_t> walk = heap;
     walk_order(v, doubled, walk);
     for (int r = 0; r < n; ++r) {
-      std::vector<uint32_t> a(2 * F), b(2 * F);  // codes: of the heap walk, and of the tile
+      std::vector<uint32_t> a(2 * F);  // codes of the columns and of their copies
       std::vector<bool> missing(F);
       for (int f = 0; f < F; ++f) {
         missing[f]     = rng() % 8 == 0;
-        const auto& qf = pf.q_feats[f];
-        const uint32_t code = qf.is_cat ? (rng() % 5 == 0 ? Q_NO_CATEGORY : rng() % 40)
-                                        : (rng() % 9 == 0 ? Q_MAX_RANK : rng() % (qf.m + 1));
+        const uint32_t code = rng() % 9 == 0 ? Q_MAX_RANK : rng() % (pf.q_feats[f].m + 1);
         a[f]     = missing[f] ? Q_NAN_CODE : code;
-        b[f]     = missing[f] ? Q_TILE_NAN : code;
         a[F + f] = missing[f] ? Q_NAN_CODE | Q_NAN_LEFT_BIT : code;
-        b[F + f] = missing[f] ? Q_TILE_NAN | Q_TILE_NAN_LEFT : code;
       }
       for (int t = 0; t < v.n_trees; ++t) {
         const uint8_t* hb = heap.data() + static_cast<size_t>(v.q_tree_stride) * t;
         const uint8_t* wb = walk.data() + stride * t;
         uint32_t i = 1, place = 0;
         for (int l = 0; l < D; ++l) {
-          uint32_t node, set = 0;
+          uint32_t node;
           std::memcpy(&node, hb + i * 4, 4);
           const uint32_t f = (node & Q_FEATURE_FIELD) >> Q_FEATURE_SHIFT;
           bool right       = static_cast<int32_t>(node - (a[f] << Q_RANK_SHIFT)) < 0;
-          if (v.q_has_cat && (node >> Q_RANK_SHIFT == Q_MAX_RANK_FIELD || node >> Q_RANK_SHIFT == Q_MAX_RANK_FIELD - 1)) {
-            std::memcpy(&set, hb + width * 4 + i * 4, 4);
-            if (a[f] < 32 && (set << a[f]) >> 31) right = true;
-          }
           if (!doubled && missing[f]) right = (node & Q_DEFAULT_RIGHT) != 0;
           i = 2 * i + (right ? 1 : 0);
 
@@ -79,14 +70,9 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
           std::memcpy(&node, wb + at, 4);
           const uint32_t g   = (node & Q_FEATURE_FIELD) >> Q_FEATURE_SHIFT;
           const uint32_t hi  = node >> 16;
-          const bool cat     = static_cast<int32_t>(node) >= 0x7BFE0000;
-          const uint32_t code = b[g];
+          const uint32_t code = a[g];
           right = half_value(code) > std::fabs(half_value(hi));
-          if (cat) {
-            std::memcpy(&set, wb + walk_sets_at(D) * 4 + at, 4);
-            if (code < 32 && (set << code) >> 31) right = true;
-          }
-          if (!doubled && code == Q_TILE_NAN) right = cat ? (hi & 1) != 0 : (hi & 0x8000) == 0;
+          if (!doubled && code == Q_NAN_CODE) right = (hi & 0x8000) == 0;
           if (right) place += walk_step_words(D, l);
         }
         const size_t lb = static_cast<size_t>(v.q_leaf_bytes);
@@ -97,7 +83,6 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
   if (D >= 9 && v.q_leaf_bytes == 4) {
     // payloads for global memory: the number of a way's later steps by the kernels' shift
     std::vector<uint8_t> walk = pf.q_nodes;
-    split_category_sets(v, walk);
     walk_order(v, false, walk);
     const std::vector<uint32_t> far = far_leaves(v, walk);
     for (int i = 0; i < 4 * n; ++i) {

@@ -270,3 +270,44 @@ def test_the_variants_that_these_tests_are_about_are_launched():
     assert np.array_equal(fi.apply(x).cpu().numpy().astype(np.uint32),
                           oracle.predict(desc, X, INFER_LEAF_ID, "single"))
     assert "nan_columns" not in _lib.last_variant()
+
+
+@pytest.mark.parametrize("n_trees,max_depth,kw", [(250, 4, {}), (251, 5, {}), (173, 6, dict(vector=True, n_outputs=3)),
+                                                  (109, 10, {}), (321, 4, {})])
+def test_outputs_of_eight_trees_leave_together(n_trees, max_depth, kw):
+    """One output per row and tree from a tile per SM and 1000 visits per row on: tree counts with and without
+    rows on 16-byte boundaries, a partial last group of eight, a batch that ends inside four rows, missing
+    values; top nodes in the small parameter block and (321 trees) the large one."""
+    import numpy as np
+    import torch
+
+    from cuml_b200.fil import ForestInference, _lib
+    from cuml_b200.fil._desc import INFER_LEAF_ID, INFER_PER_TREE
+    from oracle import oracle
+
+    desc = random_forest_desc(98, n_trees=n_trees, n_features=9, max_depth=max_depth, p_leaf=0.05, **kw)
+    X = random_rows(3, 37_891, 9, np.float32, nan_frac=0.01)
+    X[5000:30_000] = np.nan_to_num(X[5000:30_000])  # most tiles hold none
+    fi = ForestInference.load_from_treelite_model(desc, storage="dense")
+    x = torch.as_tensor(X, device="cuda:0")
+    ids = fi.apply(x).cpu().numpy()
+    assert "NT=8" in _lib.last_variant() or max_depth == 10
+    assert np.array_equal(ids.astype(np.uint32), oracle.predict(desc, X, INFER_LEAF_ID, "single"))
+    per = fi.predict_per_tree(x).cpu().numpy()
+    assert np.array_equal(per.reshape(len(X), -1),
+                          oracle.predict(desc, X, INFER_PER_TREE, "single").reshape(len(X), -1))
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("max_depth,n_features,kw", [(4, 500, {}), (7, 480, {}), (8, 400, dict(vector=True, n_outputs=2)),
+                                                     (9, 440, {}), (10, 300, dict(vector=True, n_outputs=3)),
+                                                     (10, 512, {})])
+def test_few_trees_in_flight(max_depth, n_features, kw, precision):
+    """Row tiles that leave room for few trees: specialised bodies for one and two trees in flight, payloads in
+    global memory, every output kind, partial groups of trees, missing values."""
+    import numpy as np
+
+    desc = random_forest_desc(99, n_trees=19, n_features=n_features, max_depth=max_depth, p_leaf=0.02, **kw)
+    X = random_rows(4, 2_500, n_features, np.float64, nan_frac=0.002)
+    for chunk in (4, 8):
+        _all_kinds(desc, X, precision, "depth_first", "dense", chunk_size=chunk)

@@ -366,11 +366,11 @@ def test_blocks_of_a_forest_that_several_threads_cut(pack_check):
 @pytest.mark.parametrize("precision", ["single", "double"])
 @pytest.mark.parametrize("kw", [dict(max_depth=1), dict(max_depth=8, mixed_ops=True),
                                 dict(max_depth=9), dict(max_depth=10),
-                                dict(n_categorical=4), dict(max_depth=5, vector=True, n_outputs=3)])
+                                dict(max_depth=5, vector=True, n_outputs=3)])
 def test_images_in_walking_order(tmp_path_factory, kw, precision):
     """The images that the traversal kernels read (levels in the order of the ways, thresholds and codes as
     half-precision floats) lead every row of codes to the payload that the heap-ordered images lead it to:
-    missing values, categories, tests that nothing passes."""
+    missing values, tests that nothing passes."""
     import os
     import subprocess
 
@@ -385,10 +385,7 @@ def test_images_in_walking_order(tmp_path_factory, kw, precision):
     lib = C.CDLL(so)
     lib.walk_check.restype = C.c_int64
     lib.walk_check.argtypes = [C.POINTER(CForestDesc), C.POINTER(CCreateOpts), C.c_int, C.c_int]
-    if "n_categorical" in kw:
-        desc = synthetic_complete_forest(23, 6, 11, seed=31, n_categories=30, **kw)
-    else:
-        desc = random_forest_desc(31, n_trees=23, n_features=11, **kw)
+    desc = random_forest_desc(31, n_trees=23, n_features=11, **kw)
     inner = np.flatnonzero(desc.node_kind == 1)
     desc.threshold[inner[::7]] = np.nan
     cd = desc.to_c()
