@@ -1167,39 +1167,66 @@ void walk_order(const ForestView& v, bool doubled, std::vector<uint8_t>& image)
   const size_t stride   = walk_tree_stride(D, lbytes);
   const uint32_t copies = doubled ? static_cast<uint32_t>(v.n_features) : 0u;  // first copy of a column
   std::vector<uint8_t> out(stride * static_cast<size_t>(v.n_trees), 0);
-  struct Place {
-    uint32_t heap, at;  // heap index, place in the level
-  };
-  std::vector<Place> level, next;
+  // place of every heap node in its level (leaves included), the same in all trees without a test that nothing passes
+  std::vector<uint32_t> place(2 * width, 0u), at(width, 0u);
+  for (int l = 0; l < D; ++l) {
+    for (size_t h = size_t(1) << l; h < size_t(2) << l; ++h) {
+      at[h]            = walk_level_at(D, l) + place[h];
+      place[2 * h]     = place[h];
+      place[2 * h + 1] = place[h] + walk_step_words(D, l);
+    }
+  }
+  // Where such a test comes up its children change places, with all that is below them.
+  std::vector<uint32_t> own_place, own_at;
   for (int t = 0; t < v.n_trees; ++t) {
     const uint8_t* from = image.data() + static_cast<size_t>(v.q_tree_stride) * t;
     uint8_t* to         = out.data() + stride * static_cast<size_t>(t);
-    level.assign(1, Place{1, 0});
-    for (int l = 0; l < D; ++l) {
-      next.clear();
-      for (const Place& p : level) {
-        uint32_t node;
-        std::memcpy(&node, from + p.heap * 4, 4);
-        uint32_t j       = node >> Q_RANK_SHIFT;
-        uint32_t feature = (node & Q_FEATURE_FIELD) >> Q_FEATURE_SHIFT;
-        if (feature >= copies && copies > 0) feature -= copies;
-        bool left          = (node & Q_DEFAULT_RIGHT) == 0u;  // where missing values go
-        const bool swapped = j == Q_NEVER_LEFT;
-        if (swapped) {  // never left = always left of exchanged children; every code passes 0x3FFE
-          j    = Q_MAX_RANK;
-          left = !left;
-        }
-        if (left) feature += copies;
-        const uint32_t word = (j | (left ? 0x8000u : 0u)) << 16 | feature << Q_FEATURE_SHIFT;
-        const size_t at     = (walk_level_at(D, l) + p.at) * 4;
-        std::memcpy(to + at, &word, 4);
-        next.push_back({2 * p.heap + (swapped ? 1u : 0u), p.at});
-        next.push_back({2 * p.heap + (swapped ? 0u : 1u), p.at + walk_step_words(D, l)});
-      }
-      std::swap(level, next);
+    const uint32_t *to_place = place.data(), *to_at = at.data();
+    bool exchanged = false;
+    for (size_t h = 1; h < width && !exchanged; ++h) {
+      uint32_t node;
+      std::memcpy(&node, from + h * 4, 4);
+      exchanged = node >> Q_RANK_SHIFT == Q_NEVER_LEFT;
     }
-    for (const Place& p : level)
-      std::memcpy(to + leaf_to + p.at * lbytes, from + leaves + (p.heap - width) * lbytes, lbytes);
+    if (exchanged) {
+      own_place = place;
+      own_at    = at;
+      for (int l = 0; l < D; ++l) {
+        for (size_t h = size_t(1) << l; h < size_t(2) << l; ++h) {
+          uint32_t node;
+          std::memcpy(&node, from + h * 4, 4);
+          const size_t right = 2 * h + (node >> Q_RANK_SHIFT == Q_NEVER_LEFT ? 0 : 1);
+          own_at[h]              = walk_level_at(D, l) + own_place[h];
+          own_place[2 * h]       = own_place[h];
+          own_place[2 * h + 1]   = own_place[h];
+          own_place[right]      += walk_step_words(D, l);
+        }
+      }
+      to_place = own_place.data();
+      to_at    = own_at.data();
+    }
+    for (size_t h = 1; h < width; ++h) {
+      uint32_t node;
+      std::memcpy(&node, from + h * 4, 4);
+      uint32_t j       = node >> Q_RANK_SHIFT;
+      uint32_t feature = (node & Q_FEATURE_FIELD) >> Q_FEATURE_SHIFT;
+      if (feature >= copies && copies > 0) feature -= copies;
+      bool left = (node & Q_DEFAULT_RIGHT) == 0u;  // where missing values go
+      if (j == Q_NEVER_LEFT) {  // never left = always left of exchanged children; every code passes 0x3FFE
+        j    = Q_MAX_RANK;
+        left = !left;
+      }
+      if (left) feature += copies;
+      const uint32_t word = (j | (left ? 0x8000u : 0u)) << 16 | feature << Q_FEATURE_SHIFT;
+      std::memcpy(to + size_t(4) * to_at[h], &word, 4);
+    }
+    if (lbytes == 4) {
+      for (size_t s = 0; s < width; ++s)
+        std::memcpy(to + leaf_to + size_t(4) * to_place[width + s], from + leaves + s * 4, 4);
+    } else {
+      for (size_t s = 0; s < width; ++s)
+        std::memcpy(to + leaf_to + lbytes * to_place[width + s], from + leaves + s * lbytes, lbytes);
+    }
   }
   image.swap(out);
 }
