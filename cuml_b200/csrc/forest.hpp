@@ -338,7 +338,7 @@ struct ForestView {
   int32_t q_leaf_bytes;         // bytes per leaf payload: the element size (scalar, or index of the
                                 // leaf's vector), or n_outputs elements when the vectors of a
                                 // forest with few outputs sit in the tree blocks themselves
-  int32_t q_any_default_left;   // 0: missing values go right in every test
+  int32_t q_any_default_left;   // 0: missing values go right in every test, also in walking order
   int64_t q_tree_stride;        // bytes between trees: 2^D * (node bytes + leaf bytes), 16-byte multiple
   const void* q_nodes;          // [n_trees] blocks of [2^D nodes][2^D leaf payloads] of uint32 nodes,
                                 // with [2^D category sets] in between when q_has_cat

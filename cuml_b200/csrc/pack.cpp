@@ -742,7 +742,8 @@ struct Packer {
       for (int64_t i = 1; i < width && !any_left; ++i) {
         uint32_t node;
         std::memcpy(&node, src + i * qnb, 4);
-        any_left = (node & Q_DEFAULT_RIGHT) == 0u;
+        // (walk_order() exchanges the children of a test that nothing passes, and right becomes left)
+        any_left = (node & Q_DEFAULT_RIGHT) == 0u || (!has_cat && node >> Q_RANK_SHIFT == Q_NEVER_LEFT);
       }
     }
     out.view.q_any_default_left = any_left ? 1 : 0;

@@ -72,7 +72,8 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
           const uint32_t hi  = node >> 16;
           const uint32_t code = a[g];
           right = half_value(code) > std::fabs(half_value(hi));
-          if (!doubled && code == Q_NAN_CODE) right = (hi & 0x8000) == 0;
+          // (the kernels look at the direction of missing values only in forests that are marked for it)
+          if (!doubled && code == Q_NAN_CODE && v.q_any_default_left) right = (hi & 0x8000) == 0;
           if (right) place += walk_step_words(D, l);
         }
         const size_t lb = static_cast<size_t>(v.q_leaf_bytes);

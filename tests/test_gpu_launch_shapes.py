@@ -311,3 +311,19 @@ def test_few_trees_in_flight(max_depth, n_features, kw, precision):
     X = random_rows(4, 2_500, n_features, np.float64, nan_frac=0.002)
     for chunk in (4, 8):
         _all_kinds(desc, X, precision, "depth_first", "dense", chunk_size=chunk)
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("max_depth,n_features,n_trees", [(3, 11, 70), (8, 11, 61), (10, 300, 21)])
+def test_missing_values_that_all_go_right(max_depth, n_features, n_trees, precision):
+    """Forests that send every missing value right, with tests that nothing and that everything passes: in the
+    images for ranks the former send missing values to the left of exchanged children."""
+    import numpy as np
+
+    desc = random_forest_desc(100, n_trees=n_trees, n_features=n_features, max_depth=max_depth, p_leaf=0.02)
+    inner = np.flatnonzero(desc.node_kind == 1)
+    desc.threshold[inner[::5]] = np.nan
+    desc.threshold[inner[2::5]] = np.inf
+    desc.default_left[:] = 0
+    X = random_rows(6, 21_003, n_features, np.float64, nan_frac=0.02)
+    _all_kinds(desc, X, precision, "depth_first", "dense")

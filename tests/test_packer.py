@@ -363,31 +363,54 @@ def test_blocks_of_a_forest_that_several_threads_cut(pack_check):
         assert info[12] == 1 and info[4] > 200_000
 
 
-@pytest.mark.parametrize("precision", ["single", "double"])
-@pytest.mark.parametrize("kw", [dict(max_depth=1), dict(max_depth=8, mixed_ops=True),
-                                dict(max_depth=9), dict(max_depth=10),
-                                dict(max_depth=5, vector=True, n_outputs=3)])
-def test_images_in_walking_order(tmp_path_factory, kw, precision):
-    """The images that the traversal kernels read (levels in the order of the ways, thresholds and codes as
-    half-precision floats) lead every row of codes to the payload that the heap-ordered images lead it to:
-    missing values, tests that nothing passes."""
+@pytest.fixture(scope="session")
+def walk_check(tmp_path_factory):
+    """Test-only: images in walking order against the same in heap order (tests/native/walk_check.cpp)."""
     import os
     import subprocess
 
     from cuml_b200.fil._desc import CCreateOpts, CForestDesc
 
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    so = os.path.join(str(tmp_path_factory.getbasetemp()), "libwalk_check.so")
-    if not os.path.exists(so):
-        src = [os.path.join(root, "tests", "native", "walk_check.cpp"),
-               os.path.join(root, "cuml_b200", "csrc", "pack.cpp")]
-        subprocess.check_call(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-o", so, *src])
+    so = os.path.join(str(tmp_path_factory.mktemp("walk")), "libwalk_check.so")
+    src = [os.path.join(root, "tests", "native", "walk_check.cpp"),
+           os.path.join(root, "cuml_b200", "csrc", "pack.cpp")]
+    subprocess.check_call(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-pthread", "-o", so, *src])
     lib = C.CDLL(so)
     lib.walk_check.restype = C.c_int64
     lib.walk_check.argtypes = [C.POINTER(CForestDesc), C.POINTER(CCreateOpts), C.c_int, C.c_int]
+
+    def run(desc, precision):
+        cd = desc.to_c()
+        opts = CCreateOpts(0 if precision == "single" else 1, 0, 1, 0, 0, 0, 0, 0)
+        return lib.walk_check(C.byref(cd), C.byref(opts), 400, 5)
+
+    return run
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("kw", [dict(max_depth=1), dict(max_depth=8, mixed_ops=True),
+                                dict(max_depth=9), dict(max_depth=10),
+                                dict(max_depth=5, vector=True, n_outputs=3)])
+def test_images_in_walking_order(walk_check, kw, precision):
+    """The images that the traversal kernels read (levels in the order of the ways, thresholds and codes as
+    half-precision floats) lead every row of codes to the payload that the heap-ordered images lead it to:
+    missing values, tests that nothing passes."""
     desc = random_forest_desc(31, n_trees=23, n_features=11, **kw)
     inner = np.flatnonzero(desc.node_kind == 1)
     desc.threshold[inner[::97 if max(kw.values()) == 8 else 7]] = np.nan  # (97: trees without and trees with them)
-    cd = desc.to_c()
-    opts = CCreateOpts(0 if precision == "single" else 1, 0, 1, 0, 0, 0, 0, 0)
-    assert lib.walk_check(C.byref(cd), C.byref(opts), 400, 5) == 0
+    assert walk_check(desc, precision) == 0
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("kw", [dict(max_depth=1), dict(max_depth=8, mixed_ops=True), dict(max_depth=10)])
+@pytest.mark.parametrize("left", [0, 1])
+def test_walking_order_of_forests_whose_missing_values_go_one_way(walk_check, left, kw, precision):
+    """A test that nothing passes has its children exchanged in walking order, and with them the direction of
+    missing values: a forest that sends all of them right then holds a test that sends them left."""
+    desc = random_forest_desc(31, n_trees=23, n_features=11, **kw)
+    inner = np.flatnonzero(desc.node_kind == 1)
+    desc.threshold[inner[::7]] = np.nan
+    desc.threshold[inner[3::7]] = np.inf
+    desc.default_left[:] = left
+    assert walk_check(desc, precision) == 0
