@@ -942,13 +942,14 @@ int b2fil_forest_create(const b2fil_forest_desc* desc, const b2fil_create_opts* 
         split_category_sets(pf.view, *image);
         walk_order(pf.view, image == &pf.q_nodes_nan, *image);
       }
-      const size_t stride = walk_tree_stride(pf.view.dense_depth, static_cast<size_t>(pf.view.q_leaf_bytes));
-      if (!pf.view.q_has_cat) f->view.q_tree_stride = static_cast<int64_t>(stride);
-      for (size_t t = 0; 3 * t < pf.q_top.size(); ++t)  // words 1..3 of the tree, as they are now
-        std::memcpy(&pf.q_top[3 * t], pf.q_nodes.data() + stride * t + 4, 12);
+      if (q_walk_order(pf.view)) {
+        const size_t stride = walk_tree_stride(pf.view.dense_depth, static_cast<size_t>(pf.view.q_leaf_bytes));
+        f->view.q_tree_stride = static_cast<int64_t>(stride);
+        for (size_t t = 0; 3 * t < pf.q_top.size(); ++t)  // words 1..3 of the tree, as they are now
+          std::memcpy(&pf.q_top[3 * t], pf.q_nodes.data() + stride * t + 4, 12);
+      }
       // (leaves far: see q_node_only_stride)
-      if (pf.view.format == FMT_DENSE_F && pf.view.leaf_vector_len == 1 && !pf.view.q_has_cat &&
-          (pf.view.dense_depth == 9 || pf.view.dense_depth == 10)) {
+      if (q_walk_order(pf.view) && pf.view.leaf_vector_len == 1 && pf.view.dense_depth >= 9) {
         far          = far_leaves(pf.view, pf.q_nodes);
         far_tests    = far_nodes(pf.view, pf.q_nodes);
         far_tests_nan = far_nodes(pf.view, pf.q_nodes_nan);

@@ -18,8 +18,8 @@ namespace {
 // where there is room for two while the tile before it is being walked (forests whose trees last
 // only a few microseconds per tile spend a fifth of them waiting for it otherwise);
 // tree batches stream through the stage ring exactly as in dense_kernel.  A node is 4 bytes, a test one
-// half-precision compare and a step one predicated addition (forest.hpp), or, in forests with categorical
-// tests, one signed subtraction and a funnel shift.
+// half-precision compare and a step one predicated addition (forest.hpp), or, in heap order, one signed
+// subtraction and a funnel shift.
 constexpr int NAN_NONE = 0, NAN_TESTED = 1, NAN_COLUMNS = 2;
 
 constexpr int kBarTileFull  = 2 * kMaxStages;      // mbarrier slots after the stage ring: two each
@@ -125,7 +125,16 @@ __device__ __forceinline__ uint32_t shift_if_categorical(uint32_t node, uint32_t
 }
 
 // DEPTH > 0 fixes the tree depth at compile time (the level loop is fully unrolled); DEPTH == 0
-// reads it from the forest.  TOPC: the first two levels take their nodes from `top`.
+// reads it from the forest.
+// HEAP: the image is in heap order (words 2i and 2i + 1 of a tree's block are the children of word i); a
+// test is one signed subtraction whose sign goes into the heap index with one funnel shift.  Otherwise it is
+// in walking order, which pays where levels are constants (q_walk_order()): with the depth read at run time two
+// places have to be worked out per level, and the same kernels took 1.15 to 1.4 of the time in heap order (300
+// depth-6 trees x 50 features, fp64, 150,000 rows: 181 us against 141; 100 depth-11 trees, fp32: 161 against 119).
+// CAT (heap order): forests with categorical tests.  A category set takes part in the subtraction by a shift;
+// with compares and predicates it took as many instructions in walking order, and a longer way from the
+// rank to the next node (5000 depth-6 trees, 150,000 rows: 1894 us against 1871).
+// TOPC: the first two levels take their nodes from `top`.
 // PAIR: the walk for launch shapes that shared memory keeps small (few warps, few trees in
 // flight), where the latency of one step, not the shared-memory pipe, is the limit: both children
 // of the current node are requested together
@@ -139,7 +148,7 @@ __device__ __forceinline__ uint32_t shift_if_categorical(uint32_t node, uint32_t
 // arrays of their own: a stage is one copy (a copy per tree was 20 us slower with 2000 trees of depth 10 on
 // 200,000 rows), and the payloads of ways that part late are neighbours (180 us: in the order of the
 // blocks, whose last steps are the longest, every row fetched another sector).
-template <typename T, int MODE, int NT, int DEPTH, bool TOPC, bool PAIR = false, bool LEAFG = false>
+template <typename T, int MODE, int NT, int DEPTH, bool CAT, bool HEAP, bool TOPC, bool PAIR, bool LEAFG>
 struct DenseQWalker {
   using TR = Traits<T>;
   // Walk the warp's 32 rows through all trees.  A stage of the ring holds K sub-batches of G * NT
@@ -157,18 +166,22 @@ struct DenseQWalker {
                                               uint32_t copy_off)
   {
     constexpr bool NANS = MISSING == NAN_TESTED;
-    static_assert(!TOPC || DEPTH >= 2, "top nodes need two levels");
-    static_assert(!PAIR || (!TOPC && MODE == MODE_SCALAR && sizeof(T) == 4),
+    static_assert(HEAP || (!CAT && sizeof(T) == 4 && (DEPTH >= 4 || PAIR)), "forests in walking order");
+    static_assert(!TOPC || (DEPTH >= 2 && !HEAP), "top nodes need two levels, and are in walking order");
+    static_assert(!PAIR || (!CAT && !TOPC && MODE == MODE_SCALAR && sizeof(T) == 4),
                   "the child-pair walk exists for fp32 scalar leaves without categorical tests");
-    static_assert(!LEAFG || (!PAIR && MODE == MODE_SCALAR && sizeof(T) == 4),
+    static_assert(!LEAFG || (!HEAP && !PAIR && MODE == MODE_SCALAR && sizeof(T) == 4),
                   "payloads outside the stages exist for fp32 scalar leaves without categorical tests");
     const ForestView& f    = p.f;
     const int D            = DEPTH > 0 ? DEPTH : f.dense_depth;
-    const uint32_t leaves_at = 4u * walk_leaves_at(D);  // from the start of a tree to its payloads
+    // HEAP: from a node to its category set
+    const uint32_t sets_at = 4u << D;
+    // from the start of a tree to its payloads
+    const uint32_t leaves_at = HEAP ? (CAT ? 8u : 4u) << D : 4u * walk_leaves_at(D);
     // bytes between two trees of a stage
     constexpr uint32_t kStride = LEAFG ? walk_nodes_stride(DEPTH)
                                        : static_cast<uint32_t>(walk_tree_stride(DEPTH, TR::ES));
-    constexpr bool known_stride = MODE == MODE_SCALAR && DEPTH > 0;
+    constexpr bool known_stride = MODE == MODE_SCALAR && DEPTH > 0 && !HEAP;
     const uint32_t tstride      = known_stride ? kStride : static_cast<uint32_t>(f.q_tree_stride);
     // bytes per leaf payload: the element size, except where vector leaves sit in the tree block
     const uint32_t lbytes  = MODE == MODE_SCALAR ? TR::ES : static_cast<uint32_t>(f.q_leaf_bytes);
@@ -178,24 +191,6 @@ struct DenseQWalker {
     const int per_batch    = per_sub * K;
     const uint32_t mine    = static_cast<uint32_t>(g * NT) * tstride;  // this warp's trees in a sub-batch
     const uint32_t sub_b   = static_cast<uint32_t>(per_sub) * tstride;
-    // bytes from the start of a tree to a level, and of a step to the right on it (`lvl` is a number, or, where
-    // DEPTH is a constant, a constant)
-    auto level_at = [&](auto lvl) {
-      if constexpr (std::is_same_v<decltype(lvl), int>) {
-        return 4u * walk_level_at(D, lvl);
-      } else {
-        constexpr uint32_t at = 4u * walk_level_at(DEPTH, decltype(lvl)::value);
-        return at;
-      }
-    };
-    auto step_bytes = [&](auto lvl) {
-      if constexpr (std::is_same_v<decltype(lvl), int>) {
-        return 4u * walk_step_words(D, lvl);
-      } else {
-        constexpr uint32_t step = 4u * walk_step_words(DEPTH, decltype(lvl)::value);
-        return step;
-      }
-    };
     bool ok                = true;
     uint32_t seen          = 0u;  // what release_stage() cannot tell from the sums, folded
 
@@ -219,12 +214,62 @@ struct DenseQWalker {
       using Each = std::make_integer_sequence<int, NT>;
       // slots past the end of the forest repeat the last live tree; results are dropped
       auto slot = [&](int k) { return static_cast<uint32_t>(FULL ? k : min(k, n_act - 1)) * tstride; };
-      uint32_t a[NT];  // start of the tree's block (the first one's, TS > 0) + 4 * place in the level
+      // walking order: start of the tree's block (the first one's, TS > 0) + 4 * place in the level;
+      // heap order: address of the node, its heap index, and start of the block
+      uint32_t a[NT], idx[NT], base[NT];
 #pragma unroll
-      for (int k = 0; k < NT; ++k) a[k] = TS ? base0 : base0 + slot(k);
+      for (int k = 0; k < NT; ++k) {
+        a[k] = TS ? base0 : base0 + slot(k);
+        if (HEAP) {
+          base[k] = a[k];
+          idx[k]  = 1u;
+          a[k] += 4u;
+        }
+      }
       // the NT walks are independent: all node loads are issued first, then all rank loads,
       // so that their shared-memory latencies overlap inside one warp.
-      // step(): the rows' ranks against NT nodes of level `lvl` (a constant where DEPTH is).
+      // heap_level(): a level in heap order.  The sign bit of d[k] is the step to the right.
+      auto heap_test = [&](const uint32_t(&node)[NT], uint32_t(&d)[NT]) {
+        uint32_t q[NT], bits[NT];
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          // (see step())
+          q[k] = lds_u16(__dp2a_lo(node[k], fstride, row_addr));
+        }
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          if (CAT) bits[k] = lds_if_categorical<DEPTH ? 4u << DEPTH : 0u>(node[k], a[k] + (DEPTH ? 0u : sets_at));
+        }
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          // rank j in the high half: x < T[j] <=> rank(x) <= j, so right <=> j - rank < 0
+          d[k] = rank_diff(node[k], q[k]);
+          // the code of a categorical value is its category and the node's set is stored
+          // bit-reversed: the clamped funnel shift by the code moves the category's bit to the sign
+          // position, and leaves d for every code of 32 and above (no category, NaN), which the
+          // large rank of a categorical node has made non-negative, or right for a missing value
+          // of a doubled column.  Predicated: the walk has no data-dependent branch.
+          if (CAT) d[k] = shift_if_categorical(node[k], d[k], bits[k], q[k]);
+          // the missing-goes-right flag sits 15 bits below the sign.  (Both forms compute the same; each
+          // kernel family keeps the one it was measured fastest with: the two walks of a kernel share
+          // its register allocation.)
+          if (NANS && CAT && q[k] == Q_NAN_CODE) d[k] = node[k] << 15;
+          if (NANS && !CAT && q[k] == Q_NAN_CODE) d[k] = (node[k] & Q_DEFAULT_RIGHT) ? 0x80000000u : 0u;
+        }
+      };
+      auto heap_level = [&]() {
+        uint32_t node[NT], d[NT];
+#pragma unroll
+        for (int k = 0; k < NT; ++k) node[k] = lds_u32(a[k]);
+        heap_test(node, d);
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          // heap index 2i + right in one funnel shift: (i << 1) | (d >> 31)
+          idx[k] = __funnelshift_l(d[k], idx[k], 1);
+          a[k]   = idx[k] * 4u + base[k];
+        }
+      };
+      // step(): the rows' ranks against NT nodes in walking order.
       auto step = [&](const uint32_t(&node)[NT], auto from_param, auto&& move) {
         constexpr bool PARAM = decltype(from_param)::value;
         uint32_t q[NT];
@@ -241,43 +286,57 @@ struct DenseQWalker {
 #pragma unroll
         for (int k = 0; k < NT; ++k) move(k, node[k], q[k]);
       };
+      // `lvl`: a constant
       auto level = [&](auto lvl) {
+        constexpr int LVL = decltype(lvl)::value;
         uint32_t node[NT];
-        if constexpr (DEPTH > 0) {
-          for_each_constant(
-            [&](auto kc) {
-              constexpr int k = decltype(kc)::value, L = decltype(lvl)::value;
-              node[k] = lds_u32_at<k * TS + 4u * walk_level_at(DEPTH, L)>(a[k]);
-            },
-            Each{});
-        } else {
-#pragma unroll
-          for (int k = 0; k < NT; ++k) node[k] = lds_u32(a[k] + level_at(lvl));
-        }
+        for_each_constant(
+          [&](auto kc) {
+            constexpr int k = decltype(kc)::value;
+            node[k] = lds_u32_at<k * TS + 4u * walk_level_at(DEPTH, LVL)>(a[k]);
+          },
+          Each{});
         step(node, std::false_type{}, [&](int k, uint32_t n, uint32_t q) {
-          walk_step<NANS>(a[k], n, q, step_bytes(lvl));
+          walk_step<NANS>(a[k], n, q, 4u * walk_step_words(DEPTH, LVL));
         });
       };
       if constexpr (PAIR) {
         uint32_t node[NT];
 #pragma unroll
-        for (int k = 0; k < NT; ++k) node[k] = lds_u32(a[k] + 4u);  // the root
+        for (int k = 0; k < NT; ++k) node[k] = lds_u32(HEAP ? a[k] : a[k] + 4u);  // the root
 #pragma unroll 2
         for (int lvl = 0; lvl < D; ++lvl) {
           // both children; below the last level these are the two leaf payloads (4-byte payloads go on
           // behind the nodes)
-          const uint32_t inc = step_bytes(lvl), at = lvl + 1 < D ? level_at(lvl + 1) : leaves_at;
           uint32_t left[NT], right[NT];
+          if constexpr (HEAP) {
+            uint32_t d[NT];
 #pragma unroll
-          for (int k = 0; k < NT; ++k) {
-            left[k]  = lds_u32(a[k] + at);
-            right[k] = lds_u32(a[k] + at + inc);
+            for (int k = 0; k < NT; ++k) {
+              const uint2 pair = lds_u32x2(base[k] + idx[k] * 8u);
+              left[k]          = pair.x;
+              right[k]         = pair.y;
+            }
+            heap_test(node, d);
+#pragma unroll
+            for (int k = 0; k < NT; ++k) {
+              idx[k]  = __funnelshift_l(d[k], idx[k], 1);
+              node[k] = static_cast<int32_t>(d[k]) < 0 ? right[k] : left[k];
+            }
+          } else {
+            const uint32_t inc = 4u * walk_step_words(D, lvl);
+            const uint32_t at  = lvl + 1 < D ? 4u * walk_level_at(D, lvl + 1) : leaves_at;
+#pragma unroll
+            for (int k = 0; k < NT; ++k) {
+              left[k]  = lds_u32(a[k] + at);
+              right[k] = lds_u32(a[k] + at + inc);
+            }
+            step(node, std::false_type{}, [&](int k, uint32_t n, uint32_t q) {
+              const uint32_t before = a[k];
+              walk_step<NANS>(a[k], n, q, inc);
+              node[k] = a[k] != before ? right[k] : left[k];
+            });
           }
-          step(node, std::false_type{}, [&](int k, uint32_t n, uint32_t q) {
-            const uint32_t before = a[k];
-            walk_step<NANS>(a[k], n, q, inc);
-            node[k] = a[k] != before ? right[k] : left[k];
-          });
         }
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
@@ -300,8 +359,21 @@ struct DenseQWalker {
              [&](int k, uint32_t n, uint32_t q) { node[k] = root_step<NANS>(a[k], n, q, n2[k], n3[k]); });
         step(node, std::true_type{}, [&](int k, uint32_t n, uint32_t q) { walk_step<NANS>(a[k], n, q, 8u); });
       }
-      uint32_t at_far[LEAFG ? NT : 1];  // LEAFG: where the walks were on level kWalkFarLevel
-      if constexpr (DEPTH > 0) {
+      [[maybe_unused]] uint32_t at_far[LEAFG ? NT : 1];  // LEAFG: where the walks were on level kWalkFarLevel
+      if constexpr (HEAP) {
+        if (DEPTH > 0) {
+#pragma unroll
+          for (int lvl = 0; lvl < DEPTH; ++lvl) heap_level();
+        } else {
+#pragma unroll 4
+          for (int lvl = 0; lvl < D; ++lvl) heap_level();
+        }
+        // fp64: the payload's address instead of the places it follows from (registers are short)
+        if (TR::ES == 8) {
+#pragma unroll
+          for (int k = 0; k < NT; ++k) a[k] = base[k] + leaves_at + (idx[k] - (1u << D)) * lbytes;
+        }
+      } else {
         constexpr int SKIP = TOPC ? 2 : 0;
         for_each_constant(
           [&](auto lc) {
@@ -313,15 +385,24 @@ struct DenseQWalker {
             level(std::integral_constant<int, L>{});
           },
           std::make_integer_sequence<int, DEPTH - SKIP>{});
-      } else {
-#pragma unroll 4
-        for (int lvl = 0; lvl < D; ++lvl) level(lvl);
       }
-      // place of the leaf * 4 in tree k, and the address of its payload
-      auto place4  = [&](int k) { return a[k] - (TS ? base0 : base0 + slot(k)); };
-      auto leaf_at = [&](int k) {
-        return lbytes == 4u ? a[k] + k * TS + leaves_at : base0 + slot(k) + leaves_at + (place4(k) >> 2) * lbytes;
+      // address of the payload, of `bytes` bytes, that walk k ended on
+      auto payload_at = [&](int k, uint32_t bytes) {
+        // (4-byte payloads go on behind the nodes in heap order, too)
+        if constexpr (HEAP && (TR::ES == 8 || (MODE == MODE_SCALAR && !CAT))) return a[k];
+        if constexpr (HEAP) return base[k] + leaves_at + (idx[k] - (1u << D)) * bytes;
+        const uint32_t start = TS ? base0 : base0 + slot(k);
+        return bytes == 4u ? a[k] + k * TS + leaves_at : base0 + slot(k) + leaves_at + (a[k] - start) * (bytes >> 2);
       };
+      auto leaf_at = [&](int k) { return payload_at(k, lbytes); };
+      // scalar leaves of a multi-class forest: trees are stored class by class, so when the
+      // first and the last tree of the sub-batch feed the class of the running sum, all do
+      bool same_class = false;
+      if (MODE == MODE_SCALAR && CAT) {
+        same_class = f.n_outputs == 1 ||
+                     (__ldg(f.tree_class + first) == run.cls &&
+                      __ldg(f.tree_class + first + n_act - 1) == run.cls);
+      }
       if constexpr (LEAFG) {
         // add the payloads that the previous sub-batch requested (they arrived during this
         // walk), then request this sub-batch's; nothing touches them until the next one is done
@@ -403,9 +484,21 @@ struct DenseQWalker {
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           if (FULL || k < n_act) {
-            const uint2 v = lds_u32x2(base0 + slot(k) + leaves_at + place4(k) * 2u);
+            const uint2 v = lds_u32x2(payload_at(k, 8u));
             run.v[0] += static_cast<T>(__uint_as_float(v.x));
             run.v[1] += static_cast<T>(__uint_as_float(v.y));
+          }
+        }
+      } else if (TR::ES == 8 && MODE == MODE_VECTOR && inline_vec) {
+        // (the same as below: fp64 kernels spill less this way, fp32 ones the other way)
+#pragma unroll
+        for (int k = 0; k < NT; ++k) {
+          if (FULL || k < n_act) {
+            const uint32_t leaf_a = leaf_at(k);
+#pragma unroll
+            for (int c = 0; c < kRegClasses; ++c) {
+              if (c < f.n_outputs) run.v[c] += TR::ld_real(leaf_a + c * TR::ES);
+            }
           }
         }
       } else {
@@ -413,237 +506,7 @@ struct DenseQWalker {
         for (int k = 0; k < NT; ++k) {
           if (FULL || k < n_act) {
             const uint32_t leaf_a = leaf_at(k);
-            if (MODE == MODE_VECTOR && inline_vec) {
-              // the leaf's vector sits in the tree block: one sum per output, in registers
-#pragma unroll
-              for (int c = 0; c < kRegClasses; ++c) {
-                if (c < f.n_outputs) run.v[c] += TR::ld_real(leaf_a + c * TR::ES);
-              }
-              continue;
-            }
-            const typename TR::Val payload = TR::ld_val(leaf_a);
-            if (MODE == MODE_VECTOR) seen ^= TR::low32(payload);
-            take_leaf<T, MODE>(p, first + k, payload, 0u, acc_group, R, r, row, run);
-          }
-        }
-      }
-    };
-
-    for (int b = b_begin; b < b_end; ++b) {
-      const uint32_t s = pos.stage;
-      if (ok) ok = mbar_wait(bars + 8u * s, pos.phase);
-      if (ok) {
-        uint32_t base0 = stages + s * stage_bytes + mine;
-        int first      = b * per_batch + g * NT;  // first tree of this warp inside the stage
-        for (int kk = 0; kk < K; ++kk, base0 += sub_b, first += per_sub) {
-          const int n_act = f.n_trees - first;
-          if (n_act >= NT) {
-            sub_batch(std::true_type{}, base0, first, NT);
-          } else if (n_act > 0) {
-            sub_batch(std::false_type{}, base0, first, n_act);
-          } else {
-            break;
-          }
-        }
-      }
-      const uint32_t empty = bars + 8u * (kMaxStages + s);
-      if (MODE >= MODE_PERTREE) {
-        release_stored_stage(empty, lane);
-      } else {
-        bool read = seen != 0xffffffffu;
-        if ((MODE == MODE_SCALAR && !LEAFG) || (MODE == MODE_VECTOR && inline_vec))
-          read = sums_known<T, MODE>(run);
-        release_stage(empty, lane, read, p.zero);
-      }
-      pos.advance(S);
-    }
-    if constexpr (LEAFG) take_pending();
-    return ok;
-  }
-};
-
-// The walk of forests with categorical tests, over the images in heap order: words 2i and 2i + 1 of a tree's block
-// are the children of word i, a test is one signed subtraction whose sign goes into the heap index with one
-// funnel shift.  A category set takes part in that sum by a shift; with compares and predicates it took as many
-// instructions in walking order, and a longer way from the rank to the next node (5000 depth-6 trees, 150,000
-// rows: 1894 us against 1871).
-template <typename T, int MODE, int NT, int DEPTH>
-struct HeapWalker {
-  using TR = Traits<T>;
-  // Walk the warp's 32 rows through all trees.  A stage of the ring holds K sub-batches of G * NT
-  // trees; the warp waits once per stage and walks its NT trees of every sub-batch.
-  // MISSING: see DenseQWalker.
-  template <int MISSING>
-  static __device__ __forceinline__ bool walk(const PredictParams& p, int G, int S, int K, int g,
-                                              int r, int64_t row, int lane, uint32_t bars,
-                                              uint32_t stages, uint32_t stage_bytes,
-                                              uint32_t row_addr, uint32_t stride_b, T* acc_group,
-                                              int R, RingPos& pos, Running<T>& run, int b_begin,
-                                              int b_end)
-  {
-    constexpr bool NANS = MISSING == NAN_TESTED;
-    const ForestView& f    = p.f;
-    const int D            = DEPTH > 0 ? DEPTH : f.dense_depth;
-    // bytes of a tree's test nodes and the category sets behind them
-    const uint32_t width_b = 8u << D;
-    const uint32_t sets_at = 4u << D;  // from a node to its category set
-    // bytes between two trees of a stage
-    const uint32_t tstride = static_cast<uint32_t>(f.q_tree_stride);
-    // bytes per leaf payload: the element size, except where vector leaves sit in the tree block
-    const uint32_t lbytes  = MODE == MODE_SCALAR ? TR::ES : static_cast<uint32_t>(f.q_leaf_bytes);
-    const bool inline_vec  = MODE != MODE_SCALAR && lbytes > TR::ES;
-    const uint32_t fstride = stride_b >> Q_FEATURE_SHIFT;  // R / 2 <= 128: fits a byte
-    const int per_sub      = G * NT;
-    const int per_batch    = per_sub * K;
-    const uint32_t mine    = static_cast<uint32_t>(g * NT) * tstride;  // this warp's trees in a sub-batch
-    const uint32_t sub_b   = static_cast<uint32_t>(per_sub) * tstride;
-    bool ok                = true;
-    uint32_t seen          = 0u;  // what release_stage() cannot tell from the sums, folded
-
-    // One sub-batch: NT trees side by side.  FULL means all NT slots hold live trees, which lets
-    // the compiler drop every per-slot guard.
-    auto sub_batch = [&](auto full_tag, uint32_t base0, int first, int n_act) {
-      constexpr bool FULL = decltype(full_tag)::value;
-      uint32_t base[NT], idx[NT], a[NT];
-#pragma unroll
-      for (int k = 0; k < NT; ++k) {
-        // slots past the end of the forest repeat the last live tree; results are dropped
-        base[k] = base0 + static_cast<uint32_t>(FULL ? k : min(k, n_act - 1)) * tstride;
-        idx[k]  = 1u;  // heap index of the root
-        a[k]    = base[k] + 4u;
-      }
-      // the NT walks are independent: all node loads are issued first, then all rank loads,
-      // so that their shared-memory latencies overlap inside one warp.
-      // test(): the rows' ranks against NT nodes; the sign bit of d[k] is the step to the right.
-      auto test = [&](const uint32_t(&node)[NT], const uint32_t(&at)[NT], uint32_t(&d)[NT]) {
-        uint32_t q[NT], bits[NT];
-#pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          // the low half of a node is feature * 4: one dot-product instruction (low half x byte 0
-          // of fstride, high half x byte 1 = 0) turns it into the address of the row's rank of
-          // that feature
-          q[k] = lds_u16(__dp2a_lo(node[k], fstride, row_addr));
-        }
-#pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          bits[k] = lds_if_categorical<DEPTH ? 4u << DEPTH : 0u>(node[k], at[k] + (DEPTH ? 0u : sets_at));
-        }
-#pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          // rank j in the high half: x < T[j] <=> rank(x) <= j, so right <=> j - rank < 0
-          d[k] = rank_diff(node[k], q[k]);
-          // the code of a categorical value is its category and the node's set is stored
-          // bit-reversed: the clamped funnel shift by the code moves the category's bit to the sign
-          // position, and leaves d for every code of 32 and above (no category, NaN), which the
-          // large rank of a categorical node has made non-negative, or right for a missing value
-          // of a doubled column.  Predicated: the walk has no data-dependent branch.
-          d[k] = shift_if_categorical(node[k], d[k], bits[k], q[k]);
-          // the missing-goes-right flag sits 15 bits below the sign
-          if (NANS && q[k] == Q_NAN_CODE) d[k] = node[k] << 15;
-        }
-      };
-      auto level = [&]() {
-        uint32_t node[NT], d[NT];
-#pragma unroll
-        for (int k = 0; k < NT; ++k) node[k] = lds_u32(a[k]);
-        test(node, a, d);
-#pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          // heap index 2i + right in one funnel shift: (i << 1) | (d >> 31)
-          idx[k] = __funnelshift_l(d[k], idx[k], 1);
-          a[k]   = idx[k] * 4u + base[k];
-        }
-      };
-      if (DEPTH > 0) {
-#pragma unroll
-        for (int lvl = 0; lvl < DEPTH; ++lvl) level();
-      } else {
-#pragma unroll 4
-        for (int lvl = 0; lvl < D; ++lvl) level();
-      }
-      // scalar leaves of a multi-class forest: trees are stored class by class, so when the
-      // first and the last tree of the sub-batch feed the class of the running sum, all do
-      bool same_class = false;
-      if (MODE == MODE_SCALAR) {
-        same_class = f.n_outputs == 1 ||
-                     (__ldg(f.tree_class + first) == run.cls &&
-                      __ldg(f.tree_class + first + n_act - 1) == run.cls);
-      }
-      if (MODE >= MODE_PERTREE) {
-        // One output per (row, tree).  The payload slot holds what is reported: the leaf value,
-        // or the leaf id when the CTA streams the image made for that (MODE_LEAFID).  With four
-        // live trees that are also the caller's trees first..first+3, a row's four outputs are
-        // contiguous and leave as 16-byte stores, or, where the rows are not aligned for that,
-        // four lanes at a time (store_quads): scalar 4-byte stores at a stride of a whole output
-        // row cost one sector request each and bound these predictions otherwise.
-        typename TR::Val val[NT];
-        uint32_t leaf_at[NT];
-#pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          const uint32_t slot = idx[k] - (1u << D);
-          leaf_at[k]          = base[k] + width_b + slot * lbytes;
-          val[k]              = TR::ld_val(leaf_at[k]);
-        }
-        const bool scalar_out = MODE == MODE_LEAFID || f.leaf_vector_len <= 1;
-        const bool quad = FULL && NT == 4 && scalar_out && f.q_trees_in_order != 0;
-        using Out = std::conditional_t<MODE == MODE_LEAFID, uint32_t, typename TR::Val>;
-        Out* out  = static_cast<Out*>(p.out);
-        if (quad && (f.n_trees & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0) {
-          if (row < p.n_rows) {
-            Out* dst = out + row * f.n_trees + first;
-            if constexpr (sizeof(Out) == 4) {
-              *reinterpret_cast<uint4*>(dst) =
-                make_uint4(TR::low32(val[0]), TR::low32(val[NT > 1 ? 1 : 0]),
-                           TR::low32(val[NT > 2 ? 2 : 0]), TR::low32(val[NT > 3 ? 3 : 0]));
-            } else {
-              *reinterpret_cast<ulonglong2*>(dst) =
-                make_ulonglong2(val[0], val[NT > 1 ? 1 : 0]);
-              *reinterpret_cast<ulonglong2*>(dst + 2) =
-                make_ulonglong2(val[NT > 2 ? 2 : 0], val[NT > 3 ? 3 : 0]);
-            }
-          }
-        } else if (quad) {
-          store_quads<Out>(out, f.n_trees, row, p.n_rows, first, static_cast<Out>(val[0]),
-                           static_cast<Out>(val[NT > 1 ? 1 : 0]), static_cast<Out>(val[NT > 2 ? 2 : 0]),
-                           static_cast<Out>(val[NT > 3 ? 3 : 0]));
-        } else {
-#pragma unroll
-          for (int k = 0; k < NT; ++k) {
-            if (FULL || k < n_act) {
-              if (MODE == MODE_LEAFID) {
-                if (row < p.n_rows) {
-                  const int orig = __ldg(f.tree_orig + first + k);
-                  static_cast<uint32_t*>(p.out)[row * f.n_trees + orig] = TR::low32(val[k]);
-                }
-              } else if (inline_vec) {
-                // per-tree outputs of vector leaves that sit in the tree block
-                if (row < p.n_rows) {
-                  const int orig = __ldg(f.tree_orig + first + k);
-                  T* out = static_cast<T*>(p.out) + (row * f.n_trees + orig) * f.n_outputs;
-                  for (int c = 0; c < f.n_outputs; ++c) out[c] = TR::ld_real(leaf_at[k] + c * TR::ES);
-                }
-              } else {
-                take_leaf<T, MODE>(p, first + k, val[k], 0u, acc_group, R, r, row, run);
-              }
-            }
-          }
-        }
-      } else if (MODE == MODE_VECTOR && inline_vec && f.n_outputs == 2 && sizeof(T) == 4) {
-        // two classes, the common random-forest classifier: one 8-byte load per leaf
-#pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          if (FULL || k < n_act) {
-            const uint2 v = lds_u32x2(base[k] + width_b + (idx[k] - (1u << D)) * 8u);
-            run.v[0] += static_cast<T>(__uint_as_float(v.x));
-            run.v[1] += static_cast<T>(__uint_as_float(v.y));
-          }
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          if (FULL || k < n_act) {
-            const uint32_t leaf_a = base[k] + width_b + (idx[k] - (1u << D)) * lbytes;
-            if (MODE == MODE_VECTOR && inline_vec) {
+            if (TR::ES == 4 && MODE == MODE_VECTOR && inline_vec) {
               // the leaf's vector sits in the tree block: one sum per output, in registers
 #pragma unroll
               for (int c = 0; c < kRegClasses; ++c) {
@@ -685,12 +548,13 @@ struct HeapWalker {
         release_stored_stage(empty, lane);
       } else {
         bool read = seen != 0xffffffffu;
-        if (MODE == MODE_SCALAR || (MODE == MODE_VECTOR && inline_vec))
+        if ((MODE == MODE_SCALAR && !LEAFG) || (MODE == MODE_VECTOR && inline_vec))
           read = sums_known<T, MODE>(run);
         release_stage(empty, lane, read, p.zero);
       }
       pos.advance(S);
     }
+    if constexpr (LEAFG) take_pending();
     return ok;
   }
 };
@@ -793,7 +657,7 @@ __device__ __forceinline__ void finish_shared_tile(const PredictParams& p, const
     finish_row<T>(p, sums, R, 1, threadIdx.x, static_cast<int64_t>(seg.tile) * R + threadIdx.x);
 }
 
-template <typename T, int MODE, int NT, int DEPTH, bool CAT, bool TOPC, bool PAIR = false,
+template <typename T, int MODE, int NT, int DEPTH, bool CAT, bool HEAP, bool TOPC, bool PAIR = false,
           bool LEAFG = false>
 __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs& q,
                                              const uint32_t* top)
@@ -952,15 +816,9 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
     if (ok) {
       const uint32_t row_addr = row_slot + at_tile;
       auto go = [&](auto missing) {
-        if constexpr (CAT) {
-          return HeapWalker<T, MODE, NT, DEPTH>::template walk<decltype(missing)::value>(
-            p, G, S, K, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b, acc_group, R,
-            pos, run, seg.begin, seg.end());
-        } else {
-          return DenseQWalker<T, MODE, NT, DEPTH, TOPC, PAIR, LEAFG>::template walk<decltype(missing)::value>(
-            p, G, S, K, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b, acc_group, R,
-            pos, run, top, seg.begin, seg.end(), tile_bytes);
-        }
+        return DenseQWalker<T, MODE, NT, DEPTH, CAT, HEAP, TOPC, PAIR, LEAFG>::template walk<decltype(missing)::value>(
+          p, G, S, K, g, r, row0 + r, lane, bars, stages, stage_bytes, row_addr, stride_b, acc_group, R,
+          pos, run, top, seg.begin, seg.end(), tile_bytes);
       };
       if (nans && !q.nan_columns) {
         ok = go(std::integral_constant<int, NAN_TESTED>{});
@@ -1001,15 +859,15 @@ template <typename T, int MODE, int NT, int DEPTH, bool CAT>
 __global__ void __launch_bounds__(NT > 4 ? 800 : 1024, 1)
 dense_q_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q)
 {
-  dense_q_body<T, MODE, NT, DEPTH, CAT, false>(p, q, nullptr);
+  dense_q_body<T, MODE, NT, DEPTH, CAT, CAT || DEPTH == 0, false>(p, q, nullptr);
 }
 
 // Same kernel with the child-pair walk (see DenseQWalker).
-template <int NT>
+template <int NT, bool HEAP>
 __global__ void __launch_bounds__(1024, 1)
 dense_q_pair_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q)
 {
-  dense_q_body<float, MODE_SCALAR, NT, 0, false, false, true>(p, q, nullptr);
+  dense_q_body<float, MODE_SCALAR, NT, 0, false, HEAP, false, true>(p, q, nullptr);
 }
 
 // Same kernel with the leaf payloads left in global memory (see DenseQWalker), and the same with the top nodes
@@ -1018,14 +876,14 @@ template <int NT, int DEPTH>
 __global__ void __launch_bounds__(1024, 1)
 dense_q_leafg_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q)
 {
-  dense_q_body<float, MODE_SCALAR, NT, DEPTH, false, false, false, true>(p, q, nullptr);
+  dense_q_body<float, MODE_SCALAR, NT, DEPTH, false, false, false, false, true>(p, q, nullptr);
 }
 template <int NT, int DEPTH, int TREES>
 __global__ void __launch_bounds__(1024, 1)
 dense_q_leafg_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q,
                      const __grid_constant__ QTop<TREES> top)
 {
-  dense_q_body<float, MODE_SCALAR, NT, DEPTH, false, true, false, true>(p, q, top.w);
+  dense_q_body<float, MODE_SCALAR, NT, DEPTH, false, false, true, false, true>(p, q, top.w);
 }
 
 // Same kernel with the top nodes of every tree in the parameter block.
@@ -1034,7 +892,7 @@ __global__ void __launch_bounds__(NT > 4 ? 800 : 1024, 1)
 dense_q_top_kernel(const __grid_constant__ PredictParams p, const __grid_constant__ QArgs q,
                    const __grid_constant__ QTop<TREES> top)
 {
-  dense_q_body<T, MODE, NT, DEPTH, false, true>(p, q, top.w);
+  dense_q_body<T, MODE, NT, DEPTH, false, false, true>(p, q, top.w);
 }
 
 // The three top nodes of every tree, which travel in the parameter block.

@@ -158,7 +158,8 @@ constexpr uint32_t Q_DEFAULT_RIGHT = 0x10000u;  // missing values go right (stor
 constexpr uint32_t Q_RANK_SHIFT    = 17;
 constexpr uint32_t Q_NEVER_LEFT    = 0x7FFFu;  // j of a test that no value passes
 constexpr uint32_t Q_MAX_RANK_FIELD = 0x3FFFu;  // j of a test that every code passes (categorical nodes)
-// Without categorical tests the kernels read this image in walking order (walk_order() before the upload):
+// Kernels that have the depth as a constant (q_walk_order()) read this image in walking order (walk_order()
+// before the upload):
 //     bits 31..16: a half-precision float, the bits of j, whose sign says that missing values go left
 //     bits 15..2: feature                    bits 1..0: zero
 // Ranks below 0x4000 are the bits of small positive floats in the same order, so one half-precision compare
@@ -339,9 +340,11 @@ struct ForestView {
                                 // leaf's vector), or n_outputs elements when the vectors of a
                                 // forest with few outputs sit in the tree blocks themselves
   int32_t q_any_default_left;   // 0: missing values go right in every test, also in walking order
-  int64_t q_tree_stride;        // bytes between trees: 2^D * (node bytes + leaf bytes), 16-byte multiple
+  int64_t q_tree_stride;        // bytes between trees, 16-byte multiple: 2^D * (node bytes + leaf bytes), or, in
+                                // walking order, walk_tree_stride()
   const void* q_nodes;          // [n_trees] blocks of [2^D nodes][2^D leaf payloads] of uint32 nodes,
-                                // with [2^D category sets] in between when q_has_cat
+                                // with [2^D category sets] in between when q_has_cat; in walking order with
+                                // the places of walk_level_at()
   const void* q_nodes_ids;      // same blocks with the leaf id (uint32) in every leaf payload slot:
                                 // what the traversal streams when it reports leaf ids
   // forests whose payloads may stay in global memory (depth 9 and 10, fp32 scalar leaves), else null:
@@ -445,7 +448,14 @@ bool build_blocks(PackedForest& pf);
 // [2^D {node, category set}] to [2^D nodes][2^D category sets], which is what the kernels read.
 void split_category_sets(const ForestView& view, std::vector<uint8_t>& image);
 
-// Before the upload of an image without categorical tests: heap order and ranks << 17 become what the kernels
+// Is the image uploaded in walking order?  Only where every kernel that may walk it knows the depth at compile
+// time: fp32, depth 4 to 10, no categorical tests.
+inline bool q_walk_order(int format, int depth, bool has_cat)
+{
+  return format == FMT_DENSE_F && depth >= 4 && depth <= 10 && !has_cat;
+}
+inline bool q_walk_order(const ForestView& v) { return q_walk_order(v.format, v.dense_depth, v.q_has_cat != 0); }
+// Before the upload of such an image (others stay as they are): heap order and ranks << 17 become what the kernels
 // walk (see above), trees of walk_tree_stride() bytes.  `doubled`: the image for doubled columns.
 void walk_order(const ForestView& view, bool doubled, std::vector<uint8_t>& image);
 // The payloads of such an image in the order for global memory, level_words(depth) of four bytes per tree.

@@ -870,11 +870,8 @@ int q_max_trees_in_flight(const ForestView& f, int mode, bool has_top)
   if (f.q_has_cat) {
     return f.format == FMT_DENSE_F && mode == MODE_SCALAR && f.dense_depth >= 4 && f.dense_depth <= 8 ? 6 : 4;
   }
-  const bool specialised = f.format == FMT_DENSE_F && (mode == MODE_SCALAR || mode == MODE_VECTOR) &&
-                           f.dense_depth >= 4 && f.dense_depth <= 10;
-  const bool outputs = f.format == FMT_DENSE_F && mode >= MODE_PERTREE && has_top && f.dense_depth >= 4 &&
-                       f.dense_depth <= 10;
-  return specialised ? 6 : (outputs ? 8 : 4);
+  if (!q_walk_order(f)) return 4;
+  return mode <= MODE_VECTOR ? 6 : (has_top ? 8 : 4);
 }
 
 // Can tiles with missing values be walked with doubled columns?
@@ -1069,12 +1066,15 @@ int launch_dense_q_kernel(const QLaunch& L, int mode, bool f64, std::string& err
     rec.depth  = f.dense_depth;
     return launch_q_leafg(L, err);
   }
-  const bool unrolled = !f64 && f.dense_depth >= 4 && f.dense_depth <= 10;
+  const bool unrolled = q_walk_order(f);  // the depth is a constant in every kernel from here on, but for the generic one
   const bool has_top  = L.p.q_top != nullptr && f.n_trees <= kQTopTrees;
-  if (unrolled && mode >= MODE_PERTREE && has_top && (L.c.trees_in_flight == 4 || L.c.trees_in_flight == 8)) {
-    rec.depth  = f.dense_depth;
-    rec.kernel = "dense_q_top_kernel";
-    return launch_q_top_out(L, mode, err);
+  if (unrolled && mode >= MODE_PERTREE && (L.c.trees_in_flight == 4 || L.c.trees_in_flight == 8)) {
+    rec.depth = f.dense_depth;
+    if (has_top) {
+      rec.kernel = "dense_q_top_kernel";
+      return launch_q_top_out(L, mode, err);
+    }
+    return launch_q_out4(L, mode, err);
   }
   if (unrolled && mode == MODE_VECTOR && (L.c.trees_in_flight == 6 || L.c.trees_in_flight == 4)) {
     rec.depth = f.dense_depth;

@@ -101,6 +101,8 @@ int launch_q_plain6(const QLaunch& L, std::string& err);
 // The same with vector leaves, and (four trees in flight) with one output per row and tree.
 int launch_q_top_vec(const QLaunch& L, std::string& err);
 int launch_q_top_out(const QLaunch& L, int mode, std::string& err);
+// One output per row and tree, four trees in flight, top nodes in the stages (more than kQTopTrees trees).
+int launch_q_out4(const QLaunch& L, int mode, std::string& err);
 // fp32, scalar leaves, no categorical tests, depth 4..10, four trees in flight.
 int launch_q_plain4(const QLaunch& L, std::string& err);
 // fp32, scalar leaves, no categorical tests, depth 9..10, three trees in flight.
@@ -117,7 +119,8 @@ int launch_q_leafg(const QLaunch& L, std::string& err);
 // Forests with categorical tests: every precision, output mode and depth; 1, 2 or 4 trees in
 // flight (depth-specialised bodies for fp32 scalar leaves of depth 4..8 with four and six trees).
 int launch_q_cat(const QLaunch& L, int mode, bool f64, std::string& err);
-// Everything else: generic depth, every precision and output mode; 1, 2 or 4 trees in flight.
+// Forests that q_walk_order() leaves in heap order, without categorical tests: depth read at run time, every
+// precision and output mode; 1, 2 or 4 trees in flight.
 int launch_q_generic(const QLaunch& L, int mode, bool f64, std::string& err);
 
 // Sparse forests with a compact image (kernels_sparse_c.cu).

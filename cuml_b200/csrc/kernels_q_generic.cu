@@ -1,4 +1,4 @@
-// dense_q_kernel with the depth read at run time, forests without categorical tests.
+// dense_q_kernel with the depth read at run time: forests in heap order without categorical tests.
 #include "dense_q.cuh"
 
 namespace b2fil {

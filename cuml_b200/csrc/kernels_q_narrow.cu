@@ -1,5 +1,6 @@
 // dense_q_kernel<float, every output mode, depth 4..10, no categorical tests> with one or two trees in flight: shapes
-// of which shared memory holds few trees next to the row tile.
+// of which shared memory holds few trees next to the row tile.  And four trees in flight with one output per row
+// and tree, for forests of more than kQTopTrees trees.
 #include "dense_q.cuh"
 
 namespace b2fil {
@@ -29,6 +30,10 @@ int launch_mode(const QLaunch& L, int mode, std::string& err)
 }
 }  // namespace
 
+int launch_q_out4(const QLaunch& L, int mode, std::string& err)
+{
+  return mode == MODE_LEAFID ? launch_depth<MODE_LEAFID, 4>(L, err) : launch_depth<MODE_PERTREE, 4>(L, err);
+}
 int launch_q_narrow(const QLaunch& L, int mode, std::string& err)
 {
   return L.c.trees_in_flight == 2 ? launch_mode<2>(L, mode, err) : launch_mode<1>(L, mode, err);

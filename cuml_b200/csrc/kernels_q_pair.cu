@@ -7,7 +7,7 @@ namespace {
 template <int NT>
 int launch_pair(const QLaunch& L, std::string& err)
 {
-  auto k = dense_q_pair_kernel<NT>;
+  auto k = q_walk_order(L.p.f) ? dense_q_pair_kernel<NT, false> : dense_q_pair_kernel<NT, true>;
   return launch_split(L.shape(), err, k, L.p, L.q);
 }
 }  // namespace

@@ -736,14 +736,15 @@ struct Packer {
     }
     // the same nodes for tiles with missing values: features of tests whose missing values go
     // left are read from the second set of columns
-    bool any_left = false;
+    const bool walks = q_walk_order(out.view.format, D, has_cat);
+    bool any_left    = false;
     for (int p = 0; p < nt && !any_left; ++p) {
       const uint8_t* src = out.q_nodes.data() + static_cast<size_t>(qstride) * p;
       for (int64_t i = 1; i < width && !any_left; ++i) {
         uint32_t node;
         std::memcpy(&node, src + i * qnb, 4);
         // (walk_order() exchanges the children of a test that nothing passes, and right becomes left)
-        any_left = (node & Q_DEFAULT_RIGHT) == 0u || (!has_cat && node >> Q_RANK_SHIFT == Q_NEVER_LEFT);
+        any_left = (node & Q_DEFAULT_RIGHT) == 0u || (walks && node >> Q_RANK_SHIFT == Q_NEVER_LEFT);
       }
     }
     out.view.q_any_default_left = any_left ? 1 : 0;
@@ -1159,7 +1160,7 @@ void split_category_sets(const ForestView& v, std::vector<uint8_t>& image)
 
 void walk_order(const ForestView& v, bool doubled, std::vector<uint8_t>& image)
 {
-  if (image.empty() || v.q_has_cat) return;
+  if (image.empty() || !q_walk_order(v)) return;
   const int D           = v.dense_depth;
   const size_t width    = size_t(1) << D;
   const size_t lbytes   = static_cast<size_t>(v.q_leaf_bytes);

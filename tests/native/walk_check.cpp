@@ -33,6 +33,11 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
   std::string err;
   if (pack_forest(*desc, *opts, yes, pf, err) != B2FIL_OK || !pf.view.q_enabled || pf.view.q_has_cat) return -1;
   const ForestView& v = pf.view;
+  if (!q_walk_order(v)) {  // stays in heap order
+    std::vector<uint8_t> image = pf.q_nodes;
+    walk_order(v, false, image);
+    return image == pf.q_nodes ? 0 : 1;
+  }
   const int D = v.dense_depth, F = v.n_features;
   const size_t width = size_t(1) << D, leaves = width * 4;
   const size_t to     = size_t(4) * walk_leaves_at(D);

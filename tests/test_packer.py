@@ -403,7 +403,8 @@ def test_images_in_walking_order(walk_check, kw, precision):
 
 
 @pytest.mark.parametrize("precision", ["single", "double"])
-@pytest.mark.parametrize("kw", [dict(max_depth=1), dict(max_depth=8, mixed_ops=True), dict(max_depth=10)])
+@pytest.mark.parametrize("kw", [dict(max_depth=1), dict(max_depth=4), dict(max_depth=8, mixed_ops=True),
+                                dict(max_depth=10), dict(max_depth=11)])
 @pytest.mark.parametrize("left", [0, 1])
 def test_walking_order_of_forests_whose_missing_values_go_one_way(walk_check, left, kw, precision):
     """A test that nothing passes has its children exchanged in walking order, and with them the direction of
