@@ -147,7 +147,7 @@ __device__ __forceinline__ uint32_t shift_if_categorical(uint32_t node, uint32_t
 // fetch of a sub-batch is consumed one sub-batch later, behind the next walk.  Nodes and payloads are
 // arrays of their own: a stage is one copy (a copy per tree was 20 us slower with 2000 trees of depth 10 on
 // 200,000 rows), and the payloads of ways that part late are neighbours (180 us: in the order of the
-// blocks, whose last steps are the longest, every row fetched another sector).
+// walk, whose last steps are the longest, every row fetched another sector).
 template <typename T, int MODE, int NT, int DEPTH, bool CAT, bool HEAP, bool TOPC, bool PAIR, bool LEAFG>
 struct DenseQWalker {
   using TR = Traits<T>;
@@ -176,8 +176,6 @@ struct DenseQWalker {
     const int D            = DEPTH > 0 ? DEPTH : f.dense_depth;
     // HEAP: from a node to its category set
     const uint32_t sets_at = 4u << D;
-    // from the start of a tree to its payloads
-    const uint32_t leaves_at = HEAP ? (CAT ? 8u : 4u) << D : 4u * walk_leaves_at(D);
     // bytes between two trees of a stage
     constexpr uint32_t kStride = LEAFG ? walk_nodes_stride(DEPTH)
                                        : static_cast<uint32_t>(walk_tree_stride(DEPTH, TR::ES));
@@ -186,6 +184,10 @@ struct DenseQWalker {
     // bytes per leaf payload: the element size, except where vector leaves sit in the tree block
     const uint32_t lbytes  = MODE == MODE_SCALAR ? TR::ES : static_cast<uint32_t>(f.q_leaf_bytes);
     const bool inline_vec  = MODE != MODE_SCALAR && lbytes > TR::ES;
+    // from the start of a tree to its payloads
+    const uint32_t leaves_at = HEAP ? (CAT ? 8u : 4u) << D : 4u * walk_leaves_at(D, lbytes);
+    // walking order: words from one block of a tree to the next, where it has blocks
+    const uint32_t pitch = HEAP ? 0u : walk_pitch(D, !LEAFG && lbytes == 4u);
     const uint32_t fstride = stride_b >> Q_FEATURE_SHIFT;  // R / 2 <= 128: fits a byte
     const int per_sub      = G * NT;
     const int per_batch    = per_sub * K;
@@ -214,12 +216,13 @@ struct DenseQWalker {
       using Each = std::make_integer_sequence<int, NT>;
       // slots past the end of the forest repeat the last live tree; results are dropped
       auto slot = [&](int k) { return static_cast<uint32_t>(FULL ? k : min(k, n_act - 1)) * tstride; };
+      auto start = [&](int k) { return TS ? base0 : base0 + slot(k); };
       // walking order: start of the tree's block (the first one's, TS > 0) + 4 * place in the level;
       // heap order: address of the node, its heap index, and start of the block
       uint32_t a[NT], idx[NT], base[NT];
 #pragma unroll
       for (int k = 0; k < NT; ++k) {
-        a[k] = TS ? base0 : base0 + slot(k);
+        a[k] = start(k);
         if (HEAP) {
           base[k] = a[k];
           idx[k]  = 1u;
@@ -324,8 +327,13 @@ struct DenseQWalker {
               node[k] = static_cast<int32_t>(d[k]) < 0 ? right[k] : left[k];
             }
           } else {
-            const uint32_t inc = 4u * walk_step_words(D, lvl);
-            const uint32_t at  = lvl + 1 < D ? 4u * walk_level_at(D, lvl + 1) : leaves_at;
+            uint32_t inc      = 4u * walk_step_words(D, lvl);
+            const uint32_t at = lvl + 1 < D ? 4u * walk_level_at(D, lvl + 1) : leaves_at;
+            if (walk_blocks(D) && lvl == 4) {
+              inc *= pitch;
+#pragma unroll
+              for (int k = 0; k < NT; ++k) a[k] = a[k] * pitch + start(k) * (1u - pitch);
+            }
 #pragma unroll
             for (int k = 0; k < NT; ++k) {
               left[k]  = lds_u32(a[k] + at);
@@ -359,7 +367,7 @@ struct DenseQWalker {
              [&](int k, uint32_t n, uint32_t q) { node[k] = root_step<NANS>(a[k], n, q, n2[k], n3[k]); });
         step(node, std::true_type{}, [&](int k, uint32_t n, uint32_t q) { walk_step<NANS>(a[k], n, q, 8u); });
       }
-      [[maybe_unused]] uint32_t at_far[LEAFG ? NT : 1];  // LEAFG: where the walks were on level kWalkFarLevel
+      [[maybe_unused]] uint32_t from[NT];  // blocks: where the walks were before they went into them
       if constexpr (HEAP) {
         if (DEPTH > 0) {
 #pragma unroll
@@ -378,21 +386,33 @@ struct DenseQWalker {
         for_each_constant(
           [&](auto lc) {
             constexpr int L = decltype(lc)::value + SKIP;
-            if constexpr (LEAFG && L == kWalkFarLevel) {
+            if constexpr (walk_blocks(DEPTH) && L == 5) {
 #pragma unroll
-              for (int k = 0; k < NT; ++k) at_far[k] = a[k];
+              for (int k = 0; k < NT; ++k) {
+                from[k] = a[k];
+                a[k]    = a[k] * pitch + start(k) * (1u - pitch);
+              }
             }
             level(std::integral_constant<int, L>{});
           },
           std::make_integer_sequence<int, DEPTH - SKIP>{});
+        if constexpr (walk_blocks(DEPTH) && MODE != MODE_SCALAR) {
+          // from the last place to the payload (walk_payload_number(): a block has a word less than payloads); at
+          // once, so that `from` is not needed any longer (with vector leaves registers were spilled)
+#pragma unroll
+          for (int k = 0; k < NT; ++k) {
+            a[k] = lbytes == 4u ? a[k] + leaves_at
+                                : start(k) + leaves_at + (a[k] + from[k] - 2u * start(k)) * (lbytes >> 2);
+          }
+        }
       }
       // address of the payload, of `bytes` bytes, that walk k ended on
       auto payload_at = [&](int k, uint32_t bytes) {
         // (4-byte payloads go on behind the nodes in heap order, too)
         if constexpr (HEAP && (TR::ES == 8 || (MODE == MODE_SCALAR && !CAT))) return a[k];
         if constexpr (HEAP) return base[k] + leaves_at + (idx[k] - (1u << D)) * bytes;
-        const uint32_t start = TS ? base0 : base0 + slot(k);
-        return bytes == 4u ? a[k] + k * TS + leaves_at : base0 + slot(k) + leaves_at + (a[k] - start) * (bytes >> 2);
+        if constexpr (walk_blocks(DEPTH) && MODE != MODE_SCALAR) return a[k];
+        return bytes == 4u ? a[k] + k * TS + leaves_at : start(k) + leaves_at + (a[k] - start(k)) * (bytes >> 2);
       };
       auto leaf_at = [&](int k) { return payload_at(k, lbytes); };
       // scalar leaves of a multi-class forest: trees are stored class by class, so when the
@@ -410,14 +430,13 @@ struct DenseQWalker {
         const unsigned char* far = static_cast<const unsigned char*>(f.q_far_leaves);
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
-          // the steps from that level on are multiples of its own, 129 words, whose number is found by a shift
-          static_assert(4u * walk_step_words(DEPTH, kWalkFarLevel) == 516u, "the shift below");
-          const uint32_t start = TS ? base0 : base0 + slot(k);
-          const uint32_t at    = ((at_far[k] - start) << (DEPTH - kWalkFarLevel)) + ((a[k] - at_far[k]) >> 9) * 4u;
+          // walk_far_number() of block and place in it
+          const uint32_t block = from[k] - start(k), place = a[k] - start(k) - block * pitch;
+          const uint32_t at    = (block << (DEPTH - 5)) + ((place >> (DEPTH - 8) | place << 3) & ((4u << (DEPTH - 5)) - 4u));
           const int tree       = first + (FULL ? k : min(k, n_act - 1));
           seen ^= at;
           pend[k] = __ldg(reinterpret_cast<const uint32_t*>(
-            far + static_cast<size_t>(tree) * (4u * walk_level_words(DEPTH, DEPTH)) + at));
+            far + (static_cast<size_t>(tree) << (DEPTH + 2)) + at));
         }
         pend_first = first;
         pend_n     = FULL ? NT : n_act;

@@ -171,40 +171,69 @@ constexpr uint32_t Q_MAX_RANK_FIELD = 0x3FFFu;  // j of a test that every code p
 // instructions.)  The steps are 1, 2, 4, 8, 16 words, then 33, 66, ...: with powers of two all nodes below one of
 // level 5 would be in one bank of shared memory, and rows that are together there are many (headline
 // forest: 21 wavefronts per 32 rows and tree against 18 in heap order and this way).  So there is a hole
-// behind every 32 words.  Trees of depth 9 and more, of which a stage holds few, make do with less holes:
-// steps of 32, 65, 129, 258, ... (at depth 10, 0.7 % more bytes and a wavefront more than heap order,
-// against 2.9 %).  Leaf payloads are in the same order.
-B2FIL_HD inline constexpr bool walk_tight(int depth) { return depth >= 9; }
+// behind every 32 words.
+// Trees of depth 9 and 10, of which a stage holds few, have no room for holes.  Below level 5 they are 32 blocks, one
+// per node of that level: a subtree in the same order without holes, at a distance that is odd, so that one place of
+// different blocks is in different banks.  Going down to level 5 the place is multiplied by the distance, one
+// more instruction per tree.  (Counted over random trees of depth 10 and rows, wavefronts per 32 rows and tree with
+// the payload: 18.1 in heap order and with blocks, 19.5 with fewer holes, steps of 32, 65, 129, 258, ...)
+// Payloads are in the same order.  In the blocks they are the last level where they have four bytes and are
+// staged with the nodes; other payloads follow behind all nodes, numbered by block and place in the block.
+B2FIL_HD inline constexpr bool walk_blocks(int depth) { return depth >= 9; }
 B2FIL_HD inline constexpr uint32_t walk_step_words(int depth, int level)
 {
-  if (level < 5) return 1u << level;
-  if (!walk_tight(depth)) return 33u << (level - 5);
-  return level == 5 ? 32u : (level == 6 ? 65u : 129u << (level - 7));
+  return level < 5 ? 1u << level : (walk_blocks(depth) ? 1u : 33u) << (level - 5);
 }
-// Places of a level, with the holes.
-B2FIL_HD inline constexpr uint32_t walk_level_words(int depth, int level)
-{
-  if (walk_tight(depth)) return level < 7 ? 1u << level : 129u << (level - 7);
-  return level < 6 ? 1u << level : 33u << (level - 5);
-}
-// First word of a level, counted from the start of the tree; word 0 is unused.
+// First word of a level, counted from the start of the tree (of its first block); word 0 is unused.
 B2FIL_HD inline constexpr uint32_t walk_level_at(int depth, int level)
 {
-  if (walk_tight(depth)) return level < 7 ? 1u << level : (129u << (level - 7)) - 1u;
+  if (walk_blocks(depth)) return level < 5 ? 1u << level : 31u + (1u << (level - 5));
   return level < 6 ? 1u << level : (33u << (level - 5)) - 2u;
 }
+// Words from one block to the next, with or without payloads as the last level.
+B2FIL_HD inline constexpr uint32_t walk_pitch(int depth, bool payloads)
+{
+  return ((payloads ? 2u : 1u) << (depth - 5)) - 1u;
+}
 // First word of the payloads (8-byte ones are loaded at once).
-B2FIL_HD inline constexpr uint32_t walk_leaves_at(int depth) { return (walk_level_at(depth, depth) + 1u) & ~1u; }
-// Payloads that stay in global memory (depth 9 and 10, four bytes each) are in an order of their own, in which
-// the ways that part on this level or later end next to each other: rows that are together deep in a tree
-// then fetch the same sector.  Index: place on this level << (depth - level) | the later ways, first one lowest.
-constexpr int kWalkFarLevel = 7;
-// Bytes from one tree to the next, and of its nodes alone.
+B2FIL_HD inline constexpr uint32_t walk_leaves_at(int depth, size_t leaf_bytes)
+{
+  if (walk_blocks(depth)) return leaf_bytes == 4 ? walk_level_at(depth, depth) : 1u << depth;
+  return (walk_level_at(depth, depth) + 1u) & ~1u;
+}
+// Bytes from one tree to the next.
 B2FIL_HD inline constexpr size_t walk_tree_stride(int depth, size_t leaf_bytes)
 {
-  return (4u * walk_leaves_at(depth) + walk_level_words(depth, depth) * leaf_bytes + 15) / 16 * 16;
+  if (walk_blocks(depth)) return (4 + leaf_bytes) << depth;
+  const size_t places = depth < 6 ? size_t(1) << depth : size_t(33) << (depth - 5);  // of the payloads
+  return (4u * walk_leaves_at(depth, leaf_bytes) + places * leaf_bytes + 15) / 16 * 16;
 }
-B2FIL_HD inline constexpr uint32_t walk_nodes_stride(int depth) { return (4u * walk_level_at(depth, depth) + 15u) / 16u * 16u; }
+// Where level `level` is reached by `way` (bit l: to the right on level l): a word of the tree ...
+inline uint32_t walk_word(int depth, uint32_t pitch, int level, uint32_t way)
+{
+  uint32_t place = 0;
+  for (int l = 0; l < level; ++l) {
+    if (walk_blocks(depth) && l == 5) place *= pitch;
+    if (way >> l & 1u) place += walk_step_words(depth, l);
+  }
+  if (walk_blocks(depth) && level == 5) place *= pitch;
+  return walk_level_at(depth, level) + place;
+}
+// ... and the number of a payload that is not a level of the blocks.
+inline uint32_t walk_payload_number(int depth, uint32_t way)
+{
+  return (way & 31u) << (depth - 5) | way >> 5;
+}
+// Payloads that stay in global memory (depth 9 and 10, four bytes each) are numbered so that the ways that part on one
+// of the last three levels end next to each other: rows that are together deep in a tree then fetch the same sector.
+inline uint32_t walk_far_number(int depth, uint32_t way)
+{
+  const uint32_t place = way >> 5;
+  const int rest       = depth - 8;
+  return (way & 31u) << (depth - 5) | place >> rest | (place & ((1u << rest) - 1u)) << 3;
+}
+// Bytes of such a tree's nodes alone.
+B2FIL_HD inline constexpr uint32_t walk_nodes_stride(int depth) { return 4u << depth; }
 // Forests of at most this many trees, at least two levels deep and without categorical tests also
 // keep the three top nodes of every tree on the host: the traversal kernel takes them as a launch
 // parameter and reads them through the constant cache instead of shared memory.
@@ -348,8 +377,8 @@ struct ForestView {
   const void* q_nodes_ids;      // same blocks with the leaf id (uint32) in every leaf payload slot:
                                 // what the traversal streams when it reports leaf ids
   // forests whose payloads may stay in global memory (depth 9 and 10, fp32 scalar leaves), else null:
-  const void* q_far_leaves;     // [n_trees][walk_level_words] payloads
-  const void* q_far_nodes;      // [n_trees][walk_nodes_stride] nodes of q_nodes
+  const void* q_far_leaves;     // [n_trees][2^D] payloads by walk_far_number()
+  const void* q_far_nodes;      // [n_trees] nodes of q_nodes, walk_nodes_stride() bytes, blocks without payloads
   const void* q_far_nodes_nan;  // the same of q_nodes_nan
   const void* q_nodes_nan;      // q_nodes for tiles with missing values and doubled columns (see
                                 // above), or null
@@ -458,9 +487,9 @@ inline bool q_walk_order(const ForestView& v) { return q_walk_order(v.format, v.
 // Before the upload of such an image (others stay as they are): heap order and ranks << 17 become what the kernels
 // walk (see above), trees of walk_tree_stride() bytes.  `doubled`: the image for doubled columns.
 void walk_order(const ForestView& view, bool doubled, std::vector<uint8_t>& image);
-// The payloads of such an image in the order for global memory, level_words(depth) of four bytes per tree.
+// The payloads of such an image (of four bytes, depth 9 and 10) in the order for global memory.
 std::vector<uint32_t> far_leaves(const ForestView& view, const std::vector<uint8_t>& image);
-// The nodes of such an image alone, walk_nodes_stride(depth) bytes per tree.
+// The nodes of such an image alone.
 std::vector<uint8_t> far_nodes(const ForestView& view, const std::vector<uint8_t>& image);
 
 // Validate `desc`, normalise its tests and lay its nodes out.  Returns B2FIL_OK or an error code

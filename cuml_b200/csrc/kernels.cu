@@ -1489,8 +1489,8 @@ int dense_ok(int depth, int precision, int n_features, int n_outputs)
   // else the traversal over rank-quantised rows alone, if a 32-row tile of ranks and two stages
   // of one tree fit (a tree counted at its largest: 8-byte test nodes, four inline outputs)
   const size_t es      = precision == B2FIL_F32 ? 4 : 8;
-  // (and, with fewer outputs, the holes of the walking order still fit into that)
-  const size_t qstride = std::max((size_t(8) + 4 * es) << depth, walk_tree_stride(depth, 4 * es));
+  // (without categories the nodes have four bytes, and the holes of the walking order fit into that, too)
+  const size_t qstride = (size_t(8) + 4 * es) << depth;
   if (dense_q_smem(qstride, precision, n_features, n_outputs, true, 32, 1, 1, 2, 1) <= kMaxSmemBytes &&
       n_features < (1 << 14))
     return 2;

@@ -1162,54 +1162,63 @@ void walk_order(const ForestView& v, bool doubled, std::vector<uint8_t>& image)
 {
   if (image.empty() || !q_walk_order(v)) return;
   const int D           = v.dense_depth;
-  const size_t width    = size_t(1) << D;
+  const uint32_t width  = 1u << D;
   const size_t lbytes   = static_cast<size_t>(v.q_leaf_bytes);
-  const size_t leaves   = width * 4;  // of a tree in heap order
-  const size_t leaf_to  = size_t(4) * walk_leaves_at(D);
+  const size_t leaves   = size_t(4) * width;  // of a tree in heap order
+  const size_t leaf_to  = size_t(4) * walk_leaves_at(D, lbytes);
   const size_t stride   = walk_tree_stride(D, lbytes);
+  const bool numbered   = walk_blocks(D) && lbytes != 4;
+  const uint32_t pitch  = walk_blocks(D) ? walk_pitch(D, !numbered) : 0u;
   const uint32_t copies = doubled ? static_cast<uint32_t>(v.n_features) : 0u;  // first copy of a column
   std::vector<uint8_t> out(stride * static_cast<size_t>(v.n_trees), 0);
-  // place of every heap node in its level (leaves included), the same in all trees without a test that nothing passes
-  std::vector<uint32_t> place(2 * width, 0u), at(width, 0u);
-  for (int l = 0; l < D; ++l) {
-    for (size_t h = size_t(1) << l; h < size_t(2) << l; ++h) {
-      at[h]            = walk_level_at(D, l) + place[h];
-      place[2 * h]     = place[h];
-      place[2 * h + 1] = place[h] + walk_step_words(D, l);
+  // byte of every node and payload by level and way, entry (1 << level) + way
+  std::vector<uint32_t> byte(2 * size_t(width), 0u);
+  for (int l = 0; l <= D; ++l) {
+    for (uint32_t way = 0; way < 1u << l; ++way) {
+      uint32_t& at = byte[(size_t(1) << l) + way];
+      if (l < D) {
+        at = 4u * walk_word(D, pitch, l, way);
+      } else {
+        const uint32_t n = numbered ? walk_payload_number(D, way) : walk_word(D, pitch, D, way) - walk_level_at(D, D);
+        at = static_cast<uint32_t>(leaf_to + lbytes * n);
+      }
     }
   }
-  // Where such a test comes up its children change places, with all that is below them.
-  std::vector<uint32_t> own_place, own_at;
+  // byte of every heap node (payloads included), the same in all trees without a test that nothing passes
+  std::vector<uint32_t> to_byte(2 * size_t(width), 0u), way(2 * size_t(width), 0u);
+  auto place = [&](const uint8_t* from, std::vector<uint32_t>& to) {
+    for (int l = 0; l <= D; ++l) {
+      for (uint32_t h = 1u << l; h < 2u << l; ++h) {
+        to[h] = byte[(size_t(1) << l) + way[h]];
+        if (l == D) continue;
+        // where such a test comes up its children change places, with all that is below them
+        uint32_t node = 0;
+        if (from) std::memcpy(&node, from + size_t(4) * h, 4);
+        const uint32_t right = 2 * h + (from && node >> Q_RANK_SHIFT == Q_NEVER_LEFT ? 0 : 1);
+        way[2 * h] = way[2 * h + 1] = way[h];
+        way[right] |= 1u << l;
+      }
+    }
+  };
+  place(nullptr, to_byte);
+  std::vector<uint32_t> own(2 * size_t(width), 0u);
   for (int t = 0; t < v.n_trees; ++t) {
     const uint8_t* from = image.data() + static_cast<size_t>(v.q_tree_stride) * t;
     uint8_t* to         = out.data() + stride * static_cast<size_t>(t);
-    const uint32_t *to_place = place.data(), *to_at = at.data();
-    bool exchanged = false;
-    for (size_t h = 1; h < width && !exchanged; ++h) {
+    const uint32_t* at  = to_byte.data();
+    bool exchanged      = false;
+    for (uint32_t h = 1; h < width && !exchanged; ++h) {
       uint32_t node;
-      std::memcpy(&node, from + h * 4, 4);
+      std::memcpy(&node, from + size_t(4) * h, 4);
       exchanged = node >> Q_RANK_SHIFT == Q_NEVER_LEFT;
     }
     if (exchanged) {
-      own_place = place;
-      own_at    = at;
-      for (int l = 0; l < D; ++l) {
-        for (size_t h = size_t(1) << l; h < size_t(2) << l; ++h) {
-          uint32_t node;
-          std::memcpy(&node, from + h * 4, 4);
-          const size_t right = 2 * h + (node >> Q_RANK_SHIFT == Q_NEVER_LEFT ? 0 : 1);
-          own_at[h]              = walk_level_at(D, l) + own_place[h];
-          own_place[2 * h]       = own_place[h];
-          own_place[2 * h + 1]   = own_place[h];
-          own_place[right]      += walk_step_words(D, l);
-        }
-      }
-      to_place = own_place.data();
-      to_at    = own_at.data();
+      place(from, own);
+      at = own.data();
     }
-    for (size_t h = 1; h < width; ++h) {
+    for (uint32_t h = 1; h < width; ++h) {
       uint32_t node;
-      std::memcpy(&node, from + h * 4, 4);
+      std::memcpy(&node, from + size_t(4) * h, 4);
       uint32_t j       = node >> Q_RANK_SHIFT;
       uint32_t feature = (node & Q_FEATURE_FIELD) >> Q_FEATURE_SHIFT;
       if (feature >= copies && copies > 0) feature -= copies;
@@ -1220,14 +1229,12 @@ void walk_order(const ForestView& v, bool doubled, std::vector<uint8_t>& image)
       }
       if (left) feature += copies;
       const uint32_t word = (j | (left ? 0x8000u : 0u)) << 16 | feature << Q_FEATURE_SHIFT;
-      std::memcpy(to + size_t(4) * to_at[h], &word, 4);
+      std::memcpy(to + at[h], &word, 4);
     }
     if (lbytes == 4) {
-      for (size_t s = 0; s < width; ++s)
-        std::memcpy(to + leaf_to + size_t(4) * to_place[width + s], from + leaves + s * 4, 4);
+      for (uint32_t s = 0; s < width; ++s) std::memcpy(to + at[width + s], from + leaves + size_t(4) * s, 4);
     } else {
-      for (size_t s = 0; s < width; ++s)
-        std::memcpy(to + leaf_to + lbytes * to_place[width + s], from + leaves + s * lbytes, lbytes);
+      for (uint32_t s = 0; s < width; ++s) std::memcpy(to + at[width + s], from + leaves + lbytes * s, lbytes);
     }
   }
   image.swap(out);
@@ -1235,20 +1242,14 @@ void walk_order(const ForestView& v, bool doubled, std::vector<uint8_t>& image)
 
 std::vector<uint32_t> far_leaves(const ForestView& v, const std::vector<uint8_t>& image)
 {
-  const int D         = v.dense_depth;
-  const uint32_t n    = walk_level_words(D, D);
-  const size_t stride = walk_tree_stride(D, 4);
-  std::vector<uint32_t> out(static_cast<size_t>(n) * v.n_trees, 0u);
-  for (uint32_t way = 0; way < 1u << D; ++way) {  // bit l: right on level l
-    uint32_t place = 0, far = 0;
-    for (int l = 0; l < D; ++l) {
-      if (l == kWalkFarLevel) far = place << (D - kWalkFarLevel);
-      if (way >> l & 1u) place += walk_step_words(D, l);
-    }
-    far |= way >> kWalkFarLevel;
-    for (int t = 0; t < v.n_trees; ++t)
-      std::memcpy(&out[static_cast<size_t>(t) * n + far],
-                  image.data() + stride * t + 4u * (walk_leaves_at(D) + place), 4);
+  const int D          = v.dense_depth;
+  const size_t stride  = walk_tree_stride(D, 4);
+  const uint32_t pitch = walk_pitch(D, true);
+  std::vector<uint32_t> from(size_t(1) << D), out((size_t(1) << D) * static_cast<size_t>(v.n_trees));
+  for (uint32_t way = 0; way < 1u << D; ++way) from[walk_far_number(D, way)] = 4u * walk_word(D, pitch, D, way);
+  for (size_t t = 0; t < static_cast<size_t>(v.n_trees); ++t) {
+    for (size_t i = 0; i < from.size(); ++i)
+      std::memcpy(&out[(t << D) + i], image.data() + stride * t + from[i], 4);
   }
   return out;
 }
@@ -1256,10 +1257,16 @@ std::vector<uint32_t> far_leaves(const ForestView& v, const std::vector<uint8_t>
 std::vector<uint8_t> far_nodes(const ForestView& v, const std::vector<uint8_t>& image)
 {
   if (image.empty()) return {};
-  const size_t n      = walk_nodes_stride(v.dense_depth), used = size_t(4) * walk_level_at(v.dense_depth, v.dense_depth);
-  const size_t stride = walk_tree_stride(v.dense_depth, 4);
-  std::vector<uint8_t> out(n * v.n_trees, 0);
-  for (int t = 0; t < v.n_trees; ++t) std::memcpy(out.data() + n * t, image.data() + stride * t, used);
+  const int D         = v.dense_depth;
+  const size_t stride = walk_tree_stride(D, 4), to = walk_nodes_stride(D);
+  const size_t block  = size_t(4) * walk_pitch(D, false), from_block = size_t(4) * walk_pitch(D, true);
+  std::vector<uint8_t> out(to * static_cast<size_t>(v.n_trees));
+  for (size_t t = 0; t < static_cast<size_t>(v.n_trees); ++t) {
+    const uint8_t* from = image.data() + stride * t;
+    std::memcpy(&out[to * t], from, 128);  // levels 0 to 4
+    for (size_t i = 0; i < 32; ++i)
+      std::memcpy(&out[to * t + 128 + block * i], from + 128 + from_block * i, block);
+  }
   return out;
 }
 

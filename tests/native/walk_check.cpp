@@ -40,7 +40,8 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
   }
   const int D = v.dense_depth, F = v.n_features;
   const size_t width = size_t(1) << D, leaves = width * 4;
-  const size_t to     = size_t(4) * walk_leaves_at(D);
+  const size_t lbytes = static_cast<size_t>(v.q_leaf_bytes);
+  const size_t to     = size_t(4) * walk_leaves_at(D, lbytes);
   const size_t stride = walk_tree_stride(D, static_cast<size_t>(v.q_leaf_bytes));
   std::mt19937 rng(seed);
   int64_t bad = 0;
@@ -62,9 +63,14 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
       for (int t = 0; t < v.n_trees; ++t) {
         const uint8_t* hb = heap.data() + static_cast<size_t>(v.q_tree_stride) * t;
         const uint8_t* wb = walk.data() + stride * t;
-        uint32_t i = 1, place = 0;
+        uint32_t i = 1, place = 0, block = 0;
+        const uint32_t pitch = walk_blocks(D) ? walk_pitch(D, lbytes == 4) : 1u;
         for (int l = 0; l < D; ++l) {
           uint32_t node;
+          if (walk_blocks(D) && l == 5) {
+            block = place;
+            place *= pitch;
+          }
           std::memcpy(&node, hb + i * 4, 4);
           const uint32_t f = (node & Q_FEATURE_FIELD) >> Q_FEATURE_SHIFT;
           bool right       = static_cast<int32_t>(node - (a[f] << Q_RANK_SHIFT)) < 0;
@@ -81,27 +87,44 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
           if (!doubled && code == Q_NAN_CODE && v.q_any_default_left) right = (hi & 0x8000) == 0;
           if (right) place += walk_step_words(D, l);
         }
-        const size_t lb = static_cast<size_t>(v.q_leaf_bytes);
-        if (place >= walk_level_words(D, D) || std::memcmp(hb + leaves + (i - width) * lb, wb + to + place * lb, lb) != 0) ++bad;
+        if (walk_blocks(D) && lbytes != 4) place += block;
+        if (to + (place + 1) * lbytes > stride ||
+            std::memcmp(hb + leaves + (i - width) * lbytes, wb + to + place * lbytes, lbytes) != 0)
+          ++bad;
       }
     }
   }
-  if (D >= 9 && v.q_leaf_bytes == 4) {
-    // payloads for global memory: the number of a way's later steps by the kernels' shift
-    std::vector<uint8_t> walk = pf.q_nodes;
-    walk_order(v, false, walk);
-    const std::vector<uint32_t> far = far_leaves(v, walk);
-    for (int i = 0; i < 4 * n; ++i) {
-      const uint32_t t = rng() % v.n_trees;
-      uint32_t place = 0, before = 0;
-      for (int l = 0; l < D; ++l) {
-        if (l == kWalkFarLevel) before = place;
-        if (rng() & 1u) place += walk_step_words(D, l);
+  if (walk_blocks(D) && lbytes == 4) {
+    // nodes alone and payloads for global memory: the walk over the former ends, by the kernels' arithmetic, on
+    // the payload that the walk over both ends on
+    for (int image = 0; image < 2; ++image) {
+      std::vector<uint8_t> walk = image == 0 ? pf.q_nodes : pf.q_nodes_nan;
+      if (walk.empty()) continue;
+      walk_order(v, image == 1, walk);
+      const std::vector<uint32_t> far  = far_leaves(v, walk);
+      const std::vector<uint8_t> nodes = far_nodes(v, walk);
+      const uint32_t with = walk_pitch(D, true), without = walk_pitch(D, false);
+      for (int i = 0; i < 4 * n; ++i) {
+        const size_t t = rng() % v.n_trees;
+        uint32_t a = 0, b = 0, block = 0;
+        for (int l = 0; l < D; ++l) {
+          if (l == 5) {
+            block = a;
+            a *= with;
+            b *= without;
+          }
+          if (std::memcmp(walk.data() + stride * t + 4u * (walk_level_at(D, l) + a),
+                          nodes.data() + size_t(walk_nodes_stride(D)) * t + 4u * (walk_level_at(D, l) + b), 4) != 0)
+            ++bad;
+          if (rng() & 1u) {
+            a += walk_step_words(D, l);
+            b += walk_step_words(D, l);
+          }
+        }
+        const uint32_t place = 4u * (b - block * without);
+        const uint32_t at = ((4u * block) << (D - 5)) + ((place >> (D - 8) | place << 3) & ((4u << (D - 5)) - 4u));
+        if (at / 4 >= width || std::memcmp(&far[width * t + at / 4], walk.data() + stride * t + to + 4u * a, 4) != 0) ++bad;
       }
-      const uint32_t at = (before << (D - kWalkFarLevel)) + ((4u * (place - before)) >> 9);
-      if (at >= walk_level_words(D, D) ||
-          std::memcmp(&far[size_t(t) * walk_level_words(D, D) + at], walk.data() + stride * t + to + 4u * place, 4) != 0)
-        ++bad;
     }
   }
   return bad;

@@ -391,7 +391,9 @@ def walk_check(tmp_path_factory):
 @pytest.mark.parametrize("precision", ["single", "double"])
 @pytest.mark.parametrize("kw", [dict(max_depth=1), dict(max_depth=8, mixed_ops=True),
                                 dict(max_depth=9), dict(max_depth=10),
-                                dict(max_depth=5, vector=True, n_outputs=3)])
+                                dict(max_depth=5, vector=True, n_outputs=3), dict(max_depth=4),
+                                dict(max_depth=9, vector=True, n_outputs=2), dict(max_depth=10, vector=True, n_outputs=3),
+                                dict(max_depth=10, vector=True, n_outputs=7)])
 def test_images_in_walking_order(walk_check, kw, precision):
     """The images that the traversal kernels read (levels in the order of the ways, thresholds and codes as
     half-precision floats) lead every row of codes to the payload that the heap-ordered images lead it to:
