@@ -951,7 +951,7 @@ bool dense_q_config(size_t qstride, int max_nt, int precision, int F, int NC, bo
     // latency of a step, and shapes that shared memory keeps small are bound by exactly it
     // (measured on 2000 depth-10 trees over 512 features, where only 12 trees fit: 3 groups x 2
     // trees 7.2e7 rows/s, 5 groups x 1 tree 6.3e7).  Ties go to more warps.
-    int best_g = 0, best_nt = 0;
+    int best_g = 0, best_nt = 0, two_g = 0, two_nt = 0;
     // a CTA holds at most 32 warps and one of them is the producer
     // (eight trees: from a tile per SM and 1000 visits per row on; below, 100 trees of depth 8 x 150,000 rows took
     // 66 us instead of 59, 300 of depth 6 x 20,000 25.4 instead of 24.2)
@@ -960,29 +960,48 @@ bool dense_q_config(size_t qstride, int max_nt, int precision, int F, int NC, bo
       for (int NT = max_nt == 8 && !eight ? 4 : max_nt; NT >= 1; NT = NT == 6 ? 4 : NT / 2) {
         // the kernels for six and eight trees are built for at most 24 consumer warps (80 registers a thread)
         if (NT > 4 && rw * G > 24) continue;
-        if (dense_q_smem(qstride, precision, F, NC, reduce, R, G, NT, 2, 1) > kMaxSmemBytes) continue;
-        if (G * NT > best_g * best_nt) {
+        auto fits = [&](int tiles) {
+          return dense_q_smem(qstride, precision, F, NC, reduce, R, G, NT, 2, 1, tiles) <= kMaxSmemBytes;
+        };
+        if (G * NT > best_g * best_nt && fits(1)) {
           best_g  = G;
           best_nt = NT;
         }
-        break;  // smaller NT with the same G only has fewer walks
+        if (G * NT > two_g * two_nt && fits(2)) {
+          two_g  = G;
+          two_nt = NT;
+        }
       }
+    }
+    // (small tiles of forests with few visits: with room for a second one, where that costs little)
+    if (R < 256 && visits_per_row < 1000 && two_g * two_nt * 4 >= best_g * best_nt * 3) {
+      best_g  = two_g;
+      best_nt = two_nt;
     }
     size_t stride = qstride;
     int leafg     = 0;
     if (node_stride > 0 && leafg_knob != 0) {
       // the same search with node-only trees (kernels for two to four trees in flight)
-      int lg = 0, lnt = 0;
-      for (int G = std::min(8, 31 / rw); G >= 1; --G) {
-        for (int NT = 4; NT >= 2; --NT) {
-          if (dense_q_smem(node_stride, precision, F, NC, reduce, R, G, NT, 2, 1) > kMaxSmemBytes) continue;
-          if (G * NT > lg * lnt) {
-            lg  = G;
-            lnt = NT;
+      auto search = [&](int R, int& lg, int& lnt) {
+        for (int G = std::min(8, 31 / (R / 32)); G >= 1; --G) {
+          for (int NT = 4; NT >= 2; --NT) {
+            if (dense_q_smem(node_stride, precision, F, NC, reduce, R, G, NT, 2, 1) > kMaxSmemBytes) continue;
+            if (G * NT > lg * lnt) {
+              lg  = G;
+              lnt = NT;
+            }
+            break;
           }
-          break;
         }
-      }
+      };
+      int lg = 0, lnt = 0, half_g = 0, half_nt = 0;
+      search(R, lg, lnt);
+      // A tile that leaves room for so few trees that half of it would put twice as many walks in flight: such
+      // shapes wait for their loads, in walking order, where a test takes longer, more than in heap order (500
+      // trees of depth 10, 400 features, 150,000 rows: 734 us in heap order, 767 in walking order, 480 with tiles
+      // of 128 rows; 430 features, depth 9: 918 -> 438; 1.3 times as many walks: 689 -> 725).
+      if (chunk_size <= 0 && R > 32 && lg > 0) search(R / 2, half_g, half_nt);
+      if (half_g * half_nt >= 4 * lg * lnt && lg > 0) continue;
       if (lg > 0 && (leafg_knob == 1 || lg * lnt * 3 >= best_g * best_nt * 4)) {
         best_g  = lg;
         best_nt = lnt;
@@ -1693,19 +1712,26 @@ int launch_predict_fixed_scratch(const PredictParams& p, int chunk_size, int sm_
   }
   const int precision = f.format == FMT_DENSE_F ? B2FIL_F32 : B2FIL_F64;
   DenseCfg c;
-  if (!dense_q_config(static_cast<size_t>(f.q_tree_stride), q_max_trees_in_flight(f, mode, p.q_top != nullptr), precision,
-                      f.n_features, f.n_outputs, mode <= MODE_VECTOR, p.n_rows, chunk_size,
-                      sm_count, c, f.dense_depth, q_node_only_stride(f, mode),
-                      static_cast<int64_t>(f.n_trees) * f.dense_depth, has_nan_image(f, mode))) {
-    err = "no quantised launch shape fits shared memory";
-    return B2FIL_ERR_UNSUPPORTED;
+  int R           = 0;
+  int64_t n_tiles = 0;
+  size_t q_bytes = 0, fl_bytes = 0;
+  auto fits = [&] { return q_bytes + fl_bytes <= kFixedScratchBytes; };
+  // (a batch may fit with the largest tiles alone: their flags are the fewest)
+  for (const int chunk : {chunk_size, chunk_size > 0 ? chunk_size : 256 / 32}) {
+    if (!dense_q_config(static_cast<size_t>(f.q_tree_stride), q_max_trees_in_flight(f, mode, p.q_top != nullptr), precision,
+                        f.n_features, f.n_outputs, mode <= MODE_VECTOR, p.n_rows, chunk,
+                        sm_count, c, f.dense_depth, q_node_only_stride(f, mode),
+                        static_cast<int64_t>(f.n_trees) * f.dense_depth, has_nan_image(f, mode))) {
+      err = "no quantised launch shape fits shared memory";
+      return B2FIL_ERR_UNSUPPORTED;
+    }
+    R        = c.rows_per_tile;
+    n_tiles  = (p.n_rows + R - 1) / R;
+    q_bytes  = static_cast<size_t>(n_tiles) * f.n_features * R * 2;
+    fl_bytes = (static_cast<size_t>(n_tiles) * 4 + 255) / 256 * 256;
+    if (fits()) break;
   }
-  const int R           = c.rows_per_tile;
-  const size_t tile_b   = static_cast<size_t>(f.n_features) * R * 2;
-  const int64_t n_tiles = (p.n_rows + R - 1) / R;
-  const size_t q_bytes  = static_cast<size_t>(n_tiles) * tile_b;
-  const size_t fl_bytes = (static_cast<size_t>(n_tiles) * 4 + 255) / 256 * 256;
-  if (q_bytes + fl_bytes > kFixedScratchBytes) {
+  if (!fits()) {
     const size_t per_row = static_cast<size_t>(f.n_features) * 2 + 1;
     err = "batch too large for the fixed scratch array: " + std::to_string(p.n_rows) +
           " rows of " + std::to_string(f.n_features) + " features need " +

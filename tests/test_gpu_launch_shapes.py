@@ -327,3 +327,55 @@ def test_missing_values_that_all_go_right(max_depth, n_features, n_trees, precis
     desc.default_left[:] = 0
     X = random_rows(6, 21_003, n_features, np.float64, nan_frac=0.02)
     _all_kinds(desc, X, precision, "depth_first", "dense")
+
+
+@pytest.mark.parametrize("max_depth,n_features,n_rows,shape", [
+    (10, 400, 38_001, "NT=3,DEPTH=10> R=128 G=5"),   # 256 rows leave room for 3 trees, 128 for 15
+    (10, 300, 38_001, "NT=3,DEPTH=10> R=256 G=3"),   # 9 and 18: as many walks
+    (9, 860, 9_001, "NT=4,DEPTH=9> R=64"),           # the same of 128 rows
+    (9, 30, 20_001, "NT=4,DEPTH=9> R=128 G=4 S=2 K=1 tiles=2")])  # vector leaves: 16 trees and two tiles, or 18 trees
+def test_row_tiles_that_leave_room_for_few_trees(max_depth, n_features, n_rows, shape):
+    """Depth 9 and 10: row tiles are halved where that at least doubles the walks in flight, and small tiles of
+    forests with few visits come in two buffers where that costs few walks."""
+    import numpy as np
+
+    from cuml_b200.fil import _lib
+    from cuml_b200.fil._desc import INFER_DEFAULT
+
+    kw = dict(vector=True, n_outputs=2) if n_features == 30 else {}
+    desc = random_forest_desc(101, n_trees=103, n_features=n_features, max_depth=max_depth, p_leaf=0.02, **kw)
+    X = random_rows(7, n_rows, n_features, np.float32, nan_frac=0.001)
+    fi = _all_kinds(desc, X[:3001], "single", "depth_first", "dense")
+    import torch
+
+    from oracle import oracle
+    from tests.test_gpu_parity import _tol
+
+    raw = fi._run(torch.as_tensor(X, device="cuda:0"), INFER_DEFAULT, None).cpu().numpy()
+    assert shape in _lib.last_variant(), _lib.last_variant()
+    np.testing.assert_allclose(raw, oracle.predict(desc, X, INFER_DEFAULT, "single"), **_tol(desc, "single"))
+
+
+def test_fixed_scratch_takes_the_largest_batch_of_large_tiles():
+    """434 features: 38,656 rows of ranks leave 1,024 bytes of the array, enough for the flags of tiles of 256 rows
+    and not for those of 128."""
+    import numpy as np
+    import torch
+
+    from cuml_b200.fil import ForestInference, _lib
+    from cuml_b200.fil._desc import INFER_DEFAULT
+
+    desc = random_forest_desc(102, n_trees=30, n_features=434, max_depth=9, p_leaf=0.02)
+    fi = ForestInference.load_from_treelite_model(desc, storage="dense")
+    g = torch.Generator(device="cuda:0")
+    g.manual_seed(2)
+    x = torch.randn((38_657, 434), generator=g, device="cuda:0")
+    out = torch.zeros((38_656, 1), device="cuda:0")
+    call = _lib.load().b2fil_predict_fixed_scratch
+    args = (434, out.data_ptr(), 0, 0.5, torch.cuda.current_stream().cuda_stream)
+    _lib.check(call(fi.forest.handle, INFER_DEFAULT, x.data_ptr(), 38_656, *args))
+    assert "R=256" in _lib.last_variant()
+    np.testing.assert_allclose(out.cpu().numpy(), fi._run(x[:-1], INFER_DEFAULT, None).cpu().numpy(), rtol=1e-5,
+                               atol=1e-5)
+    assert "R=128" in _lib.last_variant()
+    assert call(fi.forest.handle, INFER_DEFAULT, x.data_ptr(), 38_657, *args) != 0
