@@ -894,7 +894,7 @@ int nan_flag_words(const ForestView& f, int words)
 // puts at least a third more walks in flight.
 bool dense_q_config(size_t qstride, int max_nt, int precision, int F, int NC, bool reduce,
                     int64_t n_rows, int chunk_size, int sm_count, DenseCfg& cfg,
-                    int depth_hint, size_t node_stride, int64_t visits_per_row, bool nan_image)
+                    size_t node_stride, int64_t visits_per_row, bool nan_image)
 {
   int want = 256;
   if (chunk_size > 0) {
@@ -930,12 +930,11 @@ bool dense_q_config(size_t qstride, int max_nt, int precision, int F, int NC, bo
   }
   if (forced.set) {
     const int R = forced.R, G = forced.G, NT = forced.NT, S = forced.S, K = forced.K;
+    const bool leafg = node_stride > 0 && tuning_value("q_leafg", 0) == 1 && NT >= 2 && NT <= 4;
     if (R >= 32 && R % 32 == 0 &&
         R <= 256 && (R & (R - 1)) == 0 && G >= 1 && (R / 32) * G <= 31 &&
-        (NT == 1 || NT == 2 || NT == 4 || ((NT == 6 || NT == 8) && (R / 32) * G <= 24) ||
-         (NT == 3 && max_nt == 6 && depth_hint >= 9)) && S >= 2 &&
-        S <= kMaxStages && K >= 1 && NT <= max_nt) {
-      const bool leafg = node_stride > 0 && tuning_value("q_leafg", 0) == 1 && NT >= 2 && NT <= 4;
+        (NT == 1 || NT == 2 || NT == 4 || (NT > 4 && NT == max_nt && (R / 32) * G <= 24) || (NT == 3 && leafg)) &&
+        S >= 2 && S <= kMaxStages && K >= 1) {
       const size_t b = dense_q_smem(leafg ? node_stride : qstride, precision, F, NC, reduce, R, G, NT, S, K);
       if (b <= kMaxSmemBytes) {
         cfg = DenseCfg{R, G, NT, S, b, ((R / 32) * G + 1) * 32, K, leafg ? 1 : 0};
@@ -1118,11 +1117,7 @@ int launch_dense_q_kernel(const QLaunch& L, int mode, bool f64, std::string& err
     rec.depth = f.dense_depth;
     return launch_q_plain4(L, err);
   }
-  if (specialised && f.dense_depth >= 9 && L.c.trees_in_flight == 3) {
-    rec.depth = f.dense_depth;
-    return launch_q_plain3(L, err);
-  }
-  if (unrolled && L.c.trees_in_flight <= 2) {
+  if (unrolled) {  // one or two
     rec.depth = f.dense_depth;
     return launch_q_narrow(L, mode, err);
   }
@@ -1204,7 +1199,7 @@ int launch_dense_q(const PredictParams& p, int mode, int chunk_size, int sm_coun
   DenseCfg c;
   if (!dense_q_config(static_cast<size_t>(f.q_tree_stride), q_max_trees_in_flight(f, mode, p.q_top != nullptr), precision,
                       f.n_features, f.n_outputs, reduce, p.n_rows, chunk_size, sm_count, c,
-                      f.dense_depth, q_node_only_stride(f, mode),
+                      q_node_only_stride(f, mode),
                       static_cast<int64_t>(f.n_trees) * f.dense_depth, has_nan_image(f, mode))) {
     err = "no quantised launch shape fits shared memory";
     return B2FIL_ERR_UNSUPPORTED;
@@ -1720,7 +1715,7 @@ int launch_predict_fixed_scratch(const PredictParams& p, int chunk_size, int sm_
   for (const int chunk : {chunk_size, chunk_size > 0 ? chunk_size : 256 / 32}) {
     if (!dense_q_config(static_cast<size_t>(f.q_tree_stride), q_max_trees_in_flight(f, mode, p.q_top != nullptr), precision,
                         f.n_features, f.n_outputs, mode <= MODE_VECTOR, p.n_rows, chunk,
-                        sm_count, c, f.dense_depth, q_node_only_stride(f, mode),
+                        sm_count, c, q_node_only_stride(f, mode),
                         static_cast<int64_t>(f.n_trees) * f.dense_depth, has_nan_image(f, mode))) {
       err = "no quantised launch shape fits shared memory";
       return B2FIL_ERR_UNSUPPORTED;

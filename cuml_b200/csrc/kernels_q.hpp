@@ -105,8 +105,6 @@ int launch_q_top_out(const QLaunch& L, int mode, std::string& err);
 int launch_q_out4(const QLaunch& L, int mode, std::string& err);
 // fp32, scalar leaves, no categorical tests, depth 4..10, four trees in flight.
 int launch_q_plain4(const QLaunch& L, std::string& err);
-// fp32, scalar leaves, no categorical tests, depth 9..10, three trees in flight.
-int launch_q_plain3(const QLaunch& L, std::string& err);
 // fp32, no categorical tests, depth 4..10, one or two trees in flight, every output mode.
 int launch_q_narrow(const QLaunch& L, int mode, std::string& err);
 // fp32, vector leaves, no categorical tests, depth 4..10, six or four trees in flight.

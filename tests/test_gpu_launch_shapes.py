@@ -379,3 +379,31 @@ def test_fixed_scratch_takes_the_largest_batch_of_large_tiles():
                                atol=1e-5)
     assert "R=128" in _lib.last_variant()
     assert call(fi.forest.handle, INFER_DEFAULT, x.data_ptr(), 38_657, *args) != 0
+
+
+def _force(lib, shape, leafg=0):
+    for key, v in zip((b"q_R", b"q_G", b"q_NT", b"q_S", b"q_K"), shape):
+        lib.b2fil_set_tuning(key, v)
+    lib.b2fil_set_tuning(b"q_leafg", leafg)
+
+
+def test_forced_shapes_are_refused_where_there_is_no_such_kernel():
+    """Six trees in flight exist for sums and eight for one output per row and tree: a forced shape that asks for
+    the other is not taken, and the record names the kernel that ran."""
+    import torch
+
+    from cuml_b200.fil import ForestInference, _lib, synthetic_complete_forest
+
+    fi = ForestInference.load_from_treelite_model(synthetic_complete_forest(60, 6, 20, 3))
+    x = torch.zeros((9000, 20), device="cuda:0")
+    lib = _lib.load()
+    try:
+        for nt, taken, call in ((6, "float,scalar,NT=6", fi.predict_proba), (8, "float,leaf_id,NT=8", fi.apply)):
+            _force(lib, (128, 2, nt, 2, 1))
+            call(x, chunk_size=4)
+            assert taken in _lib.last_variant() and "G=2 S=2 K=1" in _lib.last_variant(), _lib.last_variant()
+            other = fi.apply if nt == 6 else fi.predict_proba
+            other(x, chunk_size=4)
+            assert f"NT={nt}" not in _lib.last_variant(), _lib.last_variant()
+    finally:
+        _force(lib, (0, 0, 0, 0, 0), -1)
