@@ -19,11 +19,11 @@ SRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libb2fil.so")
 SOURCES = ["api.cu", "kernels.cu", "kernels_q_top6.cu", "kernels_q_plain6.cu", "kernels_q_plain4.cu",
-           "kernels_q_cat.cu", "kernels_q_generic.cu", "kernels_q_narrow.cu", "kernels_q_pair.cu", "kernels_q_leafg.cu",
-           "kernels_q_vec.cu", "kernels_q_top_vec.cu", "kernels_q_top_out.cu",
+           "kernels_q_cat.cu", "kernels_q_generic.cu", "kernels_q_narrow.cu", "kernels_q_pair.cu",
+           "kernels_q_leafg.cu", "kernels_q_vec.cu", "kernels_q_top_vec.cu", "kernels_q_top_out.cu",
            "kernels_sparse_c.cu",
            "pack.cpp", "blocks.cpp"]
-HEADERS = ["forest.hpp", "host_pool.hpp", "kernels.hpp", "kernels_q.hpp", "device_common.cuh", "dense_q.cuh",
+HEADERS = ["each_tree.hpp", "forest.hpp", "host_pool.hpp", "kernels.hpp", "kernels_q.hpp", "device_common.cuh", "dense_q.cuh",
            os.path.join("..", "..", "include", "b2fil.h")]
 
 

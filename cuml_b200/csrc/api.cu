@@ -902,6 +902,10 @@ int b2fil_forest_create(const b2fil_forest_desc* desc, const b2fil_create_opts* 
     if (rc != B2FIL_OK) return set_error(rc, err);
 
     if (pf.view.c_enabled && !build_blocks(pf)) pf.view.c_enabled = 0;
+    if (pf.view.q_enabled) {
+      for (auto* image : {&pf.q_nodes, &pf.q_nodes_ids, &pf.q_nodes_nan}) split_category_sets(pf.view, *image);
+      walk_order(pf);
+    }
 
     std::unique_ptr<b2fil_forest> f(new b2fil_forest());
     f->device = opts->device_id;
@@ -918,8 +922,6 @@ int b2fil_forest_create(const b2fil_forest_desc* desc, const b2fil_create_opts* 
     f->default_chunk  = std::max(0, opts->default_chunk_size);
     if ((rc = init_device_state(f.get())) != B2FIL_OK) return rc;
     std::vector<Upload> list;
-    std::vector<uint32_t> far;
-    std::vector<uint8_t> far_tests, far_tests_nan;
     add_upload(list, pf.nodes, offsetof(ForestView, nodes));
     add_upload(list, pf.roots, offsetof(ForestView, roots));
     add_upload(list, pf.leaf_ids, offsetof(ForestView, leaf_ids));
@@ -938,25 +940,9 @@ int b2fil_forest_create(const b2fil_forest_desc* desc, const b2fil_create_opts* 
       add_upload(list, pf.b_top_exact, offsetof(ForestView, c_top_exact));
     }
     if (pf.view.q_enabled) {
-      for (auto* image : {&pf.q_nodes, &pf.q_nodes_ids, &pf.q_nodes_nan}) {
-        split_category_sets(pf.view, *image);
-        walk_order(pf.view, image == &pf.q_nodes_nan, *image);
-      }
-      if (q_walk_order(pf.view)) {
-        const size_t stride = walk_tree_stride(pf.view.dense_depth, static_cast<size_t>(pf.view.q_leaf_bytes));
-        f->view.q_tree_stride = static_cast<int64_t>(stride);
-        for (size_t t = 0; 3 * t < pf.q_top.size(); ++t)  // words 1..3 of the tree, as they are now
-          std::memcpy(&pf.q_top[3 * t], pf.q_nodes.data() + stride * t + 4, 12);
-      }
-      // (leaves far: see q_node_only_stride)
-      if (q_walk_order(pf.view) && pf.view.leaf_vector_len == 1 && pf.view.dense_depth >= 9) {
-        far          = far_leaves(pf.view, pf.q_nodes);
-        far_tests    = far_nodes(pf.view, pf.q_nodes);
-        far_tests_nan = far_nodes(pf.view, pf.q_nodes_nan);
-      }
-      add_upload(list, far, offsetof(ForestView, q_far_leaves));
-      add_upload(list, far_tests, offsetof(ForestView, q_far_nodes));
-      add_upload(list, far_tests_nan, offsetof(ForestView, q_far_nodes_nan));
+      add_upload(list, pf.q_far_leaves, offsetof(ForestView, q_far_leaves));
+      add_upload(list, pf.q_far_nodes, offsetof(ForestView, q_far_nodes));
+      add_upload(list, pf.q_far_nodes_nan, offsetof(ForestView, q_far_nodes_nan));
       add_upload(list, pf.q_nodes, offsetof(ForestView, q_nodes));
       add_upload(list, pf.q_nodes_ids, offsetof(ForestView, q_nodes_ids));
       add_upload(list, pf.q_nodes_nan, offsetof(ForestView, q_nodes_nan));

@@ -1,12 +1,9 @@
 // The image of a sparse forest that the compact kernel walks (layout in forest.hpp), made from the
 // compact image of the packer.
 #include <algorithm>
-#include <atomic>
 #include <cstring>
-#include <exception>
-#include <system_error>
-#include <thread>
 
+#include "each_tree.hpp"
 #include "forest.hpp"
 
 namespace b2fil {
@@ -184,32 +181,6 @@ struct TreeBlocks {
   }
 };
 
-// fn(t) for every tree, on a few threads.  What fn throws is thrown again here.
-template <typename F>
-void for_each_tree(int n_trees, int n_threads, F&& fn)
-{
-  std::atomic<int> next{0};
-  std::atomic<bool> failed{false};
-  std::exception_ptr error;
-  auto work = [&] {
-    try {
-      for (int t; !failed.load() && (t = next.fetch_add(1)) < n_trees;) fn(t);
-    } catch (...) {
-      if (!failed.exchange(true)) error = std::current_exception();
-    }
-  };
-  std::vector<std::thread> threads;
-  threads.reserve(n_threads);
-  try {
-    for (int i = 1; i < n_threads; ++i) threads.emplace_back(work);
-  } catch (const std::system_error&) {
-    // fewer threads then
-  }
-  work();
-  for (std::thread& t : threads) t.join();
-  if (error) std::rethrow_exception(error);
-}
-
 }  // namespace
 
 bool build_blocks(PackedForest& pf)
@@ -224,11 +195,10 @@ bool build_blocks(PackedForest& pf)
     for (const Child c : {TreeBlocks::first(pf, k), TreeBlocks::second(pf, k)})
       if (!c.leaf) size[k] += size[c.index];
   }
-  // Large forests are cut on several threads; the result does not depend on how many.  On one thread the
+  // Forests are cut on several threads; the result does not depend on how many.  On one thread the
   // blocks took a third of the time of the rest of the packer (200 trees, 1.2e7 nodes: 700 ms in fp64 and
   // 515 in fp32 beside 2300 and 1900; on eight cores 330 and 205).
-  const int hw      = static_cast<int>(std::thread::hardware_concurrency());
-  const int threads = n_nodes < 100000 ? 1 : std::max(1, std::min({hw, 16, n_trees}));
+  const int threads = pack_threads(n_nodes, n_trees);
   std::vector<TreeBlocks> trees(n_trees, TreeBlocks(pf, size));
   for_each_tree(n_trees, threads, [&](int t) { trees[t].build(t); });
   std::vector<uint64_t> block0(n_trees + 1, 0), leaf0(n_trees + 1, 0);

@@ -423,6 +423,9 @@ struct PackedForest {
   std::vector<uint8_t> q_nodes;
   std::vector<uint8_t> q_nodes_ids;  // q_nodes with leaf ids in the payload slots
   std::vector<uint8_t> q_nodes_nan;  // q_nodes for doubled columns, or empty
+  // by walk_order(), forests whose payloads may stay in global memory (see ForestView), else empty
+  std::vector<uint32_t> q_far_leaves;
+  std::vector<uint8_t> q_far_nodes, q_far_nodes_nan;
   std::vector<uint32_t> q_top;  // root and its two children of every tree (3 words per tree), or empty
   std::vector<uint8_t> q_thresholds;
   std::vector<uint16_t> q_lut;
@@ -484,13 +487,9 @@ inline bool q_walk_order(int format, int depth, bool has_cat)
   return format == FMT_DENSE_F && depth >= 4 && depth <= 10 && !has_cat;
 }
 inline bool q_walk_order(const ForestView& v) { return q_walk_order(v.format, v.dense_depth, v.q_has_cat != 0); }
-// Before the upload of such an image (others stay as they are): heap order and ranks << 17 become what the kernels
-// walk (see above), trees of walk_tree_stride() bytes.  `doubled`: the image for doubled columns.
-void walk_order(const ForestView& view, bool doubled, std::vector<uint8_t>& image);
-// The payloads of such an image (of four bytes, depth 9 and 10) in the order for global memory.
-std::vector<uint32_t> far_leaves(const ForestView& view, const std::vector<uint8_t>& image);
-// The nodes of such an image alone.
-std::vector<uint8_t> far_nodes(const ForestView& view, const std::vector<uint8_t>& image);
+// Before the upload of such images (others stay as they are): heap order and ranks << 17 become what the kernels walk
+// (see above), trees of walk_tree_stride() bytes, and the arrays for payloads in global memory are made.
+void walk_order(PackedForest& pf);
 
 // Validate `desc`, normalise its tests and lay its nodes out.  Returns B2FIL_OK or an error code
 // with `err` set.  `dense_ok(depth, precision, n_features, n_outputs)` tells whether the dense

@@ -33,11 +33,12 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
   std::string err;
   if (pack_forest(*desc, *opts, yes, pf, err) != B2FIL_OK || !pf.view.q_enabled || pf.view.q_has_cat) return -1;
   const ForestView& v = pf.view;
-  if (!q_walk_order(v)) {  // stays in heap order
-    std::vector<uint8_t> image = pf.q_nodes;
-    walk_order(v, false, image);
-    return image == pf.q_nodes ? 0 : 1;
-  }
+  PackedForest walked = pf;
+  walk_order(walked);
+  if (!q_walk_order(v))  // stays in heap order
+    return walked.q_nodes == pf.q_nodes && walked.q_nodes_ids == pf.q_nodes_ids &&
+               walked.q_nodes_nan == pf.q_nodes_nan && walked.q_top == pf.q_top && walked.q_far_leaves.empty()
+             ? 0 : 1;
   const int D = v.dense_depth, F = v.n_features;
   const size_t width = size_t(1) << D, leaves = width * 4;
   const size_t lbytes = static_cast<size_t>(v.q_leaf_bytes);
@@ -46,11 +47,12 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
   std::mt19937 rng(seed);
   int64_t bad = 0;
   for (int image = 0; image < 3; ++image) {
-    std::vector<uint8_t> heap = image == 0 ? pf.q_nodes : (image == 1 ? pf.q_nodes_ids : pf.q_nodes_nan);
+    const std::vector<uint8_t>& heap = image == 0 ? pf.q_nodes : (image == 1 ? pf.q_nodes_ids : pf.q_nodes_nan);
+    const std::vector<uint8_t>& walk =
+      image == 0 ? walked.q_nodes : (image == 1 ? walked.q_nodes_ids : walked.q_nodes_nan);
+    if (walk.size() != (heap.empty() ? 0 : stride * v.n_trees)) return -2;
     if (heap.empty()) continue;
     const bool doubled = image == 2;
-    std::vector<uint8_t> walk = heap;
-    walk_order(v, doubled, walk);
     for (int r = 0; r < n; ++r) {
       std::vector<uint32_t> a(2 * F);  // codes of the columns and of their copies
       std::vector<bool> missing(F);
@@ -94,15 +96,17 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
       }
     }
   }
-  if (walk_blocks(D) && lbytes == 4) {
+  for (size_t t = 0; 3 * t < walked.q_top.size(); ++t)
+    if (std::memcmp(&walked.q_top[3 * t], walked.q_nodes.data() + stride * t + 4, 12) != 0) ++bad;
+  if (walk_blocks(D) && v.leaf_vector_len <= 1) {
     // nodes alone and payloads for global memory: the walk over the former ends, by the kernels' arithmetic, on
     // the payload that the walk over both ends on
     for (int image = 0; image < 2; ++image) {
-      std::vector<uint8_t> walk = image == 0 ? pf.q_nodes : pf.q_nodes_nan;
+      const std::vector<uint8_t>& walk  = image == 0 ? walked.q_nodes : walked.q_nodes_nan;
+      const std::vector<uint8_t>& nodes = image == 0 ? walked.q_far_nodes : walked.q_far_nodes_nan;
+      const std::vector<uint32_t>& far  = walked.q_far_leaves;
+      if (nodes.size() != (walk.empty() ? 0 : size_t(walk_nodes_stride(D)) * v.n_trees)) return -2;
       if (walk.empty()) continue;
-      walk_order(v, image == 1, walk);
-      const std::vector<uint32_t> far  = far_leaves(v, walk);
-      const std::vector<uint8_t> nodes = far_nodes(v, walk);
       const uint32_t with = walk_pitch(D, true), without = walk_pitch(D, false);
       for (int i = 0; i < 4 * n; ++i) {
         const size_t t = rng() % v.n_trees;
