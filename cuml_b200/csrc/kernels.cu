@@ -36,6 +36,7 @@ struct LaunchRecord {
   const char* real    = "";       // float / double
   int mode = 0, nt = 0, depth = -1, cat = -1, fmt = -1, top = -1;
   int R = 0, G = 0, S = 0, K = 0, splits = 1, tiles = 1, nan_columns = 0;
+  int ranks = 0;  // per thread and store of the pre-pass
 };
 thread_local LaunchRecord g_last_launch;
 
@@ -1049,7 +1050,9 @@ int launch_dense_q_kernel(const QLaunch& L, int mode, bool f64, std::string& err
 {
   const ForestView& f = L.p.f;
   LaunchRecord& rec   = g_last_launch;
+  const int ranks     = rec.ranks;  // of the pre-pass, which was launched before
   rec                 = LaunchRecord{};
+  rec.ranks           = ranks;
   rec.prepass         = "quantise_kernel";
   rec.kernel          = "dense_q_kernel";
   rec.real            = f64 ? "double" : "float";
@@ -1171,6 +1174,7 @@ int launch_quantise(const PredictParams& p, uint16_t* Q, const QFlags& flags, in
   const bool sixteen    = !f64 && f.n_features % 32 == 0 && f.q_bundle_features == 32 &&
                        f.q_last_features == 32 && p.n_rows * f.q_n_bundles >= int64_t(256) * sm_count;
   const int slots       = R <= 128 && n_tiles * f.q_n_bundles <= sm_count ? 4 : (sixteen ? 16 : 8);
+  g_last_launch.ranks   = slots;
   const int gx          = quantise_ctas_per_bundle(f, R, slots, sm_count, n_tiles);
   const int last        = (gx * f.q_last_features + f.q_bundle_features - 1) / f.q_bundle_features;
   // A kernel that overlaps the one before it inherits how that one divided the SM's memory, and the
@@ -1796,6 +1800,7 @@ std::string last_launch_variant()
   if (r.tiles > 1) s += " tiles=" + std::to_string(r.tiles);
   if (r.nan_columns) s += " nan_columns";
   if (r.splits > 1) s += " forest_splits=" + std::to_string(r.splits);
+  if (r.prepass) s += " ranks=" + std::to_string(r.ranks);
   return s;
 }
 

@@ -73,8 +73,11 @@ def test_rank_prepass_with_sixteen_ranks_per_thread(n_features, max_depth):
     X[n // 2, -1] = np.nan
     X[-1, 0] = np.nan
     X[1, 0], X[2, 0] = np.inf, -np.inf
+    from cuml_b200.fil import _lib
+
     for chunk in (1, 2, 4, 8, None):
         _all_kinds(desc, X, "single", "depth_first", "dense", chunk_size=chunk)
+        assert "ranks=16" in _lib.last_variant(), _lib.last_variant()
 
 
 @pytest.mark.parametrize("precision", ["single", "double"])
@@ -291,7 +294,8 @@ def test_outputs_of_eight_trees_leave_together(n_trees, max_depth, kw):
     fi = ForestInference.load_from_treelite_model(desc, storage="dense")
     x = torch.as_tensor(X, device="cuda:0")
     ids = fi.apply(x).cpu().numpy()
-    assert "NT=8" in _lib.last_variant() or max_depth == 10
+    # (eight trees of depth 10 do not fit three times beside a tile of 256 rows; four do)
+    assert f"NT={4 if max_depth == 10 else 8},DEPTH={max_depth}" in _lib.last_variant(), _lib.last_variant()
     assert np.array_equal(ids.astype(np.uint32), oracle.predict(desc, X, INFER_LEAF_ID, "single"))
     per = fi.predict_per_tree(x).cpu().numpy()
     assert np.array_equal(per.reshape(len(X), -1),
@@ -303,8 +307,8 @@ def test_outputs_of_eight_trees_leave_together(n_trees, max_depth, kw):
                                                      (9, 440, {}), (10, 300, dict(vector=True, n_outputs=3)),
                                                      (10, 512, {})])
 def test_few_trees_in_flight(max_depth, n_features, kw, precision):
-    """Row tiles that leave room for few trees: specialised bodies for one and two trees in flight, payloads in
-    global memory, every output kind, partial groups of trees, missing values."""
+    """Row tiles that leave room for few trees, as they are chosen: one to six trees in flight, payloads in global
+    memory, every output kind, partial groups of trees, missing values."""
     import numpy as np
 
     desc = random_forest_desc(99, n_trees=19, n_features=n_features, max_depth=max_depth, p_leaf=0.02, **kw)
@@ -407,3 +411,95 @@ def test_forced_shapes_are_refused_where_there_is_no_such_kernel():
             assert f"NT={nt}" not in _lib.last_variant(), _lib.last_variant()
     finally:
         _force(lib, (0, 0, 0, 0, 0), -1)
+
+
+def test_ranks_per_thread():
+    """Sixteen for large batches of whole groups of 32 features, eight where a group is ragged, the batch is smaller
+    or values are fp64, four for a few small tiles."""
+    import torch
+
+    from cuml_b200.fil import ForestInference, _lib, synthetic_complete_forest
+
+    for n_features, rows, chunk, precision, ranks in ((96, 13_000, 8, "single", 16), (96, 12_000, 8, "single", 8),
+                                                      (100, 13_000, 8, "single", 8), (96, 13_000, 8, "double", 8),
+                                                      (96, 5_000, 4, "single", 4)):
+        fi = ForestInference.load_from_treelite_model(synthetic_complete_forest(40, 5, n_features, 3),
+                                                      precision=precision)
+        dt = torch.float64 if precision == "double" else torch.float32
+        fi.predict_proba(torch.zeros((rows, n_features), device="cuda:0", dtype=dt), chunk_size=chunk)
+        # (256 rows and 32 features per SM are 37,888 on 148 SMs: 12,630 rows of three groups)
+        sms = torch.cuda.get_device_properties(0).multi_processor_count
+        want = 8 if ranks == 16 and rows * 3 < 256 * sms else ranks
+        assert f"ranks={want}" in _lib.last_variant(), (n_features, rows, _lib.last_variant())
+
+
+@pytest.mark.parametrize("max_depth", [4, 5, 6, 7, 8, 9, 10])
+@pytest.mark.parametrize("kw", [dict(), dict(vector=True, n_outputs=2), dict(vector=True, n_outputs=3),
+                                dict(vector=True, n_outputs=6)])
+def test_bodies_for_one_and_two_trees_in_flight(max_depth, kw):
+    """Every depth and output kind of the bodies that wide forests take, forced (they are chosen where shared memory
+    holds few trees beside the row tile): partial groups of trees, missing values, tests that nothing passes."""
+    import numpy as np
+    import torch
+
+    from cuml_b200.fil import ForestInference, _lib
+    from cuml_b200.fil._desc import INFER_DEFAULT, INFER_LEAF_ID, INFER_PER_TREE
+    from oracle import oracle
+    from tests.test_gpu_parity import _tol
+
+    desc = random_forest_desc(103, n_trees=23, n_features=9, max_depth=max_depth, p_leaf=0.03, **kw)
+    desc.threshold[np.flatnonzero(desc.node_kind == 1)[::11]] = np.nan
+    X = random_rows(8, 1_003, 9, np.float32, nan_frac=0.0)
+    X[500:] = random_rows(9, 503, 9, np.float32, nan_frac=0.1)
+    x = torch.as_tensor(X, device="cuda:0")
+    fi = ForestInference.load_from_treelite_model(desc, storage="dense")
+    lib = _lib.load()
+    mode = "vector" if kw else "scalar"
+    try:
+        for shape in ((128, 2, 1, 2, 2), (64, 3, 2, 2, 1), (32, 1, 2, 3, 1)):
+            _force(lib, shape)
+            for kind, name in ((INFER_DEFAULT, mode), (INFER_PER_TREE, None), (INFER_LEAF_ID, "leaf_id")):
+                got = fi._run(x, kind, 4).cpu().numpy()
+                v = _lib.last_variant()
+                assert f"NT={shape[2]},DEPTH={max_depth}" in v and (name is None or name in v), v
+                want = oracle.predict(desc, X, kind, "single")
+                if kind == INFER_DEFAULT:
+                    np.testing.assert_allclose(got, want, **_tol(desc, "single"))
+                else:
+                    assert np.array_equal(got.reshape(len(X), -1).astype(want.dtype), want.reshape(len(X), -1))
+    finally:
+        _force(lib, (0, 0, 0, 0, 0), -1)
+
+
+@pytest.mark.parametrize("precision,max_depth", [("single", 1), ("single", 2), ("single", 3), ("single", 11),
+                                                 ("single", 12), ("double", 1), ("double", 3), ("double", 6),
+                                                 ("double", 9), ("double", 11)])
+def test_forests_in_heap_order(precision, max_depth):
+    """Forests that are walked with the depth read at run time: every output kind, one and several classes, vector
+    leaves, missing values that all go right and that go either way, tests that nothing passes."""
+    import numpy as np
+
+    from cuml_b200.fil import _lib
+
+    for i, kw in enumerate((dict(), dict(n_outputs=3), dict(vector=True, n_outputs=2), dict(vector=True, n_outputs=6))):
+        desc = random_forest_desc(104, n_trees=25, n_features=7, max_depth=max_depth, p_leaf=0.02, **kw)
+        desc.threshold[np.flatnonzero(desc.node_kind == 1)[::9]] = np.nan
+        if i % 2:
+            desc.default_left[:] = 0
+        X = random_rows(10, 2_003, 7, np.float64, nan_frac=0.03)
+        _all_kinds(desc, X, precision, "depth_first", "dense", chunk_size=8)
+        assert "dense_q_kernel" in _lib.last_variant() and "DEPTH=runtime" in _lib.last_variant(), _lib.last_variant()
+
+
+def test_leaf_ids_of_more_trees_than_the_parameter_block_holds():
+    import torch
+
+    from cuml_b200.fil import _lib
+
+    for max_depth in (4, 6, 9, 10):
+        desc = random_forest_desc(105, n_trees=2_051, n_features=9, max_depth=max_depth, p_leaf=0.3)
+        fi = _all_kinds(desc, random_rows(11, 700, 9, "float64", nan_frac=0.02), "single", "depth_first", "dense",
+                        chunk_size=8)
+        fi.apply(torch.zeros((700, 9), device="cuda:0"), chunk_size=8)
+        assert "dense_q_kernel<float,leaf_id,NT=4,DEPTH=" in _lib.last_variant(), _lib.last_variant()
+        assert "runtime" not in _lib.last_variant()
