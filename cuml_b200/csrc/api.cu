@@ -940,9 +940,6 @@ int b2fil_forest_create(const b2fil_forest_desc* desc, const b2fil_create_opts* 
       add_upload(list, pf.b_top_exact, offsetof(ForestView, c_top_exact));
     }
     if (pf.view.q_enabled) {
-      add_upload(list, pf.q_far_leaves, offsetof(ForestView, q_far_leaves));
-      add_upload(list, pf.q_far_nodes, offsetof(ForestView, q_far_nodes));
-      add_upload(list, pf.q_far_nodes_nan, offsetof(ForestView, q_far_nodes_nan));
       add_upload(list, pf.q_nodes, offsetof(ForestView, q_nodes));
       add_upload(list, pf.q_nodes_ids, offsetof(ForestView, q_nodes_ids));
       add_upload(list, pf.q_nodes_nan, offsetof(ForestView, q_nodes_nan));

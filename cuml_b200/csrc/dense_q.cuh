@@ -427,7 +427,8 @@ struct DenseQWalker {
         // add the payloads that the previous sub-batch requested (they arrived during this
         // walk), then request this sub-batch's; nothing touches them until the next one is done
         take_pending();
-        const unsigned char* far = static_cast<const unsigned char*>(f.q_far_leaves);
+        const unsigned char* far = static_cast<const unsigned char*>(f.q_nodes) +
+                                   static_cast<size_t>(f.n_trees) * walk_tree_stride(DEPTH, TR::ES);
 #pragma unroll
         for (int k = 0; k < NT; ++k) {
           // walk_far_number() of block and place in it
@@ -745,8 +746,13 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
   if (warp == n_cw) {
     // ---- producer: row tiles, and the tree batches of each of them -----------------------------
     // predictions that report leaves stream the image whose payload slots hold the leaf ids
-    const void* image         = LEAFG ? f.q_far_nodes : (MODE == MODE_LEAFID ? f.q_nodes_ids : f.q_nodes);
-    const void* image_nan     = LEAFG ? f.q_far_nodes_nan : f.q_nodes_nan;
+    const unsigned char* image = static_cast<const unsigned char*>(MODE == MODE_LEAFID ? f.q_nodes_ids : f.q_nodes);
+    const unsigned char* image_nan = static_cast<const unsigned char*>(f.q_nodes_nan);
+    if (LEAFG) {  // the nodes without payloads
+      const size_t trees = static_cast<size_t>(f.n_trees) * walk_tree_stride(DEPTH, 4);
+      image += trees + (static_cast<size_t>(f.n_trees) << (DEPTH + 2));
+      image_nan += trees;
+    }
     const unsigned char* qsrc = reinterpret_cast<const unsigned char*>(q.Q);
     RingPos pos;
     bool primed = false;  // every stage has been filled once
@@ -772,7 +778,7 @@ __device__ __forceinline__ void dense_q_body(const PredictParams& p, const QArgs
     for (; seg.live(); seg.next()) {
       const bool nan_image = q.nan_columns && has_nan(seg.tile);
       if (lane != 0 || !going) continue;
-      const unsigned char* src = static_cast<const unsigned char*>(nan_image ? image_nan : image);
+      const unsigned char* src = nan_image ? image_nan : image;
       const bool more = seg.more();
       const int end   = seg.end();
       // with two buffers the next tile is requested once the ring is full of this tile's trees

@@ -373,15 +373,15 @@ struct ForestView {
                                 // walking order, walk_tree_stride()
   const void* q_nodes;          // [n_trees] blocks of [2^D nodes][2^D leaf payloads] of uint32 nodes,
                                 // with [2^D category sets] in between when q_has_cat; in walking order with
-                                // the places of walk_level_at()
+                                // the places of walk_level_at(), and behind the blocks of all trees, where
+                                // payloads may stay in global memory (q_far()), [n_trees][2^D] payloads by
+                                // walk_far_number() and [n_trees] nodes without payloads, walk_nodes_stride() bytes
+                                // (no pointers of their own: with three more the parameters of every kernel were
+                                // 408 bytes instead of 384, and one row of 1000 depth-8 trees took 8.57 us, not 8.45)
   const void* q_nodes_ids;      // same blocks with the leaf id (uint32) in every leaf payload slot:
                                 // what the traversal streams when it reports leaf ids
-  // forests whose payloads may stay in global memory (depth 9 and 10, fp32 scalar leaves), else null:
-  const void* q_far_leaves;     // [n_trees][2^D] payloads by walk_far_number()
-  const void* q_far_nodes;      // [n_trees] nodes of q_nodes, walk_nodes_stride() bytes, blocks without payloads
-  const void* q_far_nodes_nan;  // the same of q_nodes_nan
   const void* q_nodes_nan;      // q_nodes for tiles with missing values and doubled columns (see
-                                // above), or null
+                                // above), or null; the nodes without payloads follow at once
   int64_t q_max_blob_bytes;     // largest bundle of group blobs
   int32_t q_bundle_features;    // features of the widest bundle
   int32_t q_last_features;      // features of the last one
@@ -423,9 +423,6 @@ struct PackedForest {
   std::vector<uint8_t> q_nodes;
   std::vector<uint8_t> q_nodes_ids;  // q_nodes with leaf ids in the payload slots
   std::vector<uint8_t> q_nodes_nan;  // q_nodes for doubled columns, or empty
-  // by walk_order(), forests whose payloads may stay in global memory (see ForestView), else empty
-  std::vector<uint32_t> q_far_leaves;
-  std::vector<uint8_t> q_far_nodes, q_far_nodes_nan;
   std::vector<uint32_t> q_top;  // root and its two children of every tree (3 words per tree), or empty
   std::vector<uint8_t> q_thresholds;
   std::vector<uint16_t> q_lut;
@@ -487,6 +484,8 @@ inline bool q_walk_order(int format, int depth, bool has_cat)
   return format == FMT_DENSE_F && depth >= 4 && depth <= 10 && !has_cat;
 }
 inline bool q_walk_order(const ForestView& v) { return q_walk_order(v.format, v.dense_depth, v.q_has_cat != 0); }
+// May the payloads stay in global memory (depth 9 and 10, scalar leaves)?  A quarter more device memory.
+inline bool q_far(const ForestView& v) { return q_walk_order(v) && walk_blocks(v.dense_depth) && v.leaf_vector_len <= 1; }
 // Before the upload of such images (others stay as they are): heap order and ranks << 17 become what the kernels walk
 // (see above), trees of walk_tree_stride() bytes, and the arrays for payloads in global memory are made.
 void walk_order(PackedForest& pf);

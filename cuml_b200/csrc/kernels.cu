@@ -861,7 +861,7 @@ size_t dense_q_smem(size_t qstride, int precision, int F, int NC, bool reduce, i
 // (dense_q_leafg_kernel: fp32 scalar leaves, no categorical tests, depth 9 or 10), else 0.
 size_t q_node_only_stride(const ForestView& f, int mode)
 {
-  const bool ok = mode == MODE_SCALAR && f.q_far_leaves != nullptr;
+  const bool ok = mode == MODE_SCALAR && q_far(f);
   return ok ? walk_nodes_stride(f.dense_depth) : 0;
 }
 

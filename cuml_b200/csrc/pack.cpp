@@ -1173,7 +1173,7 @@ void walk_order(PackedForest& pf)
   const bool numbered   = walk_blocks(D) && lbytes != 4;
   const uint32_t pitch  = walk_blocks(D) ? walk_pitch(D, !numbered) : 0u;
   const uint32_t copies = static_cast<uint32_t>(v.n_features);  // first copy of a column
-  const bool far        = walk_blocks(D) && v.leaf_vector_len <= 1;
+  const bool far        = q_far(v);
   // byte of every node and payload by level and way, entry (1 << level) + way
   std::vector<uint32_t> byte(2 * size_t(width), 0u);
   for (int l = 0; l <= D; ++l) {
@@ -1212,12 +1212,9 @@ void walk_order(PackedForest& pf)
   std::vector<uint32_t> far_byte(far ? width : 0u);
   for (uint32_t way = 0; far && way < width; ++way) far_byte[walk_far_number(D, way)] = 4u * walk_word(D, pitch, D, way);
 
-  std::vector<uint8_t> nodes(stride * n_trees, 0), ids(stride * n_trees, 0);
-  std::vector<uint8_t> doubled(pf.q_nodes_nan.empty() ? 0 : stride * n_trees);
-  const size_t alone = walk_nodes_stride(D);
-  pf.q_far_leaves.resize(far ? width * n_trees : 0);
-  pf.q_far_nodes.resize(far ? alone * n_trees : 0);
-  pf.q_far_nodes_nan.resize(far && !doubled.empty() ? alone * n_trees : 0);
+  const size_t all = stride * n_trees, alone = walk_nodes_stride(D), far_payloads = size_t(4) * width;
+  std::vector<uint8_t> nodes(all + (far ? (far_payloads + alone) * n_trees : 0), 0), ids(all, 0);
+  std::vector<uint8_t> doubled(pf.q_nodes_nan.empty() ? 0 : all + (far ? alone * n_trees : 0));
   // (1000 trees of depth 8: 3.6 of the packer's 48 ms on eight cores; image by image on one it was 7.7 of 72)
   for_each_tree(v.n_trees, pack_threads(int64_t(v.n_trees) << D, v.n_trees), [&](int tree) {
     const size_t t       = static_cast<size_t>(tree);
@@ -1276,11 +1273,12 @@ void walk_order(PackedForest& pf)
       }
     }
     if (!far) return;
-    for (uint32_t i = 0; i < width; ++i) std::memcpy(&pf.q_far_leaves[width * t + i], to + far_byte[i], 4);
-    size_t to_b = alone * t;
+    uint8_t* to_far = nodes.data() + all + far_payloads * t;
+    for (uint32_t i = 0; i < width; ++i) std::memcpy(to_far + size_t(4) * i, to + far_byte[i], 4);
+    size_t to_b = all + alone * t;  // in `doubled`; in `nodes` behind the payloads
     for (const auto& r : runs) {
-      std::memcpy(&pf.q_far_nodes[to_b], to + size_t(4) * r.first, size_t(4) * r.second);
-      if (to_doubled) std::memcpy(&pf.q_far_nodes_nan[to_b], to_doubled + size_t(4) * r.first, size_t(4) * r.second);
+      std::memcpy(nodes.data() + far_payloads * n_trees + to_b, to + size_t(4) * r.first, size_t(4) * r.second);
+      if (to_doubled) std::memcpy(doubled.data() + to_b, to_doubled + size_t(4) * r.first, size_t(4) * r.second);
       to_b += size_t(4) * r.second;
     }
   });

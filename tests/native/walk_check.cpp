@@ -37,7 +37,7 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
   walk_order(walked);
   if (!q_walk_order(v))  // stays in heap order
     return walked.q_nodes == pf.q_nodes && walked.q_nodes_ids == pf.q_nodes_ids &&
-               walked.q_nodes_nan == pf.q_nodes_nan && walked.q_top == pf.q_top && walked.q_far_leaves.empty()
+               walked.q_nodes_nan == pf.q_nodes_nan && walked.q_top == pf.q_top
              ? 0 : 1;
   const int D = v.dense_depth, F = v.n_features;
   const size_t width = size_t(1) << D, leaves = width * 4;
@@ -50,7 +50,9 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
     const std::vector<uint8_t>& heap = image == 0 ? pf.q_nodes : (image == 1 ? pf.q_nodes_ids : pf.q_nodes_nan);
     const std::vector<uint8_t>& walk =
       image == 0 ? walked.q_nodes : (image == 1 ? walked.q_nodes_ids : walked.q_nodes_nan);
-    if (walk.size() != (heap.empty() ? 0 : stride * v.n_trees)) return -2;
+    const size_t nodes_alone = q_far(v) ? walk_nodes_stride(D) : 0, payloads_alone = q_far(v) ? 4 * width : 0;
+    const size_t tree_bytes = stride + (image == 1 ? 0 : nodes_alone) + (image == 0 ? payloads_alone : 0);
+    if (walk.size() != (heap.empty() ? 0 : tree_bytes * v.n_trees)) return -2;
     if (heap.empty()) continue;
     const bool doubled = image == 2;
     for (int r = 0; r < n; ++r) {
@@ -98,15 +100,14 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
   }
   for (size_t t = 0; 3 * t < walked.q_top.size(); ++t)
     if (std::memcmp(&walked.q_top[3 * t], walked.q_nodes.data() + stride * t + 4, 12) != 0) ++bad;
-  if (walk_blocks(D) && v.leaf_vector_len <= 1) {
+  if (q_far(v)) {
     // nodes alone and payloads for global memory: the walk over the former ends, by the kernels' arithmetic, on
     // the payload that the walk over both ends on
     for (int image = 0; image < 2; ++image) {
-      const std::vector<uint8_t>& walk  = image == 0 ? walked.q_nodes : walked.q_nodes_nan;
-      const std::vector<uint8_t>& nodes = image == 0 ? walked.q_far_nodes : walked.q_far_nodes_nan;
-      const std::vector<uint32_t>& far  = walked.q_far_leaves;
-      if (nodes.size() != (walk.empty() ? 0 : size_t(walk_nodes_stride(D)) * v.n_trees)) return -2;
+      const std::vector<uint8_t>& walk = image == 0 ? walked.q_nodes : walked.q_nodes_nan;
       if (walk.empty()) continue;
+      const uint8_t* far   = walked.q_nodes.data() + stride * v.n_trees;
+      const uint8_t* nodes = walk.data() + stride * v.n_trees + (image == 0 ? size_t(4) * width * v.n_trees : 0);
       const uint32_t with = walk_pitch(D, true), without = walk_pitch(D, false);
       for (int i = 0; i < 4 * n; ++i) {
         const size_t t = rng() % v.n_trees;
@@ -118,7 +119,7 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
             b *= without;
           }
           if (std::memcmp(walk.data() + stride * t + 4u * (walk_level_at(D, l) + a),
-                          nodes.data() + size_t(walk_nodes_stride(D)) * t + 4u * (walk_level_at(D, l) + b), 4) != 0)
+                          nodes + size_t(walk_nodes_stride(D)) * t + 4u * (walk_level_at(D, l) + b), 4) != 0)
             ++bad;
           if (rng() & 1u) {
             a += walk_step_words(D, l);
@@ -127,7 +128,7 @@ extern "C" int64_t walk_check(const b2fil_forest_desc* desc, const b2fil_create_
         }
         const uint32_t place = 4u * (b - block * without);
         const uint32_t at = ((4u * block) << (D - 5)) + ((place >> (D - 8) | place << 3) & ((4u << (D - 5)) - 4u));
-        if (at / 4 >= width || std::memcmp(&far[width * t + at / 4], walk.data() + stride * t + to + 4u * a, 4) != 0) ++bad;
+        if (at / 4 >= width || std::memcmp(far + 4 * width * t + at, walk.data() + stride * t + to + 4u * a, 4) != 0) ++bad;
       }
     }
   }
