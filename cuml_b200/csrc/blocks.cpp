@@ -195,7 +195,7 @@ bool build_blocks(PackedForest& pf)
     for (const Child c : {TreeBlocks::first(pf, k), TreeBlocks::second(pf, k)})
       if (!c.leaf) size[k] += size[c.index];
   }
-  // Forests are cut on several threads; the result does not depend on how many.  On one thread the
+  // Large forests are cut on several threads; the result does not depend on how many.  On one thread the
   // blocks took a third of the time of the rest of the packer (200 trees, 1.2e7 nodes: 700 ms in fp64 and
   // 515 in fp32 beside 2300 and 1900; on eight cores 330 and 205).
   const int threads = pack_threads(n_nodes, n_trees);
